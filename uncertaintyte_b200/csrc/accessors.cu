@@ -2,7 +2,7 @@
 // the Uncertainty accessors (uncertainty.cpp:74-183: eigenvalues of every
 // camera and point block, sorted descending, and eigenvectors of the point
 // blocks and of the camera-centre 3 x 3 sub-blocks). The reference runs one
-// Eigen::EigenSolver per block on the host; here one warp owns one block.
+// Eigen::EigenSolver per block on the host; here one to nine lanes own one block (k_block_eigen).
 //
 // Input: packed upper triangles (row-major, i <= j) of src x src blocks
 // (45 values for src = 9, 6 for src = 3); the sub-block [off, off + dim) of each
@@ -18,79 +18,117 @@ namespace unc {
 namespace {
 
 constexpr int kMaxDim = 9;
-constexpr int kWarpsPerCta = 4;
 
-__global__ void __launch_bounds__(32 * kWarpsPerCta)
-    k_block_eigen(const double* __restrict__ packed, int nblk, int src, int off, int dim, double* vals,
-                  double* vecs) {
-    __shared__ double As[kWarpsPerCta][kMaxDim][kMaxDim + 1], Vs[kWarpsPerCta][kMaxDim][kMaxDim + 1];
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const int blk = blockIdx.x * kWarpsPerCta + w;
-    if (blk >= nblk) return;  // whole warps leave together
-    double(*A)[kMaxDim + 1] = As[w];
-    double(*V)[kMaxDim + 1] = Vs[w];
-    const int per = src * (src + 1) / 2;
-    const double* in = packed + (long)blk * per;
-    if (l < dim) {
-        const int i = off + l;
-        for (int c = 0; c < dim; ++c) {
-            const int j = off + c;
-            const int a = i < j ? i : j, b = i < j ? j : i;  // upper-triangle index of (a, b)
-            A[l][c] = in[a * src - a * (a - 1) / 2 + (b - a)];
-            V[l][c] = (l == c) ? 1.0 : 0.0;
-        }
-    }
-    __syncwarp();
-    for (int sweep = 0; sweep < 50; ++sweep) {
-        double off2 = 0.0, dg = 0.0;
-        if (l < dim) {
-            for (int c = 0; c < l; ++c) off2 += A[l][c] * A[l][c];
-            dg = A[l][l] * A[l][l];
+// The angle of the rotation that clears a_pq, from the tangent: entries so
+// large or small that their squares leave the FP64 range.
+__device__ __noinline__ void rotation_by_tangent(double d, double h, double& c, double& s, double& t) {
+    const double th = d / h;
+    t = fabs(th) > 1e100 ? 0.5 / th : (th >= 0.0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
+    c = 1.0 / sqrt(t * t + 1.0);
+    s = t * c;
+}
+
+// One D x D block on L lanes, everything in registers: every lane of a block
+// carries the whole upper triangle and applies every rotation to it, so the
+// rotations need no shared memory, shuffle or barrier; the rows of V are dealt
+// to the lanes (D / L each). The chain of dependent rotations bounds the
+// kernel, so a rotation takes two reciprocal square roots and no division:
+// with d = a_qq - a_pp, h = 2 a_pq and r = 1 / sqrt(d^2 + h^2),
+//   cos^2 = x = (1 + |d| r) / 2,  c = x / sqrt(x),  |s| = |h| r / (2 sqrt(x)).
+template <int D, int L>
+__global__ void __launch_bounds__(128) k_block_eigen(const double* __restrict__ packed, int nblk, int src, int off,
+                                                     double* vals, double* vecs) {
+    static_assert(D % L == 0, "whole rows of V per lane");
+    constexpr int R = D / L, kPerWarp = 32 / L;
+    const int lane = threadIdx.x & 31, part = lane % L;
+    const long blk = ((long)blockIdx.x * (128 / 32) + (threadIdx.x >> 5)) * kPerWarp + lane / L;
+    if (lane >= L * kPerWarp || blk >= nblk) return;
+    const double* in = packed + blk * (src * (src + 1) / 2);
+    double a[D][D], v[R][D];  // a: i <= j used
+#pragma unroll
+    for (int i = 0; i < D; ++i)
+#pragma unroll
+        for (int j = i; j < D; ++j) {
+            const int r = off + i;  // upper-triangle index of (off + i, off + j)
+            a[i][j] = __ldg(in + r * src - r * (r - 1) / 2 + (j - i));
         }
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            off2 += __shfl_xor_sync(0xffffffffu, off2, d);
-            dg += __shfl_xor_sync(0xffffffffu, dg, d);
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int j = 0; j < D; ++j) v[r][j] = part * R + r == j ? 1.0 : 0.0;
+    for (int sweep = 0; sweep < 50; ++sweep) {
+        double off2 = 0.0, dg = 0.0;
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+            dg += a[i][i] * a[i][i];
+#pragma unroll
+            for (int j = i + 1; j < D; ++j) off2 += a[i][j] * a[i][j];
         }
         if (off2 <= 1e-30 * dg) break;
-        for (int p = 0; p < dim - 1; ++p)
-            for (int q = p + 1; q < dim; ++q) {
-                const double apq = A[p][q], app = A[p][p], aqq = A[q][q];
-                if (apq == 0.0 || fabs(apq) <= 1e-17 * sqrt(fabs(app * aqq))) continue;
-                const double th = (aqq - app) / (2.0 * apq);
-                const double t = fabs(th) > 1e100 ? 0.5 / th
-                                                  : (th >= 0.0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
-                const double c = 1.0 / sqrt(t * t + 1.0), s = t * c;
-                __syncwarp();
-                if (l < dim) {
-                    const double x = A[l][p], y = A[l][q];
-                    A[l][p] = c * x - s * y;
-                    A[l][q] = s * x + c * y;
-                    const double vx = V[l][p], vy = V[l][q];
-                    V[l][p] = c * vx - s * vy;
-                    V[l][q] = s * vx + c * vy;
+#pragma unroll
+        for (int p = 0; p < D - 1; ++p)
+#pragma unroll
+            for (int q = p + 1; q < D; ++q) {
+                const double apq = a[p][q], app = a[p][p], aqq = a[q][q];
+                const double pr = fabs(app * aqq);
+                const bool small = fabs(apq) > 1e-140 ? apq * apq <= 1e-34 * pr : fabs(apq) <= 1e-17 * sqrt(pr);
+                if (apq == 0.0 || small) continue;
+                const double d = aqq - app, h = 2.0 * apq, m = fma(d, d, h * h);
+                double c, s, t;
+                if (m > 1e-280 && m < 1e280) {
+                    const double r = rsqrt(m), x = fma(0.5 * fabs(d), r, 0.5), rs = rsqrt(x);
+                    c = x * rs;
+                    s = 0.5 * fabs(h) * r * rs;
+                    if (d != 0.0 && (d < 0.0) != (h < 0.0)) s = -s;
+                    t = s * rs;
+                } else {
+                    rotation_by_tangent(d, h, c, s, t);
                 }
-                __syncwarp();
-                if (l < dim) {
-                    const double x = A[p][l], y = A[q][l];
-                    A[p][l] = c * x - s * y;
-                    A[q][l] = s * x + c * y;
+                a[p][p] = fma(-t, apq, app);
+                a[q][q] = fma(t, apq, aqq);
+                a[p][q] = 0.0;
+#pragma unroll
+                for (int k = 0; k < D; ++k) {
+                    if (k == p || k == q) continue;
+                    double& y = a[k < p ? k : p][k < p ? p : k];
+                    double& z = a[k < q ? k : q][k < q ? q : k];
+                    const double yk = y, zk = z;
+                    y = c * yk - s * zk;
+                    z = s * yk + c * zk;
                 }
-                __syncwarp();
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const double x = v[r][p], y = v[r][q];
+                    v[r][p] = c * x - s * y;
+                    v[r][q] = s * x + c * y;
+                }
             }
     }
-    if (l < dim) {  // descending order, ties by index
-        const double ev = A[l][l];
+    double* const w = vals + blk * D;
+    double* const e = vecs ? vecs + blk * (D * D) : nullptr;
+#pragma unroll
+    for (int j = 0; j < D; ++j) {  // descending order, ties by index
+        const double ev = a[j][j];
         int rank = 0;
-        for (int i = 0; i < dim; ++i) {
-            const double u = A[i][i];
-            rank += (u > ev) || (u == ev && i < l);
+#pragma unroll
+        for (int i = 0; i < D; ++i) rank += (a[i][i] > ev) || (a[i][i] == ev && i < j);
+        if (part == j / R) w[rank] = ev;
+        if (e) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) e[rank * D + part * R + r] = v[r][j];
         }
-        vals[(long)blk * dim + rank] = ev;
-        double* out = vecs ? vecs + (long)blk * dim * dim + (long)rank * dim : nullptr;
-        if (out)
-            for (int r = 0; r < dim; ++r) out[r] = V[r][l];
     }
+}
+
+// Lanes per block: one up to 3 x 3 (V fits beside the block, and there are as
+// many blocks as points), one per row above.
+template <int D>
+void launch_block_eigen(const double* packed, int nblk, int src, int off, double* vals, double* vecs,
+                        cudaStream_t sm) {
+    constexpr int L = D <= 3 ? 1 : D;
+    const long per_cta = 4 * (32 / L);
+    k_block_eigen<D, L><<<(unsigned)((nblk + per_cta - 1) / per_cta), 128, 0, sm>>>(packed, nblk, src, off, vals, vecs);
+    count_launch();
 }
 
 }  // namespace
@@ -108,9 +146,11 @@ extern "C" int unc_block_eigen_device(const double* d_packed, int num_blocks, in
     }
     if (num_blocks == 0) return UNC_OK;
     cudaStream_t sm = (cudaStream_t)stream;
-    k_block_eigen<<<(num_blocks + kWarpsPerCta - 1) / kWarpsPerCta, 32 * kWarpsPerCta, 0, sm>>>(
-        d_packed, num_blocks, block_params, sub_offset, sub_dim, d_values, d_vectors);
-    count_launch();
+    using Launch = void (*)(const double*, int, int, int, double*, double*, cudaStream_t);
+    static constexpr Launch by_dim[kMaxDim] = {launch_block_eigen<1>, launch_block_eigen<2>, launch_block_eigen<3>,
+                                               launch_block_eigen<4>, launch_block_eigen<5>, launch_block_eigen<6>,
+                                               launch_block_eigen<7>, launch_block_eigen<8>, launch_block_eigen<9>};
+    by_dim[sub_dim - 1](d_packed, num_blocks, block_params, sub_offset, d_values, d_vectors, sm);
     cudaError_t e = cudaStreamSynchronize(sm);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {
