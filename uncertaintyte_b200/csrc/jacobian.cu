@@ -30,29 +30,19 @@ __device__ __forceinline__ void skew(const double v[3], double W[3][3]) {
     W[2][0] = -v[1]; W[2][1] = v[0];  W[2][2] = 0.0;
 }
 
-__global__ void k_scene_jacobian(int num_cams, int num_points, int num_obs, const double* __restrict__ cams,
-                                 const double* __restrict__ pts, const int* __restrict__ obs_cam,
-                                 const int* __restrict__ obs_pt, int* __restrict__ rows, int* __restrict__ cols,
-                                 double* __restrict__ vals, int* err) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o == 0) rows[2L * num_obs] = 24 * num_obs;
-    if (o >= num_obs) return;
-    rows[2L * o] = 24 * o;
-    rows[2L * o + 1] = 24 * o + 12;
-    const int c = obs_cam[o], q = obs_pt[o];
-    int* cc = cols + 24L * o;
-    double* vv = vals + 24L * o;
-    if (c < 0 || c >= num_cams || q < 0 || q >= num_points) {
-        atomicOr(err, ERRBIT_LAYOUT);
-        for (int k = 0; k < 24; ++k) {
-            cc[k] = 0;
-            vv[k] = 0.0;
-        }
-        return;
-    }
-    const double* cam = cams + 9L * c;
+// One thread per observation forms the 24 values into shared memory (odd record
+// stride: conflict-free); the block then writes values and columns out as
+// 16-byte pieces, consecutive threads on consecutive pieces. The stores bound
+// the kernel (288 of its ~400 bytes per observation): written by each thread
+// into its own 192-byte record they cost five times the traffic's time.
+constexpr int kJacThreads = 128;
+constexpr int kJacStride = 25;
+
+// the 24 Jacobian values of one observation
+__device__ __forceinline__ void observation_values(const double* __restrict__ cam, const double* __restrict__ pt,
+                                                   double* vv) {
     const double w[3] = {cam[0], cam[1], cam[2]};
-    const double pC[3] = {pts[3L * q] - cam[3], pts[3L * q + 1] - cam[4], pts[3L * q + 2] - cam[5]};
+    const double pC[3] = {pt[0] - cam[3], pt[1] - cam[4], pt[2] - cam[5]};
     const double f = cam[6], k1 = cam[7], k2 = cam[8];
     // R(w) by Rodrigues' formula; first order below |w| = 1e-6
     double W[3][3], W2[3][3], R[3][3];
@@ -106,15 +96,63 @@ __global__ void k_scene_jacobian(int num_cams, int num_points, int num_obs, cons
     const double xy[2] = {xp, yp};
     for (int r = 0; r < 2; ++r) {
         double* row = vv + 12 * r;
-        int* cr = cc + 12 * r;
         for (int j = 0; j < 3; ++j) row[j] = -(Jp[r][0] * PJ[0][j] + Jp[r][1] * PJ[1][j] + Jp[r][2] * PJ[2][j]);
         for (int j = 0; j < 3; ++j) row[3 + j] = -Jp[r][j];
         row[6] = xy[r] * d;
         row[7] = f * xy[r] * r2;
         row[8] = f * xy[r] * r2 * r2;
         for (int j = 0; j < 3; ++j) row[9 + j] = Jp[r][j];
-        for (int k = 0; k < 9; ++k) cr[k] = 9 * c + k;
-        for (int k = 0; k < 3; ++k) cr[9 + k] = 9 * num_cams + 3 * q + k;
+    }
+}
+
+// Column e (0..23) of an observation whose first camera and point columns are f.
+__device__ __forceinline__ int column(int2 f, int e) {
+    const int j = e < 12 ? e : e - 12;
+    return f.x < 0 ? 0 : (j < 9 ? f.x + j : f.y + j - 9);
+}
+
+// kWide: cols and vals are 16-byte aligned; else the same values entry by entry.
+template <bool kWide>
+__global__ void __launch_bounds__(kJacThreads)
+    k_scene_jacobian(int num_cams, int num_points, int num_obs, const double* __restrict__ cams,
+                     const double* __restrict__ pts, const int* __restrict__ obs_cam, const int* __restrict__ obs_pt,
+                     int* __restrict__ rows, int* __restrict__ cols, double* __restrict__ vals, int* err) {
+    __shared__ double sv[kJacThreads * kJacStride];
+    __shared__ int2 first[kJacThreads];  // first camera and point column of an observation; x < 0: bad ids
+    const int o0 = blockIdx.x * kJacThreads, t = threadIdx.x, n = min(kJacThreads, num_obs - o0);
+    const int o = o0 + t;
+    if (o == 0) rows[2L * num_obs] = 24 * num_obs;
+    if (t < n) {
+        rows[2L * o] = 24 * o;
+        rows[2L * o + 1] = 24 * o + 12;
+        const int c = obs_cam[o], q = obs_pt[o];
+        double* vv = sv + t * kJacStride;
+        if (c < 0 || c >= num_cams || q < 0 || q >= num_points) {
+            atomicOr(err, ERRBIT_LAYOUT);
+            first[t] = make_int2(-1, 0);
+            for (int k = 0; k < 24; ++k) vv[k] = 0.0;
+        } else {
+            first[t] = make_int2(9 * c, 9 * num_cams + 3 * q);
+            observation_values(cams + 9L * c, pts + 3L * q, vv);
+        }
+    }
+    __syncthreads();
+    double* const v = vals + 24L * o0;
+    int* const c = cols + 24L * o0;
+    if (kWide) {
+        for (int i = t; i < 12 * n; i += kJacThreads) {
+            const double* r = sv + (i / 12) * kJacStride + 2 * (i % 12);
+            reinterpret_cast<double2*>(v)[i] = make_double2(r[0], r[1]);
+        }
+        for (int i = t; i < 6 * n; i += kJacThreads)
+            reinterpret_cast<int4*>(c)[i] = make_int4(column(first[i / 6], 4 * (i % 6)), column(first[i / 6], 4 * (i % 6) + 1),
+                                                      column(first[i / 6], 4 * (i % 6) + 2),
+                                                      column(first[i / 6], 4 * (i % 6) + 3));
+    } else {
+        for (int i = t; i < 24 * n; i += kJacThreads) {
+            v[i] = sv[(i / 24) * kJacStride + i % 24];
+            c[i] = column(first[i / 24], i % 24);
+        }
     }
 }
 
@@ -123,7 +161,8 @@ __global__ void k_scene_jacobian(int num_cams, int num_points, int num_obs, cons
 int launch_scene_jacobian(int num_cams, int num_points, int num_obs, const double* cams, const double* pts,
                           const int* obs_cam, const int* obs_pt, int* rows, int* cols, double* vals, int* err,
                           cudaStream_t st) {
-    k_scene_jacobian<<<(num_obs + 127) / 128 + (num_obs == 0), 128, 0, st>>>(
+    const auto kern = (((uintptr_t)cols | (uintptr_t)vals) & 15) == 0 ? k_scene_jacobian<true> : k_scene_jacobian<false>;
+    kern<<<(num_obs + kJacThreads - 1) / kJacThreads + (num_obs == 0), kJacThreads, 0, st>>>(
         num_cams, num_points, num_obs, cams, pts, obs_cam, obs_pt, rows, cols, vals, err);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? UNC_OK : UNC_ERR_CUDA;
