@@ -280,7 +280,9 @@ int unc_batch_set_tile_width(unc_batch* batch, int tile_n);
  * leading dimension lda >= n, lda even): inverted in place on the GPU
  * (equilibration, Cholesky with L^-1 formed on the way, then L^-T L^-1; for
  * n <= 3584 as 64 x 64 tile tasks in one persistent kernel, above by
- * recursion on halves). Scratch is allocated per call. */
+ * recursion on halves). Scratch (3 n x lda matrices) is allocated per call
+ * from a pool of the library's own: at most 1 GiB per device stays with it
+ * for later calls, until any context or batch is released or destroyed. */
 int unc_dense_inverse_device(double* d_A, int n, int lda, void* stream);
 
 /* The pseudo-inverse step of svdInverse (src/uncertaintyTE/compute.cpp:200-245)
@@ -291,7 +293,7 @@ int unc_dense_inverse_device(double* d_A, int n, int lda, void* stream);
  * eigenvectors are computed (subspace iteration on the shifted inverse), the
  * rest follows from one Cholesky inverse of the matrix with those directions
  * lifted and a two-sided projection. UNC_ERR_SINGULAR when a kept eigenvalue is
- * not positive. Scratch (4 n x ld matrices) is allocated per call. */
+ * not positive. Scratch (4 n x ld matrices) from the same pool. */
 int unc_pinv_psd_device(double* d_M, int n, int ld, int remove_n, double epsilon, void* stream);
 
 /* The SPD inverse of unc_dense_inverse_device (its recursive form), for callers that cannot
@@ -350,7 +352,7 @@ int unc_gemm_f64_device(int M, int N, int K, double alpha, const double* d_A, in
  * products run as tcgen05 int8 GEMMs with exact int32 accumulation, and the
  * levels are combined in FP64 (relative error about 2^(-7 slices) of the row
  * and column maxima). The mixed-precision Taylor products use this kernel.
- * Scratch is allocated per call. */
+ * Scratch from the library's pool (unc_dense_inverse_device). */
 int unc_gemm_mixed_device(int n, const double* d_P, const double* d_X, int ld, double* d_C, int slices,
                           void* stream);
 /* A = T^T T (n x n, column-major, leading dimension ld for both) for a lower
@@ -358,8 +360,8 @@ int unc_gemm_mixed_device(int n, const double* d_P, const double* d_X, int ld, d
  * T split into 7 int8 slices, lower 128 x 64 tiles whose k loops start at the
  * tile's first nonzero row, the result written in both triangles (per term an
  * error of about 2^-50 of the two columns' maxima, zero-mean). The last product of the mixed
- * modes' SPD inverse above N = 3584 (A^{-1} = L^{-T} L^{-1}). Scratch is
- * allocated per call. */
+ * modes' SPD inverse above N = 3584 (A^{-1} = L^{-T} L^{-1}). Scratch
+ * from the library's pool (unc_dense_inverse_device). */
 int unc_gram_lower_mixed_device(int n, const double* d_T, int ld, double* d_A, void* stream);
 
 /* Human-readable name of a status code, and the last error message of the

@@ -171,8 +171,9 @@ extern "C" int unc_block_eigen(const double* packed, int num_blocks, int block_p
     if (num_blocks == 0) return UNC_OK;
     const size_t nin = (size_t)num_blocks * block_params * (block_params + 1) / 2;
     const size_t nv = (size_t)num_blocks * sub_dim, nvec = vectors ? nv * sub_dim : 0;
-    double* d = nullptr;
-    cudaError_t e = cudaMalloc(&d, sizeof(double) * (nin + nv + nvec));
+    Scratch mem;
+    cudaError_t e = mem.alloc(sizeof(double) * (nin + nv + nvec), nullptr);
+    double* d = static_cast<double*>(mem.p);
     if (e != cudaSuccess) {
         g_last_error = std::string("unc_block_eigen: ") + cudaGetErrorString(e);
         return e == cudaErrorMemoryAllocation ? UNC_ERR_OUT_OF_MEMORY : UNC_ERR_CUDA;
@@ -185,7 +186,6 @@ extern "C" int unc_block_eigen(const double* packed, int num_blocks, int block_p
     if (e == cudaSuccess && rc == UNC_OK) e = cudaMemcpy(values, d + nin, sizeof(double) * nv, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && rc == UNC_OK && vectors)
         e = cudaMemcpy(vectors, d + nin + nv, sizeof(double) * nvec, cudaMemcpyDeviceToHost);
-    cudaFree(d);
     if (rc != UNC_OK) return rc;
     if (e != cudaSuccess) {
         g_last_error = std::string("unc_block_eigen: ") + cudaGetErrorString(e);

@@ -37,6 +37,53 @@ int device_sms() {
     cache[dev].store(v, std::memory_order_relaxed);
     return v;
 }
+
+namespace {
+constexpr int kMaxDevices = 64;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pool[kMaxDevices] = {};
+
+// The scratch pool of the current device, made at its first use (nullptr on failure).
+cudaMemPool_t scratch_pool(bool create) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    if (!g_pool[dev] && create) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) return nullptr;
+        cuuint64_t keep = kScratchKept;
+        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            return nullptr;
+        }
+        g_pool[dev] = pool;
+    }
+    return g_pool[dev];
+}
+}  // namespace
+
+cudaError_t Scratch::alloc(size_t bytes, cudaStream_t stream) {
+    st = stream;
+    cudaMemPool_t pool = scratch_pool(true);
+    cudaError_t e = pool ? cudaMallocFromPoolAsync(&p, bytes ? bytes : 16, pool, st) : cudaErrorMemoryAllocation;
+    if (e != cudaSuccess) {
+        p = nullptr;
+        cudaGetLastError();
+    }
+    return e;
+}
+
+Scratch::~Scratch() {
+    if (p) cudaFreeAsync(p, st);
+}
+
+void scratch_trim() {
+    if (cudaMemPool_t pool = scratch_pool(false)) cudaMemPoolTrimTo(pool, 0);
+}
 }  // namespace unc
 
 using namespace unc;
@@ -151,7 +198,6 @@ size_t carve(char* base, const Plan& pl, bool host_io, long long nnz, int nrows,
     b.g = c.take<double>(nn);
     b.dmax = c.take<unsigned long long>(24);
     b.e = c.take<double>(pl.N);
-    b.gjws = c.take<double>(chol_small_doubles(pl.N));
     b.dag_state = c.take<int>(spd_task_state_ints(pl.N));
     b.sig = c.take<double>((size_t)pl.C * 81);
     if (pl.svd_schur) {
@@ -596,27 +642,21 @@ int run_pipeline(unc_context* ctx, const unc_options* o, int num_rows, long long
     const size_t slice_region = mixed ? (size_t)nbuf * ((mixed_slice_bytes(N, slices) + 255) & ~size_t(255)) : 0;
     const bool gram = mixed && !tasks && mixed_gram_bytes(N) <= slice_region;
     int* gram_exps = mixed ? opa[kX].exps : nullptr;
-    if (tasks)
-        if (int r = spd_tasks_prepare(N)) return fail(r, "tile-task inverse: cannot upload the task list");
+    if (int r = spd_prepare(N)) return fail(r, "tile-task inverse: cannot upload the task list");
+    const SpdScratch scratch{b.iZ, b.add, b.tmp, b.dag_state, ctx->task_ctas};
     auto inverse_stage = [&]() -> int {
-        launch_shift_equilibrate(b.Z, N, ld, lambda, b.e, s.err, sm);
-        if (tasks) {
-            if (int r = chol_inverse_tasks(b.Z, N, ld, b.iZ, b.add, b.dag_state, s.err, sm, ctx->task_ctas))
-                return r;
-            launch_unequilibrate_from(b.add, b.Z, N, ld, b.e, b.iZ, sm);  // X in Z, iZ = X
-        } else if (gram) {
+        if (gram) {
             // mixed: T = L^{-1} in FP64 (its products feed the pivots), A^{-1} = T^T T
             // from int8 slices of T on the tensor cores
-            chol_lower_inverse(b.Z, N, ld, b.iZ, b.add, b.tmp, s.err, sm);
+            launch_shift_equilibrate(b.Z, N, ld, lambda, b.e, s.err, sm);
+            if (int r = chol_lower_inverse(b.Z, N, ld, scratch, s.err, sm)) return r;
             CK(cudaMemsetAsync(ctx->mp, 0, mixed_gram_bytes(N), sm));  // slice padding must be zero
             if (!mixed_gram_lower_tri(b.iZ, N, ld, reinterpret_cast<int8_t*>(ctx->mp), gram_exps, b.Z, ld, s.err, sm))
                 return fail(UNC_ERR_CUDA, "tensor-map encoding failed");
             launch_unequilibrate(b.Z, N, ld, b.e, b.iZ, sm);  // X in Z, iZ = X
-        } else {
-            chol_inverse(b.Z, N, ld, b.iZ, b.add, b.tmp, b.gjws, s.err, sm);
-            launch_unequilibrate(b.Z, N, ld, b.e, b.iZ, sm);  // X in Z, iZ = X
+            return UNC_OK;
         }
-        return UNC_OK;
+        return spd_inverse(b.Z, N, ld, lambda, b.e, scratch, b.iZ, s.err, sm);  // X in Z, iZ = X
     };
     auto taylor_stage = [&]() -> int {
         double* add = b.add;
@@ -704,7 +744,7 @@ int run_pipeline(unc_context* ctx, const unc_options* o, int num_rows, long long
         // recorded inside a graph are not available); per-product profiling
         // runs the stages directly
         GraphKey key = {1ULL, (unsigned long long)N, (unsigned long long)ld, lam_bits,
-                        (unsigned long long)(uintptr_t)b.Z, (unsigned long long)(uintptr_t)b.gjws,
+                        (unsigned long long)(uintptr_t)b.Z, (unsigned long long)(uintptr_t)b.dag_state,
                         (unsigned long long)(uintptr_t)s.err, 0ULL};
         size_t none = 0;
         if (int r = ctx->prof ? inverse_stage() : run_stage(ctx, key, sm, inverse_stage, none)) return r;
@@ -779,34 +819,20 @@ int dense_inverse(double* d_A, int n, int lda, void* stream, long long poll_limi
     if (!d_A || n <= 0 || lda < n || (lda & 1)) return fail(UNC_ERR_INVALID_ARG, "bad matrix arguments");
     cudaStream_t sm = (cudaStream_t)stream;
     const size_t mat = (size_t)lda * n;
-    // n <= 3584: the tile-task inverse (one persistent kernel), else the recursive form
-    const bool tasks = spd_tasks_apply(n);
-    if (tasks)
-        if (int r = spd_tasks_prepare(n)) return fail(r, "tile-task inverse: cannot upload the task list");
-    const size_t small_d = std::max(chol_small_doubles(n), (spd_task_state_ints(n) + 1) / 2);
-    const size_t wsd = 3 * mat + small_d + (size_t)n + 64;
-    double* ws = nullptr;
-    CK(cudaMalloc(&ws, wsd * sizeof(double) + 256));
-    double *T = ws, *W = ws + mat, *Tt = ws + 2 * mat, *small = ws + 3 * mat;
-    double* e = small + small_d;
+    if (int r = spd_prepare(n)) return fail(r, "tile-task inverse: cannot upload the task list");
+    const size_t state_d = (spd_task_state_ints(n) + 1) / 2;
+    const size_t wsd = 3 * mat + state_d + (size_t)n + 64;
+    Scratch mem;
+    CK(mem.alloc(wsd * sizeof(double) + 256, sm));
+    double* ws = static_cast<double*>(mem.p);
+    SpdScratch scratch{ws, ws + mat, ws + 2 * mat, reinterpret_cast<int*>(ws + 3 * mat), device_sms(), poll_limit, skip_task};
+    double* e = ws + 3 * mat + state_d;
     int* err = reinterpret_cast<int*>(ws + wsd);
     int h_err = 0;
     cudaError_t ce = cudaMemsetAsync(ws, 0, wsd * sizeof(double) + 256, sm);
-    if (ce == cudaSuccess) {
-        launch_shift_equilibrate(d_A, n, lda, 0.0, e, err, sm);
-        if (tasks) {
-            if (chol_inverse_tasks(d_A, n, lda, T, W, reinterpret_cast<int*>(small), err, sm, device_sms(),
-                                   poll_limit, skip_task) != UNC_OK)
-                ce = cudaErrorUnknown;
-            launch_unequilibrate_from(W, d_A, n, lda, e, nullptr, sm);
-        } else {
-            chol_inverse(d_A, n, lda, T, W, Tt, small, err, sm);
-            launch_unequilibrate(d_A, n, lda, e, nullptr, sm);
-        }
-        if (ce == cudaSuccess) ce = cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, sm);
-    }
+    if (ce == cudaSuccess && spd_inverse(d_A, n, lda, 0.0, e, scratch, nullptr, err, sm) != UNC_OK) ce = cudaErrorUnknown;
+    if (ce == cudaSuccess) ce = cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, sm);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(sm);
-    cudaFree(ws);
     if (ce != cudaSuccess) return fail(UNC_ERR_CUDA, cudaGetErrorString(ce));
     if (h_err & ERRBIT_TIMEOUT) return fail(UNC_ERR_CUDA, "a bounded device wait of the tile-task inverse ran out");
     if (h_err & (ERRBIT_SINGULAR | ERRBIT_NONFINITE)) return fail(UNC_ERR_SINGULAR, "matrix is not positive definite");
@@ -910,6 +936,7 @@ int unc_context_release(unc_context* c) {
         *sizes[i] = 0;
     }
     CK(cudaStreamSynchronize(c->stream));
+    scratch_trim();
     return UNC_OK;
 }
 
@@ -1325,19 +1352,18 @@ int unc_gemm_mixed_device(int n, const double* d_P, const double* d_X, int ld, d
         return fail(UNC_ERR_INVALID_ARG, "bad mixed GEMM arguments");
     cudaStream_t sm = (cudaStream_t)stream;
     const size_t sb = mixed_slice_bytes(n, slices);
-    char* ws = nullptr;
     const size_t exp_off = 2 * ((sb + 255) & ~size_t(255));
-    CK(cudaMalloc(&ws, exp_off + 2 * sizeof(int) * ((size_t)n + 64) + 256));
+    Scratch mem;
+    CK(mem.alloc(exp_off + 2 * sizeof(int) * ((size_t)n + 64) + 256, sm));
+    char* ws = static_cast<char*>(mem.p);
     int8_t* bufP = reinterpret_cast<int8_t*>(ws);
     int8_t* bufX = reinterpret_cast<int8_t*>(ws + (exp_off / 2));
     int* eP = reinterpret_cast<int*>(ws + exp_off);
     int* eX = eP + n + 64;
     int* err = eX + n + 64;
     MixedOperand a, b;
-    if (!mixed_plan(a, bufP, eP, n, slices, false) || !mixed_plan(b, bufX, eX, n, slices, true)) {
-        cudaFree(ws);
+    if (!mixed_plan(a, bufP, eP, n, slices, false) || !mixed_plan(b, bufX, eX, n, slices, true))
         return fail(UNC_ERR_CUDA, "tensor-map encoding failed");
-    }
     int h_err = 0;
     cudaError_t ce = cudaMemsetAsync(ws, 0, exp_off + 2 * sizeof(int) * ((size_t)n + 64) + 256, sm);
     if (ce == cudaSuccess) {
@@ -1347,7 +1373,6 @@ int unc_gemm_mixed_device(int n, const double* d_P, const double* d_X, int ld, d
         ce = cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, sm);
     }
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(sm);
-    cudaFree(ws);
     if (ce != cudaSuccess) return fail(UNC_ERR_CUDA, cudaGetErrorString(ce));
     if (h_err & ERRBIT_TIMEOUT) return fail(UNC_ERR_CUDA, "tensor-core pipeline wait timed out");
     return UNC_OK;
@@ -1359,20 +1384,17 @@ int unc_gram_lower_mixed_device(int n, const double* d_T, int ld, double* d_A, v
     cudaStream_t sm = (cudaStream_t)stream;
     const size_t sb = mixed_gram_bytes(n);
     const size_t total = sb + sizeof(int) * ((size_t)n + 64) + 256;
-    char* ws = nullptr;
-    CK(cudaMalloc(&ws, total));
+    Scratch mem;
+    CK(mem.alloc(total, sm));
+    char* ws = static_cast<char*>(mem.p);
     int* ex = reinterpret_cast<int*>(ws + sb);
     int* err = ex + n + 64;
     int h_err = 0;
     cudaError_t ce = cudaMemsetAsync(ws, 0, total, sm);
-    if (ce == cudaSuccess && !mixed_gram_lower_tri(d_T, n, ld, reinterpret_cast<int8_t*>(ws), ex, d_A, ld, err, sm)) {
-        cudaStreamSynchronize(sm);
-        cudaFree(ws);
+    if (ce == cudaSuccess && !mixed_gram_lower_tri(d_T, n, ld, reinterpret_cast<int8_t*>(ws), ex, d_A, ld, err, sm))
         return fail(UNC_ERR_CUDA, "tensor-map encoding failed");
-    }
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, sm);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(sm);
-    cudaFree(ws);
     if (ce != cudaSuccess) return fail(UNC_ERR_CUDA, cudaGetErrorString(ce));
     if (h_err & ERRBIT_TIMEOUT) return fail(UNC_ERR_CUDA, "tensor-core pipeline wait timed out");
     return UNC_OK;

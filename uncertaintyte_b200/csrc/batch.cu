@@ -740,6 +740,7 @@ int unc_batch_destroy(unc_batch* b) {
     }
     if (b->fork) cudaEventDestroy(b->fork);
     if (b->stream) cudaStreamDestroy(b->stream);
+    scratch_trim();
     delete b;
     return UNC_OK;
 }
@@ -821,6 +822,7 @@ int unc_batch_release(unc_batch* b) {
     b->ws_bytes = 0;
     BCK(cudaStreamSynchronize(b->stream));
     if (b->single) unc_context_release(b->single);
+    scratch_trim();
     return UNC_OK;
 }
 

@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <vector>
 
 #include "chol_leaf.cuh"
@@ -345,8 +346,9 @@ __global__ void __launch_bounds__(DAG_THREADS, 1)
     }
 }
 
-// The task list of nt x nt tiles in the order described above.
-std::vector<int4> build_tasks(int nt) {
+// The task list of nt x nt tiles in the order described above; without the
+// product, T = L^{-1} only (no PACC).
+std::vector<int4> build_tasks(int nt, bool product = true) {
     std::vector<int4> v;
     auto add = [&v](int ty, int i, int j, int k) { v.push_back(make_int4(ty, i, j, k)); };
     // POTRF(k) also applies UPDATE(k,k,k-1) first and computes TRSM(k+1,k) last
@@ -367,7 +369,7 @@ std::vector<int4> build_tasks(int nt) {
             for (int r = s; r < nt; ++r)
                 for (int c = 0; c < s; ++c) add(K_TACC, r, c, s - 1);
         for (int c = 0; c < s; ++c) add(K_TFIN, s, c, 0);
-        for (int r = 0; r <= s; ++r)
+        for (int r = 0; product && r <= s; ++r)
             for (int c = 0; c <= r; ++c) add(K_PACC, r, c, s);
     }
     return v;
@@ -375,7 +377,7 @@ std::vector<int4> build_tasks(int nt) {
 
 struct TaskLists {
     std::mutex mu;
-    std::map<std::pair<int, int>, std::pair<int4*, int>> lists;  // (device, nt) -> device copy
+    std::map<std::tuple<int, int, bool>, std::pair<int4*, int>> lists;  // (device, nt, product) -> device copy
     std::map<int, cudaStream_t> upload;                          // device -> upload stream
 };
 TaskLists& task_lists() {
@@ -392,15 +394,15 @@ size_t spd_task_state_ints(int n) {
     return 4 + 5 * nt * (nt + 1) / 2;
 }
 
-int spd_tasks_prepare(int n) {
+int spd_tasks_prepare(int n, bool product) {
     if (!spd_tasks_apply(n)) return UNC_ERR_INVALID_ARG;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return UNC_ERR_CUDA;
     const int nt = (n + TB - 1) / TB;
     TaskLists& tl = task_lists();
     std::lock_guard<std::mutex> lock(tl.mu);
-    if (tl.lists.count({dev, nt})) return UNC_OK;
-    const std::vector<int4> h = build_tasks(nt);
+    if (tl.lists.count({dev, nt, product})) return UNC_OK;
+    const std::vector<int4> h = build_tasks(nt, product);
     // upload on a private non-blocking stream: a copy on the legacy default
     // stream would wait for every other stream's work (a serving process runs
     // several requests at once)
@@ -424,7 +426,7 @@ int spd_tasks_prepare(int n) {
         return cudaFuncSetAttribute(k_spd_inverse_tasks, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)DAG_SMEM) == cudaSuccess;
     });
-    tl.lists[{dev, nt}] = {d, (int)h.size()};
+    tl.lists[{dev, nt, product}] = {d, (int)h.size()};
     return UNC_OK;
 }
 
@@ -437,7 +439,7 @@ int chol_inverse_tasks(double* A, int n, int lda, double* T, double* O, int* sta
     {
         TaskLists& tl = task_lists();
         std::lock_guard<std::mutex> lock(tl.mu);
-        auto it = tl.lists.find({dev, nt});
+        auto it = tl.lists.find({dev, nt, O != nullptr});
         if (it == tl.lists.end()) return UNC_ERR_INVALID_ARG;  // spd_tasks_prepare first (outside any capture)
         list = it->second;
     }
@@ -446,7 +448,7 @@ int chol_inverse_tasks(double* A, int n, int lda, double* T, double* O, int* sta
     const long spin = poll_limit > 0 ? (long)std::min<long long>(poll_limit, kDagSpin) : kDagSpin;
     int4* own = nullptr;  // a schedule with one task left out (tests of the bounded waits)
     if (skip_task >= 0 && skip_task < list.second) {
-        std::vector<int4> h = build_tasks(nt);
+        std::vector<int4> h = build_tasks(nt, O != nullptr);
         h.erase(h.begin() + skip_task);
         if (cudaMallocAsync(reinterpret_cast<void**>(&own), sizeof(int4) * h.size(), st) != cudaSuccess)
             return UNC_ERR_OUT_OF_MEMORY;

@@ -1,11 +1,12 @@
 // dense.cu - FP64 dense kernels for the inverse of the camera Schur
 // complement (sm_100a):
 //   * gemm_f64      : C = alpha*A*B + beta*C on DMMA (mma.sync m8n8k4 f64),
-//                     3-stage cp.async pipeline of 32-deep K tiles, optional fused max|C| for the
+//                     4-stage cp.async pipeline of 16-deep K tiles, optional fused max|C| for the
 //                     Taylor stop rule (ScaledDenseMatrix.cpp:207-216,314-353),
 //                     lower-tile and triangular-operand (k range per tile) modes.
-//   * chol_inverse  : SPD inverse by recursive Cholesky that forms T = L^{-1}
-//                     on the way, then A^{-1} = T^T T; every step is a GEMM
+//   * spd_inverse   : SPD inverse by recursive Cholesky that forms T = L^{-1}
+//                     on the way, then A^{-1} = T^T T; every step is a GEMM above
+//                     the blocks that the tile tasks (dag.cu) take
 //                     (replaces dgetrf+dgetri in SDM::inv, ScaledDenseMatrix.cpp:232-279).
 //   * shift/equilibrate, un-equilibrate, axpy (iZupdate, compute.cpp:64-71),
 //     camera output with the reference's (a + b/2) quirk (compute.cpp:168-183).
@@ -20,36 +21,32 @@ namespace unc {
 // GEMM
 // ------------------------------------------------------------------------
 namespace {
-constexpr int BK = 32, STAGES = 3, GEMM_THREADS = 256;  // 32-deep K stages: half the barriers of 16
-constexpr int LDB_S = BK + 4;  // Bs[n][k]: 36 doubles per n row (8 mod 32 banks: conflict-free fragment reads)
-
-// Output tile BM x BN computed by 8 warps of WM x WN (FM x FN fragments of
-// the 8 x 8 DMMA result). Shared-memory rows of A (and of the transposed B)
-// are padded by 4 doubles: a fragment read takes rows kk + t (t = 0..3) at 8
-// doubles apart in bank space (row pitch = 8 mod 32 banks), so each half-warp
-// hits 16 distinct bank pairs; cp.async rows stay 16-byte aligned.
-template <int BM_, int BN_, int WM_, int WN_>
-struct GemmCfg {
-    static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_;
-    static constexpr int WARPS_M = BM / WM;
-    static_assert((BM / WM) * (BN / WN) == GEMM_THREADS / 32, "8 warps per CTA");
-    static constexpr int FM = WM / 8, FN = WN / 8;
-    static constexpr int LDA_S = BM + 4;   // As[k][m]
-    static constexpr int LDBT_S = BN + 4;  // Bs[k][n] (transposed B)
-    static_assert((2 * LDA_S) % 32 == 8 && (2 * LDBT_S) % 32 == 8, "conflict-free fragment rows");
-    static constexpr int A_STAGE = BK * LDA_S;
-    static constexpr int B_STAGE = (BN * LDB_S > BK * LDBT_S) ? BN * LDB_S : BK * LDBT_S;
-    static constexpr size_t SMEM = sizeof(double) * (size_t)STAGES * (A_STAGE + B_STAGE);
-    static constexpr int A_CHUNKS = BM * BK / 2 / GEMM_THREADS;  // 16-byte copies per thread
-    static constexpr int B_CHUNKS = BN * BK / 2 / GEMM_THREADS;
+// Output tile 2W x 2W by four warps of W x W (fragments of the 8 x 8 DMMA
+// result), k stages of 16, three CTAs per SM. The FP64 pipe bounds the kernel
+// (one DMMA is 16 cycles of a quarter SM), so what counts is that some warp
+// always has one to issue: three independent CTAs cover each other's barriers
+// and fragment loads. W = 32; W = 16 where 64 x 64 tiles are fewer than the SMs
+// (a tile's time is its k range on one SM's FP64 pipe, so smaller tiles finish
+// four times sooner).
+constexpr int BK = 16, STAGES = 4, GEMM_THREADS = 128, GEMM_CTAS = 3;
+template <int W>
+struct GemmTile {
+    static constexpr int B = 2 * W, F = W / 8;
+    // Shared-memory operand tiles. Operands contiguous along m (n): rows of k, pitch
+    // B + 4 doubles; a thread reads two neighbouring m (n) of one k as 16 bytes.
+    // Operands contiguous along k: rows of m (n), pitch 18. Both pitches make the
+    // fragment reads conflict-free (rows 2 g of a group at 8 g words).
+    static constexpr int LDM = B + 4, LDK = BK + 2;
+    static_assert((2 * LDM) % 32 == 8 && (4 * LDK) % 32 == 8, "conflict-free fragment rows");
+    static constexpr int OP_STAGE = B * LDK > BK * LDM ? B * LDK : BK * LDM;  // doubles of one operand tile
+    static constexpr size_t SMEM = sizeof(double) * 2 * STAGES * OP_STAGE;
+    static constexpr int COPIES = B * BK / 2 / GEMM_THREADS;  // 16-byte copies per thread and operand tile
 };
-using CfgBig = GemmCfg<128, 128, 32, 64>;   // 1 CTA per SM (212 KB shared)
-using CfgSmall = GemmCfg<64, 64, 16, 32>;   // small outputs: 4x the CTAs (108 KB shared, 2 per SM)
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool pred) {
+// 16-byte asynchronous copy of `bytes` (0, 8 or 16) valid bytes, the rest zero
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int bytes) {
     unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    int sz = pred ? 16 : 0;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(sz));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
@@ -58,14 +55,16 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // Accumulation. By default the products accumulate in the MMA's own C
-// operand over the whole k range. With GEMM_SHORT_ACC they accumulate there
-// over two 8 x 8 x 4 steps only (k = 8), starting from zero, and those partial
-// sums are added to the running sums with ordinary FP64 additions (IEEE
-// round to nearest): accumulating in the C operand over the thousands of
-// steps of a long dot product carried a one-sided rounding into the SPD
-// inverse's Cholesky pivots (the last ones are ~lambda, formed by cancellation
-// from O(1) entries, and set the inverse's largest, gauge, components), so the
-// products that feed pivots (L21 = A21 T11^T and A22 -= L21 L21^T) take it.
+// operand over the whole k range: one rounding per k step at the size of the
+// running sum. With GEMM_SHORT_ACC they accumulate there over 32 steps of k
+// (two stages), starting from zero, and those partial sums are added to the
+// running sums: k / 32 roundings at that size. The SPD inverse's last Cholesky
+// pivots (~lambda, formed by cancellation from O(1) entries) set the inverse's
+// largest, gauge, components, so the products that feed pivots
+// (L21 = A21 T11^T and A22 -= L21 L21^T) take it. A partial sum is added when
+// its registers are needed again, one k step of other fragments later, so that
+// no addition waits for an MMA in flight (n = 6144: 32.1 TFLOP/s; 25.5 with
+// partial sums of 8 added at once).
 __device__ __forceinline__ void dmma0(double& t0, double& t1, double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%4};\n"
                  : "=d"(t0), "=d"(t1)
@@ -76,64 +75,118 @@ __device__ __forceinline__ void dmma_acc(double& d0, double& d1, double a, doubl
                  : "+d"(d0), "+d"(d1)
                  : "d"(a), "d"(b));
 }
-}  // namespace
 
-// Tile loader: A tile (BM rows x BK cols of column-major A), B tile (BK rows
-// x BN cols of column-major B). Out-of-range chunks are zero-filled. Rows
-// past M (or K for B) inside the allocation are read as 16-byte pairs; the
-// values there only meet zero-filled partners or land in unstored rows, so
-// they must merely be finite.
-template <class Cfg, bool kTransB>
-__device__ __forceinline__ void load_tiles(double* As, double* Bs, const double* __restrict__ A,
-                                           long lda, const double* __restrict__ B, long ldb, int M,
-                                           int N, int K, int m0, int n0, int k0, int tid) {
-    constexpr int AH = Cfg::BM / 2, BH = Cfg::BN / 2;
+// This thread's copies of one operand's tiles: B rows (m or n) from r0, BK
+// steps of k at a time, of an operand with extent R x K. kAlongK: X(r, k) =
+// X[k + r ld], else X[r + k ld]. Everything past K is zero. Along m (n) the
+// 16-byte pair at R - 1 may include one element past R, which only reaches
+// results that are not stored.
+template <int W, bool kAlongK>
+struct OperandCopy {
+    using T = GemmTile<W>;
+    const double* src;
+    long step, next;   // between this thread's copies of a tile, from one tile to the next
+    int dst, rows_ok;  // rows_ok: bit q set when copy q's row exists
+    int k;             // k of the first copy in the next tile
+
+    __device__ __forceinline__ OperandCopy(const double* X, long ld, int R, int r0, int kt, int tid) {
+        rows_ok = 0;
+        if (kAlongK) {
+            const int r = tid / (BK / 2);
+            k = kt * BK + (tid % (BK / 2)) * 2;
+            src = X + k + (long)(r0 + r) * ld;
+            step = (long)(GEMM_THREADS / (BK / 2)) * ld;
+            next = BK;
+            dst = r * T::LDK + (tid % (BK / 2)) * 2;
 #pragma unroll
-    for (int q = 0; q < Cfg::A_CHUNKS; ++q) {
-        int idx = tid + q * GEMM_THREADS;
-        int k = idx / AH, m2 = (idx % AH) * 2;
-        bool p = (m0 + m2 < M) && (k0 + k < K);
-        const double* src = p ? A + (m0 + m2) + (long)(k0 + k) * lda : A;
-        cp_async16(As + k * Cfg::LDA_S + m2, src, p);
-    }
-    if (kTransB) {
-        // B(k, n) = B[n + k * ldb]: tile stored Bs[k][n] like A
-#pragma unroll
-        for (int q = 0; q < Cfg::B_CHUNKS; ++q) {
-            int idx = tid + q * GEMM_THREADS;
-            int k = idx / BH, n2 = (idx % BH) * 2;
-            bool p = (n0 + n2 < N) && (k0 + k < K);
-            const double* src = p ? B + (n0 + n2) + (long)(k0 + k) * ldb : B;
-            cp_async16(Bs + k * Cfg::LDBT_S + n2, src, p);
+            for (int q = 0; q < T::COPIES; ++q) rows_ok |= (r0 + r + q * (GEMM_THREADS / (BK / 2)) < R) << q;
+        } else {
+            const int r2 = (tid % W) * 2;
+            k = kt * BK + tid / W;
+            src = X + (r0 + r2) + (long)k * ld;
+            step = (long)(GEMM_THREADS / W) * ld;
+            next = (long)BK * ld;
+            dst = (tid / W) * T::LDM + r2;
+            rows_ok = r0 + r2 < R ? (1 << T::COPIES) - 1 : 0;
         }
-    } else {
+    }
+    __device__ __forceinline__ void tile(double* sm, const double* __restrict__ X, int K) {
 #pragma unroll
-        for (int q = 0; q < Cfg::B_CHUNKS; ++q) {
-            int idx = tid + q * GEMM_THREADS;
-            int n = idx / (BK / 2), k2 = (idx % (BK / 2)) * 2;
-            bool p = (n0 + n < N) && (k0 + k2 < K);
-            const double* src = p ? B + (k0 + k2) + (long)(n0 + n) * ldb : B;
-            cp_async16(Bs + n * LDB_S + k2, src, p);
+        for (int q = 0; q < T::COPIES; ++q) {
+            const int left = K - (kAlongK ? k : k + q * (GEMM_THREADS / W));
+            const int bytes = !((rows_ok >> q) & 1) || left <= 0 ? 0 : (kAlongK && left == 1 ? 8 : 16);
+            cp_async16(sm + dst + q * (kAlongK ? GEMM_THREADS / (BK / 2) * T::LDK : GEMM_THREADS / W * T::LDM),
+                       bytes ? src + q * step : X, bytes);
+        }
+        src += next;
+        k += BK;
+    }
+};
+
+// The fragments of one operand at k step kk (this thread's k: kk + t).
+// Fragment f holds rows 16 (f / 2) + 2 g + f % 2 of the warp's W: a pair of
+// fragments reads neighbouring rows.
+template <int W, bool kAlongK>
+__device__ __forceinline__ void load_fragments(const double* sm, int w0, int kk, int g, int t, double (&f)[W / 8]) {
+    using T = GemmTile<W>;
+#pragma unroll
+    for (int i = 0; i < W / 8; i += 2) {
+        const int r = w0 + 8 * i + 2 * g;
+        if (kAlongK) {
+            f[i] = sm[r * T::LDK + kk + t];
+            f[i + 1] = sm[(r + 1) * T::LDK + kk + t];
+        } else {
+            const double2 v = *reinterpret_cast<const double2*>(sm + (kk + t) * T::LDM + r);
+            f[i] = v.x;
+            f[i + 1] = v.y;
         }
     }
 }
 
-template <class Cfg, bool kTransB, bool kShortAcc>
-__global__ void __launch_bounds__(GEMM_THREADS, (Cfg::BM == 128 ? 1 : 2))
+__device__ __forceinline__ double finite_abs(double v) {  // |v|, infinity for a NaN
+    const double a = fabs(v);
+    return a <= 1.7976931348623157e308 ? a : __longlong_as_double(0x7ff0000000000000LL);
+}
+
+// X[0], X[stride] = v0, v1 (one 16-byte store when wide)
+__device__ __forceinline__ void store_pair(double* X, double v0, double v1, bool wide) {
+    if (wide) {
+        *reinterpret_cast<double2*>(X) = make_double2(v0, v1);
+    } else {
+        X[0] = v0;
+        X[1] = v1;
+    }
+}
+}  // namespace
+
+// kTransA: A(m, k) = A[k + m lda]; kTransB: B(k, n) = B[n + k ldb].
+template <int W, bool kTransA, bool kTransB, bool kShortAcc>
+__global__ void __launch_bounds__(GEMM_THREADS, GEMM_CTAS)
     k_gemm_f64(int M, int N, int K, double alpha, const double* __restrict__ A, long lda,
                const double* __restrict__ B, long ldb, double beta, double* C, long ldc,
                unsigned long long* amax, int mode, double* part, const int* skip) {
-    constexpr int BM = Cfg::BM, BN = Cfg::BN, FM = Cfg::FM, FN = Cfg::FN;
+    using T = GemmTile<W>;
+    constexpr int BM = T::B, BN = T::B, FM = T::F, FN = T::F;
     if (skip && *skip) return;
+    // Tile order: groups of kGroup tile rows, each walked column by column, so that
+    // the CTAs running together share a few rows of A and columns of B in L2. Where
+    // the k range grows with m or n the walk starts at the long end (short tiles last).
+    constexpr int kGroup = 16;
+    const int gy = (M + BM - 1) / BM, gx = (N + BN - 1) / BN;
+    const int band = (int)(blockIdx.x / (unsigned)(kGroup * gx)), in = (int)(blockIdx.x - (unsigned)band * (kGroup * gx));
+    const int rows = min(kGroup, gy - band * kGroup);
+    int ty = band * kGroup + in % rows, tx = in / rows;
+    if (mode & GEMM_KHI_M) ty = gy - 1 - ty;
+    if (mode & GEMM_KHI_N) tx = gx - 1 - tx;
+    const int m0 = ty * BM, n0 = tx * BN;
     // GEMM_LOWER: tiles strictly above the diagonal of C are skipped (SYRK-style update)
-    if ((mode & GEMM_LOWER) && (int)(blockIdx.x * BN) > (int)(blockIdx.y * BM) + BM - 1) return;
+    if ((mode & GEMM_LOWER) && n0 > m0 + BM - 1) return;
     extern __shared__ __align__(16) double smem[];
     double* As = smem;
-    double* Bs = smem + STAGES * Cfg::A_STAGE;
+    double* Bs = smem + STAGES * T::OP_STAGE;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = (warp % Cfg::WARPS_M) * Cfg::WM, wn = (warp / Cfg::WARPS_M) * Cfg::WN;
+    const int wm = (warp & 1) * W, wn = (warp >> 1) * W;
     const int g = lane >> 2, t = lane & 3;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const bool wact = (m0 + wm < M) && (n0 + wn < N);
     // triangular operands: the k range of this tile outside which a product term is zero
     int kbeg = 0, kend = K;
@@ -143,125 +196,130 @@ __global__ void __launch_bounds__(GEMM_THREADS, (Cfg::BM == 128 ? 1 : 2))
     if (mode & GEMM_KHI_N) kend = min(kend, n0 + BN);
     int kt0 = kbeg / BK;
     int KT = kend > kbeg ? (kend + BK - 1) / BK - kt0 : 0;  // k tiles of this output tile
-    if (gridDim.z > 1) {  // split-K: a contiguous share of the k tiles, partial sums to part
-        const int chunk = (KT + gridDim.z - 1) / gridDim.z;
-        const int b0 = min(KT, (int)blockIdx.z * chunk);
+    if (gridDim.y > 1) {  // split-K: a contiguous share of the k tiles, partial sums to part
+        const int chunk = (KT + gridDim.y - 1) / gridDim.y;
+        const int b0 = min(KT, (int)blockIdx.y * chunk);
         KT = min(KT, b0 + chunk) - b0;
         kt0 += b0;
     }
 
-    double acc[FM][FN][2];
+    double acc[FM][FN][2], p[FM][FN][2];
 #pragma unroll
     for (int i = 0; i < FM; ++i)
 #pragma unroll
-        for (int j = 0; j < FN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+        for (int j = 0; j < FN; ++j) acc[i][j][0] = acc[i][j][1] = p[i][j][0] = p[i][j][1] = 0.0;
 
+    OperandCopy<W, kTransA> copy_a(A, lda, M, m0, kt0, tid);
+    OperandCopy<W, !kTransB> copy_b(B, ldb, N, n0, kt0, tid);
+    auto load_stage = [&](int s) {
+        copy_a.tile(As + s * T::OP_STAGE, A, K);
+        copy_b.tile(Bs + s * T::OP_STAGE, B, K);
+    };
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) {
-        if (s < KT)
-            load_tiles<Cfg, kTransB>(As + s * Cfg::A_STAGE, Bs + s * Cfg::B_STAGE, A, lda, B, ldb, M, N, K, m0,
-                                     n0, (kt0 + s) * BK, tid);
+        if (s < KT) load_stage(s);
         cp_async_commit();
     }
-    for (int kt = 0; kt < KT; ++kt) {
+    constexpr int kUnroll = kShortAcc ? 2 : 1;  // a partial sum spans two stages
+    auto stage = [&](int kt, bool opens) {
         cp_async_wait<STAGES - 2>();
         __syncthreads();
-        int pf = kt + STAGES - 1;
-        if (pf < KT) {
-            int ps = pf % STAGES;
-            load_tiles<Cfg, kTransB>(As + ps * Cfg::A_STAGE, Bs + ps * Cfg::B_STAGE, A, lda, B, ldb, M, N, K,
-                                     m0, n0, (kt0 + pf) * BK, tid);
-        }
+        if (kt + STAGES - 1 < KT) load_stage((kt + STAGES - 1) % STAGES);
         cp_async_commit();
-        const double* as = As + (kt % STAGES) * Cfg::A_STAGE;
-        const double* bs = Bs + (kt % STAGES) * Cfg::B_STAGE;
-        if (!wact) continue;  // this warp's sub-tile lies outside C
-        if (kShortAcc) {
-#pragma unroll 1
-            for (int kk = 0; kk < BK; kk += 8) {  // two 4-deep steps: a partial sum from zero, then added
-                double af[2][FM], bf[2][FN];
+        if (!wact) return;  // this warp's sub-tile lies outside C
+        const double* as = As + (kt % STAGES) * T::OP_STAGE;
+        const double* bs = Bs + (kt % STAGES) * T::OP_STAGE;
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
+        for (int kk = 0; kk < BK; kk += 4) {
+            double af[FM], bf[FN];
+            load_fragments<W, kTransA>(as, wm, kk, g, t, af);
+            load_fragments<W, !kTransB>(bs, wn, kk, g, t, bf);
 #pragma unroll
-                    for (int i = 0; i < FM; ++i) af[h][i] = as[(kk + 4 * h + t) * Cfg::LDA_S + wm + i * 8 + g];
+            for (int i = 0; i < FM; ++i)
 #pragma unroll
-                    for (int j = 0; j < FN; ++j)
-                        bf[h][j] = kTransB ? bs[(kk + 4 * h + t) * Cfg::LDBT_S + wn + j * 8 + g]
-                                           : bs[(wn + j * 8 + g) * LDB_S + kk + 4 * h + t];
-                }
-                constexpr int FH = FN >= 8 ? FN / 2 : FN;  // fragments per group (register pressure)
-#pragma unroll
-                for (int i = 0; i < FM; ++i)  // FH partial sums at a time, then added
-#pragma unroll
-                    for (int j0 = 0; j0 < FN; j0 += FH) {
-                        double p[FH][2];
-#pragma unroll
-                        for (int j = 0; j < FH; ++j) dmma0(p[j][0], p[j][1], af[0][i], bf[0][j0 + j]);
-#pragma unroll
-                        for (int j = 0; j < FH; ++j) dmma_acc(p[j][0], p[j][1], af[1][i], bf[1][j0 + j]);
-#pragma unroll
-                        for (int j = 0; j < FH; ++j) {
-                            acc[i][j0 + j][0] += p[j][0];
-                            acc[i][j0 + j][1] += p[j][1];
-                        }
+                for (int j = 0; j < FN; ++j) {
+                    if (!kShortAcc) {
+                        dmma_acc(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
+                    } else if (kk == 0 && opens) {  // a new partial sum; the finished one is added
+                        acc[i][j][0] += p[i][j][0];
+                        acc[i][j][1] += p[i][j][1];
+                        dmma0(p[i][j][0], p[i][j][1], af[i], bf[j]);
+                    } else {
+                        dmma_acc(p[i][j][0], p[i][j][1], af[i], bf[j]);
                     }
-            }
-        } else {
-#pragma unroll
-            for (int kk = 0; kk < BK; kk += 4) {
-                double af[FM], bf[FN];
-#pragma unroll
-                for (int i = 0; i < FM; ++i) af[i] = as[(kk + t) * Cfg::LDA_S + wm + i * 8 + g];
-#pragma unroll
-                for (int j = 0; j < FN; ++j)
-                    bf[j] = kTransB ? bs[(kk + t) * Cfg::LDBT_S + wn + j * 8 + g]
-                                    : bs[(wn + j * 8 + g) * LDB_S + kk + t];
-#pragma unroll
-                for (int i = 0; i < FM; ++i)
-#pragma unroll
-                    for (int j = 0; j < FN; ++j) dmma_acc(acc[i][j][0], acc[i][j][1], af[i], bf[j]);
-            }
+                }
         }
+    };
+    for (int kt = 0; kt < KT; kt += kUnroll) {
+        stage(kt, true);
+        if (kUnroll == 2 && kt + 1 < KT) stage(kt + 1, false);
     }
     cp_async_wait<0>();
+    if (kShortAcc) {
+#pragma unroll
+        for (int i = 0; i < FM; ++i)
+#pragma unroll
+            for (int j = 0; j < FN; ++j) {
+                acc[i][j][0] += p[i][j][0];
+                acc[i][j][1] += p[i][j][1];
+            }
+    }
 
-    if (part) {  // raw partial tile of split blockIdx.z (M x N slab, leading dimension M)
-        double* P = part + (size_t)blockIdx.z * M * N;
+    if (part) {  // raw partial tile of split blockIdx.y (M x N slab, leading dimension M)
+        double* P = part + (size_t)blockIdx.y * M * N;
 #pragma unroll
         for (int i = 0; i < FM; ++i) {
-            int row = m0 + wm + i * 8 + g;
+            const int row = m0 + wm + 16 * (i / 2) + 2 * g + i % 2;
 #pragma unroll
             for (int j = 0; j < FN; ++j)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    int col = n0 + wn + j * 8 + t * 2 + h;
+                    const int col = n0 + wn + 16 * (j / 2) + 2 * (2 * t + h) + j % 2;
                     if (row < M && col < N) P[row + (size_t)col * M] = acc[i][j][h];
                 }
         }
         return;
     }
 
+    // each 2 x 2 group of fragment elements (rows r, r + 1, columns c, c + 1)
+    const bool wide = ((reinterpret_cast<uintptr_t>(C) | (uintptr_t)(ldc * 8)) & 15) == 0;
+    const bool mirror = (mode & GEMM_MIRROR) != 0;
     double mx = 0.0;
 #pragma unroll
-    for (int i = 0; i < FM; ++i) {
-        int row = m0 + wm + i * 8 + g;
+    for (int i = 0; i < FM; i += 2)
 #pragma unroll
-        for (int j = 0; j < FN; ++j) {
+        for (int j = 0; j < FN; j += 2)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                int col = n0 + wn + j * 8 + t * 2 + h;
-                if (row < M && col < N && (!(mode & GEMM_MIRROR) || row >= col)) {
-                    double* c = C + row + (long)col * ldc;
-                    double v = alpha * acc[i][j][h];
-                    if (beta != 0.0) v += beta * *c;
-                    *c = v;
-                    if ((mode & GEMM_MIRROR) && row > col) C[col + (long)row * ldc] = v;
-                    double av = fabs(v);
-                    mx = fmax(mx, av <= 1.7976931348623157e308 ? av : __longlong_as_double(0x7ff0000000000000LL));
+                const int r = m0 + wm + 8 * i + 2 * g, c = n0 + wn + 8 * j + 2 * (2 * t + h);
+                double v[2][2];  // [row][column]
+#pragma unroll
+                for (int a = 0; a < 2; ++a)
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        const bool in_c = r + a < M && c + b < N && (!mirror || r + a >= c + b);
+                        v[a][b] = alpha * acc[i + a][j + b][h];
+                        if (in_c && beta != 0.0) v[a][b] += beta * C[(r + a) + (long)(c + b) * ldc];
+                        if (in_c) mx = fmax(mx, finite_abs(v[a][b]));
+                    }
+                if (r + 1 < M && c + 1 < N && (!mirror || r > c + 1)) {  // the whole group, strictly below the diagonal
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) store_pair(C + r + (long)(c + b) * ldc, v[0][b], v[1][b], wide);
+                    if (mirror) {
+#pragma unroll
+                        for (int a = 0; a < 2; ++a) store_pair(C + c + (long)(r + a) * ldc, v[a][0], v[a][1], wide);
+                    }
+                } else {
+#pragma unroll
+                    for (int a = 0; a < 2; ++a)
+#pragma unroll
+                        for (int b = 0; b < 2; ++b)
+                            if (r + a < M && c + b < N && (!mirror || r + a >= c + b)) {
+                                C[(r + a) + (long)(c + b) * ldc] = v[a][b];
+                                if (mirror && r + a > c + b) C[(c + b) + (long)(r + a) * ldc] = v[a][b];
+                            }
                 }
             }
-        }
-    }
     if (amax) {
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, d));
@@ -270,17 +328,17 @@ __global__ void __launch_bounds__(GEMM_THREADS, (Cfg::BM == 128 ? 1 : 2))
 }
 
 // C = alpha * sum_s part[s] + beta * C over the tiles the GEMM computed
-// (tile size bm x bn), the splits summed in a fixed order (deterministic),
+// (tiles of b x b), the splits summed in a fixed order (deterministic),
 // max|C| folded into amax.
 __global__ void k_splitk_reduce(int M, int N, int splits, const double* __restrict__ part, double alpha,
-                                double beta, double* C, long ldc, unsigned long long* amax, int mode, int bm,
-                                int bn, const int* skip) {
+                                double beta, double* C, long ldc, unsigned long long* amax, int mode, int b,
+                                const int* skip) {
     if (skip && *skip) return;
     const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
     double mx = 0.0;
     if (idx < (long)M * N) {
         const int col = (int)(idx / M), row = (int)(idx - (long)col * M);
-        if (!((mode & GEMM_LOWER) && (col / bn) * bn > (row / bm) * bm + bm - 1) &&
+        if (!((mode & GEMM_LOWER) && col / b > row / b) &&
             !((mode & GEMM_MIRROR) && row < col)) {
             double v = 0.0;
             for (int s = 0; s < splits; ++s) v += part[(size_t)s * M * N + idx];
@@ -302,41 +360,40 @@ __global__ void k_splitk_reduce(int M, int N, int splits, const double* __restri
 }
 
 namespace {
-template <class Cfg>
-int active_tiles(dim3 grid, int mode) {
-    if (!(mode & GEMM_LOWER)) return (int)(grid.x * grid.y);
+int active_tiles(int M, int N, int b, int mode) {
+    const int gy = (M + b - 1) / b, gx = (N + b - 1) / b;
+    if (!(mode & GEMM_LOWER)) return gy * gx;
     int tiles = 0;
-    for (unsigned by = 0; by < grid.y; ++by)
-        for (unsigned bx = 0; bx < grid.x; ++bx) tiles += (int)(bx * Cfg::BN) <= (int)(by * Cfg::BM) + Cfg::BM - 1;
+    for (int y = 0; y < gy; ++y) tiles += std::min(gx, y + 1);
     return tiles;
 }
 
-template <class Cfg>
+template <int W, bool kTransA, bool kTransB, bool kShortAcc>
+bool gemm_smem() {
+    return cudaFuncSetAttribute(k_gemm_f64<W, kTransA, kTransB, kShortAcc>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GemmTile<W>::SMEM) == cudaSuccess;
+}
+
+template <int W>
 void gemm_attr() {
     static std::atomic<unsigned long long> attr{0};
     once_per_device(attr, [] {
-        return cudaFuncSetAttribute(k_gemm_f64<Cfg, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)Cfg::SMEM) == cudaSuccess &&
-               cudaFuncSetAttribute(k_gemm_f64<Cfg, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)Cfg::SMEM) == cudaSuccess &&
-               cudaFuncSetAttribute(k_gemm_f64<Cfg, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)Cfg::SMEM) == cudaSuccess &&
-               cudaFuncSetAttribute(k_gemm_f64<Cfg, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)Cfg::SMEM) == cudaSuccess;
+        return gemm_smem<W, false, false, false>() && gemm_smem<W, false, true, false>() &&
+               gemm_smem<W, false, true, true>() && gemm_smem<W, true, false, false>();
     });
 }
 
-template <class Cfg>
+template <int W>
 void launch_gemm(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb, double beta,
                  double* C, int ldc, unsigned long long* amax, int mode, cudaStream_t st, double* ws,
                  size_t ws_doubles, const int* skip) {
-    gemm_attr<Cfg>();
-    dim3 grid((N + Cfg::BN - 1) / Cfg::BN, (M + Cfg::BM - 1) / Cfg::BM);
+    gemm_attr<W>();
     // split-K when the output has too few tiles to fill the SMs: each split
     // keeps at least kMinSplitTiles k tiles, the partial slabs fit in ws
-    const int tiles = active_tiles<Cfg>(grid, mode);
-    constexpr int kSMs = 148, kMinSplitTiles = 3, kMaxSplits = 16;
-    const int slots = kSMs * (Cfg::BM == 128 ? 1 : 2);
+    constexpr int B_ = GemmTile<W>::B;
+    const int tiles = active_tiles(M, N, B_, mode);
+    constexpr int kMinSplitTiles = 6, kMaxSplits = 16;
+    const int slots = device_sms() * GEMM_CTAS;
     int splits = 1;
     const int kt = (K + BK - 1) / BK;
     if (ws && tiles > 0 && tiles < slots && kt >= 2 * kMinSplitTiles) {
@@ -345,17 +402,19 @@ void launch_gemm(int M, int N, int K, double alpha, const double* A, int lda, co
         while (splits > 1 && (size_t)splits * slab > ws_doubles) --splits;
     }
     double* part = splits > 1 ? ws : nullptr;
-    grid.z = splits;
-    const bool tb = (mode & GEMM_TRANS_B) != 0, sa = (mode & GEMM_SHORT_ACC) != 0;
-    auto kern = tb ? (sa ? k_gemm_f64<Cfg, true, true> : k_gemm_f64<Cfg, true, false>)
-                   : (sa ? k_gemm_f64<Cfg, false, true> : k_gemm_f64<Cfg, false, false>);
-    kern<<<grid, GEMM_THREADS, Cfg::SMEM, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, amax, mode, part,
-                                                skip);
+    const dim3 grid((unsigned)((M + B_ - 1) / B_) * (unsigned)((N + B_ - 1) / B_), splits);
+    // GEMM_SHORT_ACC comes with GEMM_TRANS_B, GEMM_TRANS_A without it
+    const auto kern = (mode & GEMM_TRANS_A)      ? k_gemm_f64<W, true, false, false>
+                      : !(mode & GEMM_TRANS_B)   ? k_gemm_f64<W, false, false, false>
+                      : (mode & GEMM_SHORT_ACC) ? k_gemm_f64<W, false, true, true>
+                                                : k_gemm_f64<W, false, true, false>;
+    kern<<<grid, GEMM_THREADS, GemmTile<W>::SMEM, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, amax, mode, part,
+                                                        skip);
     count_launch();
     if (part) {
         const long total = (long)M * N;
         k_splitk_reduce<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(M, N, splits, part, alpha, beta, C, ldc,
-                                                                          amax, mode, Cfg::BM, Cfg::BN, skip);
+                                                                          amax, mode, B_, skip);
         count_launch();
     }
 }
@@ -365,12 +424,10 @@ void gemm_f64_mode(int M, int N, int K, double alpha, const double* A, int lda, 
                    double beta, double* C, int ldc, unsigned long long* amax, int mode, cudaStream_t st,
                    double* ws, size_t ws_doubles, const int* skip) {
     if (M <= 0 || N <= 0) return;
-    // 64 x 64 tiles when 128 x 128 tiles would leave most SMs idle
-    const dim3 g128((N + 127) / 128, (M + 127) / 128);
-    if (active_tiles<CfgBig>(g128, mode) * 4 <= 148)
-        launch_gemm<CfgSmall>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, amax, mode, st, ws, ws_doubles, skip);
+    if (active_tiles(M, N, GemmTile<32>::B, mode) < device_sms())
+        launch_gemm<16>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, amax, mode, st, ws, ws_doubles, skip);
     else
-        launch_gemm<CfgBig>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, amax, mode, st, ws, ws_doubles, skip);
+        launch_gemm<32>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, amax, mode, st, ws, ws_doubles, skip);
 }
 
 void gemm_f64_ex(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
@@ -390,60 +447,19 @@ void gemm_f64_tri(int M, int N, int K, double alpha, const double* A, int lda, c
     gemm_f64_ex(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, nullptr, true, st, false);
 }
 
-// Copy the strict lower triangle onto the upper one (32 x 32 tiles).
-__global__ void k_mirror_lower(double* Z, int n, long ld, const int* skip) {
-    if (skip && *skip) return;
-    __shared__ double t[32][33];
-    const int bi = blockIdx.y, bj = blockIdx.x;  // tile row, tile col of the source (lower) tile
-    if (bj > bi) return;
-    for (int r = threadIdx.y; r < 32; r += 8) {
-        int i = bi * 32 + r, j = bj * 32 + threadIdx.x;
-        t[r][threadIdx.x] = (i < n && j < n) ? Z[i + (long)j * ld] : 0.0;
-    }
-    __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += 8) {
-        int j = bj * 32 + r, i = bi * 32 + threadIdx.x;  // target (j, i) = source (i, j), i > j
-        if (i < n && j < n && i > j) Z[j + (long)i * ld] = t[threadIdx.x][r];
-    }
-}
-
-void launch_mirror_lower(double* Z, int n, int ld, cudaStream_t st, const int* skip) {
-    if (n == 0) return;
-    dim3 g((n + 31) / 32, (n + 31) / 32);
-    k_mirror_lower<<<g, dim3(32, 8), 0, st>>>(Z, n, ld, skip);
-    count_launch();
-}
-
 // ------------------------------------------------------------------------
 // SPD inverse: recursive Cholesky A = L L^T that forms T = L^{-1} on the
 // way, then A^{-1} = T^T T
 // ------------------------------------------------------------------------
-size_t chol_small_doubles(int n) { (void)n; return (size_t)NB * NB + 64; }
-
 __global__ void __launch_bounds__(LEAF_THREADS) k_chol_leaf(const double* __restrict__ A, long lda, int k0,
                                                             int kb, double* T, long ldt, int* err) {
     extern __shared__ __align__(16) double lsm[];
     chol_leaf_tile(A, lda, k0, kb, T, ldt, err, lsm);
 }
 
-// Tt = T^T (n x n), 32 x 32 tiles through shared memory.
-__global__ void k_transpose(const double* __restrict__ T, long ldt, int n, double* Tt, long ldo) {
-    __shared__ double t[32][33];
-    int bx = blockIdx.x * 32, by = blockIdx.y * 32;
-    for (int r = threadIdx.y; r < 32; r += 8) {
-        int i = by + r, j = bx + threadIdx.x;
-        if (i < n && j < n) t[r][threadIdx.x] = T[i + (long)j * ldt];
-    }
-    __syncthreads();
-    for (int r = threadIdx.y; r < 32; r += 8) {
-        int j = bx + r, i = by + threadIdx.x;  // out(j, i) = T(i, j)
-        if (i < n && j < n) Tt[j + (long)i * ldo] = t[threadIdx.x][r];
-    }
-}
-
 void prepare_dense_kernels() {
-    gemm_attr<CfgBig>();
-    gemm_attr<CfgSmall>();
+    gemm_attr<32>();
+    gemm_attr<16>();
     static std::atomic<unsigned long long> attr{0};
     once_per_device(attr, [] {
         return cudaFuncSetAttribute(k_chol_leaf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LEAF_SMEM) ==
@@ -452,6 +468,12 @@ void prepare_dense_kernels() {
 }
 
 namespace {
+
+// Where the recursion splits [r0, r1): the first half a multiple of 64.
+int chol_split(int r0, int r1) {
+    const int m = r0 + (((r1 - r0) / 2 + NB - 1) / NB) * NB;
+    return m >= r1 ? r1 - NB : m;
+}
 
 // Factor A[r0:r1, r0:r1] (already updated by the earlier panels) and write
 // T[r0:r1, r0:r1] = L^{-1}. With the split [r0, m) [m, r1):
@@ -462,47 +484,67 @@ namespace {
 //   T21 = -T22 X                    (T22 lower triangular)
 // Every product is a GEMM whose k loop skips the zero triangle of its
 // triangular operand, so the whole recursion costs n^3 / 3 + n^3 / 3 flops.
-void chol_rec(double* A, int lda, double* T, double* W, double* ws, size_t wsd, int r0, int r1, int* err,
-              cudaStream_t st) {
+// Blocks that the tile tasks take (up to n = 3584) end the recursion: down to
+// single leaves each 64 rows cost a leaf and five small dependent launches
+// (n = 5401: 5.5 of 13.8 ms), as tasks one diagonal task of their chain.
+int chol_rec(double* A, int lda, const SpdScratch& s, size_t wsd, int r0, int r1, int* err, cudaStream_t st) {
     const int n = r1 - r0;
+    double* T = s.T;
+    if (s.state && spd_tasks_apply(n)) {
+        const long at = r0 + (long)r0 * lda;
+        return chol_inverse_tasks(A + at, n, lda, T + at, nullptr, s.state, err, st, s.max_ctas);
+    }
     if (n <= NB) {
         prepare_dense_kernels();
         k_chol_leaf<<<1, LEAF_THREADS, LEAF_SMEM, st>>>(A, lda, r0, n, T, lda, err);
         count_launch();
-        return;
+        return UNC_OK;
     }
-    int m = r0 + ((n / 2 + NB - 1) / NB) * NB;
-    if (m >= r1) m = r1 - NB;
+    const int m = chol_split(r0, r1);
     const int h1 = m - r0, h2 = r1 - m;
-    chol_rec(A, lda, T, W, ws, wsd, r0, m, err, st);
+    if (int r = chol_rec(A, lda, s, wsd, r0, m, err, st)) return r;
     double* A21 = A + m + (long)r0 * lda;
     const double* T11 = T + r0 + (long)r0 * lda;
-    gemm_f64_mode(h2, h1, h1, 1.0, A21, lda, T11, lda, 0.0, W, lda, nullptr,
-                  GEMM_TRANS_B | GEMM_KHI_N | GEMM_SHORT_ACC, st, ws, wsd);
-    gemm_f64_mode(h2, h2, h1, -1.0, W, lda, W, lda, 1.0, A + m + (long)m * lda, lda, nullptr,
-                  GEMM_TRANS_B | GEMM_LOWER | GEMM_SHORT_ACC, st, ws, wsd);
-    gemm_f64_mode(h2, h1, h1, 1.0, W, lda, T11, lda, 0.0, A21, lda, nullptr, GEMM_KLO_N, st, ws, wsd);
-    chol_rec(A, lda, T, W, ws, wsd, m, r1, err, st);
+    gemm_f64_mode(h2, h1, h1, 1.0, A21, lda, T11, lda, 0.0, s.W, lda, nullptr,
+                  GEMM_TRANS_B | GEMM_KHI_N | GEMM_SHORT_ACC, st, s.ws, wsd);
+    gemm_f64_mode(h2, h2, h1, -1.0, s.W, lda, s.W, lda, 1.0, A + m + (long)m * lda, lda, nullptr,
+                  GEMM_TRANS_B | GEMM_LOWER | GEMM_SHORT_ACC, st, s.ws, wsd);
+    gemm_f64_mode(h2, h1, h1, 1.0, s.W, lda, T11, lda, 0.0, A21, lda, nullptr, GEMM_KLO_N, st, s.ws, wsd);
+    if (int r = chol_rec(A, lda, s, wsd, m, r1, err, st)) return r;
     gemm_f64_mode(h2, h1, h2, -1.0, T + m + (long)m * lda, lda, A21, lda, 0.0, T + m + (long)r0 * lda, lda,
-                  nullptr, GEMM_KHI_M, st, ws, wsd);
+                  nullptr, GEMM_KHI_M, st, s.ws, wsd);
+    return UNC_OK;
+}
+
+int prepare_rec(int r0, int r1) {
+    if (spd_tasks_apply(r1 - r0)) return spd_tasks_prepare(r1 - r0, false);
+    const int m = chol_split(r0, r1);
+    if (int r = prepare_rec(r0, m)) return r;
+    return prepare_rec(m, r1);
 }
 }  // namespace
 
-void chol_lower_inverse(double* A, int n, int lda, double* T, double* W, double* ws, int* err, cudaStream_t st) {
-    chol_rec(A, lda, T, W, ws, (size_t)n * lda, 0, n, err, st);
+int spd_prepare(int n) { return spd_tasks_apply(n) ? spd_tasks_prepare(n, true) : prepare_rec(0, n); }
+
+int chol_lower_inverse(double* A, int n, int lda, const SpdScratch& s, int* err, cudaStream_t st) {
+    return chol_rec(A, lda, s, (size_t)n * lda, 0, n, err, st);
 }
 
-void chol_inverse(double* A, int n, int lda, double* T, double* W, double* Tt, double* small, int* err,
-                  cudaStream_t st) {
-    (void)small;
-    // Tt is free until the final product: split-K partial sums of the recursion
-    chol_lower_inverse(A, n, lda, T, W, Tt, err, st);
-    // A^{-1} = T^T T: lower tiles, k >= the tile's first row (T lower triangular), then mirror
-    dim3 g((n + 31) / 32, (n + 31) / 32);
-    k_transpose<<<g, dim3(32, 8), 0, st>>>(T, lda, n, Tt, lda);
-    count_launch();
-    gemm_f64_mode(n, n, n, 1.0, Tt, lda, T, lda, 0.0, A, lda, nullptr, GEMM_LOWER | GEMM_KLO_M, st);
-    launch_mirror_lower(A, n, lda, st);
+int spd_inverse(double* A, int n, int lda, double shift, double* e, const SpdScratch& s, double* Y, int* err,
+                cudaStream_t st) {
+    launch_shift_equilibrate(A, n, lda, shift, e, err, st);
+    if (s.state && spd_tasks_apply(n)) {
+        if (int r = chol_inverse_tasks(A, n, lda, s.T, s.W, s.state, err, st, s.max_ctas, s.poll_limit, s.skip_task))
+            return r;
+        launch_unequilibrate_from(s.W, A, n, lda, e, Y, st);
+        return UNC_OK;
+    }
+    if (int r = chol_lower_inverse(A, n, lda, s, err, st)) return r;
+    // A^{-1} = T^T T: lower tiles, k >= the tile's first row (T lower triangular), written in both triangles
+    gemm_f64_mode(n, n, n, 1.0, s.T, lda, s.T, lda, 0.0, A, lda, nullptr,
+                  GEMM_LOWER | GEMM_KLO_M | GEMM_TRANS_A | GEMM_MIRROR, st);
+    launch_unequilibrate(A, n, lda, e, Y, st);
+    return UNC_OK;
 }
 
 // ------------------------------------------------------------------------

@@ -51,6 +51,23 @@ void once_per_device(std::atomic<unsigned long long>& done, F&& f) {
     if (done.load(std::memory_order_relaxed) & bit) return;
     if (f()) done.fetch_or(bit, std::memory_order_release);
 }
+// Device scratch of one call, allocated in stream order from the library's own
+// memory pool of the current device and freed in stream order when it goes out
+// of scope. Between calls the pool keeps at most kScratchKept bytes, so that a
+// repeated call neither maps nor unmaps memory (cudaMalloc, cudaFree and their
+// implicit synchronisation cost 0.4 to 4 ms beside kernels of 0.5 to 15 ms);
+// more than that goes back at the next synchronisation, everything when
+// scratch_trim is called (a context or batch is released or destroyed).
+// Thread-safe; streams may differ from call to call.
+constexpr unsigned long long kScratchKept = 1ULL << 30;
+struct Scratch {
+    void* p = nullptr;
+    cudaStream_t st = nullptr;
+    cudaError_t alloc(size_t bytes, cudaStream_t stream);
+    ~Scratch();
+};
+void scratch_trim();  // of the current device
+
 // Per-device set-up of the kernels' shared-memory attributes (current device).
 void prepare_assembly_kernels();
 void prepare_dense_kernels();
@@ -133,15 +150,15 @@ size_t scan_tmp_ints(int n);
 void gemm_f64(int M, int N, int K, double alpha, const double* A, int lda, const double* B,
               int ldb, double beta, double* C, int ldc, unsigned long long* amax, cudaStream_t st);
 // General form: lower_only skips output tiles strictly above the diagonal
-// (symmetric results; mirror afterwards with launch_mirror_lower).
+// (symmetric results; GEMM_MIRROR of gemm_f64_mode writes the other triangle too).
 // trans_b: B(k, n) is read from B[n + k * ldb] (the transpose of a column-major matrix).
 void gemm_f64_ex(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
                  double beta, double* C, int ldc, unsigned long long* amax, bool lower_only, cudaStream_t st,
                  bool trans_b = false);
 // Mode bits of gemm_f64_mode. The k-range bits restrict the k loop of the
 // output tile at (m0, n0) when an operand is triangular (terms outside the
-// range are zero): KLO_M k >= m0, KLO_N k >= n0, KHI_M k < m0 + 128,
-// KHI_N k < n0 + 128 (tile size 128 x 128).
+// range are zero): KLO_M k >= m0, KLO_N k >= n0, KHI_M k < m0 + 64,
+// KHI_N k < n0 + 64 (tile size 64 x 64).
 enum : int {
     GEMM_LOWER = 1,
     GEMM_TRANS_B = 2,
@@ -150,8 +167,9 @@ enum : int {
     GEMM_KHI_M = 16,
     GEMM_KHI_N = 32,
     GEMM_MIRROR = 64,  // symmetric C: write the lower triangle at (i, j) and (j, i), nothing above it directly
-    GEMM_SHORT_ACC = 128,  // partial sums over k = 8 from zero, added with ordinary FP64 additions (the
-                           // products that feed Cholesky pivots: see k_gemm_f64)
+    GEMM_SHORT_ACC = 128,  // partial sums over k = 32 from zero, added to the running sums (the products
+                           // that feed Cholesky pivots: see k_gemm_f64); with GEMM_TRANS_B only
+    GEMM_TRANS_A = 256,    // A(m, k) is read from A[k + m * lda]; without GEMM_TRANS_B only
 };
 // ws (ws_doubles): optional scratch that enables split-K for outputs with
 // fewer tiles than SMs (partials summed in a fixed order by a second kernel).
@@ -160,21 +178,30 @@ enum : int {
 void gemm_f64_mode(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
                    double beta, double* C, int ldc, unsigned long long* amax, int mode, cudaStream_t st,
                    double* ws = nullptr, size_t ws_doubles = 0, const int* skip = nullptr);
-void launch_mirror_lower(double* Z, int n, int ld, cudaStream_t st, const int* skip = nullptr);
 // Same, skipping output tiles strictly above the diagonal (symmetric updates).
 void gemm_f64_tri(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
                   double beta, double* C, int ldc, cudaStream_t st);
-// In-place inverse of an SPD matrix (n x n, lda): recursive Cholesky that
-// forms T = L^{-1} directly (64 x 64 leaves, GEMM merges), then A^{-1} = T^T T.
-// T, W, Tt: n x lda scratch matrices, all finite, T zero on entry; small:
-// chol_small_doubles(n) doubles (unused by the recursive form, kept for the
-// workspace layout). Sets ERRBIT_SINGULAR in err.
-size_t chol_small_doubles(int n);
-void chol_inverse(double* A, int n, int lda, double* T, double* W, double* Tt, double* small, int* err,
-                  cudaStream_t st);
-// The recursion of chol_inverse alone: T = L^{-1} (lower triangle; T zero on
-// entry), A overwritten; ws: n x lda doubles of split-K scratch.
-void chol_lower_inverse(double* A, int n, int lda, double* T, double* W, double* ws, int* err, cudaStream_t st);
+// Scratch of an SPD inverse of order n: T (receives L^{-1}; its tiles above the
+// diagonal are neither read nor written) and W, n x lda each; ws: n x lda doubles of split-K
+// partial sums, or unused by the tile tasks; state: spd_task_state_ints(n) ints
+// of the tile tasks (dag.cu), nullptr to run without them (nothing uploaded).
+struct SpdScratch {
+    double *T, *W, *ws;
+    int* state;
+    int max_ctas = 148;        // grid bound of the tile tasks
+    long long poll_limit = 0;  // as chol_inverse_tasks
+    int skip_task = -1;
+};
+// Uploads the task lists that an inverse of order n uses (once per device and
+// size; outside any stream capture).
+int spd_prepare(int n);
+// In-place inverse of A + shift I (SPD, n x n, lda, both triangles), Jacobi
+// equilibrated (e: n doubles): tile tasks up to n = 3584, above by recursion on
+// halves. Y (optional): a copy of the result. Sets ERRBIT_SINGULAR in err.
+int spd_inverse(double* A, int n, int lda, double shift, double* e, const SpdScratch& s, double* Y, int* err,
+                cudaStream_t st);
+// The recursion alone: T = L^{-1} (lower triangle), A overwritten.
+int chol_lower_inverse(double* A, int n, int lda, const SpdScratch& s, int* err, cudaStream_t st);
 // A <- A + lambda*I and symmetric Jacobi equilibration: A_s = E A E, E = diag(A_ii)^-1/2.
 void launch_shift_equilibrate(double* A, int n, int lda, double lambda, double* e, int* err,
                               cudaStream_t st);
@@ -189,10 +216,10 @@ void launch_unequilibrate_from(const double* S, double* X, int n, int lda, const
 // A (lower triangle) is overwritten by L, T receives L^{-1} (lower tiles) and
 // O = A^{-1} (both triangles). state: spd_task_state_ints(n) ints.
 // spd_tasks_prepare uploads the task list of this size once per device (call it
-// outside stream capture).
+// outside stream capture). O == nullptr (prepared with product = false): T only.
 bool spd_tasks_apply(int n);
 size_t spd_task_state_ints(int n);
-int spd_tasks_prepare(int n);
+int spd_tasks_prepare(int n, bool product = true);
 // max_ctas bounds the persistent grid (at most one CTA per SM is used anyway);
 // the task order and every tile's update order do not depend on it, so neither
 // do the results.
@@ -423,6 +450,7 @@ struct PinvBuffers {
     double *X, *Y, *MX, *MX2;      // n x 32 subspace blocks
     double *H, *Wr, *S;            // 32 x 32
     double *theta, *res, *e;
+    int* state;                    // counters of the tile tasks
     int* err;
     unsigned long long* dmax;
 };

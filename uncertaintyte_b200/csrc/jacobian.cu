@@ -182,14 +182,14 @@ extern "C" int unc_jacobian_device(int num_cams, int num_points, int num_obs, co
         return UNC_ERR_INVALID_ARG;
     }
     cudaStream_t sm = (cudaStream_t)stream;
-    int* err = nullptr;
-    if (cudaMallocAsync((void**)&err, sizeof(int), sm) != cudaSuccess) return UNC_ERR_OUT_OF_MEMORY;
+    Scratch mem;
+    if (mem.alloc(sizeof(int), sm) != cudaSuccess) return UNC_ERR_OUT_OF_MEMORY;
+    int* err = static_cast<int*>(mem.p);
     cudaMemsetAsync(err, 0, sizeof(int), sm);
     int rc = launch_scene_jacobian(num_cams, num_points, num_obs, d_cams, d_points, d_obs_cam, d_obs_pt, d_rows,
                                    d_cols, d_values, err, sm);
     int h = 0;
     cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, sm);
-    cudaFreeAsync(err, sm);
     cudaError_t e = cudaStreamSynchronize(sm);
     if (rc != UNC_OK || e != cudaSuccess) {
         g_last_error = std::string("unc_jacobian_device: ") + cudaGetErrorString(e);

@@ -30,9 +30,8 @@ namespace {
 
 constexpr int kNoAllocMaxN = 512;                                    // largest n and lda
 constexpr size_t kMat = (size_t)kNoAllocMaxN * kNoAllocMaxN;        // one n x lda matrix
-constexpr size_t kSmall = (size_t)64 * 64 + 64;                      // >= chol_small_doubles(n)
 constexpr size_t kEq = (size_t)kNoAllocMaxN + 64;                    // equilibration scales
-constexpr size_t kScratchDoubles = 3 * kMat + kSmall + kEq + 8;      // + the error word
+constexpr size_t kScratchDoubles = 3 * kMat + kEq + 8;      // + the error word
 
 // The scratch: host code may only use its name to look up the device address.
 __device__ __align__(256) double g_inverse_scratch[kScratchDoubles];
@@ -115,10 +114,6 @@ extern "C" int unc_dense_inverse_noalloc(double* d_A, int n, int lda, void* stre
         g_last_error = "unc_dense_inverse_noalloc: n and lda must be at most 512 (static scratch size)";
         return UNC_ERR_TOO_LARGE;
     }
-    if (chol_small_doubles(n) > kSmall) {
-        g_last_error = "static scratch too small for the panel buffers";
-        return UNC_ERR_TOO_LARGE;
-    }
     double* ws = nullptr;
     int rc = scratch_for_current_device(&ws);
     if (rc != UNC_OK) return rc;
@@ -127,20 +122,18 @@ extern "C" int unc_dense_inverse_noalloc(double* d_A, int n, int lda, void* stre
     double* T = ws;
     double* W = ws + kMat;
     double* Tt = ws + 2 * kMat;
-    double* small = ws + 3 * kMat;
-    double* e = small + kSmall;
+    double* e = ws + 3 * kMat;
     int* err = reinterpret_cast<int*>(e + kEq);
     // the previous call's contents stay in the array: clear what must start at
     // zero (T above its diagonal blocks, the padding rows, the error word)
     cudaError_t ce = cudaMemsetAsync(T, 0, sizeof(double) * mat, sm);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(W, 0, sizeof(double) * mat, sm);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(Tt, 0, sizeof(double) * mat, sm);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(small, 0, sizeof(double) * (kSmall + kEq + 8), sm);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(e, 0, sizeof(double) * (kEq + 8), sm);
     int h_err = 0;
     if (ce == cudaSuccess) {
-        launch_shift_equilibrate(d_A, n, lda, 0.0, e, err, sm);
-        chol_inverse(d_A, n, lda, T, W, Tt, small, err, sm);
-        launch_unequilibrate(d_A, n, lda, e, nullptr, sm);
+        // no tile tasks: their list would have to be uploaded into allocated memory
+        spd_inverse(d_A, n, lda, 0.0, e, SpdScratch{T, W, Tt, nullptr}, nullptr, err, sm);
         ce = cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, sm);
     }
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(sm);

@@ -303,15 +303,15 @@ int read_err(const int* d_err, int* h, cudaStream_t sm) {
 }
 
 // In-place SPD inverse with equilibration (the inverse of the Taylor path).
-int spd_inverse(double* A, int n, int ld, const PinvBuffers& b, cudaStream_t sm) {
-    const size_t mat = (size_t)n * ld;
-    SVD_CK(cudaMemsetAsync(b.T, 0, sizeof(double) * mat, sm));
+SpdScratch spd_scratch(const PinvBuffers& b) { return SpdScratch{b.T, b.W, b.Tt, b.state, device_sms()}; }
+
+int inverse_in_place(double* A, int n, int ld, const PinvBuffers& b, cudaStream_t sm) {
     SVD_CK(cudaMemsetAsync(b.err, 0, sizeof(int), sm));
-    launch_shift_equilibrate(A, n, ld, 0.0, b.e, b.err, sm);
-    chol_inverse(A, n, ld, b.T, b.W, b.Tt, nullptr, b.err, sm);
-    launch_unequilibrate(A, n, ld, b.e, nullptr, sm);
+    if (int rc = spd_inverse(A, n, ld, 0.0, b.e, spd_scratch(b), nullptr, b.err, sm))
+        return svd_fail(rc, "SPD inverse: launch failed");
     int e = 0;
     if (int rc = read_err(b.err, &e, sm)) return rc;
+    if (e & ERRBIT_TIMEOUT) return svd_fail(UNC_ERR_CUDA, "a bounded device wait of the tile-task inverse ran out");
     if (e & (ERRBIT_SINGULAR | ERRBIT_NONFINITE)) return svd_fail(UNC_ERR_SINGULAR, "matrix is not positive definite");
     return UNC_OK;
 }
@@ -335,6 +335,7 @@ size_t pinv_carve(char* base, int n, int ld, PinvBuffers& b) {
     b.theta = c.take<double>(kMaxBlock);
     b.res = c.take<double>(kMaxBlock);
     b.e = c.take<double>((size_t)n + 64);
+    b.state = c.take<int>(spd_task_state_ints(n));
     b.err = c.take<int>(4);
     b.dmax = c.take<unsigned long long>(1);
     return c.off + 256;
@@ -348,6 +349,7 @@ int pinv_psd(double* M, int n, int ld, int remove_n, double eps, const PinvBuffe
     if (n <= 0 || ld < n || (ld & 1)) return svd_fail(UNC_ERR_INVALID_ARG, "bad matrix arguments");
     if (remove_n > kMaxBlock - 1)
         return svd_fail(UNC_ERR_UNSUPPORTED, "at most 31 singular values can be removed");
+    if (int rc = spd_prepare(n)) return svd_fail(rc, "tile-task inverse: cannot upload the task list");
     const size_t mat = (size_t)n * ld, blk = (size_t)ld * kMaxBlock;
     // every scratch matrix starts finite (the GEMM reads padding rows in pairs)
     SVD_CK(cudaMemsetAsync(b.W, 0, sizeof(double) * mat, sm));
@@ -363,7 +365,7 @@ int pinv_psd(double* M, int n, int ld, int remove_n, double eps, const PinvBuffe
 
     if (remove_n == 0) {  // nothing removed: the plain inverse
         inf.removed = 0;
-        return spd_inverse(M, n, ld, b, sm);
+        return inverse_in_place(M, n, ld, b, sm);
     }
     k_diag_absmax<<<(n + 255) / 256, 256, 0, sm>>>(M, n, ld, b.dmax);
     count_launch();
@@ -384,13 +386,12 @@ int pinv_psd(double* M, int n, int ld, int remove_n, double eps, const PinvBuffe
     bool ok = false;
     for (int attempt = 0; attempt < 4 && !ok; ++attempt) {
         SVD_CK(cudaMemcpyAsync(b.G, M, sizeof(double) * mat, cudaMemcpyDeviceToDevice, sm));
-        SVD_CK(cudaMemsetAsync(b.T, 0, sizeof(double) * mat, sm));
         SVD_CK(cudaMemsetAsync(b.err, 0, sizeof(int), sm));
-        launch_shift_equilibrate(b.G, n, ld, s, b.e, b.err, sm);
-        chol_inverse(b.G, n, ld, b.T, b.W, b.Tt, nullptr, b.err, sm);
-        launch_unequilibrate(b.G, n, ld, b.e, nullptr, sm);
+        if (int rc = spd_inverse(b.G, n, ld, s, b.e, spd_scratch(b), nullptr, b.err, sm))
+            return svd_fail(rc, "SPD inverse: launch failed");
         int e = 0;
         if (int rc = read_err(b.err, &e, sm)) return rc;
+        if (e & ERRBIT_TIMEOUT) return svd_fail(UNC_ERR_CUDA, "a bounded device wait of the tile-task inverse ran out");
         ok = !(e & (ERRBIT_SINGULAR | ERRBIT_NONFINITE));
         if (!ok) s *= 100.0;
     }
@@ -452,7 +453,7 @@ int pinv_psd(double* M, int n, int ld, int remove_n, double eps, const PinvBuffe
     if (remove_n < 0 && kk > p - 4)
         return svd_fail(UNC_ERR_UNSUPPORTED, "more than 20 singular values at or below epsilon");
     inf.removed = kk;
-    if (kk == 0) return spd_inverse(M, n, ld, b, sm);
+    if (kk == 0) return inverse_in_place(M, n, ld, b, sm);
     if (kk >= n) {
         SVD_CK(cudaMemsetAsync(M, 0, sizeof(double) * mat, sm));
         return UNC_OK;
@@ -469,7 +470,7 @@ int pinv_psd(double* M, int n, int ld, int remove_n, double eps, const PinvBuffe
 
     // 3. B = M + c V_R V_R^T, inverted in place
     gemm_f64_mode(n, n, kk, c, b.X, ld, b.X, ld, 1.0, M, ld, nullptr, GEMM_TRANS_B, sm);
-    if (int rc = spd_inverse(M, n, ld, b, sm)) return rc;
+    if (int rc = inverse_in_place(M, n, ld, b, sm)) return rc;
 
     // 4. P B^{-1} P = B^{-1} - Z V^T - V Z^T + V (V^T Z) V^T, Z = B^{-1} V
     gemm_f64(n, kk, n, 1.0, M, ld, b.X, ld, 0.0, b.Y, ld, nullptr, sm);
@@ -641,11 +642,10 @@ extern "C" int unc_pinv_psd_device(double* d_M, int n, int ld, int remove_n, dou
     cudaStream_t sm = (cudaStream_t)stream;
     PinvBuffers b;
     const size_t bytes = pinv_carve(nullptr, n, ld, b);
-    char* ws = nullptr;
-    SVD_CK(cudaMalloc(&ws, bytes));
-    pinv_carve(ws, n, ld, b);
+    Scratch mem;
+    SVD_CK(mem.alloc(bytes, sm));
+    pinv_carve(static_cast<char*>(mem.p), n, ld, b);
     int rc = pinv_psd(d_M, n, ld, remove_n, epsilon < 0 ? 1e-10 : epsilon, b, sm, nullptr);
     cudaStreamSynchronize(sm);
-    cudaFree(ws);
     return rc;
 }
