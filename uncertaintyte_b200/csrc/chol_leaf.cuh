@@ -9,229 +9,270 @@ constexpr int NB = 64;  // leaf size
 
 // Leaf: Cholesky of the kb x kb (kb <= 64) diagonal block of A at (k0, k0)
 // and T_kk = L_kk^{-1}, written as a full kb x kb block of T (zeros above the
-// diagonal). One CTA of 512 threads; the block (S) and its inverse (Ts) sit in
-// shared memory, padded to 64 x 64 with an identity tail (the factor and
-// inverse of blockdiag(A, I) are blockdiag(L, I) and blockdiag(L^-1, I), so
-// every step has fixed shapes). Four 16-column panels:
-//  (A) warp 0 factors the 16 x 16 diagonal block in registers (lane = row,
-//      column p broadcast by shuffle; the pivot check is folded into a flag so
-//      that the dependent chain carries no branch), 1 / L(p, p) kept in rinv;
-//  (B) the rows below solve x L_qq^T = A_iq by forward substitution, one
-//      thread per row;
-//  (C) the trailing lower triangle takes the rank-16 update in 2 x 2 register
-//      tiles.
-// Then T = L^{-1} from the diagonal inverses D_q = L_qq^{-1} (D_0..D_2 are
-// formed beside the last panel's factorisation): T_{q+1,q} = -D_{q+1} L_{q+1,q}
-// D_q for the two 16-row pairs, then T21 = -T1 (L21 T0) for the 32-row halves.
-// Intermediate products are kept transposed in the unused upper blocks of Ts,
-// and only the lower triangle is written out.
+// diagonal). One CTA of 256 threads; the block (S) and its inverse (Ts) sit in
+// shared memory, column-major with a stride of 68 doubles (fragment reads in
+// both orientations and lane = row reads are conflict-free), padded to 64 x 64
+// with an identity tail (the factor and inverse of blockdiag(A, I) are
+// blockdiag(L, I) and blockdiag(L^-1, I), so every step has fixed shapes).
+//
+// The leaf is a chain of dependent operations, so everything but that chain
+// runs beside it. Four 16-column panels q:
+//  (A) warp 0 factors the 16 x 16 diagonal block in registers, two columns per
+//      step: with pivot d, e below it and f the next diagonal entry,
+//      1/L(p,p) = d^-1/2 and 1/L(p+1,p+1) = (d f - e^2)^-1/2 d^1/2, whose two
+//      reciprocal square roots run side by side, and the next step's d, e, f are
+//      formed by every lane from broadcast values (one shuffle latency per
+//      step). Lanes 0..15 hold the block's rows, lanes 16..31 the rows of the
+//      identity, which the same instructions turn into D_q = L_qq^{-1}.
+//  (B) the rows below: X = A_iq D_q^T on the FP64 tensor cores (DMMA);
+//  (C) the next diagonal block takes its rank-16 update; the rest of the
+//      trailing update and the blocks of T = L^{-1} (block forward
+//      substitution: W_ij = sum_k L_ik T_kj in the T_ij slot, T_ij = -D_i W_ij)
+//      are done by the other warps during the next panel's (A).
 // Non-positive or non-finite pivots set ERRBIT_SINGULAR.
-constexpr int LEAF_THREADS = 512;
-constexpr int LEAF_LD = NB + 1;
+constexpr int LEAF_THREADS = 256;
+constexpr int LEAF_LD = NB + 4;
 constexpr int LEAF_PW = 16;
-constexpr size_t LEAF_SMEM = sizeof(double) * (2 * NB * LEAF_LD + NB);
+constexpr int LEAF_TILE = NB * LEAF_LD;                      // doubles of one 64 x 64 shared tile
+constexpr size_t LEAF_SMEM = sizeof(double) * 2 * LEAF_TILE;  // S, Ts
 
-// lane = column of D_q = L_qq^{-1} (lanes 16..31 idle)
-__device__ __forceinline__ void diag_inverse(const double* S, double* Ts, const double* rinv, int c0, int lane) {
-    double t[LEAF_PW];
+__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
+}
+
+// Barrier `id` (1..15) over `threads` threads of the block.
+__device__ __forceinline__ void named_barrier(int id, int threads) {
+    asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+
+// c = A B over k = 16 for one 8 x 8 fragment of shared tiles (column-major,
+// stride LEAF_LD): A(m, k) = a[k LD + m], B(k, n) = kBT ? b[k LD + n] :
+// b[n LD + k]. Lane (g, t) gets C(g, 2t), C(g, 2t + 1).
+template <bool kBT>
+__device__ __forceinline__ void leaf_mma(const double* a, const double* b, int g, int t, double (&c)[2]) {
+    double u[2] = {0.0, 0.0}, v[2] = {0.0, 0.0};  // two chains of two steps
 #pragma unroll
-    for (int r = 0; r < LEAF_PW; ++r) {
-        double s0 = (r == lane) ? 1.0 : 0.0, s1 = 0.0;
+    for (int h = 0; h < 2; ++h) {
+        const int k = 4 * h + t;
+        dmma(u[0], u[1], a[k * LEAF_LD + g], kBT ? b[k * LEAF_LD + g] : b[g * LEAF_LD + k]);
+        dmma(v[0], v[1], a[(8 + k) * LEAF_LD + g], kBT ? b[(8 + k) * LEAF_LD + g] : b[g * LEAF_LD + 8 + k]);
+    }
+    c[0] = u[0] + v[0];
+    c[1] = u[1] + v[1];
+}
+
+// The 16 x 16 block (r, c) (in units of 16) of a shared tile.
+__device__ __forceinline__ double* leaf_block(double* M, int r, int c) {
+    return M + (c * LEAF_LD + r) * LEAF_PW;
+}
+
+// Fragment (fi, fj) of the block Cb -= Xi Xj^T.
+__device__ __forceinline__ void leaf_update(double* Cb, const double* Xi, const double* Xj, int fi, int fj, int g,
+                                            int t) {
+    double c[2];
+    leaf_mma<true>(Xi + 8 * fi, Xj + 8 * fj, g, t, c);
+    double* z = Cb + (8 * fj + 2 * t) * LEAF_LD + 8 * fi + g;
+    z[0] -= c[0];
+    z[LEAF_LD] -= c[1];
+}
+
+// Rows 8 fi .. 8 fi + 7 of the block X <- X D^T, in place (one warp).
+__device__ __forceinline__ void leaf_solve(double* X, const double* D, int fi, int g, int t) {
+    double c[2][2];
 #pragma unroll
-        for (int k = 0; k < r; ++k) {
-            const double v = S[(c0 + r) * LEAF_LD + c0 + k] * t[k];
-            if (k & 1) s1 -= v; else s0 -= v;
+    for (int fj = 0; fj < 2; ++fj) leaf_mma<true>(X + 8 * fi, D + 8 * fj, g, t, c[fj]);
+    __syncwarp();
+#pragma unroll
+    for (int fj = 0; fj < 2; ++fj) {
+        double* z = X + (8 * fj + 2 * t) * LEAF_LD + 8 * fi + g;
+        z[0] = c[fj][0];
+        z[LEAF_LD] = c[fj][1];
+    }
+}
+
+// Fragment (fi, fj) of the block W (+)= L Tb.
+__device__ __forceinline__ void leaf_gather(double* W, const double* L, const double* Tb, bool first, int fi, int fj,
+                                            int g, int t) {
+    double c[2];
+    leaf_mma<false>(L + 8 * fi, Tb + 8 * fj * LEAF_LD, g, t, c);
+    double* z = W + (8 * fj + 2 * t) * LEAF_LD + 8 * fi + g;
+    z[0] = first ? c[0] : z[0] + c[0];
+    z[LEAF_LD] = first ? c[1] : z[LEAF_LD] + c[1];
+}
+
+// Columns 8 fj .. 8 fj + 7 of the block W <- -D W, in place (one warp).
+__device__ __forceinline__ void leaf_finish(double* W, const double* D, int fj, int g, int t) {
+    double c[2][2];
+#pragma unroll
+    for (int fi = 0; fi < 2; ++fi) leaf_mma<false>(D + 8 * fi, W + 8 * fj * LEAF_LD, g, t, c[fi]);
+    __syncwarp();
+#pragma unroll
+    for (int fi = 0; fi < 2; ++fi) {
+        double* z = W + (8 * fj + 2 * t) * LEAF_LD + 8 * fi + g;
+        z[0] = -c[fi][0];
+        z[LEAF_LD] = -c[fi][1];
+    }
+}
+
+// 1 / sqrt(d) for a normal d > 0: the hardware's approximation (about 2^-22) and one
+// third-order Householder step, y (1 + e/2 + 3 e^2/8) with e = 1 - d y^2. No
+// branch, so that two of them overlap in the panel's dependent chain.
+__device__ __forceinline__ double rsqrt_step(double d) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(d));
+    const double e = fma(-(d * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// (A): one warp; the diagonal block Sb becomes L_qq, Db receives L_qq^{-1}.
+__device__ __forceinline__ void leaf_panel(double* Sb, double* Db, int lane, int* err) {
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr double kTiny = 2.2250738585072014e-308, kHuge = 1.7976931348623157e308;  // normal pivots
+    double a[LEAF_PW];
+#pragma unroll
+    for (int j = 0; j < LEAF_PW; ++j)
+        a[j] = lane < LEAF_PW ? (j <= lane ? Sb[j * LEAF_LD + lane] : 0.0) : (j == lane - LEAF_PW ? 1.0 : 0.0);
+    bool bad = false;
+    double d = __shfl_sync(kAll, a[0], 0), e = __shfl_sync(kAll, a[0], 1), f = __shfl_sync(kAll, a[1], 1);
+#pragma unroll
+    for (int h = 0; h < LEAF_PW / 2; ++h) {
+        const int p = 2 * h;
+        // the next step's entries before this step's update
+        double dn = 0.0, en = 0.0, fn = 0.0;
+        if (p + 2 < LEAF_PW) {
+            dn = __shfl_sync(kAll, a[p + 2], p + 2);
+            en = __shfl_sync(kAll, a[p + 2], p + 3);
+            fn = __shfl_sync(kAll, a[p + 3], p + 3);
         }
-        t[r] = (r >= lane) ? (s0 + s1) * rinv[c0 + r] : 0.0;
+        const double r0 = rsqrt_step(d), det = fma(d, f, -(e * e)), rd = rsqrt_step(det);
+        bad |= !(d >= kTiny && det >= kTiny && d <= kHuge && det <= kHuge);
+        const double r1 = rd * (d * r0);
+        const double x0 = a[p] * r0;
+        const double x1 = fma(-x0, e * r0, a[p + 1]) * r1;
+        a[p] = x0;
+        a[p + 1] = x1;
+#pragma unroll
+        for (int j = p + 2; j < LEAF_PW; ++j) {
+            const double m0 = __shfl_sync(kAll, x0, j), m1 = __shfl_sync(kAll, x1, j);
+            a[j] = fma(-x1, m1, fma(-x0, m0, a[j]));
+            if (j == p + 2) {
+                dn = fma(-m1, m1, fma(-m0, m0, dn));
+                e = m0;  // rows p + 2 of the two columns, for the entry below the next pivot
+                f = m1;
+            }
+            if (j == p + 3) {
+                en = fma(-m1, f, fma(-m0, e, en));
+                fn = fma(-m1, m1, fma(-m0, m0, fn));
+            }
+        }
+        d = dn;
+        e = en;
+        f = fn;
     }
-    if (lane < LEAF_PW) {
+    if (lane == 0 && bad) atomicOr(err, ERRBIT_SINGULAR);
+    double* out = lane < LEAF_PW ? Sb + lane : Db + (lane - LEAF_PW) * LEAF_LD;  // row of L, column of D
+    const int step = lane < LEAF_PW ? LEAF_LD : 1;
 #pragma unroll
-        for (int r = 0; r < LEAF_PW; ++r) Ts[(c0 + r) * LEAF_LD + c0 + lane] = t[r];
-    }
-}
-
-// X = L_{b+1,b} D_b (16 x 16, b0 = 16 b), stored transposed in the upper block: Ts(b0 + j, b0 + 16 + i)
-__device__ __forceinline__ void pair_x(const double* S, double* Ts, int b0, int e) {
-    const int i = e >> 4, j = e & 15;
-    double s = 0.0;
-#pragma unroll
-    for (int k = 0; k < LEAF_PW; ++k) s = fma(S[(b0 + 16 + i) * LEAF_LD + b0 + k], Ts[(b0 + k) * LEAF_LD + b0 + j], s);
-    Ts[(b0 + j) * LEAF_LD + b0 + 16 + i] = s;
-}
-// T_{b+1,b} = -D_{b+1} X
-__device__ __forceinline__ void pair_t(double* Ts, int b0, int e) {
-    const int i = e >> 4, j = e & 15;
-    double s = 0.0;
-#pragma unroll
-    for (int k = 0; k < LEAF_PW; ++k) s = fma(Ts[(b0 + 16 + i) * LEAF_LD + b0 + 16 + k], Ts[(b0 + j) * LEAF_LD + b0 + 16 + k], s);
-    Ts[(b0 + 16 + i) * LEAF_LD + b0 + j] = -s;
+    for (int j = 0; j < LEAF_PW; ++j)
+        if (lane >= LEAF_PW || j <= lane) out[j * step] = a[j];
 }
 
 // Load phase: the kb x kb diagonal block of A at (k0, k0) into S (lower
-// triangle; the upper one zero; identity tail) and Ts cleared. A is read
-// through L2 only (ld.global.cg), so that a persistent caller never sees a
-// stale L1 line of a tile another CTA rewrote. The caller synchronises.
-__device__ __forceinline__ void chol_leaf_load(const double* A, long lda, int k0, int kb, double* lsm) {
-    double* S = lsm;
-    double* Ts = lsm + NB * LEAF_LD;
+// triangle, identity tail). A is read through L2 only (ld.global.cg), so that a
+// persistent caller never sees a stale L1 line of a tile another CTA rewrote.
+// The caller synchronises.
+__device__ __forceinline__ void chol_leaf_load(const double* A, long lda, int k0, int kb, double* S) {
     const int tid = threadIdx.x;
     constexpr int kPer = NB * NB / LEAF_THREADS;
-    double v[kPer];
     const int i = tid & (NB - 1);
+    double v[kPer];
 #pragma unroll
     for (int u = 0; u < kPer; ++u) {
         const int j = (tid >> 6) + u * (LEAF_THREADS / NB);
         v[u] = (i < kb && j < kb) ? (j <= i ? __ldcg(A + (k0 + i) + (long)(k0 + j) * lda) : 0.0) : (i == j ? 1.0 : 0.0);
     }
 #pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-        const int j = (tid >> 6) + u * (LEAF_THREADS / NB);
-        S[i * LEAF_LD + j] = v[u];
-        Ts[i * LEAF_LD + j] = 0.0;
-    }
+    for (int u = 0; u < kPer; ++u) S[((tid >> 6) + u * (LEAF_THREADS / NB)) * LEAF_LD + i] = v[u];
 }
 
 // Factorisation of the block in S (after chol_leaf_load and a barrier), T_kk
-// written to T at (k0, k0). One 512-thread CTA, lsm: LEAF_SMEM bytes.
-__device__ __forceinline__ void chol_leaf_factor(int k0, int kb, double* T, long ldt, int* err, double* lsm) {
-    double* S = lsm;
-    double* Ts = lsm + NB * LEAF_LD;
-    double* rinv = Ts + NB * LEAF_LD;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    for (int q = 0; q < NB / LEAF_PW; ++q) {
-        const int c0 = q * LEAF_PW;
-        if (warp == 0) {  // (A) Cholesky of the diagonal block in registers, lane = row
-            double a[LEAF_PW];
-#pragma unroll
-            for (int j = 0; j < LEAF_PW; ++j) a[j] = (lane < LEAF_PW && j <= lane) ? S[(c0 + lane) * LEAF_LD + c0 + j] : 0.0;
-            bool bad = false;
-#pragma unroll
-            for (int p = 0; p < LEAF_PW; ++p) {
-                const double d = __shfl_sync(0xffffffffu, a[p], p);
-                const double r = rsqrt(d);
-                if (lane == p) rinv[c0 + p] = r;
-                bad |= !(d > 0.0 && d <= 1.7976931348623157e308);
-                a[p] = (lane == p) ? d * r : a[p] * r;
-                const double lp = a[p];
-#pragma unroll
-                for (int j = p + 1; j < LEAF_PW; ++j) {
-                    const double ljp = __shfl_sync(0xffffffffu, lp, j);
-                    a[j] = fma(-lp, ljp, a[j]);
-                }
+// in Ts (lower 16 x 16 blocks, the diagonal ones with zeros above the diagonal)
+// and written to T at (k0, k0). One CTA of LEAF_THREADS threads. Warp 4 calls
+// beside(q) during panel q: the caller's own work (no block barrier in it).
+template <class F>
+__device__ __forceinline__ void chol_leaf_factor(int k0, int kb, double* T, long ldt, int* err, double* S, double* Ts,
+                                                 F&& beside) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    // the warps beside (A): 1, 2, 3, 5, 6, 7 (warp 4 shares warp 0's scheduler and FP64 pipe)
+    const int worker = warp < 4 ? warp - 1 : warp - 2;
+    constexpr int kWorkers = 6, kSideThreads = LEAF_THREADS - 32;
+    auto S_ = [S](int r, int c) { return leaf_block(S, r, c); };
+    auto T_ = [Ts](int r, int c) { return leaf_block(Ts, r, c); };
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q) {
+        if (warp == 0) {
+            leaf_panel(S_(q, q), T_(q, q), lane, err);
+        } else if (warp == 4) {
+            beside(q);
+            if (q > 0) named_barrier(1, kSideThreads);
+        } else if (q > 0) {
+            // beside panel q: the updates of panel p = q - 1 that panel q does not need
+            const int p = q - 1;
+            {
+                int item = 0;
+                // T_pj = -D_p W_pj, then (after the barrier) W_ij += L_ip T_pj
+                for (int j = 0; j < p; ++j)
+                    for (int fj = 0; fj < 2; ++fj)
+                        if (item++ % kWorkers == worker) leaf_finish(T_(p, j), T_(p, p), fj, g, t);
+                for (int i = q; i < 4; ++i)
+                    for (int j = q; j <= i; ++j) {
+                        if (i == q) continue;  // the diagonal block (q, q) was updated before the panel
+                        for (int f = 0; f < 4; ++f)
+                            if (item++ % kWorkers == worker)
+                                leaf_update(S_(i, j), S_(i, p), S_(j, p), f & 1, f >> 1, g, t);
+                    }
+                for (int i = q; i < 4; ++i)
+                    for (int f = 0; f < 4; ++f)
+                        if (item++ % kWorkers == worker)
+                            leaf_gather(T_(i, p), S_(i, p), T_(p, p), true, f & 1, f >> 1, g, t);
             }
-            if (lane == 0 && bad) atomicOr(err, ERRBIT_SINGULAR);
-            if (lane < LEAF_PW) {
-#pragma unroll
-                for (int j = 0; j < LEAF_PW; ++j)
-                    if (j <= lane) S[(c0 + lane) * LEAF_LD + c0 + j] = a[j];
-            }
-        } else if (q == NB / LEAF_PW - 1 && warp < NB / LEAF_PW) {
-            diag_inverse(S, Ts, rinv, (warp - 1) * LEAF_PW, lane);  // D_0 .. D_2 beside the last factorisation
-        }
-        __syncthreads();
-        const int r0 = c0 + LEAF_PW, m = NB - r0;
-        if (m == 0) break;
-        // (B) rows below: forward substitution x L_qq^T = A_iq, one thread per row
-        if (tid < m) {
-            double* row = S + (r0 + tid) * LEAF_LD + c0;
-            double x[LEAF_PW];
-#pragma unroll
-            for (int j = 0; j < LEAF_PW; ++j) {
-                double s = row[j];
-#pragma unroll
-                for (int k = 0; k < j; ++k) s = fma(-x[k], S[(c0 + j) * LEAF_LD + c0 + k], s);
-                x[j] = s * rinv[c0 + j];
-            }
-#pragma unroll
-            for (int j = 0; j < LEAF_PW; ++j) row[j] = x[j];
-        }
-        __syncthreads();
-        // (C) trailing update, lower 2 x 2 tiles: S(i, j) -= sum_k L(i, c0 + k) L(j, c0 + k)
-        {
-            const int mt = m / 2, ntile = mt * (mt + 1) / 2;
-            if (tid < ntile) {
-                int ti = (int)((sqrtf(8.0f * tid + 1.0f) - 1.0f) * 0.5f);
-                while (ti * (ti + 1) / 2 > tid) --ti;
-                while ((ti + 1) * (ti + 2) / 2 <= tid) ++ti;
-                const int tj = tid - ti * (ti + 1) / 2;
-                const int i0 = r0 + 2 * ti, j0 = r0 + 2 * tj;
-                const double* a0 = S + i0 * LEAF_LD + c0;
-                const double* a1 = a0 + LEAF_LD;
-                const double* b0 = S + j0 * LEAF_LD + c0;
-                const double* b1 = b0 + LEAF_LD;
-                double c00 = 0.0, c01 = 0.0, c10 = 0.0, c11 = 0.0;
-#pragma unroll
-                for (int k = 0; k < LEAF_PW; ++k) {
-                    const double x0 = a0[k], x1 = a1[k], y0 = b0[k], y1 = b1[k];
-                    c00 = fma(x0, y0, c00);
-                    c01 = fma(x0, y1, c01);
-                    c10 = fma(x1, y0, c10);
-                    c11 = fma(x1, y1, c11);
-                }
-                double* z = S + i0 * LEAF_LD + j0;
-                z[0] -= c00;
-                z[1] -= c01;
-                z[LEAF_LD] -= c10;
-                z[LEAF_LD + 1] -= c11;
+            named_barrier(1, kSideThreads);
+            {
+                int item = 0;
+                for (int i = q; i < 4; ++i)
+                    for (int j = 0; j < p; ++j)
+                        for (int f = 0; f < 4; ++f)
+                            if (item++ % kWorkers == worker)
+                                leaf_gather(T_(i, j), S_(i, p), T_(p, j), false, f & 1, f >> 1, g, t);
             }
         }
         __syncthreads();
+        if (q == 3) break;
+        // (B): 8-row strips of the blocks below, the next block row first
+        for (int s = warp; s < 2 * (3 - q); s += LEAF_THREADS / 32) leaf_solve(S_(q + 1 + s / 2, q), T_(q, q), s & 1, g, t);
+        __syncthreads();
+        // (C), the next diagonal block's lower fragments
+        if (warp < 3) leaf_update(S_(q + 1, q + 1), S_(q + 1, q), S_(q + 1, q), warp > 0, warp > 1, g, t);
+        __syncthreads();
     }
-    // T = L^{-1} from the four D_q: 16-level pairs, then the 32-level block. Intermediate
-    // products sit transposed in the (unused) upper blocks of Ts.
-    if (warp == 0)
-        diag_inverse(S, Ts, rinv, 48, lane);
-    else if (warp < 9)
-        pair_x(S, Ts, 0, tid - 32);
+    for (int s = warp; s < 6; s += LEAF_THREADS / 32) leaf_finish(T_(3, s >> 1), T_(3, 3), s & 1, g, t);
     __syncthreads();
-    if (tid < 256)
-        pair_t(Ts, 0, tid);
-    else
-        pair_x(S, Ts, 32, tid - 256);
-    __syncthreads();
-    if (tid < 256) pair_t(Ts, 32, tid);
-    {  // X = L21 T0 (32 x 32), stored transposed: Ts(j, 32 + i)
-        const int j = tid & 31, i0 = 2 * (tid >> 5);
-        double s0 = 0.0, s1 = 0.0;
-#pragma unroll 8
-        for (int k = 0; k < 32; ++k) {
-            const double t = k >= j ? Ts[k * LEAF_LD + j] : 0.0;  // the upper block holds X of the first pair
-            s0 = fma(S[(32 + i0) * LEAF_LD + k], t, s0);
-            s1 = fma(S[(33 + i0) * LEAF_LD + k], t, s1);
-        }
-        Ts[j * LEAF_LD + 32 + i0] = s0;
-        Ts[j * LEAF_LD + 33 + i0] = s1;
-    }
-    __syncthreads();
-    {  // T21 = -T1 X
-        const int j = tid & 31, i0 = 2 * (tid >> 5);
-        double s0 = 0.0, s1 = 0.0;
-#pragma unroll 4
-        for (int k = 0; k < i0 + 2; ++k) {
-            const double x = Ts[j * LEAF_LD + 32 + k];
-            s0 = fma(Ts[(32 + i0) * LEAF_LD + 32 + k], x, s0);
-            s1 = fma(Ts[(33 + i0) * LEAF_LD + 32 + k], x, s1);
-        }
-        Ts[(32 + i0) * LEAF_LD + j] = -s0;
-        Ts[(33 + i0) * LEAF_LD + j] = -s1;
-    }
-    __syncthreads();
-    {
-        const int i = tid & (NB - 1);
+    const int i = tid & (NB - 1);
 #pragma unroll
-        for (int u = 0; u < NB * NB / LEAF_THREADS; ++u) {
-            const int j = (tid >> 6) + u * (LEAF_THREADS / NB);
-            if (i < kb && j < kb) T[(k0 + i) + (long)(k0 + j) * ldt] = i >= j ? Ts[i * LEAF_LD + j] : 0.0;
-        }
+    for (int u = 0; u < NB * NB / LEAF_THREADS; ++u) {
+        const int j = (tid >> 6) + u * (LEAF_THREADS / NB);
+        if (i < kb && j < kb) T[(k0 + i) + (long)(k0 + j) * ldt] = i >= j ? Ts[j * LEAF_LD + i] : 0.0;
     }
 }
 
-// The whole leaf: load, barrier, factorisation.
+// The whole leaf: load, barrier, factorisation (lsm: LEAF_SMEM bytes).
 __device__ __forceinline__ void chol_leaf_tile(const double* A, long lda, int k0, int kb, double* T, long ldt,
                                                int* err, double* lsm) {
     chol_leaf_load(A, lda, k0, kb, lsm);
     __syncthreads();
-    chol_leaf_factor(k0, kb, T, ldt, err, lsm);
+    chol_leaf_factor(k0, kb, T, ldt, err, lsm, lsm + LEAF_TILE, [](int) {});
 }
 
 }  // namespace unc

@@ -16,14 +16,23 @@
 // topological order that puts each diagonal factorisation right after the
 // tasks it waits for (look-ahead).
 // CTAs claim tasks from a global cursor in list order, wait (thread 0, with an
-// iteration limit) on per-tile counters, run the task with all 512 threads
+// iteration limit) on per-tile counters, run the task with all 256 threads
 // and publish its counter. Every dependency of a claimed task was claimed
 // earlier by a running CTA that waits only on still earlier tasks, so the
 // schedule completes with any number of resident CTAs; updates of one tile
 // are applied in a fixed order, so the result is bitwise repeatable. Tile data
-// written by other CTAs is read through L2 only (ld.global.cg).
+// written by other CTAs is read through L2 only (ld.global.cg, cp.async.cg).
+// One matrix alone: the CTA that claims POTRF(0) runs every POTRF(k) itself, one
+// after the other (run_chain), and the other CTAs pass over those entries. The
+// chain bounds the whole inverse at these sizes; kept in one CTA, L(k+1,k) is
+// in shared memory when POTRF(k+1) needs it and the next tiles are fetched
+// beside the leaf, and the SM's second CTA leaves it the FP64 pipe (it retires
+// once a CTA elsewhere takes tasks). The other CTAs' tasks still depend only on
+// earlier entries and on the chain, so one resident CTA beside the chain's is
+// enough to complete.
 //
-// Counters (ints, zeroed before the launch): cursor, abort flag, then per
+// Counters (ints, zeroed before the launch): cursor, abort flag, 1 + the SM of the
+// chain, CTAs on other SMs, then per
 // lower tile: ver (updates applied to A), lrdy (L final / T(k,k) ready),
 // tacc (W accumulations), trdy (T final), pacc (O accumulations).
 #include <algorithm>
@@ -40,9 +49,12 @@ namespace {
 
 constexpr int TB = NB;                   // tile size (the leaf size)
 constexpr int DAG_THREADS = LEAF_THREADS;
-constexpr int TLD = TB + 4;              // shared tile stride: fragment reads conflict-free in both orientations
-constexpr size_t TILE_SMEM = sizeof(double) * 2 * TB * TLD;
-constexpr size_t DAG_SMEM = TILE_SMEM + LEAF_SMEM;  // two operand tiles, then the leaf's block
+constexpr int TLD = LEAF_LD;             // shared tile stride: fragment reads conflict-free in both orientations
+// Two CTAs of 256 threads per SM, so that one loads its tiles, waits or stores
+// while the other computes: two operand tiles and the leaf's block (whose
+// inverse takes the second operand tile) are 104 KB.
+constexpr int DAG_CTAS = 2;
+constexpr size_t DAG_SMEM = sizeof(double) * 3 * LEAF_TILE;
 constexpr long kDagSpin = 1L << 22;      // polls of one dependency before the kernel gives up
 constexpr int kMaxTilesN = 56;           // tasks are used up to n = 56 * 64
 
@@ -67,36 +79,36 @@ __device__ bool wait_ge(const int* flag, int v, const int* abort, long spin) {
     return false;
 }
 
-__device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
-
 // Tile X (column-major, leading dimension ld; rows < vr and columns < vc
-// valid, the rest read as zero) into shared memory as sm[c * TLD + r].
-__device__ __forceinline__ void load_tile(double* sm, const double* X, long ld, int vr, int vc, int tid) {
-#pragma unroll
-    for (int u = 0; u < TB * TB / 2 / DAG_THREADS; ++u) {
-        const int q = tid + u * DAG_THREADS;
+// valid, the rest zero) into shared memory as sm[c * TLD + r], asynchronously
+// and past L1, by `threads` threads; tile_wait() before the barrier that
+// publishes it.
+__device__ __forceinline__ void load_tile(double* sm, const double* X, long ld, int vr, int vc, int tid,
+                                          int threads = DAG_THREADS) {
+    for (int q = tid; q < TB * TB / 2; q += threads) {
         const int c = q >> 5, r2 = (q & 31) * 2;
-        double2 v = make_double2(0.0, 0.0);
-        if (c < vc && r2 < vr) v = __ldcg(reinterpret_cast<const double2*>(X + r2 + (long)c * ld));
-        if (r2 + 1 >= vr) v.y = 0.0;
-        *reinterpret_cast<double2*>(sm + c * TLD + r2) = v;
+        const int left = c < vc ? vr - r2 : 0;
+        const int bytes = left >= 2 ? 16 : (left == 1 ? 8 : 0);
+        const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(sm + c * TLD + r2));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst),
+                     "l"(bytes ? X + r2 + (long)c * ld : X), "r"(bytes)
+                     : "memory");
     }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
+__device__ __forceinline__ void tile_wait() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// acc += op(A) op(B) over k in [kb, ke) (multiples of 4) for this warp's 16 x 16
+// acc += op(A) op(B) over k in [kb, ke) (multiples of 4) for this warp's 32 x 16
 // block (rows wm.., columns wn..). op(A)(m, k) = kTA ? A(k, m) : A(m, k),
 // op(B)(k, n) = kTB ? B(n, k) : B(k, n), tiles as left by load_tile.
+using Acc = double[4][2][2];
 template <bool kTA, bool kTB>
 __device__ __forceinline__ void tile_mma(const double* As, const double* Bs, int wm, int wn, int g, int t, int kb,
-                                         int ke, double (&acc)[2][2][2]) {
+                                         int ke, Acc& acc) {
     for (int kk = kb; kk < ke; kk += 4) {
-        double a[2], b[2];
+        double a[4], b[2];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < 4; ++i) {
             const int m = wm + 8 * i + g, k = kk + t;
             a[i] = kTA ? As[m * TLD + k] : As[k * TLD + m];
         }
@@ -106,184 +118,255 @@ __device__ __forceinline__ void tile_mma(const double* As, const double* Bs, int
             b[j] = kTB ? Bs[k * TLD + n] : Bs[n * TLD + k];
         }
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int j = 0; j < 2; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
     }
 }
 
-// X(r, c) = alpha acc + (accumulate ? X(r, c) : 0) for r < vr, c < vc; with
-// Xm, also Xm(c, r) = the same value (the transposed tile).
-__device__ __forceinline__ void store_tile(double* X, long ld, int vr, int vc, const double (&acc)[2][2][2],
-                                           double alpha, bool accumulate, double* Xm, int wm, int wn, int g,
-                                           int t) {
+// f(row, column, element of x) over this thread's elements of the warp's block
+// that lie in the vr x vc valid part of the tile.
+template <class F>
+__device__ __forceinline__ void tile_elements(int vr, int vc, int wm, int wn, int g, int t, Acc& x, F&& f) {
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int r = wm + 8 * i + g, c = wn + 8 * j + 2 * t + h;
-                if (r < vr && c < vc) {
-                    double v = alpha * acc[i][j][h];
-                    if (accumulate) v += __ldcg(X + r + (long)c * ld);
-                    X[r + (long)c * ld] = v;
-                    if (Xm) Xm[c + (long)r * ld] = v;
-                }
+                if (r < vr && c < vc) f(r, c, x[i][j][h]);
             }
 }
 
-// One tile task (type, i, j, k) of the n x n matrix whose tiles A, T, O and
-// counters (`state`, laid out as described at the top) are given, run by all
-// DAG_THREADS threads of the block; thread 0 waits for its dependencies first.
-// Returns false when a wait gave up (ERRBIT_TIMEOUT and the abort flag are
-// set): the caller stops taking tasks.
-__device__ __forceinline__ bool run_task(double* A, double* T, double* O, int n, long ld, int* state, int ntri,
-                                         int* err, int* abort, long spin, int type, int i, int j, int k, double* sm,
-                                         int& s_ok) {
-    int* const ver = state + 4;
-    int* const lrdy = ver + ntri;
-    int* const tacc = lrdy + ntri;
-    int* const trdy = tacc + ntri;
-    int* const pacc = trdy + ntri;
+// prev = X where valid: issued before the products, so that its latency is
+// covered by the operand loads and the products.
+__device__ __forceinline__ void load_prev(const double* X, long ld, int vr, int vc, int wm, int wn, int g, int t,
+                                          Acc& prev) {
+    tile_elements(vr, vc, wm, wn, g, t, prev, [&](int r, int c, double& v) { v = __ldcg(X + r + (long)c * ld); });
+}
+
+// X(r, c) = alpha acc + prev for r < vr, c < vc; with Xm, also Xm(c, r) = the
+// same value (the transposed tile).
+__device__ __forceinline__ void store_tile(double* X, long ld, int vr, int vc, Acc& acc, double alpha, const Acc& prev,
+                                           double* Xm, int wm, int wn, int g, int t) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) acc[i][j][h] = fma(alpha, acc[i][j][h], prev[i][j][h]);
+    tile_elements(vr, vc, wm, wn, g, t, acc, [&](int r, int c, double& v) {
+        X[r + (long)c * ld] = v;
+        if (Xm) Xm[c + (long)r * ld] = v;
+    });
+}
+
+// The n x n matrix of a task: tiles of A, T, O and the counters (laid out as
+// described at the top).
+struct TaskMatrix {
+    double *A, *T, *O;
+    int n;
+    long ld;
+    int *ver, *lrdy, *tacc, *trdy, *pacc;
+    int* err;
+    int* abort;
+    long spin;
+
+    __device__ __forceinline__ TaskMatrix(double* A_, double* T_, double* O_, int n_, long ld_, int* state, int ntri,
+                                          int* err_, int* abort_, long spin_)
+        : A(A_), T(T_), O(O_), n(n_), ld(ld_), ver(state + 4), lrdy(ver + ntri), tacc(lrdy + ntri), trdy(tacc + ntri),
+          pacc(trdy + ntri), err(err_), abort(abort_), spin(spin_) {}
+    __device__ __forceinline__ int ext(int b) const { return min(TB, n - TB * b); }
+    __device__ __forceinline__ int kext(int b) const { return (ext(b) + 3) & ~3; }  // K extent of a partial tile, DMMA steps
+    __device__ __forceinline__ int tiles() const { return (n + TB - 1) / TB; }
+    __device__ __forceinline__ double* tile(double* M, int i, int j) const { return M + (long)TB * i + (long)TB * j * ld; }
+    // thread 0 only
+    __device__ __forceinline__ bool wait(const int* flag, int v) const { return wait_ge(flag, v, abort, spin); }
+    __device__ __forceinline__ bool give_up() const {
+        atomicOr(err, ERRBIT_TIMEOUT);
+        atomicExch(abort, 1);
+        return false;
+    }
+};
+
+// POTRF(k): A(k,k) -= L(k,k-1) L(k,k-1)^T, the leaf, T(k,k) published, then
+// L(k+1,k) = A(k+1,k) T(k,k)^T with T(k,k) still in shared memory (Bs), published.
+// A(k+1,k) is fetched beside the leaf once its updates are in. chained: called
+// in order by one CTA: L(k,k-1) is left in As by the call before, which also
+// fetched A(k,k) into S when diag_in. Otherwise the caller has waited for both.
+// flag: three shared ints. False when a wait gave up.
+__device__ bool potrf(const TaskMatrix& m, int k, bool chained, bool& diag_in, double* sm, int* flag) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    const int wm = (warp & 1) * 32, wn = (warp >> 1) * 16;
+    double *As = sm, *Bs = sm + LEAF_TILE, *S = sm + 2 * LEAF_TILE;
+    const bool below = k + 1 < m.tiles();
+    if (chained && k > 0 && !diag_in) {
+        if (tid == 0) flag[0] = m.wait(m.ver + tri(k, k), k - 1) || m.give_up();
+        __syncthreads();
+        if (!flag[0]) return false;
+    }
+    if (!diag_in) chol_leaf_load(m.A, m.ld, TB * k, m.ext(k), S);
+    if (k > 0 && !chained) load_tile(As, m.tile(m.A, k, k - 1), m.ld, m.ext(k), m.ext(k - 1), tid);
+    tile_wait();
+    __syncthreads();
+    Acc acc = {};
+    if (k > 0) {
+        if (wn < wm + 32) tile_mma<false, true>(As, As, wm, wn, g, t4, 0, TB, acc);  // lower blocks only
+        tile_elements(TB, TB, wm, wn, g, t4, acc, [&](int r, int c, double& v) {
+            if (c <= r) S[c * TLD + r] -= v;
+        });
+    }
+    if (tid == 0) flag[0] = 0;
+    __syncthreads();
+    bool fetched = false;  // warp 4: A(k+1,k) is on its way into As
+    chol_leaf_factor(TB * k, m.ext(k), m.T, m.ld, m.err, S, Bs, [&](int q) {
+        if (!below || fetched || q == 0) return;
+        int ready = 0;
+        if (lane == 0) ready = ld_acquire(m.ver + tri(k + 1, k)) >= k;
+        fetched = __shfl_sync(0xffffffffu, ready, 0) != 0;
+        if (!fetched) return;
+        load_tile(As, m.tile(m.A, k + 1, k), m.ld, m.ext(k + 1), m.ext(k), lane, 32);
+        if (lane == 0) flag[0] = 1;
+    });
+    tile_wait();
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        atomicExch(m.lrdy + tri(k, k), 1);
+        atomicExch(m.trdy + tri(k, k), 1);
+    }
+    if (!below) return true;
+    if (!flag[0]) {
+        if (tid == 0) flag[1] = m.wait(m.ver + tri(k + 1, k), k) || m.give_up();
+        __syncthreads();
+        if (!flag[1]) return false;
+        load_tile(As, m.tile(m.A, k + 1, k), m.ld, m.ext(k + 1), m.ext(k), tid);
+        tile_wait();
+    }
+    // the next diagonal tile, when its updates but the last are in (a partial
+    // one takes its identity tail from chol_leaf_load)
+    if (tid == 32) flag[2] = chained && m.ext(k + 1) == TB && ld_acquire(m.ver + tri(k + 1, k + 1)) >= k;
+    __syncthreads();
+    diag_in = flag[2];
+    if (diag_in) load_tile(S, m.tile(m.A, k + 1, k + 1), m.ld, TB, TB, tid);
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+    tile_mma<false, true>(As, Bs, wm, wn, g, t4, 0, wn + 16, acc);
+    if (chained) {
+        __syncthreads();  // As is read no more
+        tile_elements(TB, TB, wm, wn, g, t4, acc, [&](int r, int c, double& v) { As[c * TLD + r] = v; });
+    }
+    double* L = m.tile(m.A, k + 1, k);
+    tile_elements(m.ext(k + 1), m.ext(k), wm, wn, g, t4, acc, [&](int r, int c, double& v) { L[r + (long)c * m.ld] = v; });
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        atomicExch(m.lrdy + tri(k + 1, k), 1);
+    }
+    return true;
+}
+
+// Every POTRF(k) of one matrix, in order, by the calling CTA.
+__device__ bool run_chain(const TaskMatrix& m, double* sm, int* flag) {
+    bool diag_in = false;
+    for (int k = 0; k < m.tiles(); ++k)
+        if (!potrf(m, k, true, diag_in, sm, flag)) return false;
+    return true;
+}
+
+// One tile task (type, i, j, k), run by all DAG_THREADS threads of the block;
+// thread 0 waits for its dependencies first. Returns false when a wait gave up
+// (ERRBIT_TIMEOUT and the abort flag are set): the caller stops taking tasks.
+__device__ __forceinline__ bool run_task(const TaskMatrix& m, int type, int i, int j, int k, double* sm, int* flag) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t4 = lane & 3;
-    const int wm = (warp & 3) * 16, wn = (warp >> 2) * 16;
+    const int wm = (warp & 1) * 32, wn = (warp >> 1) * 16;
     double* As = sm;
-    double* Bs = sm + TB * TLD;
-    auto ext = [n](int b) { return min(TB, n - TB * b); };
-    auto kext = [n](int b) { return (min(TB, n - TB * b) + 3) & ~3; };  // K extent of a partial tile, DMMA steps
-    auto tile = [ld](double* M, int i, int j) { return M + (long)TB * i + (long)TB * j * ld; };
+    double* Bs = sm + LEAF_TILE;
+    const long ld = m.ld;
     if (tid == 0) {
         bool ok = true;
         switch (type) {
             case K_POTRF:  // its last update (from panel k-1) is applied inside the task
-                ok = k == 0 || (wait_ge(ver + tri(k, k), k - 1, abort, spin) &&
-                                wait_ge(lrdy + tri(k, k - 1), 1, abort, spin));
+                ok = k == 0 || (m.wait(m.ver + tri(k, k), k - 1) && m.wait(m.lrdy + tri(k, k - 1), 1));
                 break;
             case K_TRSM:
-                ok = wait_ge(ver + tri(i, k), k, abort, spin) && wait_ge(lrdy + tri(k, k), 1, abort, spin);
+                ok = m.wait(m.ver + tri(i, k), k) && m.wait(m.lrdy + tri(k, k), 1);
                 break;
             case K_UPDATE:
-                ok = wait_ge(ver + tri(i, j), k, abort, spin) && wait_ge(lrdy + tri(i, k), 1, abort, spin) &&
-                     wait_ge(lrdy + tri(j, k), 1, abort, spin);
+                ok = m.wait(m.ver + tri(i, j), k) && m.wait(m.lrdy + tri(i, k), 1) && m.wait(m.lrdy + tri(j, k), 1);
                 break;
             case K_TACC:
-                ok = wait_ge(tacc + tri(i, j), k - j, abort, spin) && wait_ge(lrdy + tri(i, k), 1, abort, spin) &&
-                     wait_ge(trdy + tri(k, j), 1, abort, spin);
+                ok = m.wait(m.tacc + tri(i, j), k - j) && m.wait(m.lrdy + tri(i, k), 1) && m.wait(m.trdy + tri(k, j), 1);
                 break;
             case K_TFIN:
-                ok = wait_ge(tacc + tri(i, j), i - j, abort, spin) && wait_ge(trdy + tri(i, i), 1, abort, spin);
+                ok = m.wait(m.tacc + tri(i, j), i - j) && m.wait(m.trdy + tri(i, i), 1);
                 break;
             default:  // K_PACC
-                ok = wait_ge(pacc + tri(i, j), k - i, abort, spin) && wait_ge(trdy + tri(k, i), 1, abort, spin) &&
-                     wait_ge(trdy + tri(k, j), 1, abort, spin);
+                ok = m.wait(m.pacc + tri(i, j), k - i) && m.wait(m.trdy + tri(k, i), 1) && m.wait(m.trdy + tri(k, j), 1);
                 break;
         }
-        if (!ok) {
-            atomicOr(err, ERRBIT_TIMEOUT);
-            atomicExch(abort, 1);
-        }
-        s_ok = ok;
+        flag[0] = ok || m.give_up();
     }
     __syncthreads();
-    if (!s_ok) return false;
+    if (!flag[0]) return false;
     if (type == K_POTRF) {
-        // A(k,k) -= L(k,k-1) L(k,k-1)^T applied to the leaf's block (both tiles loaded
-        // together), the leaf, T(k,k) published, then L(k+1,k) = A(k+1,k) T(k,k)^T with
-        // T(k,k) still in shared memory
-        double* lsm = sm + 2 * TB * TLD;
-        chol_leaf_load(A, ld, TB * k, ext(k), lsm);
-        if (k > 0) {
-            double acc[2][2][2] = {};
-            load_tile(As, tile(A, k, k - 1), ld, ext(k), ext(k - 1), tid);
+        bool diag_in = false;
+        return potrf(m, k, false, diag_in, sm, flag);
+    }
+    Acc acc = {}, prev = {};
+    switch (type) {
+        case K_TRSM:  // L(i,k) = A(i,k) T(k,k)^T; T(k,k) lower: terms k' <= n only
+            load_tile(As, m.tile(m.A, i, k), ld, m.ext(i), m.ext(k), tid);
+            load_tile(Bs, m.tile(m.T, k, k), ld, m.ext(k), m.ext(k), tid);
+            tile_wait();
             __syncthreads();
-            if (wn <= wm) tile_mma<false, true>(As, As, wm, wn, g, t4, 0, TB, acc);  // lower blocks only
-#pragma unroll
-            for (int a = 0; a < 2; ++a)
-#pragma unroll
-                for (int b = 0; b < 2; ++b)
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int r = wm + 8 * a + g, c = wn + 8 * b + 2 * t4 + h;
-                        if (c <= r) lsm[r * LEAF_LD + c] -= acc[a][b][h];
-                    }
-        }
-        __syncthreads();
-        chol_leaf_factor(TB * k, ext(k), T, ld, err, lsm);
-        __syncthreads();
-        if (tid == 0) {
-            __threadfence();
-            atomicExch(lrdy + tri(k, k), 1);
-            atomicExch(trdy + tri(k, k), 1);
-        }
-        if (k + 1 >= (n + TB - 1) / TB) return true;
-        if (tid == 0) {
-            const bool ok = wait_ge(ver + tri(k + 1, k), k, abort, spin);
-            if (!ok) {
-                atomicOr(err, ERRBIT_TIMEOUT);
-                atomicExch(abort, 1);
-            }
-            s_ok = ok;
-        }
-        const double* Tl = lsm + NB * LEAF_LD;  // T(r, c) at Tl[r * LEAF_LD + c], lower triangle valid
-        for (int e = tid; e < TB * TB; e += DAG_THREADS) {
-            const int r = e & (TB - 1), c = e >> 6;
-            Bs[c * TLD + r] = r >= c ? Tl[r * LEAF_LD + c] : 0.0;
-        }
-        __syncthreads();
-        if (!s_ok) return false;
-        load_tile(As, tile(A, k + 1, k), ld, ext(k + 1), ext(k), tid);
-        __syncthreads();
-        double acc[2][2][2] = {};
-        tile_mma<false, true>(As, Bs, wm, wn, g, t4, 0, wn + 16, acc);
-        store_tile(tile(A, k + 1, k), ld, ext(k + 1), ext(k), acc, 1.0, false, nullptr, wm, wn, g, t4);
-    } else {
-        double acc[2][2][2] = {};
-        switch (type) {
-            case K_TRSM:  // L(i,k) = A(i,k) T(k,k)^T; T(k,k) lower: terms k' <= n only
-                load_tile(As, tile(A, i, k), ld, ext(i), ext(k), tid);
-                load_tile(Bs, tile(T, k, k), ld, ext(k), ext(k), tid);
-                __syncthreads();
-                tile_mma<false, true>(As, Bs, wm, wn, g, t4, 0, min(wn + 16, kext(k)), acc);
-                __syncthreads();
-                store_tile(tile(A, i, k), ld, ext(i), ext(k), acc, 1.0, false, nullptr, wm, wn, g, t4);
-                break;
-            case K_UPDATE:  // A(i,j) -= L(i,k) L(j,k)^T
-                load_tile(As, tile(A, i, k), ld, ext(i), ext(k), tid);
-                load_tile(Bs, tile(A, j, k), ld, ext(j), ext(k), tid);
-                __syncthreads();
-                tile_mma<false, true>(As, Bs, wm, wn, g, t4, 0, kext(k), acc);
-                store_tile(tile(A, i, j), ld, ext(i), ext(j), acc, -1.0, true, nullptr, wm, wn, g, t4);
-                break;
-            case K_TACC:  // W(i,j) += L(i,k) T(k,j); T(j,j) lower: terms k' >= n only
-                load_tile(As, tile(A, i, k), ld, ext(i), ext(k), tid);
-                load_tile(Bs, tile(T, k, j), ld, ext(k), ext(j), tid);
-                __syncthreads();
-                tile_mma<false, false>(As, Bs, wm, wn, g, t4, k == j ? wn : 0, kext(k), acc);
-                store_tile(tile(T, i, j), ld, ext(i), ext(j), acc, 1.0, k > j, nullptr, wm, wn, g, t4);
-                break;
-            case K_TFIN:  // T(i,j) = -T(i,i) W(i,j); T(i,i) lower: terms k' <= m only
-                load_tile(As, tile(T, i, i), ld, ext(i), ext(i), tid);
-                load_tile(Bs, tile(T, i, j), ld, ext(i), ext(j), tid);
-                __syncthreads();
-                tile_mma<false, false>(As, Bs, wm, wn, g, t4, 0, min(wm + 16, kext(i)), acc);
-                __syncthreads();
-                store_tile(tile(T, i, j), ld, ext(i), ext(j), acc, -1.0, false, nullptr, wm, wn, g, t4);
-                break;
-            default: {  // K_PACC: O(i,j) += T(k,i)^T T(k,j); diagonal T tiles lower
-                load_tile(As, tile(T, k, i), ld, ext(k), ext(i), tid);
-                load_tile(Bs, tile(T, k, j), ld, ext(k), ext(j), tid);
-                __syncthreads();
-                int kb = 0;
-                if (k == i) kb = wm;
-                if (k == j) kb = max(kb, wn);
-                tile_mma<true, false>(As, Bs, wm, wn, g, t4, kb, kext(k), acc);
-                const bool last = k == (n + TB - 1) / TB - 1;
-                store_tile(tile(O, i, j), ld, ext(i), ext(j), acc, 1.0, k > i,
-                           (last && i > j) ? tile(O, j, i) : nullptr, wm, wn, g, t4);
-                break;
-            }
+            tile_mma<false, true>(As, Bs, wm, wn, g, t4, 0, min(wn + 16, m.kext(k)), acc);
+            store_tile(m.tile(m.A, i, k), ld, m.ext(i), m.ext(k), acc, 1.0, prev, nullptr, wm, wn, g, t4);
+            break;
+        case K_UPDATE:  // A(i,j) -= L(i,k) L(j,k)^T
+            load_tile(As, m.tile(m.A, i, k), ld, m.ext(i), m.ext(k), tid);
+            load_tile(Bs, m.tile(m.A, j, k), ld, m.ext(j), m.ext(k), tid);
+            load_prev(m.tile(m.A, i, j), ld, m.ext(i), m.ext(j), wm, wn, g, t4, prev);
+            tile_wait();
+            __syncthreads();
+            tile_mma<false, true>(As, Bs, wm, wn, g, t4, 0, m.kext(k), acc);
+            store_tile(m.tile(m.A, i, j), ld, m.ext(i), m.ext(j), acc, -1.0, prev, nullptr, wm, wn, g, t4);
+            break;
+        case K_TACC:  // W(i,j) += L(i,k) T(k,j); T(j,j) lower: terms k' >= n only
+            load_tile(As, m.tile(m.A, i, k), ld, m.ext(i), m.ext(k), tid);
+            load_tile(Bs, m.tile(m.T, k, j), ld, m.ext(k), m.ext(j), tid);
+            if (k > j) load_prev(m.tile(m.T, i, j), ld, m.ext(i), m.ext(j), wm, wn, g, t4, prev);
+            tile_wait();
+            __syncthreads();
+            tile_mma<false, false>(As, Bs, wm, wn, g, t4, k == j ? wn : 0, m.kext(k), acc);
+            store_tile(m.tile(m.T, i, j), ld, m.ext(i), m.ext(j), acc, 1.0, prev, nullptr, wm, wn, g, t4);
+            break;
+        case K_TFIN:  // T(i,j) = -T(i,i) W(i,j); T(i,i) lower: terms k' <= m only
+            load_tile(As, m.tile(m.T, i, i), ld, m.ext(i), m.ext(i), tid);
+            load_tile(Bs, m.tile(m.T, i, j), ld, m.ext(i), m.ext(j), tid);
+            tile_wait();
+            __syncthreads();
+            tile_mma<false, false>(As, Bs, wm, wn, g, t4, 0, min(wm + 32, m.kext(i)), acc);
+            store_tile(m.tile(m.T, i, j), ld, m.ext(i), m.ext(j), acc, -1.0, prev, nullptr, wm, wn, g, t4);
+            break;
+        default: {  // K_PACC: O(i,j) += T(k,i)^T T(k,j); diagonal T tiles lower
+            load_tile(As, m.tile(m.T, k, i), ld, m.ext(k), m.ext(i), tid);
+            load_tile(Bs, m.tile(m.T, k, j), ld, m.ext(k), m.ext(j), tid);
+            if (k > i) load_prev(m.tile(m.O, i, j), ld, m.ext(i), m.ext(j), wm, wn, g, t4, prev);
+            tile_wait();
+            __syncthreads();
+            int kb = 0;
+            if (k == i) kb = wm;
+            if (k == j) kb = max(kb, wn);
+            tile_mma<true, false>(As, Bs, wm, wn, g, t4, kb, m.kext(k), acc);
+            const bool last = k == m.tiles() - 1;
+            store_tile(m.tile(m.O, i, j), ld, m.ext(i), m.ext(j), acc, 1.0, prev,
+                       (last && i > j) ? m.tile(m.O, j, i) : nullptr, wm, wn, g, t4);
+            break;
         }
     }
     // release: the barrier orders every thread's tile writes before thread 0's
@@ -292,31 +375,57 @@ __device__ __forceinline__ bool run_task(double* A, double* T, double* O, int n,
     if (tid == 0) {
         __threadfence();
         switch (type) {
-            case K_POTRF: atomicExch(lrdy + tri(k + 1, k), 1); break;  // the fused L(k+1,k)
-            case K_TRSM: atomicExch(lrdy + tri(i, k), 1); break;
-            case K_UPDATE: atomicAdd(ver + tri(i, j), 1); break;
-            case K_TACC: atomicAdd(tacc + tri(i, j), 1); break;
-            case K_TFIN: atomicExch(trdy + tri(i, j), 1); break;
-            default: atomicAdd(pacc + tri(i, j), 1); break;
+            case K_TRSM: atomicExch(m.lrdy + tri(i, k), 1); break;
+            case K_UPDATE: atomicAdd(m.ver + tri(i, j), 1); break;
+            case K_TACC: atomicAdd(m.tacc + tri(i, j), 1); break;
+            case K_TFIN: atomicExch(m.trdy + tri(i, j), 1); break;
+            default: atomicAdd(m.pacc + tri(i, j), 1); break;
         }
     }
     return true;
 }
 
-__global__ void __launch_bounds__(DAG_THREADS, 1)
+__device__ __forceinline__ int sm_id() {
+    unsigned id;
+    asm volatile("mov.u32 %0, %%smid;\n" : "=r"(id));
+    return (int)id;
+}
+
+__global__ void __launch_bounds__(DAG_THREADS, DAG_CTAS)
     k_spd_inverse_tasks(double* A, double* T, double* O, int n, long ld, const int4* __restrict__ tasks, int ntasks,
                         int* state, int ntri, int* err, long spin) {
     extern __shared__ __align__(16) double sm[];
-    __shared__ int s_task, s_ok;
+    __shared__ int s_task, flag[3];
     int* const cursor = state;
-    int* const abort = state + 1;
+    int* const chain_sm = state + 2;  // 1 + the SM that runs the chain
+    int* const others = state + 3;    // CTAs that take tasks on other SMs until the list is done
+    const TaskMatrix m(A, T, O, n, ld, state, ntri, err, state + 1, spin);
+    bool counted = false, chain = false;  // thread 0
     while (true) {
-        if (threadIdx.x == 0) s_task = atomicAdd(cursor, 1);
+        if (threadIdx.x == 0) {
+            const int at = ld_acquire(chain_sm), here = sm_id() + 1;
+            if (at != 0 && at != here && !counted) {
+                atomicAdd(others, 1);
+                counted = true;
+            }
+            // beside the chain, unless nobody else is there to do the tasks
+            const bool retire = at == here && !chain && ld_acquire(others) > 0;
+            s_task = retire ? ntasks : atomicAdd(cursor, 1);
+        }
         __syncthreads();
         const int task = s_task;
         if (task >= ntasks) break;
         const int4 tk = tasks[task];
-        if (!run_task(A, T, O, n, ld, state, ntri, err, abort, spin, tk.x, tk.y, tk.z, tk.w, sm, s_ok)) break;
+        if (tk.x != K_POTRF) {
+            if (!run_task(m, tk.x, tk.y, tk.z, tk.w, sm, flag)) break;
+        } else if (tk.w == 0) {
+            if (threadIdx.x == 0) {
+                chain = true;
+                atomicExch(chain_sm, sm_id() + 1);
+            }
+            if (!run_chain(m, sm, flag)) break;
+        }
+        __syncthreads();  // s_task and flag are rewritten
     }
 }
 
@@ -328,21 +437,21 @@ __global__ void __launch_bounds__(DAG_THREADS, 1)
 // earlier in the list and the launch completes with any number of resident
 // CTAs; each task does exactly the arithmetic of the single-matrix kernel, so
 // the results are bitwise those of one launch per matrix.
-__global__ void __launch_bounds__(DAG_THREADS, 1)
+__global__ void __launch_bounds__(DAG_THREADS, DAG_CTAS)
     k_spd_inverse_tasks_grouped(const SpdTaskMatrix* __restrict__ mats, const int4* __restrict__ tasks, int ntasks,
                                 int* ctl, long spin) {
     extern __shared__ __align__(16) double sm[];
-    __shared__ int s_task, s_ok;
+    __shared__ int s_task, flag[3];
     while (true) {
         if (threadIdx.x == 0) s_task = atomicAdd(ctl, 1);
         __syncthreads();
         const int task = s_task;
         if (task >= ntasks) break;
         const int4 tk = tasks[task];
-        const SpdTaskMatrix& m = mats[tk.x >> 3];
-        if (!run_task(m.A, m.T, m.O, m.n, m.ld, m.state, m.ntri, m.err, ctl + 1, spin, tk.x & 7, tk.y, tk.z, tk.w, sm,
-                      s_ok))
-            break;
+        const SpdTaskMatrix& d = mats[tk.x >> 3];
+        const TaskMatrix m(d.A, d.T, d.O, d.n, d.ld, d.state, d.ntri, d.err, ctl + 1, spin);
+        if (!run_task(m, tk.x & 7, tk.y, tk.z, tk.w, sm, flag)) break;
+        __syncthreads();
     }
 }
 
@@ -459,7 +568,7 @@ int chol_inverse_tasks(double* A, int n, int lda, double* T, double* O, int* sta
         }
         list = {own, (int)h.size()};
     }
-    const int grid = std::max(1, std::min(std::min(device_sms(), max_ctas), list.second));
+    const int grid = std::max(1, std::min(DAG_CTAS * std::min(device_sms(), max_ctas), list.second));
     k_spd_inverse_tasks<<<grid, DAG_THREADS, DAG_SMEM, st>>>(A, T, O, n, lda, list.first, list.second, state, ntri,
                                                              err, spin);
     count_launch();
@@ -508,7 +617,7 @@ int chol_inverse_tasks_grouped(const SpdTaskMatrix* d_mats, const int4* d_tasks,
     if (ntasks <= 0) return UNC_OK;
     prepare_task_kernels();
     const long spin = poll_limit > 0 ? (long)std::min<long long>(poll_limit, kDagSpin) : kDagSpin;
-    const int grid = std::max(1, std::min(std::min(device_sms(), max_ctas), ntasks));
+    const int grid = std::max(1, std::min(DAG_CTAS * std::min(device_sms(), max_ctas), ntasks));
     k_spd_inverse_tasks_grouped<<<grid, DAG_THREADS, DAG_SMEM, st>>>(d_mats, d_tasks, ntasks, ctl, spin);
     count_launch();
     return UNC_OK;

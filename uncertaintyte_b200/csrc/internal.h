@@ -188,7 +188,7 @@ void gemm_f64_tri(int M, int N, int K, double alpha, const double* A, int lda, c
 struct SpdScratch {
     double *T, *W, *ws;
     int* state;
-    int max_ctas = 148;        // grid bound of the tile tasks
+    int max_ctas = 148;        // SMs that the tile tasks may cover
     long long poll_limit = 0;  // as chol_inverse_tasks
     int skip_task = -1;
 };
@@ -220,7 +220,7 @@ void launch_unequilibrate_from(const double* S, double* X, int n, int lda, const
 bool spd_tasks_apply(int n);
 size_t spd_task_state_ints(int n);
 int spd_tasks_prepare(int n, bool product = true);
-// max_ctas bounds the persistent grid (at most one CTA per SM is used anyway);
+// max_ctas bounds the SMs that the persistent grid covers (two CTAs each);
 // the task order and every tile's update order do not depend on it, so neither
 // do the results.
 // poll_limit (> 0): polls of one dependency before a wait gives up (default
