@@ -10,6 +10,12 @@
 //   TFIN(i,j)     T(i,j) = -T(i,i) W(i,j)                     (block forward substitution)
 //   PACC(i,j,k)   O(i,j) += T(k,i)^T T(k,j)                   (k >= i >= j; the last term also
 //                                                             writes the transposed tile)
+// UPDATE, TACC and PACC take 1 to 4 consecutive values of their last index in one
+// task (its k field: first value + count << 16): a single one where the chain of
+// diagonal tiles or of T's rows waits for it, groups of four elsewhere. A task
+// streams its operands in slices of 32 k through three shared-memory stages and
+// reads and writes its own tile once, so a group costs its products and not one
+// load-compute-store round trip per 64 k.
 // POTRF(k) also applies the last update of its tile (from panel k-1) before
 // factoring and computes TRSM(k+1,k) after it, so the dependent chain from one
 // diagonal tile to the next is one task. The host lists the tasks in a
@@ -50,11 +56,15 @@ namespace {
 constexpr int TB = NB;                   // tile size (the leaf size)
 constexpr int DAG_THREADS = LEAF_THREADS;
 constexpr int TLD = LEAF_LD;             // shared tile stride: fragment reads conflict-free in both orientations
-// Two CTAs of 256 threads per SM, so that one loads its tiles, waits or stores
-// while the other computes: two operand tiles and the leaf's block (whose
-// inverse takes the second operand tile) are 104 KB.
+// Two CTAs of 256 threads per SM, so that one waits, loads or stores while the
+// other computes. Shared memory of a CTA: two operand tiles and the leaf's block
+// (whose inverse takes the second operand tile), or the stages of a stream.
 constexpr int DAG_CTAS = 2;
-constexpr size_t DAG_SMEM = sizeof(double) * 3 * LEAF_TILE;
+constexpr int SLICE = 32, STREAM_STAGES = 3;      // k of a slice
+constexpr int SLD = SLICE + 4;                    // stride of a slice of rows (k contiguous)
+constexpr int SLOT = TB * SLD > SLICE * TLD ? TB * SLD : SLICE * TLD;  // doubles of one operand's slice
+constexpr size_t DAG_SMEM = sizeof(double) * (2 * STREAM_STAGES * SLOT > 3 * LEAF_TILE ? 2 * STREAM_STAGES * SLOT : 3 * LEAF_TILE);
+constexpr int GROUP = 4;                          // consecutive k of a group
 constexpr long kDagSpin = 1L << 22;      // polls of one dependency before the kernel gives up
 constexpr int kMaxTilesN = 56;           // tasks are used up to n = 56 * 64
 
@@ -68,8 +78,8 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
     return v;
 }
 
-// thread 0 only: wait until *flag >= v (or the abort flag is raised / the
-// limit of `spin` polls runs out)
+// One thread: wait until *flag >= v (or the abort flag is raised / the limit of
+// `spin` polls runs out)
 __device__ bool wait_ge(const int* flag, int v, const int* abort, long spin) {
     for (long it = 0; it < spin; ++it) {
         if (ld_acquire(flag) >= v) return true;
@@ -79,13 +89,24 @@ __device__ bool wait_ge(const int* flag, int v, const int* abort, long spin) {
     return false;
 }
 
+// One warp: the same for one flag per lane (nullptr: none), polled together.
+__device__ bool wait_all(const int* flag, int v, const int* abort, long spin) {
+    for (long it = 0; it < spin; ++it) {
+        const bool ok = !flag || ld_acquire(flag) >= v;
+        if (__all_sync(0xffffffffu, ok)) return true;
+        if (ld_acquire(abort)) return false;
+        __nanosleep(32);
+    }
+    return false;
+}
+
 // Tile X (column-major, leading dimension ld; rows < vr and columns < vc
 // valid, the rest zero) into shared memory as sm[c * TLD + r], asynchronously
 // and past L1, by `threads` threads; tile_wait() before the barrier that
-// publishes it.
+// publishes it. cols: columns of the tile that are copied.
 __device__ __forceinline__ void load_tile(double* sm, const double* X, long ld, int vr, int vc, int tid,
-                                          int threads = DAG_THREADS) {
-    for (int q = tid; q < TB * TB / 2; q += threads) {
+                                          int threads = DAG_THREADS, int cols = TB) {
+    for (int q = tid; q < cols * (TB / 2); q += threads) {
         const int c = q >> 5, r2 = (q & 31) * 2;
         const int left = c < vc ? vr - r2 : 0;
         const int bytes = left >= 2 ? 16 : (left == 1 ? 8 : 0);
@@ -98,29 +119,89 @@ __device__ __forceinline__ void load_tile(double* sm, const double* X, long ld, 
 }
 __device__ __forceinline__ void tile_wait() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
-// acc += op(A) op(B) over k in [kb, ke) (multiples of 4) for this warp's 32 x 16
-// block (rows wm.., columns wn..). op(A)(m, k) = kTA ? A(k, m) : A(m, k),
-// op(B)(k, n) = kTB ? B(n, k) : B(k, n), tiles as left by load_tile.
+// A tile of a matrix: its first element and its valid rows and columns.
+struct TileRef {
+    const double* p;
+    int rows, cols;
+};
+
+// acc += A op(B) over k in [kb, ke) (multiples of 4) for this warp's 32 x 16
+// block (rows wm.., columns wn..), op(B)(k, n) = B(n, k), whole tiles as left by
+// load_tile.
 using Acc = double[4][2][2];
-template <bool kTA, bool kTB>
 __device__ __forceinline__ void tile_mma(const double* As, const double* Bs, int wm, int wn, int g, int t, int kb,
                                          int ke, Acc& acc) {
     for (int kk = kb; kk < ke; kk += 4) {
         double a[4], b[2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int m = wm + 8 * i + g, k = kk + t;
-            a[i] = kTA ? As[m * TLD + k] : As[k * TLD + m];
-        }
+        for (int i = 0; i < 4; ++i) a[i] = As[(kk + t) * TLD + wm + 8 * i + g];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int n = wn + 8 * j + g, k = kk + t;
-            b[j] = kTB ? Bs[k * TLD + n] : Bs[n * TLD + k];
-        }
+        for (int j = 0; j < 2; ++j) b[j] = Bs[(kk + t) * TLD + wn + 8 * j + g];
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int j = 0; j < 2; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+    }
+}
+
+// One operand of a stream: tile(kt) is its tile at k tile kt, of rows x cols
+// valid elements. kRows: k runs along the tile's rows, else along its columns.
+template <bool kRows>
+__device__ __forceinline__ void load_slice(double* sm, const double* X, long ld, int vr, int vc, int half, int tid) {
+#pragma unroll
+    for (int u = 0; u < TB * SLICE / 2 / DAG_THREADS; ++u) {
+        const int q = tid + u * DAG_THREADS;
+        const int c = kRows ? q / (SLICE / 2) : q / (TB / 2) + half * SLICE;
+        const int r2 = kRows ? (q % (SLICE / 2)) * 2 + half * SLICE : (q % (TB / 2)) * 2;
+        const int left = c < vc ? vr - r2 : 0;
+        const int bytes = left >= 2 ? 16 : (left == 1 ? 8 : 0);
+        double* d = kRows ? sm + c * SLD + (r2 - half * SLICE) : sm + (c - half * SLICE) * TLD + r2;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(
+                         static_cast<unsigned>(__cvta_generic_to_shared(d))),
+                     "l"(bytes ? X + r2 + (long)c * ld : X), "r"(bytes)
+                     : "memory");
+    }
+}
+
+// acc += sum over k tiles k0 .. k0 + count - 1 of op(A) op(B): fa(kt), fb(kt)
+// give the operands' tiles (pointer, valid rows, valid columns). op(A)(m, k) =
+// kRowsA ? A(k, m) : A(m, k), op(B)(k, n) = kRowsB ? B(k, n) : B(n, k). klim:
+// this warp's products stop at that k of a tile (a triangular operand).
+template <bool kRowsA, bool kRowsB, class FA, class FB>
+__device__ __forceinline__ void stream_mma(double* sm, long ld, int k0, int count, FA&& fa, FB&& fb, int wm, int wn,
+                                           int g, int t, int klim, int tid, Acc& acc) {
+    const int n = 2 * count;
+    auto issue = [&](int it) {
+        if (it < n) {
+            double* st = sm + (it % STREAM_STAGES) * 2 * SLOT;
+            const TileRef a = fa(k0 + it / 2), b = fb(k0 + it / 2);
+            load_slice<kRowsA>(st, a.p, ld, a.rows, a.cols, it & 1, tid);
+            load_slice<kRowsB>(st + SLOT, b.p, ld, b.rows, b.cols, it & 1, tid);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    issue(0);
+    issue(1);
+    for (int it = 0; it < n; ++it) {
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        __syncthreads();
+        issue(it + 2);
+        const double* As = sm + (it % STREAM_STAGES) * 2 * SLOT;
+        const double* Bs = As + SLOT;
+        const int ke = min(SLICE, klim - (it & 1) * SLICE);
+#pragma unroll 4
+        for (int kk = 0; kk < ke; kk += 4) {
+            double a[4], b[2];
+            const int k = kk + t;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = kRowsA ? As[(wm + 8 * i + g) * SLD + k] : As[k * TLD + wm + 8 * i + g];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) b[j] = kRowsB ? Bs[(wn + 8 * j + g) * SLD + k] : Bs[k * TLD + wn + 8 * j + g];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+        }
     }
 }
 
@@ -178,7 +259,6 @@ struct TaskMatrix {
         : A(A_), T(T_), O(O_), n(n_), ld(ld_), ver(state + 4), lrdy(ver + ntri), tacc(lrdy + ntri), trdy(tacc + ntri),
           pacc(trdy + ntri), err(err_), abort(abort_), spin(spin_) {}
     __device__ __forceinline__ int ext(int b) const { return min(TB, n - TB * b); }
-    __device__ __forceinline__ int kext(int b) const { return (ext(b) + 3) & ~3; }  // K extent of a partial tile, DMMA steps
     __device__ __forceinline__ int tiles() const { return (n + TB - 1) / TB; }
     __device__ __forceinline__ double* tile(double* M, int i, int j) const { return M + (long)TB * i + (long)TB * j * ld; }
     // thread 0 only
@@ -212,22 +292,27 @@ __device__ bool potrf(const TaskMatrix& m, int k, bool chained, bool& diag_in, d
     __syncthreads();
     Acc acc = {};
     if (k > 0) {
-        if (wn < wm + 32) tile_mma<false, true>(As, As, wm, wn, g, t4, 0, TB, acc);  // lower blocks only
+        if (wn < wm + 32) tile_mma(As, As, wm, wn, g, t4, 0, TB, acc);  // lower blocks only
         tile_elements(TB, TB, wm, wn, g, t4, acc, [&](int r, int c, double& v) {
             if (c <= r) S[c * TLD + r] -= v;
         });
     }
     if (tid == 0) flag[0] = 0;
     __syncthreads();
-    bool fetched = false;  // warp 4: A(k+1,k) is on its way into As
+    // warp 4: A(k+1,k) into As in two halves of 32 columns, beside two panels (a
+    // whole tile takes this one warp longer than a panel)
+    int halves = 0;
     chol_leaf_factor(TB * k, m.ext(k), m.T, m.ld, m.err, S, Bs, [&](int q) {
-        if (!below || fetched || q == 0) return;
-        int ready = 0;
-        if (lane == 0) ready = ld_acquire(m.ver + tri(k + 1, k)) >= k;
-        fetched = __shfl_sync(0xffffffffu, ready, 0) != 0;
-        if (!fetched) return;
-        load_tile(As, m.tile(m.A, k + 1, k), m.ld, m.ext(k + 1), m.ext(k), lane, 32);
-        if (lane == 0) flag[0] = 1;
+        if (!below || halves == 2 || q == 0) return;
+        if (halves == 0) {
+            int ready = 0;
+            if (lane == 0) ready = ld_acquire(m.ver + tri(k + 1, k)) >= k;
+            if (!__shfl_sync(0xffffffffu, ready, 0)) return;
+            if (lane == 0) flag[0] = 1;
+        }
+        for (const int stop = q == 3 ? 2 : halves + 1; halves < stop; ++halves)
+            load_tile(As + halves * 32 * TLD, m.tile(m.A, k + 1, k) + halves * 32 * m.ld, m.ld, m.ext(k + 1),
+                      m.ext(k) - halves * 32, lane, 32, 32);
     });
     tile_wait();
     __syncthreads();
@@ -254,7 +339,7 @@ __device__ bool potrf(const TaskMatrix& m, int k, bool chained, bool& diag_in, d
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int b = 0; b < 2; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-    tile_mma<false, true>(As, Bs, wm, wn, g, t4, 0, wn + 16, acc);
+    tile_mma(As, Bs, wm, wn, g, t4, 0, wn + 16, acc);
     if (chained) {
         __syncthreads();  // As is read no more
         tile_elements(TB, TB, wm, wn, g, t4, acc, [&](int r, int c, double& v) { As[c * TLD + r] = v; });
@@ -277,39 +362,44 @@ __device__ bool run_chain(const TaskMatrix& m, double* sm, int* flag) {
     return true;
 }
 
-// One tile task (type, i, j, k), run by all DAG_THREADS threads of the block;
-// thread 0 waits for its dependencies first. Returns false when a wait gave up
-// (ERRBIT_TIMEOUT and the abort flag are set): the caller stops taking tasks.
-__device__ __forceinline__ bool run_task(const TaskMatrix& m, int type, int i, int j, int k, double* sm, int* flag) {
+// One tile task (type, i, j, k with its count), run by all DAG_THREADS threads of
+// the block; warp 0 waits for its dependencies first. Returns false when a wait
+// gave up (ERRBIT_TIMEOUT and the abort flag are set): the caller stops taking
+// tasks.
+__device__ __forceinline__ bool run_task(const TaskMatrix& m, int type, int i, int j, int kc, double* sm, int* flag) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t4 = lane & 3;
     const int wm = (warp & 1) * 32, wn = (warp >> 1) * 16;
-    double* As = sm;
-    double* Bs = sm + LEAF_TILE;
+    const int k = kc & 0xffff, count = kc >> 16;
     const long ld = m.ld;
-    if (tid == 0) {
-        bool ok = true;
+    if (warp == 0) {
+        // lane 0: the tile's own counter; lanes 1 .. count and count + 1 .. 2 count: the operands of each k
+        const int *own = nullptr, *first = nullptr, *second = nullptr;
+        int v = 0;
+        const int q = lane > count ? lane - count - 1 : lane - 1;
         switch (type) {
             case K_POTRF:  // its last update (from panel k-1) is applied inside the task
-                ok = k == 0 || (m.wait(m.ver + tri(k, k), k - 1) && m.wait(m.lrdy + tri(k, k - 1), 1));
+                if (k > 0) {
+                    own = m.ver + tri(k, k);
+                    v = k - 1;
+                    first = m.lrdy + tri(k, k - 1);
+                }
                 break;
-            case K_TRSM:
-                ok = m.wait(m.ver + tri(i, k), k) && m.wait(m.lrdy + tri(k, k), 1);
-                break;
+            case K_TRSM: own = m.ver + tri(i, k), v = k, first = m.lrdy + tri(k, k); break;
             case K_UPDATE:
-                ok = m.wait(m.ver + tri(i, j), k) && m.wait(m.lrdy + tri(i, k), 1) && m.wait(m.lrdy + tri(j, k), 1);
+                own = m.ver + tri(i, j), v = k, first = m.lrdy + tri(i, k + q), second = m.lrdy + tri(j, k + q);
                 break;
             case K_TACC:
-                ok = m.wait(m.tacc + tri(i, j), k - j) && m.wait(m.lrdy + tri(i, k), 1) && m.wait(m.trdy + tri(k, j), 1);
+                own = m.tacc + tri(i, j), v = k - j, first = m.lrdy + tri(i, k + q), second = m.trdy + tri(k + q, j);
                 break;
-            case K_TFIN:
-                ok = m.wait(m.tacc + tri(i, j), i - j) && m.wait(m.trdy + tri(i, i), 1);
-                break;
+            case K_TFIN: own = m.tacc + tri(i, j), v = i - j, first = m.trdy + tri(i, i); break;
             default:  // K_PACC
-                ok = m.wait(m.pacc + tri(i, j), k - i) && m.wait(m.trdy + tri(k, i), 1) && m.wait(m.trdy + tri(k, j), 1);
+                own = m.pacc + tri(i, j), v = k - i, first = m.trdy + tri(k + q, i), second = m.trdy + tri(k + q, j);
                 break;
         }
-        flag[0] = ok || m.give_up();
+        const int* f = lane == 0 ? own : (lane <= count ? first : (lane <= 2 * count ? second : nullptr));
+        const bool ok = wait_all(f, lane == 0 ? v : 1, m.abort, m.spin);
+        if (lane == 0) flag[0] = ok || m.give_up();
     }
     __syncthreads();
     if (!flag[0]) return false;
@@ -317,53 +407,36 @@ __device__ __forceinline__ bool run_task(const TaskMatrix& m, int type, int i, i
         bool diag_in = false;
         return potrf(m, k, false, diag_in, sm, flag);
     }
+    auto ref = [&](double* M, int r, int c) { return TileRef{m.tile(M, r, c), m.ext(r), m.ext(c)}; };
     Acc acc = {}, prev = {};
     switch (type) {
         case K_TRSM:  // L(i,k) = A(i,k) T(k,k)^T; T(k,k) lower: terms k' <= n only
-            load_tile(As, m.tile(m.A, i, k), ld, m.ext(i), m.ext(k), tid);
-            load_tile(Bs, m.tile(m.T, k, k), ld, m.ext(k), m.ext(k), tid);
-            tile_wait();
-            __syncthreads();
-            tile_mma<false, true>(As, Bs, wm, wn, g, t4, 0, min(wn + 16, m.kext(k)), acc);
+            stream_mma<false, false>(sm, ld, k, 1, [&](int) { return ref(m.A, i, k); },
+                                     [&](int) { return ref(m.T, k, k); }, wm, wn, g, t4, wn + 16, tid, acc);
             store_tile(m.tile(m.A, i, k), ld, m.ext(i), m.ext(k), acc, 1.0, prev, nullptr, wm, wn, g, t4);
             break;
         case K_UPDATE:  // A(i,j) -= L(i,k) L(j,k)^T
-            load_tile(As, m.tile(m.A, i, k), ld, m.ext(i), m.ext(k), tid);
-            load_tile(Bs, m.tile(m.A, j, k), ld, m.ext(j), m.ext(k), tid);
             load_prev(m.tile(m.A, i, j), ld, m.ext(i), m.ext(j), wm, wn, g, t4, prev);
-            tile_wait();
-            __syncthreads();
-            tile_mma<false, true>(As, Bs, wm, wn, g, t4, 0, m.kext(k), acc);
+            stream_mma<false, false>(sm, ld, k, count, [&](int q) { return ref(m.A, i, q); },
+                                     [&](int q) { return ref(m.A, j, q); }, wm, wn, g, t4, TB, tid, acc);
             store_tile(m.tile(m.A, i, j), ld, m.ext(i), m.ext(j), acc, -1.0, prev, nullptr, wm, wn, g, t4);
             break;
-        case K_TACC:  // W(i,j) += L(i,k) T(k,j); T(j,j) lower: terms k' >= n only
-            load_tile(As, m.tile(m.A, i, k), ld, m.ext(i), m.ext(k), tid);
-            load_tile(Bs, m.tile(m.T, k, j), ld, m.ext(k), m.ext(j), tid);
+        case K_TACC:  // W(i,j) += L(i,k) T(k,j)
             if (k > j) load_prev(m.tile(m.T, i, j), ld, m.ext(i), m.ext(j), wm, wn, g, t4, prev);
-            tile_wait();
-            __syncthreads();
-            tile_mma<false, false>(As, Bs, wm, wn, g, t4, k == j ? wn : 0, m.kext(k), acc);
+            stream_mma<false, true>(sm, ld, k, count, [&](int q) { return ref(m.A, i, q); },
+                                    [&](int q) { return ref(m.T, q, j); }, wm, wn, g, t4, TB, tid, acc);
             store_tile(m.tile(m.T, i, j), ld, m.ext(i), m.ext(j), acc, 1.0, prev, nullptr, wm, wn, g, t4);
             break;
         case K_TFIN:  // T(i,j) = -T(i,i) W(i,j); T(i,i) lower: terms k' <= m only
-            load_tile(As, m.tile(m.T, i, i), ld, m.ext(i), m.ext(i), tid);
-            load_tile(Bs, m.tile(m.T, i, j), ld, m.ext(i), m.ext(j), tid);
-            tile_wait();
-            __syncthreads();
-            tile_mma<false, false>(As, Bs, wm, wn, g, t4, 0, min(wm + 32, m.kext(i)), acc);
+            stream_mma<false, true>(sm, ld, i, 1, [&](int) { return ref(m.T, i, i); },
+                                    [&](int) { return ref(m.T, i, j); }, wm, wn, g, t4, wm + 32, tid, acc);
             store_tile(m.tile(m.T, i, j), ld, m.ext(i), m.ext(j), acc, -1.0, prev, nullptr, wm, wn, g, t4);
             break;
-        default: {  // K_PACC: O(i,j) += T(k,i)^T T(k,j); diagonal T tiles lower
-            load_tile(As, m.tile(m.T, k, i), ld, m.ext(k), m.ext(i), tid);
-            load_tile(Bs, m.tile(m.T, k, j), ld, m.ext(k), m.ext(j), tid);
+        default: {  // K_PACC: O(i,j) += T(k,i)^T T(k,j)
             if (k > i) load_prev(m.tile(m.O, i, j), ld, m.ext(i), m.ext(j), wm, wn, g, t4, prev);
-            tile_wait();
-            __syncthreads();
-            int kb = 0;
-            if (k == i) kb = wm;
-            if (k == j) kb = max(kb, wn);
-            tile_mma<true, false>(As, Bs, wm, wn, g, t4, kb, m.kext(k), acc);
-            const bool last = k == m.tiles() - 1;
+            stream_mma<true, true>(sm, ld, k, count, [&](int q) { return ref(m.T, q, i); },
+                                   [&](int q) { return ref(m.T, q, j); }, wm, wn, g, t4, TB, tid, acc);
+            const bool last = k + count == m.tiles();
             store_tile(m.tile(m.O, i, j), ld, m.ext(i), m.ext(j), acc, 1.0, prev,
                        (last && i > j) ? m.tile(m.O, j, i) : nullptr, wm, wn, g, t4);
             break;
@@ -376,10 +449,10 @@ __device__ __forceinline__ bool run_task(const TaskMatrix& m, int type, int i, i
         __threadfence();
         switch (type) {
             case K_TRSM: atomicExch(m.lrdy + tri(i, k), 1); break;
-            case K_UPDATE: atomicAdd(m.ver + tri(i, j), 1); break;
-            case K_TACC: atomicAdd(m.tacc + tri(i, j), 1); break;
+            case K_UPDATE: atomicAdd(m.ver + tri(i, j), count); break;
+            case K_TACC: atomicAdd(m.tacc + tri(i, j), count); break;
             case K_TFIN: atomicExch(m.trdy + tri(i, j), 1); break;
-            default: atomicAdd(m.pacc + tri(i, j), 1); break;
+            default: atomicAdd(m.pacc + tri(i, j), count); break;
         }
     }
     return true;
@@ -418,7 +491,7 @@ __global__ void __launch_bounds__(DAG_THREADS, DAG_CTAS)
         const int4 tk = tasks[task];
         if (tk.x != K_POTRF) {
             if (!run_task(m, tk.x, tk.y, tk.z, tk.w, sm, flag)) break;
-        } else if (tk.w == 0) {
+        } else if (tk.y == 0) {
             if (threadIdx.x == 0) {
                 chain = true;
                 atomicExch(chain_sm, sm_id() + 1);
@@ -456,32 +529,66 @@ __global__ void __launch_bounds__(DAG_THREADS, DAG_CTAS)
 }
 
 // The task list of nt x nt tiles in the order described above; without the
-// product, T = L^{-1} only (no PACC).
+// product, T = L^{-1} only (no PACC). At step s panel s, T's row s - 1 and the
+// product terms of T's row s become available. A tile that is not needed in the
+// next two steps takes its terms in groups of GROUP, whose ends fall on another
+// step for each of GROUP neighbouring tiles, so that every step has its share of
+// them and none floods the CTAs that the chain waits for; one that is needed in
+// the step after next takes the rest of its group, so that only a single term is
+// left when the next step waits for it. The last two product terms are single
+// ones (a short tail). Below kGroupTiles the CTAs keep up with single terms and a
+// group would only delay its tile (n = 600: 173 us single, 188 us in groups; equal at 1800;
+// n = 2752: 1606 and 1102 us).
+constexpr int kGroupTiles = 32;
 std::vector<int4> build_tasks(int nt, bool product = true) {
     std::vector<int4> v;
-    auto add = [&v](int ty, int i, int j, int k) { v.push_back(make_int4(ty, i, j, k)); };
+    auto add = [&v](int ty, int i, int j, int first, int last) {
+        v.push_back(make_int4(ty, i, j, first | (last - first + 1) << 16));
+    };
+    const int size = nt < kGroupTiles ? 1 : GROUP;
+    // tile (i, j): terms first_of(i, j, s) .. s are one group at step s when ends(i, j, s)
+    auto ends = [size](int i, int j, int s) { return (s + i + j) % size == size - 1; };
+    auto first_of = [size](int i, int j, int s) { return std::max(0, s - (s + i + j) % size); };
     // POTRF(k) also applies UPDATE(k,k,k-1) first and computes TRSM(k+1,k) last
-    add(K_POTRF, 0, 0, 0);
-    for (int i = 2; i < nt; ++i) add(K_TRSM, i, 0, 0);
+    add(K_POTRF, 0, 0, 0, 0);
+    for (int i = 2; i < nt; ++i) add(K_TRSM, i, 0, 0, 0);
     for (int s = 0; s < nt; ++s) {
         if (s + 1 < nt) {
-            if (s + 2 < nt) add(K_UPDATE, s + 2, s + 1, s);  // the input of the fused TRSM(s+2,s+1)
-            add(K_POTRF, s + 1, s + 1, s + 1);
+            if (s + 2 < nt) add(K_UPDATE, s + 2, s + 1, s, s);  // the input of the fused TRSM(s+2,s+1)
+            add(K_POTRF, s + 1, s + 1, s + 1, s + 1);
+            if (s + 2 < nt) add(K_UPDATE, s + 2, s + 2, first_of(s + 2, s + 2, s), s);  // the next diagonal tile
             for (int i = s + 3; i < nt; ++i) {
-                add(K_UPDATE, i, s + 1, s);
-                add(K_TRSM, i, s + 1, s + 1);
+                add(K_UPDATE, i, s + 1, s, s);
+                add(K_TRSM, i, s + 1, s + 1, s + 1);
             }
             for (int j = s + 2; j < nt; ++j)
-                for (int i = j; i < nt; ++i) add(K_UPDATE, i, j, s);
+                for (int i = j + (j == s + 2); i < nt; ++i)
+                    if (j == s + 2 || ends(i, j, s)) add(K_UPDATE, i, j, first_of(i, j, s), s);
         }
-        if (s >= 1)
-            for (int r = s; r < nt; ++r)
-                for (int c = 0; c < s; ++c) add(K_TACC, r, c, s - 1);
-        for (int c = 0; c < s; ++c) add(K_TFIN, s, c, 0);
+        if (s >= 1) {
+            const int p = s - 1;  // T's row p is final
+            for (int c = 0; c < s; ++c) add(K_TACC, s, c, p, p);
+            for (int r = s + 1; r < nt; ++r)
+                for (int c = 0; c < s; ++c)
+                    if (r == s + 1 || ends(r, c, p)) add(K_TACC, r, c, std::max(c, first_of(r, c, p)), p);
+        }
+        for (int c = 0; c < s; ++c) add(K_TFIN, s, c, 0, 0);
         for (int r = 0; product && r <= s; ++r)
-            for (int c = 0; c <= r; ++c) add(K_PACC, r, c, s);
+            for (int c = 0; c <= r; ++c) {
+                const bool last = s == nt - 1;
+                if (last || s == nt - 2 || ends(r, c, s))
+                    add(K_PACC, r, c, last ? s : std::max(r, first_of(r, c, s)), s);
+            }
     }
     return v;
+}
+
+// The same with every group as its single terms, one after the other.
+std::vector<int4> single_tasks(const std::vector<int4>& v) {
+    std::vector<int4> out;
+    for (const int4& t : v)
+        for (int q = 0; q < t.w >> 16; ++q) out.push_back(make_int4(t.x, t.y, t.z, ((t.w & 0xffff) + q) | 1 << 16));
+    return out;
 }
 
 struct TaskLists {
@@ -556,8 +663,8 @@ int chol_inverse_tasks(double* A, int n, int lda, double* T, double* O, int* sta
     if (cudaMemsetAsync(state, 0, sizeof(int) * spd_task_state_ints(n), st) != cudaSuccess) return UNC_ERR_CUDA;
     const long spin = poll_limit > 0 ? (long)std::min<long long>(poll_limit, kDagSpin) : kDagSpin;
     int4* own = nullptr;  // a schedule with one task left out (tests of the bounded waits)
-    if (skip_task >= 0 && skip_task < list.second) {
-        std::vector<int4> h = build_tasks(nt, O != nullptr);
+    if (skip_task >= 0 && skip_task < unc_spd_task_list(n, nullptr, 0)) {
+        std::vector<int4> h = single_tasks(build_tasks(nt, O != nullptr));
         h.erase(h.begin() + skip_task);
         if (cudaMallocAsync(reinterpret_cast<void**>(&own), sizeof(int4) * h.size(), st) != cudaSuccess)
             return UNC_ERR_OUT_OF_MEMORY;
@@ -635,13 +742,13 @@ extern "C" int unc_spd_task_list(int n, int* out, int capacity) {
         unc::g_last_error = "unc_spd_task_list: n must be in 1..3584";
         return UNC_ERR_INVALID_ARG;
     }
-    const std::vector<int4> v = unc::build_tasks((n + unc::NB - 1) / unc::NB);
+    const std::vector<int4> v = unc::single_tasks(unc::build_tasks((n + unc::NB - 1) / unc::NB));
     if (out && capacity >= (int)v.size())
         for (size_t q = 0; q < v.size(); ++q) {
             out[4 * q] = v[q].x;
             out[4 * q + 1] = v[q].y;
             out[4 * q + 2] = v[q].z;
-            out[4 * q + 3] = v[q].w;
+            out[4 * q + 3] = v[q].w & 0xffff;
         }
     return (int)v.size();
 }
