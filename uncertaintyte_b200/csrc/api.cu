@@ -172,15 +172,15 @@ size_t carve(char* base, const Plan& pl, bool host_io, long long nnz, int nrows,
     s.cam_ptr = c.take<int>((size_t)pl.C + 1);
     s.cam_obs = c.take<int>(pl.nobs);
     s.pt_ptr = c.take<int>((size_t)pl.P + 1);
-    s.pt_obs = c.take<int>(pl.nobs);
-    s.cursor = c.take<int>((size_t)pl.C + pl.P + 1);
-    s.scan_tmp = c.take<int>(scan_tmp_ints(std::max(pl.C, pl.P)));
+    s.pt_list = c.take<int2>(pl.nobs);
+    s.pt_tmp = c.take<int2>(pl.nobs);
+    s.pos_list = c.take<int2>(pl.nobs);
+    s.index_tmp = c.take<int>(index_scratch_ints(pl.C, pl.P));
     s.s_cam = c.take<double>((size_t)pl.C * 9);
-    s.s_pt = c.take<double>((size_t)pl.P * 3);
+    s.is_cam = c.take<double>((size_t)pl.C * 9);
     s.Vraw = c.take<double>((size_t)pl.P * 6);
-    s.iVs = c.take<double>((size_t)pl.P * 6);
-    s.Ws = c.take<double>((size_t)pl.nobs * 27);
-    s.Ys = c.take<double>((size_t)pl.nobs * 27);
+    s.Mp = c.take<double>((size_t)pl.P * 6);
+    s.Q = c.take<double>((size_t)pl.nobs * 27);
     s.cam_part = c.take<double>(45 * camera_tile_slots(pl.C, pl.nobs));
     s.Ucam = c.take<double>(81 * (size_t)pl.C);
     s.err = c.take<int>(4);
@@ -402,10 +402,9 @@ int sparse_stage(const unc_options* o, const Plan& pl, long long nnz, const int*
     if (int r = mark(2)) return r;
     // zero the dense work buffers once (padding rows must stay finite for the GEMM loads)
     CK(cudaMemsetAsync(b.iZ, 0, (size_t)((char*)(b.tmp + (size_t)ld * N) - (char*)b.iZ), sm));
-    launch_camera_blocks(s, sm);
     launch_point_blocks(s, sm);
     if (int r = mark(3)) return r;
-    launch_obs_blocks(s, sm);
+    launch_camera_blocks(s, sm);
     if (int r = mark(4)) return r;
     CK(cudaMemsetAsync(b.Z, 0, sizeof(double) * (size_t)ld * N, sm));
     if (launch_schur_columns(s, b.Z, ld, sm) != UNC_OK)
@@ -806,8 +805,6 @@ int run_pipeline(unc_context* ctx, const unc_options* o, int num_rows, long long
         return fail(UNC_ERR_SINGULAR, "non-positive pivot or non-finite value while inverting Z + lambda*I");
     if (err & ERRBIT_TIMEOUT)
         return fail(UNC_ERR_CUDA, "a bounded device wait ran out (tensor-core pipeline or tile-task inverse)");
-    if (err & ERRBIT_SCHUR_CAP)
-        return fail(UNC_ERR_TOO_LARGE, "an observation shares its point with more observations than the Schur stage holds");
     if (te.bad) return fail(UNC_ERR_SINGULAR, "non-finite Taylor-series power");
     return UNC_OK;
 }
@@ -868,6 +865,7 @@ int unc_context_create(int device, unc_context** out) {
         c->sm_count = device_sms();
         c->task_ctas = c->sm_count;
         prepare_assembly_kernels();
+        prepare_point_kernels();
         prepare_dense_kernels();
         prepare_mixed_kernels();
         e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
@@ -1229,12 +1227,11 @@ int unc_jtj_crs(int num_rows, int num_cols, const int* rows, const int* cols, co
     CK(dal((void**)&s.cam_ptr, sizeof(int) * ((size_t)C + 1)));
     CK(dal((void**)&s.cam_obs, sizeof(int) * (size_t)nobs));
     CK(dal((void**)&s.pt_ptr, sizeof(int) * ((size_t)P + 1)));
-    CK(dal((void**)&s.pt_obs, sizeof(int) * (size_t)nobs));
-    CK(dal((void**)&s.cursor, sizeof(int) * ((size_t)C + P + 1)));
-    CK(dal((void**)&s.scan_tmp, sizeof(int) * scan_tmp_ints(std::max(C, P))));
-    CK(dal((void**)&s.s_pt, sizeof(double) * 3 * (size_t)P));
+    CK(dal((void**)&s.pt_list, sizeof(int2) * (size_t)nobs));
+    CK(dal((void**)&s.pt_tmp, sizeof(int2) * (size_t)nobs));
+    CK(dal((void**)&s.pos_list, sizeof(int2) * (size_t)nobs));
+    CK(dal((void**)&s.index_tmp, sizeof(int) * index_scratch_ints(C, P)));
     CK(dal((void**)&s.Vraw, sizeof(double) * 6 * (size_t)P));
-    CK(dal((void**)&s.iVs, sizeof(double) * 6 * (size_t)P));
     CK(dal((void**)&s.err, sizeof(int) * 4));
     CK(dal((void**)&d_U, sizeof(double) * 81 * (size_t)C));
     CK(dal((void**)&d_W, sizeof(double) * 27 * (size_t)nobs));

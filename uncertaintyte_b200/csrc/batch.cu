@@ -664,7 +664,6 @@ int run_group(unc_batch* b, GroupRun& g, const int* const* rows, const int* cons
         if (err & ERRBIT_LAYOUT) rc = UNC_ERR_LAYOUT;
         else if (err & (ERRBIT_SINGULAR | ERRBIT_NONFINITE)) rc = UNC_ERR_SINGULAR;
         else if (err & ERRBIT_TIMEOUT) rc = UNC_ERR_CUDA;
-        else if (err & ERRBIT_SCHUR_CAP) rc = UNC_ERR_TOO_LARGE;
         else if (te.bad) rc = UNC_ERR_SINGULAR;
         status[s.idx] = rc;
         if (stats) {
@@ -704,6 +703,7 @@ int unc_batch_create(int device, unc_batch** out) {
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) {
         prepare_assembly_kernels();
+        prepare_point_kernels();
         prepare_dense_kernels();
         prepare_mixed_kernels();
         prepare_task_kernels();

@@ -18,9 +18,7 @@ enum : int {
     ERRBIT_LAYOUT = 1,      // observation rows not 12 entries / columns out of range
     ERRBIT_SINGULAR = 2,    // non-positive or non-finite pivot
     ERRBIT_NONFINITE = 4,   // NaN / Inf produced
-    ERRBIT_SORT_CAP = 8,    // a segment was too long to sort (order left nondeterministic)
     ERRBIT_TIMEOUT = 16,    // a bounded device wait ran out (tensor-core pipeline)
-    ERRBIT_SCHUR_CAP = 32,  // an observation has more Schur partners than one chunk holds (Z incomplete)
 };
 
 constexpr int kCamParams = 9;
@@ -105,17 +103,18 @@ struct SceneDev {
     int* obs_cam;         // per observation camera id (-1 = dropped)
     int* obs_pt;          // per observation point id (-1 = dropped: fixed point or no point)
     int* cam_ptr;         // num_cams + 1
-    int* cam_obs;         // observation ids grouped by camera (ascending within a camera)
+    int* cam_obs;         // observation ids grouped by camera (ascending within a camera): the camera order
     int* pt_ptr;          // num_points + 1
-    int* pt_obs;          // observation ids grouped by point (ascending within a point)
-    int* cursor;          // scratch: max(num_cams, num_points) + 1 ints
-    int* scan_tmp;        // scratch for the scan
+    int2* pt_list;        // per point its observations: (position in the camera order, camera), ascending
+    int2* pt_tmp;         // scratch: the lists in arrival order
+    int2* pos_list;       // per position: the start of its point's list, its rank in it
+    int* index_tmp;       // scratch: index_scratch_ints(num_cams, num_points)
     double* s_cam;        // 9*num_cams column norms of J (camera columns)
-    double* s_pt;         // 3*num_points column norms (point columns)
+    double* is_cam;       // 9*num_cams their inverses (1 for a zero norm)
     double* Vraw;         // 6*num_points upper triangle of the unscaled point block J_p^T J_p
-    double* iVs;          // 6*num_points upper triangle of the inverse of the scaled point block
-    double* Ws;           // 27*num_obs scaled W_o = (J_c^T J_p)/(s s), 9x3 row-major
-    double* Ys;           // 27*num_obs Y_o = W_o * iV_p, 9x3 row-major
+    double* Mp;           // 6*num_points M_p, M_p M_p^T = V_p^{-1} (k_point_blocks), or nullptr
+    double* Q;            // 27*num_obs by position: Q_o = W_o M_p, 9x3 row-major (W_o = J_c^T J_p); after the
+                          // Schur stage 6 per position: the observation's share of its point's covariance
     double* cam_part;     // 45 * camera_tile_slots(): per-tile partial sums of the camera blocks
     double* Ucam;         // 81*num_cams scaled camera blocks U (9 x 9, column-major)
     int* err;             // device error bits
@@ -125,10 +124,12 @@ void launch_validate_obs(const SceneDev& s, cudaStream_t st);
 // Camera observations are processed in tiles of 256; slots = C + num_obs/256 + 1.
 size_t camera_tile_slots(int num_cams, int num_obs);
 void launch_build_index(SceneDev& s, cudaStream_t st);
-// U blocks (scaled) into s.Ucam, column norms into s.s_cam.
-void launch_camera_blocks(const SceneDev& s, cudaStream_t st);
+size_t index_scratch_ints(int num_cams, int num_points);
+// Point blocks and, unless s.Mp is nullptr, their inverse factors.
 void launch_point_blocks(const SceneDev& s, cudaStream_t st);
-void launch_obs_blocks(const SceneDev& s, cudaStream_t st);
+// U blocks (scaled) into s.Ucam, column norms into s.s_cam / s.is_cam, the Q
+// records (after the point blocks).
+void launch_camera_blocks(const SceneDev& s, cudaStream_t st);
 // The Schur complement Z = U - W V^-1 W^T (schur.cu) over a zeroed Z: the
 // diagonal blocks from s.Ucam, every co-visible camera-pair block written in
 // both triangles, bitwise symmetric. UNC_ERR_TOO_LARGE above kSchurMaxCams.
@@ -141,8 +142,6 @@ void launch_repack_generic(int num_obs, int cam_off, const int* rows, const int*
                            const double* vals, double* J, int* obs_cam, int* obs_pt, int* err,
                            cudaStream_t st);
 void launch_unscaled_blocks(const SceneDev& s, double* U, double* W, cudaStream_t st);
-void exclusive_scan(const int* in, int* out, int n, int* tmp, cudaStream_t st);
-size_t scan_tmp_ints(int n);
 
 // ---------------- dense.cu ----------------
 // C = alpha*A*B + beta*C, column-major, FP64 on DMMA. If amax != nullptr the
@@ -479,5 +478,6 @@ int launch_scene_jacobian(int num_cams, int num_points, int num_obs, const doubl
 
 // ---------------- points.cu ----------------
 void launch_point_cov(const SceneDev& s, const double* sig, double* pt_unc, cudaStream_t st);
+void prepare_point_kernels();  // kernel attributes (before any stream capture)
 
 }  // namespace unc

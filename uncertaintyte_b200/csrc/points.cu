@@ -13,11 +13,67 @@
 //
 //   Sigma_pt = D^+ + D^+ (sum_o W_o^T Sigma_cam(o) W_o) D^+,   W_o = J_cam,o^T A_o
 //
-// evaluated per point in FP64 registers: no 2n x 11n matrices, no O(P*obs)
-// scan (the reference rescans every Jacobian row per point, :393).
-#include "internal.h"
+// in two steps: per observation the six values of W_o^T Sigma_cam(o) W_o, by
+// camera tiles (the camera's block in shared memory, the records staged), and
+// per point the sum of its observations' six values and the 3 x 3 algebra. No
+// 2n x 11n matrices, no O(P*obs) scan (the reference rescans every Jacobian row
+// per point, :393).
+#include "obs_tiles.cuh"
 
 namespace unc {
+
+// One thread per observation of a camera tile: S = W^T Sigma W (symmetric: 00 01
+// 02 11 12 22) by position. Gathering the camera's 81 values per observation
+// instead cost as many cache lines as there are lanes on every load (100 us for
+// 342k observations, of which the records' bytes are 15).
+constexpr size_t kSigTileSmem = sizeof(double) * kObsTile * kRecStride;
+__global__ void __launch_bounds__(kObsTile, 2)
+    k_camera_sig_tiles(int num_cams, const double* __restrict__ J, const int* __restrict__ cam_ptr,
+                       const int* __restrict__ cam_obs, const double* __restrict__ sig, double* __restrict__ S) {
+    extern __shared__ __align__(16) double sj[];
+    __shared__ int ids[kObsTile];
+    __shared__ double sg[81];
+    ObsTile tile;
+    if (!find_tile(cam_ptr, num_cams, blockIdx.x, tile)) return;
+    const int n = tile.end - tile.begin, t = threadIdx.x;
+    if (t < 81) sg[t] = sig[81L * tile.cam + t];
+    stage_records(sj, ids, J, cam_obs, tile);
+    if (t >= n) return;
+    const double* r = sj + t * kRecStride;
+    double W[9][3];
+    {
+        const double a0 = r[9], a1 = r[10], a2 = r[11], b0 = r[21], b1 = r[22], b2 = r[23];
+#pragma unroll
+        for (int j = 0; j < 9; ++j) {
+            const double u = r[j], v = r[12 + j];
+            W[j][0] = u * a0 + v * b0;
+            W[j][1] = u * a1 + v * b1;
+            W[j][2] = u * a2 + v * b2;
+        }
+    }
+    double s00 = 0, s01 = 0, s02 = 0, s11 = 0, s12 = 0, s22 = 0;
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+        double t0 = 0, t1 = 0, t2 = 0;  // (Sigma W)(j, :)
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const double x = sg[9 * j + k];
+            t0 = fma(x, W[k][0], t0);
+            t1 = fma(x, W[k][1], t1);
+            t2 = fma(x, W[k][2], t2);
+        }
+        s00 = fma(W[j][0], t0, s00);
+        s01 = fma(W[j][0], t1, s01);
+        s02 = fma(W[j][0], t2, s02);
+        s11 = fma(W[j][1], t1, s11);
+        s12 = fma(W[j][1], t2, s12);
+        s22 = fma(W[j][2], t2, s22);
+    }
+    double2* out = reinterpret_cast<double2*>(S + 6L * (tile.begin + t));
+    out[0] = make_double2(s00, s01);
+    out[1] = make_double2(s02, s11);
+    out[2] = make_double2(s12, s22);
+}
 
 // Pseudo-inverse of a symmetric PSD 3x3 (a00 a01 a02 a11 a12 a22) through a
 // cyclic Jacobi eigen-decomposition. Eigenvalues below 64*eps*max are
@@ -69,75 +125,37 @@ __device__ void sym3_pinv(const double in[6], double out[3][3]) {
             out[i][j] = v[i][0] * v[j][0] * iw[0] + v[i][1] * v[j][1] * iw[1] + v[i][2] * v[j][2] * iw[2];
 }
 
-// Four threads per point: thread q of the quad sums observations b + q,
-// b + q + 4, ... of the point into its S; the quad then adds its four partial
-// S in a fixed butterfly order (bitwise repeatable) and thread 0 finishes.
-constexpr int kPointLanes = 4;
-__global__ void __launch_bounds__(128) k_point_cov(int num_points, int3 fix, int has_fix,
-                                                   const double* __restrict__ J,
-                                                   const int* __restrict__ pt_ptr,
-                                                   const int* __restrict__ pt_obs,
-                                                   const int* __restrict__ obs_cam,
-                                                   const double* __restrict__ Vraw,
-                                                   const double* __restrict__ sig,
-                                                   double* __restrict__ pt_unc) {
-    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
-    const int p = gt / kPointLanes, q = gt % kPointLanes;
-    const unsigned quad = 0xfu << (threadIdx.x & 28);
-    if (p >= num_points) return;  // whole quads leave together
+// One thread per point: its observations' S in list order, then the algebra.
+__global__ void __launch_bounds__(128) k_point_cov(int num_points, int3 fix, int has_fix, const int* __restrict__ pt_ptr,
+                                                   const int2* __restrict__ pt_list, const double* __restrict__ So,
+                                                   const double* __restrict__ Vraw, double* __restrict__ pt_unc) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= num_points) return;
     if (has_fix && (p == fix.x || p == fix.y || p == fix.z)) return;  // fixed points are skipped
     double* out = pt_unc + 6L * p;
     const int b = pt_ptr[p], e = pt_ptr[p + 1];
     if (b == e) {  // pinv of an empty A: zero covariance
-        if (q == 0) out[0] = out[1] = out[2] = out[3] = out[4] = out[5] = 0.0;
+        out[0] = out[1] = out[2] = out[3] = out[4] = out[5] = 0.0;
         return;
     }
-    double S[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    for (int i = b + q; i < e; i += kPointLanes) {
-        int o = pt_obs[i];
-        const double* r = J + 24L * o;
-        const double2* qv = reinterpret_cast<const double2*>(r);
-        double v[24];
+    double s6[6] = {0, 0, 0, 0, 0, 0};
+    for (int i0 = b; i0 < e; i0 += 4) {  // four records in flight
+        double2 x[4][3];
 #pragma unroll
-        for (int k = 0; k < 12; ++k) {
-            double2 x = __ldg(qv + k);
-            v[2 * k] = x.x;
-            v[2 * k + 1] = x.y;
+        for (int q = 0; q < 4; ++q) {
+            const double2* src = reinterpret_cast<const double2*>(So + 6L * (i0 + q < e ? pt_list[i0 + q].x : 0));
+#pragma unroll
+            for (int k = 0; k < 3; ++k) x[q][k] = i0 + q < e ? __ldg(src + k) : make_double2(0.0, 0.0);
         }
-        // W = Jc^T Jp (9x3)
-        double W[9][3];
 #pragma unroll
-        for (int j = 0; j < 9; ++j)
+        for (int q = 0; q < 4; ++q)
 #pragma unroll
-            for (int k = 0; k < 3; ++k) W[j][k] = v[j] * v[9 + k] + v[12 + j] * v[21 + k];
-        const double* sg = sig + 81L * obs_cam[o];
-        // S += W^T Sig W  (Sig row-major 9x9: sg[9*j + k] = Sigma(j, k))
-#pragma unroll
-        for (int j = 0; j < 9; ++j) {
-            double t0 = 0, t1 = 0, t2 = 0;  // (Sig W)(j, :)
-#pragma unroll
-            for (int k = 0; k < 9; ++k) {
-                double s = __ldg(sg + 9 * j + k);
-                t0 += s * W[k][0];
-                t1 += s * W[k][1];
-                t2 += s * W[k][2];
+            for (int k = 0; k < 3; ++k) {
+                s6[2 * k] += x[q][k].x;
+                s6[2 * k + 1] += x[q][k].y;
             }
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                S[a][0] += W[j][a] * t0;
-                S[a][1] += W[j][a] * t1;
-                S[a][2] += W[j][a] * t2;
-            }
-        }
     }
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            S[a][c] += __shfl_xor_sync(quad, S[a][c], 1);
-            S[a][c] += __shfl_xor_sync(quad, S[a][c], 2);
-        }
-    if (q != 0) return;
+    const double S[3][3] = {{s6[0], s6[1], s6[2]}, {s6[1], s6[3], s6[4]}, {s6[2], s6[4], s6[5]}};
     double Dp[3][3];
     sym3_pinv(Vraw + 6L * p, Dp);
     // Sigma_pt = D^+ + D^+ S D^+
@@ -160,14 +178,24 @@ __global__ void __launch_bounds__(128) k_point_cov(int num_points, int3 fix, int
     out[5] = R[2][2];
 }
 
+void prepare_point_kernels() {
+    static std::atomic<unsigned long long> attr{0};
+    once_per_device(attr, [] {
+        return cudaFuncSetAttribute(k_camera_sig_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSigTileSmem) ==
+               cudaSuccess;
+    });
+}
+
 void launch_point_cov(const SceneDev& s, const double* sig, double* pt_unc, cudaStream_t st) {
     if (s.num_points == 0) return;
+    prepare_point_kernels();
     int3 fix = make_int3(s.fix[0], s.fix[1], s.fix[2]);
-    const long threads = (long)s.num_points * kPointLanes;
-    k_point_cov<<<(unsigned)((threads + 127) / 128), 128, 0, st>>>(s.num_points, fix, s.has_fix, s.J,
-                                                            s.pt_ptr, s.pt_obs, s.obs_cam, s.Vraw,
-                                                            sig, pt_unc);
-    count_launch();
+    double* So = s.Q;  // the Q records are not needed any more
+    k_camera_sig_tiles<<<(unsigned)camera_tile_slots(s.num_cams, s.num_obs), kObsTile, kSigTileSmem, st>>>(
+        s.num_cams, s.J, s.cam_ptr, s.cam_obs, sig, So);
+    k_point_cov<<<(s.num_points + 127) / 128, 128, 0, st>>>(s.num_points, fix, s.has_fix, s.pt_ptr, s.pt_list, So, s.Vraw,
+                                                            pt_unc);
+    count_launch(2);
 }
 
 }  // namespace unc

@@ -110,13 +110,13 @@ __global__ void k_dense_pt(const double* __restrict__ Vraw, int P, long b0, doub
 // so a camera seeing the point twice is summed deterministically; the thread
 // owns the point's three columns (upper right) and three rows (lower left).
 __global__ void k_dense_w(const double* __restrict__ W, const int* __restrict__ obs_cam,
-                          const int* __restrict__ pt_ptr, const int* __restrict__ pt_obs, int P, long b0,
-                          double* M, long ld) {
+                          const int* __restrict__ pt_ptr, const int2* __restrict__ pt_list,
+                          const int* __restrict__ cam_obs, int P, long b0, double* M, long ld) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= P) return;
     const long r = b0 + 3L * p;
     for (int q = pt_ptr[p]; q < pt_ptr[p + 1]; ++q) {
-        const int o = pt_obs[q], c = obs_cam[o];
+        const int o = cam_obs[pt_list[q].x], c = obs_cam[o];
         if (c < 0) continue;
         const double* w = W + 27L * o;
         for (int i = 0; i < 9; ++i)
@@ -513,12 +513,11 @@ size_t svd_carve(char* base, int C, int P, int nobs, bool host_io, long long nnz
     s.cam_ptr = c.take<int>((size_t)C + 1);
     s.cam_obs = c.take<int>(nobs);
     s.pt_ptr = c.take<int>((size_t)P + 1);
-    s.pt_obs = c.take<int>(nobs);
-    s.cursor = c.take<int>((size_t)C + P + 1);
-    s.scan_tmp = c.take<int>(scan_tmp_ints(std::max(C, P)));
-    s.s_pt = c.take<double>((size_t)P * 3);
+    s.pt_list = c.take<int2>(nobs);
+    s.pt_tmp = c.take<int2>(nobs);
+    s.pos_list = c.take<int2>(nobs);
+    s.index_tmp = c.take<int>(index_scratch_ints(C, P));
     s.Vraw = c.take<double>((size_t)P * 6);
-    s.iVs = c.take<double>((size_t)P * 6);
     s.err = c.take<int>(4);
     L.U = c.take<double>((size_t)C * 81);
     L.Wb = c.take<double>((size_t)nobs * 27);
@@ -586,7 +585,7 @@ int svd_pipeline(char* ws, const unc_options* o, int num_rows, long long nnz, co
     k_dense_cam<<<C, 96, 0, sm>>>(L.U, C, L.M, ld);
     if (P > 0) {
         k_dense_pt<<<(P + 127) / 128, 128, 0, sm>>>(s.Vraw, P, b0, L.M, ld);
-        k_dense_w<<<(P + 127) / 128, 128, 0, sm>>>(L.Wb, s.obs_cam, s.pt_ptr, s.pt_obs, P, b0, L.M, ld);
+        k_dense_w<<<(P + 127) / 128, 128, 0, sm>>>(L.Wb, s.obs_cam, s.pt_ptr, s.pt_list, s.cam_obs, P, b0, L.M, ld);
     }
     count_launch(P > 0 ? 3 : 1);
     int err = 0;
