@@ -195,7 +195,7 @@ size_t carve(char* base, const Plan& pl, bool host_io, long long nnz, int nrows,
     b.p8 = c.take<double>(nn);
     b.p12 = c.take<double>(nn);
     b.p16 = c.take<double>(nn);
-    b.g = c.take<double>(nn);
+    b.pblk = c.take<double>(16 * (size_t)kPowerPairs * pl.C);
     b.dmax = c.take<unsigned long long>(24);
     b.e = c.take<double>(pl.N);
     b.dag_state = c.take<int>(spd_task_state_ints(pl.N));
@@ -400,8 +400,6 @@ int sparse_stage(const unc_options* o, const Plan& pl, long long nnz, const int*
     if (int r = mark(1)) return r;
     launch_build_index(s, sm);
     if (int r = mark(2)) return r;
-    // zero the dense work buffers once (padding rows must stay finite for the GEMM loads)
-    CK(cudaMemsetAsync(b.iZ, 0, (size_t)((char*)(b.tmp + (size_t)ld * N) - (char*)b.iZ), sm));
     launch_point_blocks(s, sm);
     if (int r = mark(3)) return r;
     launch_camera_blocks(s, sm);
@@ -413,8 +411,23 @@ int sparse_stage(const unc_options* o, const Plan& pl, long long nnz, const int*
     return UNC_OK;
 }
 
-void output_stage(const Plan& pl, Buffers& b, double* cam_out, double* pt_out, cudaStream_t sm) {
-    launch_camera_output(b.iZ, pl.ld, b.s.s_cam, pl.C, cam_out, b.sig, sm);
+PowerSet power_set(const Plan& pl, const Buffers& b) {
+    PowerSet ps{};
+    double* const m[7] = {b.Z, b.add, b.tmp, b.p4, b.p8, b.p12, b.p16};
+    std::copy(m, m + 7, ps.M);
+    ps.blk = b.pblk;
+    ps.n = pl.N;
+    ps.ld = pl.ld;
+    ps.dmax = b.dmax;
+    ps.te = b.te;
+    return ps;
+}
+
+void output_stage(const Plan& pl, Buffers& b, bool powers, double* cam_out, double* pt_out, cudaStream_t sm) {
+    if (powers)
+        launch_power_output(power_set(pl, b), b.s.s_cam, cam_out, b.sig, sm);
+    else
+        launch_camera_output(b.iZ, pl.ld, b.s.s_cam, pl.C, cam_out, b.sig, sm);
     if (pl.P > 3) cudaMemsetAsync(pt_out, 0, sizeof(double) * 6 * ((size_t)pl.P - 3), sm);
     launch_point_cov(b.s, b.sig, pt_out, sm);
 }
@@ -482,6 +495,10 @@ int run_stage(unc_context* ctx, const GraphKey& key, cudaStream_t sm, F&& stage,
     return UNC_OK;
 }
 
+
+// Slice buffers of the mixed modes: X, the A operand of the moment and, with the
+// blocked powers, X^4 and X^8.
+int slice_buffers(const unc_options* o) { return o->taylor_eval == UNC_TAYLOR_SEQUENTIAL ? 2 : 4; }
 
 float ev_s(cudaEvent_t a, cudaEvent_t b) {
     float ms = 0;
@@ -551,11 +568,11 @@ int run_pipeline(unc_context* ctx, const unc_options* o, int num_rows, long long
     const bool mixed = o->precision != UNC_PRECISION_FP64;
     const bool powers = o->taylor_eval != UNC_TAYLOR_SEQUENTIAL;
     const int slices = o->precision == UNC_PRECISION_MIXED4 ? 4 : (o->precision == UNC_PRECISION_MIXED3 ? 3 : 5);
-    // slice buffers: X, the A operand of the moment, and (powers) X^4, X^8, X^12, X^16
-    constexpr int kX = 0, kA = 1, k4 = 2, k8 = 3, k12 = 4, k16 = 5;
-    const int nbuf = powers ? 6 : 2;
-    MixedOperand opa[6], opb[6];  // each buffer as the A (128-row boxes) and as the B operand
-    MixedOperand opa_k[6][6], opb_k[6][6];  // [buffer][k]: its first k slices
+    // slice buffers: X, the A operand of the moment, and (powers) X^4, X^8
+    constexpr int kX = 0, kA = 1, k4 = 2, k8 = 3;
+    const int nbuf = slice_buffers(o);
+    MixedOperand opa[4], opb[4];  // each buffer as the A (128-row boxes) and as the B operand
+    MixedOperand opa_k[4][6], opb_k[4][6];  // [buffer][k]: its first k slices
     size_t mp_need = 0;
     if (mixed) {  // host-side preparation: buffers and tensor maps
         const size_t sb = (mixed_slice_bytes(N, slices) + 255) & ~size_t(255);
@@ -610,18 +627,18 @@ int run_pipeline(unc_context* ctx, const unc_options* o, int num_rows, long long
         }
         return prof_mark();
     };
-    // blocked powers: out (+)= A B, A and B powers of X (symmetric, commuting)
+    // blocked powers: out = A B, A and B powers of X (symmetric, commuting)
     // given as FP64 matrices and, in mixed mode, as slice buffers ia / ib;
     // q: the product's index in power_product_slices
-    auto power_product = [&](int q, const double* A, int ia, const double* B, int ib, double* out, bool acc,
+    auto power_product = [&](int q, const double* A, int ia, const double* B, int ib, double* out,
                              const int* skip) -> int {
         if (int r = prof_mark()) return r;
         if (mixed) {
             const int k = power_product_slices(q, slices);
-            mixed_gemm(opa_k[ia][k], opb_k[ib][k], out, ld, nullptr, true, s.err, sm, skip, true, acc);
+            mixed_gemm(opa_k[ia][k], opb_k[ib][k], out, ld, nullptr, true, s.err, sm, skip, true);
         } else
-            gemm_f64_mode(N, N, N, 1.0, A, ld, B, ld, acc ? 1.0 : 0.0, out, ld, nullptr, GEMM_LOWER | GEMM_MIRROR,
-                          sm, nullptr, 0, skip);
+            gemm_f64_mode(N, N, N, 1.0, A, ld, B, ld, 0.0, out, ld, nullptr, GEMM_LOWER | GEMM_MIRROR, sm, nullptr, 0,
+                          skip);
         return prof_mark();
     };
     auto slice = [&](const double* A, int q, const int* skip) {
@@ -643,28 +660,25 @@ int run_pipeline(unc_context* ctx, const unc_options* o, int num_rows, long long
     int* gram_exps = mixed ? opa[kX].exps : nullptr;
     if (int r = spd_prepare(N)) return fail(r, "tile-task inverse: cannot upload the task list");
     const SpdScratch scratch{b.iZ, b.add, b.tmp, b.dag_state, ctx->task_ctas};
+    double* const copy = powers ? nullptr : b.iZ;  // X comes out in Z; one product per iteration: iZ = X too
     auto inverse_stage = [&]() -> int {
         if (gram) {
             // mixed: T = L^{-1} in FP64 (its products feed the pivots), A^{-1} = T^T T
             // from int8 slices of T on the tensor cores
             launch_shift_equilibrate(b.Z, N, ld, lambda, b.e, s.err, sm);
             if (int r = chol_lower_inverse(b.Z, N, ld, scratch, s.err, sm)) return r;
-            CK(cudaMemsetAsync(ctx->mp, 0, mixed_gram_bytes(N), sm));  // slice padding must be zero
             if (!mixed_gram_lower_tri(b.iZ, N, ld, reinterpret_cast<int8_t*>(ctx->mp), gram_exps, b.Z, ld, s.err, sm))
                 return fail(UNC_ERR_CUDA, "tensor-map encoding failed");
-            launch_unequilibrate(b.Z, N, ld, b.e, b.iZ, sm);  // X in Z, iZ = X
+            launch_unequilibrate(b.Z, N, ld, b.e, copy, sm);
             return UNC_OK;
         }
-        return spd_inverse(b.Z, N, ld, lambda, b.e, scratch, b.iZ, s.err, sm);  // X in Z, iZ = X
+        return spd_inverse(b.Z, N, ld, lambda, b.e, scratch, copy, s.err, sm);
     };
     auto taylor_stage = [&]() -> int {
         double* add = b.add;
         double* tmp = b.tmp;
-        if (mixed) {
-            CK(cudaMemsetAsync(ctx->mp, 0, mp_need, sm));  // slice padding must be zero
-            mixed_slice(X, ld, opa[kX], sm);
-        }
-        launch_te_init(b.te, sm);
+        if (mixed) mixed_slice(X, ld, opa[kX], sm);
+        launch_te_init(b.te, nullptr, sm);
         const int* skip = &b.te->done;
         CK(cudaMemsetAsync(b.amax, 0, 8, sm));
         if (int r = product(X, add, nullptr)) return r;
@@ -680,55 +694,29 @@ int run_pipeline(unc_context* ctx, const unc_options* o, int num_rows, long long
     };
     // The blocked-power evaluation (powers.cu): X^2, X^3, X^4, X^8, X^12 and
     // X^16 (skipped on the device unless the rule passes iteration 15); the
-    // stop rule from their diagonal maxima; iZ = G_0 + sum_q X^(4q) G_q, the
-    // products on the camera blocks only, with the blocks whose coefficients
-    // are all zero skipped on the device.
-    PowerSet ps{};
-    ps.M[0] = b.Z;
-    ps.M[1] = b.add;
-    ps.M[2] = b.tmp;
-    ps.M[3] = b.p4;
-    ps.M[4] = b.p8;
-    ps.M[5] = b.p12;
-    ps.M[6] = b.p16;
-    ps.iZ = b.iZ;
-    ps.G = b.g;
-    ps.n = N;
-    ps.ld = ld;
-    ps.dmax = b.dmax;
-    ps.te = b.te;
+    // camera blocks and diagonals of their products, the stop rule. The sum is
+    // formed with the outputs.
+    const PowerSet ps = power_set(pl, b);
     TaylorCoefs kc{};
     for (int i = 1; i < 20; ++i) kc.k[i - 1] = pow(lambda, i) / factorial_i32(i - 1);
     auto powers_stage = [&]() -> int {
         const int* sk = b.te->skip;
-        if (ld != N)  // padding rows of the extra power buffers must stay finite for the product loads
-            for (double* m : {b.p4, b.p8, b.p12, b.p16, b.g})
-                CK(cudaMemset2DAsync(m + N, sizeof(double) * (size_t)ld, 0, sizeof(double) * (size_t)(ld - N), N, sm));
-        if (mixed) {
-            CK(cudaMemsetAsync(ctx->mp, 0, mp_need, sm));  // slice padding must be zero
-            slice(X, kX, nullptr);
-        }
-        launch_te_init(b.te, sm);
-        CK(cudaMemsetAsync(b.dmax, 0, sizeof(unsigned long long) * 24, sm));
-        if (int r = power_product(0, X, kX, X, kX, b.add, false, nullptr)) return r;  // X^2
+        slice(X, kX, nullptr);
+        launch_te_init(b.te, b.dmax, sm);
+        if (int r = power_product(0, X, kX, X, kX, b.add, nullptr)) return r;  // X^2
         slice(b.add, kA, nullptr);
-        if (int r = power_product(1, b.add, kA, X, kX, b.tmp, false, nullptr)) return r;  // X^3
+        if (int r = power_product(1, b.add, kA, X, kX, b.tmp, nullptr)) return r;  // X^3
         slice(b.tmp, kA, nullptr);
-        if (int r = power_product(2, b.tmp, kA, X, kX, b.p4, false, nullptr)) return r;  // X^4
+        if (int r = power_product(2, b.tmp, kA, X, kX, b.p4, nullptr)) return r;  // X^4
         slice(b.p4, k4, nullptr);
-        if (int r = power_product(3, b.p4, k4, b.p4, k4, b.p8, false, nullptr)) return r;  // X^8
+        if (int r = power_product(3, b.p4, k4, b.p4, k4, b.p8, nullptr)) return r;  // X^8
         slice(b.p8, k8, nullptr);
-        if (int r = power_product(4, b.p8, k8, b.p4, k4, b.p12, false, nullptr)) return r;  // X^12
-        slice(b.p12, k12, nullptr);
-        launch_power_diag(ps, 2, 16, nullptr, sm);
+        if (int r = power_product(4, b.p8, k8, b.p4, k4, b.p12, nullptr)) return r;  // X^12
+        launch_power_blocks(ps, false, nullptr, sm);
         launch_power_decide(b.te, b.dmax, kc, 1, 15, sm);
-        if (int r = power_product(5, b.p8, k8, b.p8, k8, b.p16, false, sk)) return r;  // X^16
-        slice(b.p16, k16, sk);
-        launch_power_diag(ps, 17, 20, sk, sm);
+        if (int r = power_product(5, b.p8, k8, b.p8, k8, b.p16, sk)) return r;  // X^16
+        launch_power_blocks(ps, true, sk, sm);
         launch_power_decide(b.te, b.dmax, kc, 16, 19, sm);
-        launch_power_combine(ps, 0, b.iZ, nullptr, sm);  // iZ = G_0
-        // iZ += X^(4q) G_q on the camera blocks, the only part of iZ that is read after
-        launch_taylor_blocks(ps, sm);
         return UNC_OK;
     };
     while (ctx->prof && ctx->pev.size() < 2 * 20 + 2) {  // events exist before any capture
@@ -744,7 +732,9 @@ int run_pipeline(unc_context* ctx, const unc_options* o, int num_rows, long long
         // runs the stages directly
         GraphKey key = {1ULL, (unsigned long long)N, (unsigned long long)ld, lam_bits,
                         (unsigned long long)(uintptr_t)b.Z, (unsigned long long)(uintptr_t)b.dag_state,
-                        (unsigned long long)(uintptr_t)s.err, 0ULL};
+                        (unsigned long long)(uintptr_t)s.err,
+                        // what the inverse's launches depend on besides: T^T T by int8 (and its buffer), a copy of X
+                        (gram ? (unsigned long long)(uintptr_t)ctx->mp : 0ULL) | (copy ? 1ULL : 0ULL)};
         size_t none = 0;
         if (int r = ctx->prof ? inverse_stage() : run_stage(ctx, key, sm, inverse_stage, none)) return r;
         CK(cudaEventRecord(ev[6], sm));
@@ -758,7 +748,7 @@ int run_pipeline(unc_context* ctx, const unc_options* o, int num_rows, long long
         CK(cudaEventRecord(ev[7], sm));
     }
 
-    output_stage(pl, b, cam_out, pt_out, sm);
+    output_stage(pl, b, powers, cam_out, pt_out, sm);
     CK(cudaEventRecord(ev[8], sm));
 
     int err = 0;
@@ -769,12 +759,10 @@ int run_pipeline(unc_context* ctx, const unc_options* o, int num_rows, long long
     CK(cudaGetLastError());
     const int iters = te.iters;
     // products actually computed. Sequential: the first one and one per
-    // performed iteration. Powers: X^2..X^12 (5), X^16 unless skipped, one per
-    // non-zero block.
+    // performed iteration. Powers: X^2..X^12 (5), X^16 unless skipped.
     std::vector<bool> ran(npev / 2, false);
     for (size_t q = 0; q < ran.size(); ++q)
-        ran[q] = powers ? (q < 5 || (q == 5 && !te.skip[0]) || (q > 5 && q < 10 && !te.skip[q - 5]))
-                        : q < (size_t)iters + 1;
+        ran[q] = powers ? q < 5 || !te.skip[0] : q < (size_t)iters + 1;
     for (size_t q = 0; q < ran.size(); ++q) {
         if (!ran[q]) continue;
         ctx->prof_seconds += ev_s(ctx->pev[2 * q], ctx->pev[2 * q + 1]);
@@ -826,7 +814,7 @@ int dense_inverse(double* d_A, int n, int lda, void* stream, long long poll_limi
     double* e = ws + 3 * mat + state_d;
     int* err = reinterpret_cast<int*>(ws + wsd);
     int h_err = 0;
-    cudaError_t ce = cudaMemsetAsync(ws, 0, wsd * sizeof(double) + 256, sm);
+    cudaError_t ce = cudaMemsetAsync(err, 0, sizeof(int), sm);
     if (ce == cudaSuccess && spd_inverse(d_A, n, lda, 0.0, e, scratch, nullptr, err, sm) != UNC_OK) ce = cudaErrorUnknown;
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, sm);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(sm);
@@ -970,9 +958,9 @@ long long unc_request_bytes(const unc_options* o, int num_rows, int num_cols, co
     Plan pl = make_plan(o, num_rows);
     Buffers b;
     long long bytes = (long long)carve(nullptr, pl, true, nnz, num_rows, b);
-    if (o->precision != UNC_PRECISION_FP64) {  // slice buffers: 6 (blocked powers) or 2 (sequential)
+    if (o->precision != UNC_PRECISION_FP64) {
         const int slices = o->precision == UNC_PRECISION_MIXED4 ? 4 : (o->precision == UNC_PRECISION_MIXED3 ? 3 : 5);
-        const long long nbuf = o->taylor_eval == UNC_TAYLOR_SEQUENTIAL ? 2 : 6;
+        const long long nbuf = slice_buffers(o);
         bytes += nbuf * ((long long)((mixed_slice_bytes(pl.N, slices) + 255) & ~size_t(255)) +
                          (long long)((4 * ((size_t)pl.N + 64) + 255) & ~size_t(255))) + 256;
     }
@@ -1362,7 +1350,7 @@ int unc_gemm_mixed_device(int n, const double* d_P, const double* d_X, int ld, d
     if (!mixed_plan(a, bufP, eP, n, slices, false) || !mixed_plan(b, bufX, eX, n, slices, true))
         return fail(UNC_ERR_CUDA, "tensor-map encoding failed");
     int h_err = 0;
-    cudaError_t ce = cudaMemsetAsync(ws, 0, exp_off + 2 * sizeof(int) * ((size_t)n + 64) + 256, sm);
+    cudaError_t ce = cudaMemsetAsync(err, 0, sizeof(int), sm);
     if (ce == cudaSuccess) {
         mixed_slice(d_P, ld, a, sm);
         mixed_slice(d_X, ld, b, sm);
@@ -1387,7 +1375,7 @@ int unc_gram_lower_mixed_device(int n, const double* d_T, int ld, double* d_A, v
     int* ex = reinterpret_cast<int*>(ws + sb);
     int* err = ex + n + 64;
     int h_err = 0;
-    cudaError_t ce = cudaMemsetAsync(ws, 0, total, sm);
+    cudaError_t ce = cudaMemsetAsync(err, 0, sizeof(int), sm);
     if (ce == cudaSuccess && !mixed_gram_lower_tri(d_T, n, ld, reinterpret_cast<int8_t*>(ws), ex, d_A, ld, err, sm))
         return fail(UNC_ERR_CUDA, "tensor-map encoding failed");
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, sm);

@@ -75,8 +75,8 @@ struct Scene {
     double* out_cam;
     double* out_pt;
     size_t in_off[3], out_off[2];  // byte offsets in the staging areas
-    int8_t* buf[6];  // slices of X, of the A operand of the moment, of X^4, X^8, X^12, X^16
-    int* ex[6];      // their row exponents
+    int8_t* buf[4];  // slices of X, of the A operand of the moment, of X^4, X^8
+    int* ex[4];      // their row exponents
 };
 
 struct Layout {
@@ -200,13 +200,11 @@ int slices_of(int precision) {
     return precision == UNC_PRECISION_MIXED4 ? 4 : (precision == UNC_PRECISION_MIXED3 ? 3 : 5);
 }
 
-// per scene: X (A, B), A operand (A), X^4 (A, B), X^8 (A, B), X^12 (B), X^16 (B), and X^4, X^8, X^12, X^16
-// as B operands of 128-column tiles (the products with fewer slices than the group's)
-constexpr int kMaps = 13;
-// descriptor sets (the last four of each are laid out but not launched: the
-// block terms X^(4q) G_q are formed on the camera blocks, launch_taylor_blocks)
-constexpr int kSliceSets = 11;  // X, X^2, X^3, X^4, X^8, X^12, X^16, G_1..G_4
-constexpr int kGemmSets = 10;   // X^2, X^3, X^4, X^8, X^12, X^16, X^4 G_1 .. X^16 G_4
+// per scene: X (A, B), A operand (A), X^4 (A, B), X^8 (A, B), and X^4, X^8 as B operands of 128-column
+// tiles (the products with fewer slices than the group's)
+constexpr int kMaps = 9;
+constexpr int kSliceSets = 5;  // X, X^2, X^3, X^4, X^8
+constexpr int kGemmSets = 6;   // X^2, X^3, X^4, X^8, X^12, X^16
 
 // Device addresses of the descriptor region, in lay_out's order.
 struct Desc {
@@ -279,8 +277,8 @@ void lay_out(char* base, std::vector<Scene>& sc, int slices, int nt, Layout& L, 
     L.mixed_off = c.off;
     for (auto& s : sc) {
         const size_t sb = mixed_slice_bytes_nt(s.pl.N, slices, nt);
-        for (int q = 0; q < 6; ++q) s.buf[q] = c.take<int8_t>(sb);
-        for (int q = 0; q < 6; ++q) s.ex[q] = c.take<int>((size_t)s.pl.N + 64);
+        for (int q = 0; q < 4; ++q) s.buf[q] = c.take<int8_t>(sb);
+        for (int q = 0; q < 4; ++q) s.ex[q] = c.take<int>((size_t)s.pl.N + 64);
     }
     c.off = (c.off + 255) & ~size_t(255);
     L.mixed_bytes = c.off - L.mixed_off;
@@ -340,18 +338,12 @@ int launch_group(unc_batch* b, GroupRun& g) {
         int fx[3];
         if (int r = sparse_stage(&s.opt, s.pl, s.nnz, s.in_rows, s.in_cols, s.in_vals, s.b, fx, nullptr, br))
             return r;
-        const int N = s.pl.N, ld = s.pl.ld;
-        if (ld != N)  // padding rows of the extra power buffers must stay finite for the product loads
-            for (double* m : {s.b.p4, s.b.p8, s.b.p12, s.b.p16, s.b.g})
-                BCK(cudaMemset2DAsync(m + N, sizeof(double) * (size_t)ld, 0, sizeof(double) * (size_t)(ld - N), N,
-                                      br));
     }
     for (int k = 0; k < kBranches; ++k) {
         BCK(cudaEventRecord(b->join[k], b->branch[k]));
         BCK(cudaStreamWaitEvent(sm, b->join[k], 0));
     }
     // the dense stage, grouped (compute.cpp:121-166)
-    BCK(cudaMemsetAsync(g.dbase + g.L.mixed_off, 0, g.L.mixed_bytes, sm));  // slice padding must be zero
     BCK(cudaMemsetAsync(g.dbase + g.L.zero_off, 0, g.L.zero_bytes, sm));
     launch_shift_equilibrate_grouped(g.dd.dense, n, g.dd.blk_rows, g.nblk_rows, g.dd.blk_elems, g.nblk_elems, sm);
     int* ctl = reinterpret_cast<int*>(g.dbase + g.L.zero_off + g.L.zero_bytes - 256);
@@ -380,20 +372,15 @@ int launch_group(unc_batch* b, GroupRun& g) {
     gemm(3);  // X^8
     slice(4);
     gemm(4);  // X^12
-    slice(5);
-    launch_power_diag_grouped(g.dd.powers, n, g.dd.blk_cols, g.nblk_cols, 2, 16, false, sm);
+    launch_power_blocks_grouped(g.dd.powers, n, g.dd.blk_cols, g.nblk_cols, false, sm);
     launch_power_decide_grouped(g.dd.powers, n, g.dd.kpow, 1, 15, sm);
     gemm(5);  // X^16 (skipped per scene)
-    slice(6);
-    launch_power_diag_grouped(g.dd.powers, n, g.dd.blk_cols, g.nblk_cols, 17, 20, true, sm);
+    launch_power_blocks_grouped(g.dd.powers, n, g.dd.blk_cols, g.nblk_cols, true, sm);
     launch_power_decide_grouped(g.dd.powers, n, g.dd.kpow, 16, 19, sm);
-    launch_power_combine_grouped(g.dd.powers, n, g.dd.blk_elems, g.nblk_elems, 0, sm);  // iZ = G_0
-    // iZ += X^(4q) G_q on the camera blocks (the per-scene path's device function)
-    launch_taylor_blocks_grouped(g.dd.powers, n, g.dd.blk_cols, g.nblk_cols, sm);
     // outputs (compute.cpp:168-183, 370-455)
     BCK(cudaEventRecord(b->fork, sm));
     for (int k = 0; k < kBranches; ++k) BCK(cudaStreamWaitEvent(b->branch[k], b->fork, 0));
-    for (int i = 0; i < n; ++i) output_stage(g.sc[i].pl, g.sc[i].b, g.sc[i].out_cam, g.sc[i].out_pt,
+    for (int i = 0; i < n; ++i) output_stage(g.sc[i].pl, g.sc[i].b, true, g.sc[i].out_cam, g.sc[i].out_pt,
                                              b->branch[i % kBranches]);
     for (int k = 0; k < kBranches; ++k) {
         BCK(cudaEventRecord(b->join[k], b->branch[k]));
@@ -465,78 +452,56 @@ int prepare_group(unc_batch* b, GroupRun& g, int nt) {
         const long ld = s.pl.ld;
         const int nt64 = (N + 63) / 64;
         hdd.mats[i] = SpdTaskMatrix{s.b.Z, s.b.iZ, s.b.add, ld, N, nt64 * (nt64 + 1) / 2, s.b.dag_state, s.b.s.err};
-        // tensor maps: X (A, B), A operand (A), X^4 (A, B), X^8 (A, B), X^12 (B), X^16 (B); then
-        // X^4, X^8, X^12, X^16 as B operands with 128-row boxes (same buffers and plane stride)
-        const int mbuf[kMaps] = {0, 0, 1, 2, 2, 3, 3, 4, 5, 2, 3, 4, 5};
-        const bool mb[kMaps] = {false, true, false, false, true, false, true, true, true, true, true, true, true};
+        // tensor maps: X (A, B), A operand (A), X^4 (A, B), X^8 (A, B); then X^4, X^8 as B operands with
+        // 128-row boxes (same buffers and plane stride)
+        const int mbuf[kMaps] = {0, 0, 1, 2, 2, 3, 3, 2, 3};
+        const bool mb[kMaps] = {false, true, false, false, true, false, true, true, true};
         MixedOperand op[kMaps];
         for (int m = 0; m < kMaps; ++m) {
             bool ok = mixed_plan_nt(op[m], s.buf[mbuf[m]], s.ex[mbuf[m]], N, g.slices, mb[m], nt);
-            if (ok && m >= 9) op[m] = mixed_fewer_slices(op[m], 2, true, &ok);  // 128-row boxes
+            if (ok && m >= 7) op[m] = mixed_fewer_slices(op[m], 2, true, &ok);  // 128-row boxes
             if (!ok) return bfail(UNC_ERR_CUDA, "tensor-map encoding failed");
             hdd.maps[kMaps * i + m] = op[m].map;
         }
         const int rows = op[0].rows, kp = op[0].kp;
-        hdd.dense[i] = DenseJob{s.b.Z, s.b.iZ, s.b.add, s.b.e, ld, N, s.lambda, s.b.s.err, s.b.te, s.b.amax};
+        hdd.dense[i] = DenseJob{s.b.Z, s.b.add, s.b.e, ld, N, s.lambda, s.b.s.err, s.b.te, s.b.amax};
         hdd.blk_rows[i] = br;
         hdd.blk_elems[i] = be;
         hdd.blk_cols[i] = bc;
         br += (N + 255) / 256;
-        be += ((long)N * N + 255) / 256;
+        be += scale_blocks_grouped(N);
         bc += N;
         hdd.row_start[i] = rs;
         rs += N;
-        // slicing sets (powers.cu's order): X, X^2, X^3, X^4, X^8, X^12, X^16, G_1..G_4
+        // slicing sets (powers.cu's order): X, X^2, X^3, X^4, X^8
         const int* sk = s.b.te->skip;
         struct SliceDef {
             const double* src;
             int buf;
-            const int* skip;
         };
-        const SliceDef sd[kSliceSets] = {{s.b.Z, 0, nullptr},  {s.b.add, 1, nullptr}, {s.b.tmp, 1, nullptr},
-                                         {s.b.p4, 2, nullptr}, {s.b.p8, 3, nullptr},  {s.b.p12, 4, nullptr},
-                                         {s.b.p16, 5, sk},     {s.b.g, 1, sk + 1},    {s.b.g, 1, sk + 2},
-                                         {s.b.g, 1, sk + 3},   {s.b.g, 1, sk + 4}};
+        const SliceDef sd[kSliceSets] = {{s.b.Z, 0}, {s.b.add, 1}, {s.b.tmp, 1}, {s.b.p4, 2}, {s.b.p8, 3}};
         for (int q = 0; q < kSliceSets; ++q)
             hdd.slice[(size_t)q * n + i] = MixedSliceJob{sd[q].src, ld, N, g.slices, s.buf[sd[q].buf], rows, kp,
-                                                         s.ex[sd[q].buf], nullptr, nullptr, sd[q].skip};
-        // products: A map, B map, A / B exponent buffers, output, accumulate, skip
+                                                         s.ex[sd[q].buf], nullptr, nullptr, nullptr};
+        // products: A map, B map, A / B exponent buffers, output, skip
         const CUtensorMap* dm = g.dd.maps + kMaps * i;
         struct GemmDef {
             int a, b, b128, ea, eb;  // b128: the B map with 128-row boxes (-1: always full slices)
             double* C;
-            int acc;
             const int* skip;
         };
         const GemmDef gd[kGemmSets] = {
-            {0, 1, -1, 0, 0, s.b.add, 0, nullptr}, {2, 1, -1, 1, 0, s.b.tmp, 0, nullptr},
-            {2, 1, -1, 1, 0, s.b.p4, 0, nullptr},  {3, 4, 9, 2, 2, s.b.p8, 0, nullptr},
-            {5, 4, 9, 3, 2, s.b.p12, 0, nullptr},  {5, 6, 10, 3, 3, s.b.p16, 0, sk},
-            {2, 4, 9, 1, 2, s.b.iZ, 1, sk + 1},    {2, 6, 10, 1, 3, s.b.iZ, 1, sk + 2},
-            {2, 7, 11, 1, 4, s.b.iZ, 1, sk + 3},   {2, 8, 12, 1, 5, s.b.iZ, 1, sk + 4}};
+            {0, 1, -1, 0, 0, s.b.add, nullptr}, {2, 1, -1, 1, 0, s.b.tmp, nullptr}, {2, 1, -1, 1, 0, s.b.p4, nullptr},
+            {3, 4, 7, 2, 2, s.b.p8, nullptr},   {5, 4, 7, 3, 2, s.b.p12, nullptr},  {5, 6, 8, 3, 3, s.b.p16, sk}};
         for (int q = 0; q < kGemmSets; ++q) {
             const bool narrow = power_product_slices(q, g.slices) != g.slices && nt != 128;
             const int bm = narrow ? gd[q].b128 : gd[q].b;
             if (bm < 0) return bfail(UNC_ERR_UNSUPPORTED, "slice schedule and map table disagree");
             hdd.gemm[(size_t)q * n + i] = MixedGemmJob{dm + gd[q].a,   dm + bm,        N,          kp, rows, rows,
                                                        s.ex[gd[q].ea], s.ex[gd[q].eb], gd[q].C,    ld, nullptr,
-                                                       s.b.s.err,      gd[q].skip,     gd[q].acc};
+                                                       s.b.s.err,      gd[q].skip};
         }
-        PowerSet ps{};
-        ps.M[0] = s.b.Z;
-        ps.M[1] = s.b.add;
-        ps.M[2] = s.b.tmp;
-        ps.M[3] = s.b.p4;
-        ps.M[4] = s.b.p8;
-        ps.M[5] = s.b.p12;
-        ps.M[6] = s.b.p16;
-        ps.iZ = s.b.iZ;
-        ps.G = s.b.g;
-        ps.n = N;
-        ps.ld = ld;
-        ps.dmax = s.b.dmax;
-        ps.te = s.b.te;
-        hdd.powers[i] = ps;
+        hdd.powers[i] = power_set(s.pl, s.b);
         for (int it = 1; it <= kTaylorIters; ++it)
             hdd.kpow[19L * i + it - 1] = pow(s.lambda, it) / factorial_i32(it - 1);
     }

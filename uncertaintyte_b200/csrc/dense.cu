@@ -567,58 +567,53 @@ __global__ void k_shift_diag_scale(double* A, int n, long lda, double lambda, do
     shift_diag_one(A, i, lda, lambda, e, err);
 }
 
-// element idx of a column-major n x n matrix: A <- A e_r e_c (and Y = the same)
-__device__ __forceinline__ void scale_sym_one(double* A, long idx, int n, long lda, const double* __restrict__ e,
-                                              double* Y, long ldy) {
-    int c = (int)(idx / n), r = (int)(idx - (long)c * n);
-    double v = A[r + c * lda] * e[r] * e[c];
-    A[r + c * lda] = v;
-    if (Y) Y[r + c * ldy] = v;
+// Element-wise launches over an n x n matrix: blockIdx.y = first column, kScaleRows rows
+// per block (no division per element).
+constexpr int kScaleThreads = 256, kScaleRows = 4 * kScaleThreads;
+dim3 scale_grid(int n) { return dim3((unsigned)((n + kScaleRows - 1) / kScaleRows), (unsigned)std::min(n, 65535)); }
+
+// The rows r0 .. of column c: X(r, c) = S(r, c) e_r e_c (and Y the same), from row `first` on.
+__device__ __forceinline__ void scale_column(const double* S, double* X, int n, long ld, int c, int r0, int first,
+                                             const double* __restrict__ e, double* Y) {
+    const double ec = e[c];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int r = r0 + (int)threadIdx.x + u * kScaleThreads;
+        if (r < n && r >= first) {
+            const double v = S[r + c * ld] * e[r] * ec;
+            X[r + c * ld] = v;
+            if (Y) Y[r + c * ld] = v;
+        }
+    }
 }
 
-__global__ void k_scale_sym(double* A, int n, long lda, const double* __restrict__ e,
-                            double* Y, long ldy) {
-    long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    long total = (long)n * n;
-    if (idx >= total) return;
-    scale_sym_one(A, idx, n, lda, e, Y, ldy);
+// lower: the lower triangle only (all that a Cholesky factorisation reads)
+__global__ void __launch_bounds__(kScaleThreads)
+    k_scale_sym(const double* S, double* X, int n, long ld, const double* __restrict__ e, double* Y, int lower) {
+    for (int c = blockIdx.y; c < n; c += gridDim.y)
+        scale_column(S, X, n, ld, c, blockIdx.x * kScaleRows, lower ? c : 0, e, Y);
+}
+
+static void launch_scale(const double* S, double* X, int n, int lda, const double* e, double* Y, bool lower,
+                         cudaStream_t st) {
+    k_scale_sym<<<scale_grid(n), kScaleThreads, 0, st>>>(S, X, n, lda, e, Y, lower ? 1 : 0);
+    count_launch();
 }
 
 void launch_shift_equilibrate(double* A, int n, int lda, double lambda, double* e, int* err,
                               cudaStream_t st) {
     k_shift_diag_scale<<<(n + 255) / 256, 256, 0, st>>>(A, n, lda, lambda, e, err);
-    long total = (long)n * n;
-    k_scale_sym<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(A, n, lda, e, nullptr, 0);
-    count_launch(2);
-}
-
-__device__ __forceinline__ void scale_sym_from_one(const double* __restrict__ S, double* A, long idx, int n,
-                                                   long lda, const double* __restrict__ e, double* Y, long ldy) {
-    int c = (int)(idx / n), r = (int)(idx - (long)c * n);
-    double v = S[r + c * lda] * e[r] * e[c];
-    A[r + c * lda] = v;
-    if (Y) Y[r + c * ldy] = v;
-}
-
-__global__ void k_scale_sym_from(const double* __restrict__ S, double* A, int n, long lda,
-                                 const double* __restrict__ e, double* Y, long ldy) {
-    long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    long total = (long)n * n;
-    if (idx >= total) return;
-    scale_sym_from_one(S, A, idx, n, lda, e, Y, ldy);
+    count_launch();
+    launch_scale(A, A, n, lda, e, nullptr, true, st);
 }
 
 void launch_unequilibrate_from(const double* S, double* X, int n, int lda, const double* e, double* Y,
                                cudaStream_t st) {
-    long total = (long)n * n;
-    k_scale_sym_from<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(S, X, n, lda, e, Y, lda);
-    count_launch();
+    launch_scale(S, X, n, lda, e, Y, false, st);
 }
 
 void launch_unequilibrate(double* X, int n, int lda, const double* e, double* Y, cudaStream_t st) {
-    long total = (long)n * n;
-    k_scale_sym<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(X, n, lda, e, Y, lda);
-    count_launch();
+    launch_scale(X, X, n, lda, e, Y, false, st);
 }
 
 __global__ void k_axpy(double* Y, const double* __restrict__ X, double k, int n, long ld) {
@@ -668,9 +663,9 @@ __device__ __forceinline__ void te_init_one(TeState* s) {
     for (int i = 0; i < 8; ++i) s->skip[i] = 0;
 }
 
-__global__ void k_te_init(TeState* s) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    te_init_one(s);
+__global__ void k_te_init(TeState* s, unsigned long long* dmax) {
+    if (dmax && threadIdx.x < 24) dmax[threadIdx.x] = 0ULL;
+    if (threadIdx.x == 0) te_init_one(s);
 }
 
 // ---- grouped forms over the dense stages of many matrices (a batch) ----
@@ -691,18 +686,18 @@ __global__ void k_shift_diag_scale_grouped(const DenseJob* __restrict__ jobs, in
     if (i < j.n) shift_diag_one(j.Z, (int)i, j.ld, j.lambda, j.e, j.err);
 }
 
-__global__ void k_scale_sym_grouped(const DenseJob* __restrict__ jobs, int njobs, const long* __restrict__ blk) {
-    const int m = job_of_block(blk, njobs, blockIdx.x);
-    const DenseJob& j = jobs[m];
-    const long idx = (blockIdx.x - blk[m]) * (long)blockDim.x + threadIdx.x;
-    if (idx < (long)j.n * j.n) scale_sym_one(j.Z, idx, j.n, j.ld, j.e, nullptr, 0);
+// Element-wise over kScaleRows x kScaleCols pieces: block b - blk[m] of job m.
+constexpr int kScaleCols = 8;
+__host__ __device__ constexpr long scale_blocks(int n) {
+    return (long)((n + kScaleRows - 1) / kScaleRows) * ((n + kScaleCols - 1) / kScaleCols);
 }
-
-__global__ void k_unequilibrate_grouped(const DenseJob* __restrict__ jobs, int njobs, const long* __restrict__ blk) {
+__global__ void __launch_bounds__(kScaleThreads)
+    k_scale_sym_grouped(const DenseJob* __restrict__ jobs, int njobs, const long* __restrict__ blk, int back) {
     const int m = job_of_block(blk, njobs, blockIdx.x);
     const DenseJob& j = jobs[m];
-    const long idx = (blockIdx.x - blk[m]) * (long)blockDim.x + threadIdx.x;
-    if (idx < (long)j.n * j.n) scale_sym_from_one(j.add, j.Z, idx, j.n, j.ld, j.e, j.iZ, j.ld);
+    const int rows = (j.n + kScaleRows - 1) / kScaleRows, b = (int)(blockIdx.x - blk[m]);
+    for (int c = b / rows * kScaleCols; c < min(j.n, (b / rows + 1) * kScaleCols); ++c)
+        scale_column(back ? j.add : j.Z, j.Z, j.n, j.ld, c, b % rows * kScaleRows, back ? 0 : c, j.e, nullptr);
 }
 
 __global__ void k_te_init_grouped(const DenseJob* __restrict__ jobs, int njobs) {
@@ -719,16 +714,18 @@ void launch_shift_equilibrate_grouped(const DenseJob* d_jobs, int njobs, const l
                                       const long* d_blk_elems, long nblk_elems, cudaStream_t st) {
     if (njobs <= 0) return;
     k_shift_diag_scale_grouped<<<(unsigned)nblk_rows, 256, 0, st>>>(d_jobs, njobs, d_blk_rows);
-    k_scale_sym_grouped<<<(unsigned)nblk_elems, 256, 0, st>>>(d_jobs, njobs, d_blk_elems);
+    k_scale_sym_grouped<<<(unsigned)nblk_elems, kScaleThreads, 0, st>>>(d_jobs, njobs, d_blk_elems, 0);
     count_launch(2);
 }
 
 void launch_unequilibrate_grouped(const DenseJob* d_jobs, int njobs, const long* d_blk_elems, long nblk_elems,
                                   cudaStream_t st) {
     if (njobs <= 0) return;
-    k_unequilibrate_grouped<<<(unsigned)nblk_elems, 256, 0, st>>>(d_jobs, njobs, d_blk_elems);
+    k_scale_sym_grouped<<<(unsigned)nblk_elems, kScaleThreads, 0, st>>>(d_jobs, njobs, d_blk_elems, 1);
     count_launch();
 }
+
+long scale_blocks_grouped(int n) { return scale_blocks(n); }
 
 void launch_te_init_grouped(const DenseJob* d_jobs, int njobs, cudaStream_t st) {
     if (njobs <= 0) return;
@@ -742,8 +739,8 @@ void launch_te_decide_grouped(const DenseJob* d_jobs, int njobs, const double* d
     count_launch();
 }
 
-void launch_te_init(TeState* s, cudaStream_t st) {
-    k_te_init<<<1, 32, 0, st>>>(s);
+void launch_te_init(TeState* s, unsigned long long* dmax, cudaStream_t st) {
+    k_te_init<<<1, 32, 0, st>>>(s, dmax);
     count_launch();
 }
 

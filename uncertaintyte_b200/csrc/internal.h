@@ -264,81 +264,71 @@ struct TeState {
     double change[20];      // cycle_change record
     // blocked-power evaluation (powers.cu): the series' coefficients c[0] = 1,
     // c[i] = k_i for the performed iterations, 0 after; skip[0]: X^16 is not
-    // needed, skip[q] (q = 1..4): the block X^(4q) G_q is zero
+    // needed, skip[q] (q = 1..4): the terms c[4q .. 4q + 3] are all zero
     double c[20];
     int skip[8];
 };
 // One thread: change = |k * max(amax, DBL_MIN)|; stop when change < 1e-5 or
 // change > old_change, else record it and publish k for the axpy.
 void launch_te_decide(TeState* s, const unsigned long long* amax, double k, cudaStream_t st);
-// Reset the state (not done, no iteration, old change = DBL_MAX).
-void launch_te_init(TeState* s, cudaStream_t st);
+// Reset the state (not done, no iteration, old change = DBL_MAX) and the 24
+// words of dmax (optional).
+void launch_te_init(TeState* s, unsigned long long* dmax, cudaStream_t st);
 // ---------------- powers.cu ----------------
 // The Taylor series iZ = X + sum_{i=1..m} k_i X^(i+1) (compute.cpp:141-160)
-// evaluated from the powers X^2, X^3, X^4, X^8, X^12 (X^16 when m >= 15):
-// the stop rule's max|X^j| is the largest diagonal entry of the SPD power X^j,
-// the dot product of columns of two lower powers; the sum is formed in blocks
-// iZ = G_0 + X^4 G_1 + X^8 G_2 + X^12 G_3 + X^16 G_4, G_q = sum_r c_(4q+r) X^(r+1).
-// 8 products for m <= 15 instead of m + 1.
+// evaluated from the powers X^2, X^3, X^4, X^8, X^12 (X^16 when m >= 15) on the
+// camera blocks of iZ: the stop rule's max|X^j| is the largest diagonal entry of
+// the SPD power X^j, the dot product of columns of two lower powers, and the
+// camera blocks of X^(4q + r + 1) are products of nine columns of X^(4q) and
+// X^(r+1). 5 products for m <= 15 instead of m + 1.
+constexpr int kPowerPairs = 45;  // lower triangle of a 9 x 9 block
 struct PowerSet {
     double* M[7];  // X, X^2, X^3, X^4, X^8, X^12, X^16
-    double *iZ, *G;
+    double* blk;   // [camera][4 (q - 1) + r][45]: camera blocks of X^(4q) X^(r+1), q = 1..4, r = 0..3
     int n;
-    long ld;
+    long ld;       // even, the matrices 16-byte aligned
     unsigned long long* dmax;  // 21 words: max diag of X^j, j = 0..20 (bits of a non-negative double)
     TeState* te;
 };
 // Slices of the int8-sliced products of the blocked-power evaluation (mixed
-// modes with S slices). Product q: 0..5 = X^2, X^3, X^4, X^8, X^12, X^16;
-// 6..9 = X^4 G_1, X^8 G_2, X^12 G_3, X^16 G_4 (counts kept for the int8
-// product entry points; the solves form these four on the camera blocks in
-// FP64, launch_taylor_blocks). Z is positive semi-definite,
-// so the eigenvalues of X = (Z + lambda I)^-1 are at most 1/lambda and the
-// series term lambda^i / (i-1)! X^(i+1) = X (lambda X)^i / (i-1)! has norm at
-// most ||X|| / (i-1)! (32-bit factorial). G_2 (terms 8..11) therefore adds at
-// most 2.3e-4 ||X||, G_3 3e-8 and G_4 1e-8 (the factorial wraps there): their
-// products keep the absolute error of the full-slice ones with 2 and 3 slices
-// (7 bits each) fewer. X^8, X^12 and X^16 feed only those blocks and the stop
-// rule's diagonal maxima (relative error ~2^-28 with one slice fewer). The
-// digits are rounded greedily, so the first k slices of an operand are its
-// k-slice form: the same slice buffers serve every count.
-inline int power_product_slices(int q, int S) {
-    const int drop = (q >= 3 && q <= 5) ? 1 : (q == 7 ? 2 : (q >= 8 ? 3 : 0));
-    return S - drop < 2 ? (S < 2 ? S : 2) : S - drop;
-}
+// modes with S slices). Product q: 0..5 = X^2, X^3, X^4, X^8, X^12, X^16. Z is
+// positive semi-definite, so the eigenvalues of X = (Z + lambda I)^-1 are at
+// most 1/lambda and the series term lambda^i / (i-1)! X^(i+1) = X (lambda X)^i /
+// (i-1)! has norm at most ||X|| / (i-1)! (32-bit factorial): the terms past
+// X^8, which alone come from X^8, X^12 and X^16, add at most 2.3e-4 ||X||, so
+// those three take one slice (7 bits) fewer; for the stop rule's diagonal maxima
+// that is a relative error of ~2^-28. The digits are rounded greedily, so the
+// first k slices of an operand are its k-slice form: the same slice buffers
+// serve every count.
+inline int power_product_slices(int q, int S) { return q >= 3 && S > 2 ? S - 1 : S; }
 // k[i - 1] = lambda^i / factorial(i - 1), i = 1..19 (host values)
 struct TaylorCoefs {
     double k[19];
 };
-// The powers' diagonal maxima for j in [jlo, jhi] (2..16 or 17..20), unless *skip.
-void launch_power_diag(const PowerSet& ps, int jlo, int jhi, const int* skip, cudaStream_t st);
+// The camera blocks and diagonal maxima from X .. X^12 (past_15: those with
+// X^16), unless *skip; grouped: over the cameras of every set (d_blk_cols: the
+// sets' column offsets).
+void launch_power_blocks(const PowerSet& ps, bool past_15, const int* skip, cudaStream_t st);
+void launch_power_blocks_grouped(const PowerSet* d_sets, int nsets, const long* d_blk_cols, long nblk_cols, bool past_15,
+                                 cudaStream_t st);
 // The stop rule over iterations [ilo, ihi] from the diagonal maxima (a
 // non-finite one marks the state bad); the coefficients c[i] of the performed
 // iterations; after ilo..15 the X^16 skip word, after ..19 the block skip words.
 void launch_power_decide(TeState* te, const unsigned long long* dmax, const TaylorCoefs& k, int ilo, int ihi,
                          cudaStream_t st);
-// out = c[4q] X + c[4q+1] X^2 + c[4q+2] X^3 + c[4q+3] X^4 (q = 0: into iZ), unless skipped.
-void launch_power_combine(const PowerSet& ps, int q, double* out, const int* skip, cudaStream_t st);
-// The 9 x 9 camera blocks of iZ += X^(4q) G_q, q = 1..4 (skipped blocks left out);
-// grouped: over the cameras of every set (d_blk_cols: the sets' column offsets).
-void launch_taylor_blocks(const PowerSet& ps, cudaStream_t st);
-void launch_taylor_blocks_grouped(const PowerSet* d_sets, int nsets, const long* d_blk_cols, long nblk_cols,
-                                  cudaStream_t st);
-// Grouped forms over many matrices (a batch): one block per column (diag) or
-// per 256 elements (combine) of set m with blk[m] <= b < blk[m + 1].
-void launch_power_diag_grouped(const PowerSet* d_sets, int nsets, const long* d_blk_cols, long nblk, int jlo,
-                               int jhi, bool skip_if_done_early, cudaStream_t st);
 // d_k: 19 coefficients per set (set-major)
 void launch_power_decide_grouped(const PowerSet* d_sets, int nsets, const double* d_k, int ilo, int ihi,
                                  cudaStream_t st);
-void launch_power_combine_grouped(const PowerSet* d_sets, int nsets, const long* d_blk_elems, long nblk, int q,
-                                  cudaStream_t st);
+// The camera output and the unscaled 9x9 camera covariance blocks (as
+// launch_camera_output) of the series' sum.
+void launch_power_output(const PowerSet& ps, const double* s_cam, double* cam_unc, double* sig, cudaStream_t st);
 
 // Grouped dense-stage kernels over many matrices (a batch). Element-wise
 // launches: block b belongs to job m with blk[m] <= b < blk[m + 1] (blk: njobs
-// + 1 longs; 256 threads per block over the job's rows, or n^2 elements).
+// + 1 longs; 256 threads per block over the job's rows, or
+// scale_blocks_grouped(n) blocks over its elements).
 struct DenseJob {
-    double *Z, *iZ, *add, *e;  // Z (in: Schur complement, out: X), iZ (T, then X), add (O = inverse)
+    double *Z, *add, *e;  // Z (in: Schur complement, out: X), add (O = inverse)
     long ld;
     int n;
     double lambda;
@@ -349,9 +339,10 @@ struct DenseJob {
 // Z += lambda I and the symmetric equilibration of every job (as launch_shift_equilibrate).
 void launch_shift_equilibrate_grouped(const DenseJob* d_jobs, int njobs, const long* d_blk_rows, long nblk_rows,
                                       const long* d_blk_elems, long nblk_elems, cudaStream_t st);
-// Z = E add E, iZ = Z for every job (as launch_unequilibrate_from(add, Z, ..., iZ)).
+// Z = E add E for every job (as launch_unequilibrate_from(add, Z, ...)).
 void launch_unequilibrate_grouped(const DenseJob* d_jobs, int njobs, const long* d_blk_elems, long nblk_elems,
                                   cudaStream_t st);
+long scale_blocks_grouped(int n);
 void launch_te_init_grouped(const DenseJob* d_jobs, int njobs, cudaStream_t st);
 // the stop rule of every job with its coefficient d_k[m]
 void launch_te_decide_grouped(const DenseJob* d_jobs, int njobs, const double* d_k, cudaStream_t st);
@@ -367,7 +358,7 @@ void launch_camera_output(const double* iZ, int ldz, const double* s_cam, int nu
 // (kind::i8) products, with its TMA descriptor and per-row exponents.
 struct MixedOperand {
     CUtensorMap map;
-    int8_t* buf;   // slices x rows x kp bytes, zero padding
+    int8_t* buf;   // slices x rows x kp bytes, zeros past column n
     int* exps;     // n row exponents
     int n, slices, rows, kp;
 };
@@ -412,7 +403,6 @@ struct MixedGemmJob {  // one lower-triangle symmetric product C = P X (mirrored
     unsigned long long* amax;
     int* err;
     const int* skip;
-    int accumulate;  // C += P X
 };
 // block b of the launch slices row b - row_start[m] of job m (row_start: njobs + 1 ints)
 void mixed_slice_grouped(const MixedSliceJob* d_jobs, int njobs, const int* d_row_start, int total_rows,
@@ -423,8 +413,8 @@ void mixed_lower_tiles(int job, int n, int nt, std::vector<int4>& out);
 // slices; for 5, 64 or 96 by the single-scene cost model over all the tiles
 int mixed_group_tile_n(int slices, const std::vector<int>& ns);
 // A = T^T T (lower tiles, mirrored) for lower-triangular n x n T from
-// kGramSlices int8 slices of T's columns; buf holds mixed_gram_bytes(n) bytes
-// whose padding is zero, exps n + 64 ints. false: tensor-map encoding failed.
+// kGramSlices int8 slices of T's columns; buf holds mixed_gram_bytes(n) bytes,
+// exps n + 64 ints. false: tensor-map encoding failed.
 constexpr int kGramSlices = 7;
 size_t mixed_gram_bytes(int n);
 bool mixed_gram_lower_tri(const double* T, int n, int ld, int8_t* buf, int* exps, double* A, int lda, int* err,
@@ -432,15 +422,14 @@ bool mixed_gram_lower_tri(const double* T, int n, int ld, int8_t* buf, int* exps
 void mixed_gemm_grouped(int slices, int nt, const MixedGemmJob* d_jobs, const int4* d_tiles, int ntiles,
                         cudaStream_t st);
 // Y, te (optional): Y += te->coef * A while A is sliced, unless te->done.
+// lower: A is lower triangular (the elements above its diagonal are not read).
 void mixed_slice(const double* A, int lda, MixedOperand& op, cudaStream_t st, const int* skip = nullptr,
-                 double* Y = nullptr, const TeState* te = nullptr);
+                 double* Y = nullptr, const TeState* te = nullptr, bool lower = false);
 // C = P * X from the slices of P (a) and X (b); lower_only: tiles on/below the
 // diagonal; mirror: the result's lower triangle is also written transposed
 // into the upper one (a symmetric product needs no separate mirror pass).
-// accumulate: C += P X (C symmetric, with mirror) instead of C = P X.
 void mixed_gemm(const MixedOperand& a, const MixedOperand& b, double* C, int ldc, unsigned long long* amax,
-                bool lower_only, int* err, cudaStream_t st, const int* skip = nullptr, bool mirror = false,
-                bool accumulate = false);
+                bool lower_only, int* err, cudaStream_t st, const int* skip = nullptr, bool mirror = false);
 
 // ---------------- svd.cu ----------------
 // Scratch of the PSD pseudo-inverse (n x ld matrices and p x n blocks).

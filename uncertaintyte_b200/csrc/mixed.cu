@@ -151,38 +151,69 @@ struct Shape {
 
 using namespace mp;
 
-// Slice rows of a symmetric FP64 matrix (row j = column j, contiguous) into S
-// int8 planes out[s][j][k] (pitch kp bytes, plane stride rows_pad * kp) of
-// round-to-nearest digits in [-64, 64], and the row exponents e[j] with
-// max_k |A[j,k]| 2^-e < 1/2. One CTA per row.
 // 2^e exactly (bit pattern for normal exponents): v * pow2(e) == ldexp(v, e)
 __device__ __forceinline__ double pow2(int e) {
     return (e >= -1022 && e <= 1023) ? __longlong_as_double((long long)(e + 1023) << 52) : ldexp(1.0, e);
 }
 
+// Slice rows of a symmetric FP64 matrix (row j = column j, contiguous) into S
+// int8 planes out[s][j][k] (pitch kp bytes, plane stride rows_pad * kp) of
+// round-to-nearest digits in [-64, 64], and the row exponents e[j] with
+// max_k |A[j,k]| 2^-e < 1/2. One CTA of 256 threads per row; the row's padding
+// up to kp is written as zeros (the K padding of the products; padding rows stay
+// as they are: they only reach results that are not stored). lower: the matrix is
+// lower triangular, so row j starts at k = j (zeros before it from the products'
+// first k on, a multiple of 128).
+// Digit s of x, |x| < 1/2, is rint of its remainder in units of 2^-7s: adding
+// 1.5 2^(52 - 7s) rounds the remainder to that unit (to nearest, ties to even)
+// and leaves the digit in the sum's low bits, so a digit is three additions and
+// no conversion; the row stays in registers between its maximum and its digits
+// up to kSliceKept elements. n = 1800, five slices: 19 -> 8 us.
 // Y (optional): Y += te->coef * A on the way (the Taylor update iZ += k add of
-// the power being sliced, compute.cpp:64-71), unless te->done.
-// Row j of one matrix, all 256 threads of the block (red: 8 shared doubles).
+// the power being sliced, compute.cpp:64-71).
+constexpr int kSlicePasses = 4;  // 1024 elements each
 __device__ __forceinline__ void slice_row(int j, const double* __restrict__ A, long lda, int n, int S,
                                           int8_t* __restrict__ out, int rows_pad, int kp, int* __restrict__ exps,
-                                          double* Y, const TeState* te, double* red) {
+                                          double* Y, const TeState* te, bool lower, double* red) {
     const double* col = A + (long)j * lda;
-    double m = 0.0;
-    for (int k = threadIdx.x; k < n; k += 256) m = fmax(m, fabs(col[k]));
+    const bool wide = (reinterpret_cast<uintptr_t>(col) & 15) == 0;
+    const int first = lower ? j : 0, start = lower ? j / 128 * 128 : 0;
+    const int k_at = start + 4 * threadIdx.x;
+    auto load = [&](int k, double (&v)[4]) {
+        if (wide && k >= first && k + 3 < n) {
+            const double2 x = *reinterpret_cast<const double2*>(col + k), y = *reinterpret_cast<const double2*>(col + k + 2);
+            v[0] = x.x;
+            v[1] = x.y;
+            v[2] = y.x;
+            v[3] = y.y;
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = k + u >= first && k + u < n ? col[k + u] : 0.0;
+        }
+    };
+    double kept[kSlicePasses][4], m = 0.0;
+#pragma unroll
+    for (int p = 0; p < kSlicePasses; ++p) {
+        load(k_at + 1024 * p, kept[p]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) m = fmax(m, fabs(kept[p][u]));
+    }
+    for (int k = k_at + 1024 * kSlicePasses; k < n; k += 1024) {
+        double v[4];
+        load(k, v);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) m = fmax(m, fabs(v[u]));
+    }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, d));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
-    if (threadIdx.x < 32) {
-        double v = threadIdx.x < 8 ? red[threadIdx.x] : 0.0;
+    m = red[0];
 #pragma unroll
-        for (int d = 4; d > 0; d >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, d));
-        if (threadIdx.x == 0) red[0] = v;
-    }
-    __syncthreads();
+    for (int w = 1; w < 8; ++w) m = fmax(m, red[w]);
     int e = 0;
-    if (red[0] > 0.0 && red[0] <= 1.7976931348623157e308) frexp(red[0], &e);  // max * 2^-e in [0.5, 1)
-    e += 1;                                                                     // max * 2^-e in [0.25, 0.5)
+    if (m > 0.0 && m <= 1.7976931348623157e308) frexp(m, &e);  // max * 2^-e in [0.5, 1)
+    e += 1;                                                     // max * 2^-e in [0.25, 0.5)
     if (threadIdx.x == 0) exps[j] = e;
     if (Y) {
         const double c = te->coef;
@@ -192,40 +223,39 @@ __device__ __forceinline__ void slice_row(int j, const double* __restrict__ A, l
     const double sc = pow2(-e);
     const size_t plane = (size_t)rows_pad * kp;
     int8_t* row = out + (size_t)j * kp;
-    for (int k0 = 4 * threadIdx.x; k0 < n; k0 += 4 * 256) {
-        double v[4];
+    auto digits = [&](int k, double (&v)[4]) {
+        if (k >= kp) return;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = (k0 + u < n) ? col[k0 + u] * sc : 0.0;
+        for (int u = 0; u < 4; ++u) v[u] *= sc;
+        double unit = 1.5 * 35184372088832.0;  // 1.5 2^45
         for (int s = 0; s < S; ++s) {
-            char4 q;
-            signed char qs[4];
+            unsigned word = 0;
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                v[u] *= 128.0;
-                const double t = rint(v[u]);  // |v| <= 64 before, |v - t| <= 1/2 after
-                v[u] -= t;
-                qs[u] = (signed char)(int)t;
+                const double r = v[u] + unit;
+                v[u] -= r - unit;
+                word |= ((unsigned)__double2loint(r) & 0xffu) << (8 * u);
             }
-            q.x = qs[0];
-            q.y = qs[1];
-            q.z = qs[2];
-            q.w = qs[3];
-            if (k0 + 3 < n) {
-                *reinterpret_cast<char4*>(row + s * plane + k0) = q;
-            } else {
-                for (int u = 0; u < 4 && k0 + u < n; ++u) row[s * plane + k0 + u] = qs[u];
-            }
+            *reinterpret_cast<unsigned*>(row + s * plane + k) = word;
+            unit *= 1.0 / 128.0;
         }
+    };
+#pragma unroll
+    for (int p = 0; p < kSlicePasses; ++p) digits(k_at + 1024 * p, kept[p]);
+    for (int k = k_at + 1024 * kSlicePasses; k < kp; k += 1024) {
+        double v[4];
+        load(k, v);
+        digits(k, v);
     }
 }
 
 __global__ void __launch_bounds__(256) k_slice_rows(const double* __restrict__ A, long lda, int n, int S,
                                                    int8_t* __restrict__ out, int rows_pad, int kp,
                                                    int* __restrict__ exps, const int* skip, double* Y,
-                                                   const TeState* te) {
+                                                   const TeState* te, int lower) {
     if (skip && *skip) return;
     __shared__ double red[8];
-    slice_row(blockIdx.x, A, lda, n, S, out, rows_pad, kp, exps, Y, te, red);
+    slice_row(blockIdx.x, A, lda, n, S, out, rows_pad, kp, exps, Y, te, lower != 0, red);
 }
 
 // The same over the rows of many matrices (a batch): block b slices row
@@ -241,7 +271,7 @@ __global__ void __launch_bounds__(256) k_slice_rows_grouped(const MixedSliceJob*
     const MixedSliceJob& jb = jobs[lo];
     if (jb.skip && *jb.skip) return;
     __shared__ double red[8];
-    slice_row(b - row_start[lo], jb.A, jb.lda, jb.n, jb.S, jb.out, jb.rows_pad, jb.kp, jb.exps, jb.Y, jb.te, red);
+    slice_row(b - row_start[lo], jb.A, jb.lda, jb.n, jb.S, jb.out, jb.rows_pad, jb.kp, jb.exps, jb.Y, jb.te, false, red);
 }
 
 // One 128 x NT output tile at (m0, n0): TMA producer, MMA issuer, epilogue.
@@ -252,7 +282,7 @@ __device__ __forceinline__ void ozaki_tile(const CUtensorMap* tA, const CUtensor
                                            int kp, int rowsA, int rowsB, const int* __restrict__ eA,
                                            const int* __restrict__ eB, double* C, long ldc,
                                            unsigned long long* amax, int* err, int mirror, bool maps_in_global,
-                                           int accumulate, int klo = 0) {
+                                           int klo = 0) {
     using Sh = Shape<NT, S>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -365,14 +395,6 @@ __device__ __forceinline__ void ozaki_tile(const CUtensorMap* tA, const CUtensor
             int r[S][16];
 #pragma unroll
             for (int l = 0; l < S; ++l) tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(l * NT + c0), r[l]);
-            // accumulate: the previous values of C, loaded together before any store of
-            // this chunk (reads are of the lower triangle, mirrored stores go above it)
-            double prev[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const int col = n0 + c0 + j;
-                prev[j] = accumulate && row < M && col < N && (!mirror || row >= col) ? C[row + (long)col * ldc] : 0.0;
-            }
             tmem_wait_ld();
 #pragma unroll
             for (int l = 0; l < S; ++l) tmem_fence_regs(r[l]);
@@ -385,23 +407,33 @@ __device__ __forceinline__ void ozaki_tile(const CUtensorMap* tA, const CUtensor
 #pragma unroll
                 for (int j = 0; j < 16; ++j) v[j] += (double)r[l][j] * w;
             }
+            // mirror: the lower triangle is written at (row, col) and at (col, row);
+            // nothing above the diagonal is written directly
             if (row < M) {
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                     const int col = n0 + c0 + j;
                     if (col < N) {
-                        double x = v[j] * pow2(er + eB[col]);
-                        // mirror: the lower triangle is written at (row, col) and at
-                        // (col, row); nothing above the diagonal is written directly
-                        // accumulate: C += P X (C symmetric: its lower element is read)
-                        if (accumulate && (!mirror || row >= col)) x += prev[j];
+                        v[j] *= pow2(er + eB[col]);
                         if (!mirror || row >= col) {
-                            C[row + (long)col * ldc] = x;
-                            const double ax = fabs(x);
+                            C[row + (long)col * ldc] = v[j];
+                            const double ax = fabs(v[j]);
                             mx = fmax(mx, ax <= 1.7976931348623157e308 ? ax
                                                                        : __longlong_as_double(0x7ff0000000000000LL));
                         }
-                        if (mirror && row > col) C[col + (long)row * ldc] = x;
+                    }
+                }
+                if (mirror) {  // this lane's 16 columns are consecutive in the mirrored column
+                    const int col = n0 + c0;
+                    double* up = C + col + (long)row * ldc;
+                    if (row > col + 15 && ((reinterpret_cast<uintptr_t>(up) & 15) == 0)) {
+#pragma unroll
+                        for (int j = 0; j < 16; j += 2)
+                            *reinterpret_cast<double2*>(up + j) = make_double2(v[j], v[j + 1]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (row > col + j && col + j < N) up[j] = v[j];
                     }
                 }
             }
@@ -447,7 +479,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     k_ozaki_gemm(const __grid_constant__ CUtensorMap tA, const __grid_constant__ CUtensorMap tB, int M, int N,
                  int kp, int rowsA, int rowsB, const int* __restrict__ eA, const int* __restrict__ eB, double* C,
                  long ldc, unsigned long long* amax, int lower_only, int* err, const int* skip, int mirror,
-                 int accumulate, int group_m, int klo) {
+                 int group_m, int klo) {
     if (skip && *skip) return;
     int m0, n0;
     if (group_m > 0) {  // 1-D grid over exactly the lower tiles, grouped order
@@ -461,8 +493,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         n0 = blockIdx.x * NT;
         if (lower_only && n0 > m0 + BM - 1) return;
     }
-    ozaki_tile<NT, S>(&tA, &tB, m0, n0, M, N, kp, rowsA, rowsB, eA, eB, C, ldc, amax, err, mirror, false,
-                      accumulate, klo);
+    ozaki_tile<NT, S>(&tA, &tB, m0, n0, M, N, kp, rowsA, rowsB, eA, eB, C, ldc, amax, err, mirror, false, klo);
 }
 
 // The products of many matrices (a batch) in one launch: CTA b computes tile
@@ -476,7 +507,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const MixedGemmJob& j = jobs[t.x];
     if (j.skip && *j.skip) return;
     ozaki_tile<NT, S>(j.tA, j.tB, t.y, t.z, j.n, j.n, j.kp, j.rowsA, j.rowsB, j.eA, j.eB, j.C, j.ldc, j.amax, j.err,
-                      1, true, j.accumulate);
+                      1, true);
 }
 
 // ------------------------------------------------------------------------
@@ -687,8 +718,9 @@ void mixed_gemm_grouped(int slices, int nt, const MixedGemmJob* d_jobs, const in
 }
 
 void mixed_slice(const double* A, int lda, MixedOperand& op, cudaStream_t st, const int* skip, double* Y,
-                 const TeState* te) {
-    k_slice_rows<<<op.n, 256, 0, st>>>(A, lda, op.n, op.slices, op.buf, op.rows, op.kp, op.exps, skip, Y, te);
+                 const TeState* te, bool lower) {
+    k_slice_rows<<<op.n, 256, 0, st>>>(A, lda, op.n, op.slices, op.buf, op.rows, op.kp, op.exps, skip, Y, te,
+                                       lower ? 1 : 0);
     count_launch();
 }
 
@@ -702,7 +734,7 @@ static int group_rows_for(int n, int slices) {
 
 template <int NT, int S>
 static void launch_ozaki(const MixedOperand& a, const MixedOperand& b, double* C, int ldc, unsigned long long* amax,
-                         bool lower_only, int* err, cudaStream_t st, const int* skip, bool mirror, bool accumulate,
+                         bool lower_only, int* err, cudaStream_t st, const int* skip, bool mirror,
                          bool klo = false) {
     set_attr_once<NT, S>();
     const int n = a.n;
@@ -710,23 +742,23 @@ static void launch_ozaki(const MixedOperand& a, const MixedOperand& b, double* C
     dim3 grid = gm > 0 ? dim3((unsigned)lower_tiles(n, NT), 1) : dim3((n + NT - 1) / NT, (n + BM - 1) / BM);
     k_ozaki_gemm<NT, S><<<grid, THREADS, Shape<NT, S>::SMEM, st>>>(a.map, b.map, n, n, a.kp, a.rows, b.rows, a.exps,
                                                                    b.exps, C, ldc, amax, lower_only ? 1 : 0, err,
-                                                                   skip, mirror ? 1 : 0, accumulate ? 1 : 0, gm,
+                                                                   skip, mirror ? 1 : 0, gm,
                                                                    klo ? 1 : 0);
 }
 
 void mixed_gemm(const MixedOperand& a, const MixedOperand& b, double* C, int ldc, unsigned long long* amax,
-                bool lower_only, int* err, cudaStream_t st, const int* skip, bool mirror, bool accumulate) {
+                bool lower_only, int* err, cudaStream_t st, const int* skip, bool mirror) {
     const int n = a.n;
     if (a.slices == 4)
-        launch_ozaki<128, 4>(a, b, C, ldc, amax, lower_only, err, st, skip, mirror, accumulate);
+        launch_ozaki<128, 4>(a, b, C, ldc, amax, lower_only, err, st, skip, mirror);
     else if (a.slices == 5 && mixed_tile_n(5, n) == 64)
-        launch_ozaki<64, 5>(a, b, C, ldc, amax, lower_only, err, st, skip, mirror, accumulate);
+        launch_ozaki<64, 5>(a, b, C, ldc, amax, lower_only, err, st, skip, mirror);
     else if (a.slices == 5)
-        launch_ozaki<96, 5>(a, b, C, ldc, amax, lower_only, err, st, skip, mirror, accumulate);
+        launch_ozaki<96, 5>(a, b, C, ldc, amax, lower_only, err, st, skip, mirror);
     else if (a.slices == 3)
-        launch_ozaki<128, 3>(a, b, C, ldc, amax, lower_only, err, st, skip, mirror, accumulate);
+        launch_ozaki<128, 3>(a, b, C, ldc, amax, lower_only, err, st, skip, mirror);
     else
-        launch_ozaki<128, 2>(a, b, C, ldc, amax, lower_only, err, st, skip, mirror, accumulate);
+        launch_ozaki<128, 2>(a, b, C, ldc, amax, lower_only, err, st, skip, mirror);
     count_launch();
 }
 
@@ -739,14 +771,14 @@ size_t mixed_gram_bytes(int n) {
 // A^{-1} = L^{-T} L^{-1}): the columns of T sliced into kGramSlices int8
 // planes, lower 128 x 64 tiles, each tile's K loop from max(m0, n0) (the rows
 // above are zero in both of its columns), the result mirrored. buf: the
-// slice planes (mixed_gram_bytes(n)); its K and row padding must be zero.
+// slice planes (mixed_gram_bytes(n)).
 bool mixed_gram_lower_tri(const double* T, int n, int ld, int8_t* buf, int* exps, double* A, int lda, int* err,
                           cudaStream_t st) {
     MixedOperand a, b;
     if (!mixed_plan_nt(a, buf, exps, n, kGramSlices, false, 64) || !mixed_plan_nt(b, buf, exps, n, kGramSlices, true, 64))
         return false;
-    mixed_slice(T, ld, a, st);
-    launch_ozaki<64, kGramSlices>(a, b, A, lda, nullptr, true, err, st, nullptr, true, false, true);
+    mixed_slice(T, ld, a, st, nullptr, nullptr, nullptr, true);
+    launch_ozaki<64, kGramSlices>(a, b, A, lda, nullptr, true, err, st, nullptr, true, true);
     count_launch();
     return true;
 }

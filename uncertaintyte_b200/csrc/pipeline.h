@@ -16,7 +16,8 @@ struct Buffers {
     double *cam_out, *pt_out;
     SceneDev s;
     double *Z, *iZ, *add, *tmp, *e, *sig;
-    double *p4, *p8, *p12, *p16, *g;   // blocked-power Taylor evaluation: X^4, X^8, X^12, X^16, G_q
+    double *p4, *p8, *p12, *p16;       // blocked-power Taylor evaluation: X^4, X^8, X^12, X^16
+    double* pblk;                      // and the camera blocks of its products (PowerSet::blk)
     unsigned long long* dmax;          // 24 words: the powers' diagonal maxima
     int* dag_state;  // counters of the tile-task inverse
     unsigned long long* amax;
@@ -43,9 +44,12 @@ int grow_buffer(void** p, size_t* have, size_t need, size_t want, cudaStream_t s
 int sparse_stage(const unc_options* o, const Plan& pl, long long nnz, const int* rows, const int* cols,
                  const double* vals, Buffers& b, int fx[3], cudaEvent_t* ev, cudaStream_t sm);
 
-// The camera outputs (removeScaleJ4Z, compute.cpp:168-183) from iZ and the
-// point covariances (compute.cpp:370-455, 517-527) into cam_out / pt_out.
-void output_stage(const Plan& pl, Buffers& b, double* cam_out, double* pt_out, cudaStream_t sm);
+// The blocked-power evaluation over the workspace's matrices.
+PowerSet power_set(const Plan& pl, const Buffers& b);
+// The camera outputs (removeScaleJ4Z, compute.cpp:168-183) from the powers or
+// from iZ and the point covariances (compute.cpp:370-455, 517-527) into cam_out /
+// pt_out.
+void output_stage(const Plan& pl, Buffers& b, bool powers, double* cam_out, double* pt_out, cudaStream_t sm);
 
 // The automatic lambda of teInverse (compute.cpp:124-125) for N camera parameters.
 double auto_lambda(int N);

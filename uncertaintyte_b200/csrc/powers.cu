@@ -10,17 +10,16 @@
 //     of X^a and of X^b. From X, X^2, X^3, X^4, X^8, X^12 (and X^16) every
 //     j = 2..20 is such a pair, so the stop rule runs on the device from
 //     O(N^2) column dot products;
-//   * the sum is taken in blocks of four coefficients,
-//       iZ = G_0 + X^4 G_1 + X^8 G_2 + X^12 G_3 + X^16 G_4,
-//       G_q = c_4q X + c_(4q+1) X^2 + c_(4q+2) X^3 + c_(4q+3) X^4,
-//     with c_0 = 1, c_i = k_i for the performed iterations and 0 after; the
-//     blocks whose coefficients are all zero are skipped on the device.
+//   * only the 9 x 9 diagonal camera blocks of iZ are read after the series (the
+//     camera output, compute.cpp:168-183, and the point stage's block-diagonal
+//     camera covariance, compute.cpp:422-441), and the camera blocks of
+//     X^(4q + r + 1), q = 1..4, r = 0..3, are products of 9 columns of X^(4q)
+//     and of X^(r+1): formed once, they give both the diagonal entries of the
+//     stop rule and, with the coefficients that it decides (c_0 = 1, c_i = k_i
+//     for the performed iterations and 0 after), the sum.
 // Products: X^2, X^3, X^4, X^8, X^12 (X^16 past 15 iterations): 5 for the
-// 12..15 iterations of the reference scenes, instead of 13..16. The block
-// terms X^(4q) G_q are formed on the 9 x 9 camera blocks of iZ only, the only
-// part of iZ read afterwards (k_taylor_blocks: 81 N multiply-adds per camera
-// and block instead of a full product). The polynomial, its coefficients and
-// the stop decisions are the reference's;
+// 12..15 iterations of the reference scenes, instead of 13..16. The
+// polynomial, its coefficients and the stop decisions are the reference's;
 // the results differ from the one-product-per-iteration order at the
 // rounding level. Every kernel here has a fixed summation order, so the
 // results are bitwise repeatable.
@@ -31,65 +30,130 @@
 namespace unc {
 namespace {
 
-// diag(X^j) = dot of the columns of slots slot_a(j), slot_b(j): slots 0..3 =
-// X..X^4, 4 = X^8, 5 = X^12, 6 = X^16 (j = 2..20)
-__host__ __device__ constexpr int slot_a(int j) {
-    return j == 2 || j == 3 ? 0 : (j == 4 ? 1 : (j <= 8 ? j - 5 : (j - 9) % 4));
-}
-__host__ __device__ constexpr int slot_b(int j) {
-    return j == 2 ? 0 : (j <= 4 ? 1 : (j <= 8 ? 3 : (j <= 12 ? 4 : (j <= 16 ? 5 : 6))));
-}
-static_assert(slot_a(2) == 0 && slot_b(2) == 0 && slot_a(3) == 0 && slot_b(3) == 1 && slot_a(4) == 1 &&
-                  slot_b(4) == 1 && slot_a(5) == 0 && slot_b(5) == 3 && slot_a(8) == 3 && slot_a(9) == 0 &&
-                  slot_b(9) == 4 && slot_a(16) == 3 && slot_b(16) == 5 && slot_a(20) == 3 && slot_b(20) == 6,
-              "power pairs");
+constexpr int kBlkThreads = 256;
+constexpr int kBlkPairs = kPowerPairs;
 
-constexpr int kDiagThreads = 256;
+// Element p = r (r + 1) / 2 + s of a lower triangle.
+__device__ __forceinline__ void lower_pair(int p, int& r, int& s) {
+    r = 0;
+    s = p;
+    while (s > r) s -= ++r;
+}
 
-// The diagonal entries c of X^j, j in [JLO, JHI], into dmax (max over c of the
-// non-negative values; a non-finite value becomes +inf). One block per column.
-template <int JLO, int JHI>
-__device__ __forceinline__ void power_diag_column(const PowerSet& ps, int c, double (*red)[JHI - JLO + 1]) {
-    constexpr int NJ = JHI - JLO + 1;
-    const long off = (long)c * ps.ld;
-    double acc[NJ];
+// The camera's blocks of X^(4q) X^(r+1) for q in [Q0, Q0 + NQ) and r = 0..3,
+// lower triangles, into ps.blk; their diagonals, and with Q0 = 1 those of X^2,
+// X^3, X^4, into the maxima ps.dmax (over the non-negative values; a non-finite
+// one becomes +inf). One CTA per camera, eight warps: warp (r, half) takes the
+// columns of X^(r+1) over half of the rows against those of the NQ powers: a DMMA
+// per power for the leading 8 x 8 part, ordinary multiply-adds for row 8. A
+// lane's 16-byte load holds the rows k = 8 j + 2 t and the next, which go to two
+// DMMA steps. Reading every power once bounds the kernel (the six or seven
+// matrices of the series; they were read three times when the diagonals, the
+// first four terms and the blocks were kernels of their own: 126 us at n = 1800).
+template <int Q0, int NQ>
+__device__ __forceinline__ void power_blocks(const PowerSet& ps, int cam, double (*red)[4][NQ][kBlkPairs],
+                                             double (*dia)[3][9], unsigned long long* top) {
+    const int n = ps.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int r = warp & 3, half = warp >> 2;
+    const long ld = ps.ld, c0 = 9L * cam;
+    const int steps = (n + 7) / 8, s0 = half ? steps / 2 : 0, s1 = half ? steps : steps / 2;
+    const double* const A = ps.M[r] + c0 * ld;
+    double c[NQ][2], row[NQ], corner[NQ], d[2][2];  // d: diagonals of X X (X^2 X^2 in warp r = 1) and X X^2
 #pragma unroll
-    for (int q = 0; q < NJ; ++q) acc[q] = 0.0;
-    for (int r = threadIdx.x; r < ps.n; r += kDiagThreads) {
-        double v[7];
+    for (int q = 0; q < NQ; ++q) c[q][0] = c[q][1] = row[q] = corner[q] = 0.0;
+    d[0][0] = d[0][1] = d[1][0] = d[1][1] = 0.0;
+    auto load = [&](const double* M, int col, int k) {
+        double2 v = make_double2(0.0, 0.0);
+        if (k + 1 < n) v = *reinterpret_cast<const double2*>(M + col * ld + k);
+        else if (k < n) v.x = M[col * ld + k];
+        return v;
+    };
+    for (int s = s0; s < s1; ++s) {
+        const int k = 8 * s + 2 * t;
+        const double2 a = load(A, g, k), a8 = load(A, 8, k);
+        double2 b[NQ], b8[NQ];
 #pragma unroll
-        for (int s = 0; s < 7; ++s) {
-            bool used = false;
-#pragma unroll
-            for (int j = JLO; j <= JHI; ++j) used |= (slot_a(j) == s) | (slot_b(j) == s);
-            v[s] = used ? ps.M[s][off + r] : 0.0;
+        for (int q = 0; q < NQ; ++q) {
+            const double* B = ps.M[Q0 + q + 2] + c0 * ld;
+            b[q] = load(B, g, k);
+            b8[q] = load(B, 8, k);
         }
 #pragma unroll
-        for (int j = JLO; j <= JHI; ++j) acc[j - JLO] += v[slot_a(j)] * v[slot_b(j)];
+        for (int q = 0; q < NQ; ++q) {
+            asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                         : "+d"(c[q][0]), "+d"(c[q][1])
+                         : "d"(a.x), "d"(b[q].x));
+            asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                         : "+d"(c[q][0]), "+d"(c[q][1])
+                         : "d"(a.y), "d"(b[q].y));
+            row[q] = fma(a8.y, b[q].y, fma(a8.x, b[q].x, row[q]));
+            corner[q] = fma(a8.y, b8[q].y, fma(a8.x, b8[q].x, corner[q]));
+        }
+        if (Q0 == 1 && r < 2) {
+            d[0][0] = fma(a.y, a.y, fma(a.x, a.x, d[0][0]));
+            d[0][1] = fma(a8.y, a8.y, fma(a8.x, a8.x, d[0][1]));
+            if (r == 0) {
+                const double2 x = load(ps.M[1] + c0 * ld, g, k), x8 = load(ps.M[1] + c0 * ld, 8, k);
+                d[1][0] = fma(a.y, x.y, fma(a.x, x.x, d[1][0]));
+                d[1][1] = fma(a8.y, x8.y, fma(a8.x, x8.x, d[1][1]));
+            }
+        }
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int q = 0; q < NJ; ++q) {
-        double a = acc[q];
+    for (int m = 1; m < 4; m <<= 1) {
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) a += __shfl_xor_sync(0xffffffffu, a, d);
-        if (lane == 0) red[warp][q] = a;
+        for (int q = 0; q < NQ; ++q) {
+            row[q] += __shfl_xor_sync(0xffffffffu, row[q], m);
+            corner[q] += __shfl_xor_sync(0xffffffffu, corner[q], m);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) d[i][j] += __shfl_xor_sync(0xffffffffu, d[i][j], m);
     }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        double* out = red[half][r][q];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (2 * t + h <= g) out[g * (g + 1) / 2 + 2 * t + h] = c[q][h];
+        if (t == 0) out[36 + g] = row[q];
+        if (lane == 0) out[44] = corner[q];
+    }
+    if (Q0 == 1 && r < 2 && t == 0) {  // rows of dia: X^2, X^3 (both from warp r = 0), X^4
+        dia[half][r == 0 ? 0 : 2][g] = d[0][0];
+        if (r == 0) dia[half][1][g] = d[1][0];
+        if (g == 0) {
+            dia[half][r == 0 ? 0 : 2][8] = d[0][1];
+            if (r == 0) dia[half][1][8] = d[1][1];
+        }
+    }
+    if (tid < 32) top[tid] = 0ULL;
     __syncthreads();
-    if (threadIdx.x < NJ) {
-        double t = 0.0;
-#pragma unroll
-        for (int w = 0; w < kDiagThreads / 32; ++w) t += red[w][threadIdx.x];
-        const double v = (t <= DBL_MAX) ? fmax(t, 0.0) : __longlong_as_double(0x7ff0000000000000LL);  // NaN -> inf
-        atomicMax(ps.dmax + JLO + threadIdx.x, (unsigned long long)__double_as_longlong(v));
+    auto fold = [&](int j, double v) {  // a diagonal entry of X^j
+        v = v <= DBL_MAX ? fmax(v, 0.0) : __longlong_as_double(0x7ff0000000000000LL);  // NaN -> inf
+        atomicMax(top + j, (unsigned long long)__double_as_longlong(v));
+    };
+    for (int e = tid; e < NQ * 4 * kBlkPairs; e += kBlkThreads) {
+        const int p = e % kBlkPairs, rr = e / kBlkPairs % 4, q = e / (4 * kBlkPairs);
+        const double v = red[0][rr][q][p] + red[1][rr][q][p];
+        ps.blk[((long)cam * 16 + 4 * (Q0 - 1 + q) + rr) * kBlkPairs + p] = v;
+        int i, j;
+        lower_pair(p, i, j);
+        if (i == j) fold(4 * (Q0 + q) + rr + 1, v);
     }
+    if (Q0 == 1 && tid < 27) fold(2 + tid / 9, dia[0][tid / 9][tid % 9] + dia[1][tid / 9][tid % 9]);
+    __syncthreads();
+    constexpr int jlo = Q0 == 1 ? 2 : 4 * Q0 + 1, jhi = 4 * (Q0 + NQ);
+    if (tid <= jhi - jlo) atomicMax(ps.dmax + jlo + tid, top[jlo + tid]);
 }
 
-template <int JLO, int JHI>
-__global__ void __launch_bounds__(kDiagThreads) k_power_diag(PowerSet ps, const int* skip) {
+template <int Q0, int NQ>
+__global__ void __launch_bounds__(kBlkThreads, 2) k_power_blocks(PowerSet ps, const int* skip) {
+    __shared__ double red[2][4][NQ][kBlkPairs], dia[2][3][9];
+    __shared__ unsigned long long top[32];
     if (skip && *skip) return;
-    __shared__ double red[kDiagThreads / 32][JHI - JLO + 1];
-    power_diag_column<JLO, JHI>(ps, blockIdx.x, red);
+    power_blocks<Q0, NQ>(ps, blockIdx.x, red, dia, top);
 }
 
 __device__ __forceinline__ int set_of_block(const long* __restrict__ blk, int nsets, long b) {
@@ -101,14 +165,17 @@ __device__ __forceinline__ int set_of_block(const long* __restrict__ blk, int ns
     return lo;
 }
 
-template <int JLO, int JHI>
-__global__ void __launch_bounds__(kDiagThreads) k_power_diag_grouped(const PowerSet* __restrict__ sets, int nsets,
-                                                                      const long* __restrict__ blk, int skip_done) {
-    const int m = set_of_block(blk, nsets, blockIdx.x);
+// The same over the cameras of many sets: cols holds the sets' column offsets
+// (multiples of 9), so set m owns the cameras [cols[m] / 9, cols[m + 1] / 9).
+template <int Q0, int NQ>
+__global__ void __launch_bounds__(kBlkThreads, 2)
+    k_power_blocks_grouped(const PowerSet* __restrict__ sets, int nsets, const long* __restrict__ cols) {
+    __shared__ double red[2][4][NQ][kBlkPairs], dia[2][3][9];
+    __shared__ unsigned long long top[32];
+    const int m = set_of_block(cols, nsets, 9L * blockIdx.x);
     const PowerSet ps = sets[m];
-    if (skip_done && ps.te->skip[0]) return;
-    __shared__ double red[kDiagThreads / 32][JHI - JLO + 1];
-    power_diag_column<JLO, JHI>(ps, (int)(blockIdx.x - blk[m]), red);
+    if (Q0 > 1 && ps.te->skip[0]) return;
+    power_blocks<Q0, NQ>(ps, (int)(blockIdx.x - cols[m] / 9), red, dia, top);
 }
 
 // The reference's stop rule (compute.cpp:145-155) over iterations ilo..ihi.
@@ -144,166 +211,62 @@ __global__ void k_power_decide_grouped(const PowerSet* __restrict__ sets, int ns
     if (m < nsets) power_decide_one(sets[m].te, sets[m].dmax, k + 19L * m, ilo, ihi);
 }
 
-// out(idx) = c[4q] X + c[4q+1] X^2 + c[4q+2] X^3 + c[4q+3] X^4 (element idx of the n x n matrix)
-__device__ __forceinline__ void power_combine_one(const PowerSet& ps, int q, double* out, long idx) {
-    const int col = (int)(idx / ps.n), r = (int)(idx - (long)col * ps.n);
-    const long o = r + col * ps.ld;
-    const double* c = ps.te->c + 4 * q;
-    double v = c[0] * ps.M[0][o];
-    v += c[1] * ps.M[1][o];
-    v += c[2] * ps.M[2][o];
-    v += c[3] * ps.M[3][o];
-    out[o] = v;
-}
-
-__global__ void k_power_combine(PowerSet ps, int q, double* out, const int* skip) {
-    if (skip && *skip) return;
-    const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (idx < (long)ps.n * ps.n) power_combine_one(ps, q, out, idx);
-}
-
-__global__ void k_power_combine_grouped(const PowerSet* __restrict__ sets, int nsets, const long* __restrict__ blk,
-                                        int q) {
-    const int m = set_of_block(blk, nsets, blockIdx.x);
-    const PowerSet& ps = sets[m];
-    if (q > 0 && ps.te->skip[q]) return;
-    const long idx = (blockIdx.x - blk[m]) * (long)blockDim.x + threadIdx.x;
-    if (idx < (long)ps.n * ps.n) power_combine_one(ps, q, q == 0 ? ps.iZ : ps.G, idx);
-}
-
-// The camera blocks of iZ += X^(4q) G_q, q = 1..4 (blocks whose skip word is
-// set left out). Only the 9 x 9 diagonal camera blocks of iZ are read after
-// the series (the camera output, compute.cpp:168-183, and the point stage's
-// block-diagonal camera covariance, compute.cpp:422-441), so these products
-// are formed on those blocks only: element (r, c) of camera block b, r >= c,
-// is sum_k G_q(k, r) X^(4q)(k, c) with G_q(k, r) = c_4q X + c_(4q+1) X^2 +
-// c_(4q+2) X^3 + c_(4q+3) X^4 at (k, r) (G_q and the powers are symmetric,
-// so their columns are their rows), added to iZ(r, c) in the order q = 1..4
-// and written at (r, c) and (c, r). One CTA per camera; each thread sums a
-// fixed stride of k, the partial sums are added in a fixed tree and warp
-// order, so the result is bitwise repeatable.
-constexpr int kBlkThreads = 128;
-constexpr int kBlkPairs = 45;  // lower triangle of a 9 x 9 block
-
-__device__ __forceinline__ void taylor_camera_block(const PowerSet& ps, int cam, double (*red)[kBlkPairs],
-                                                    double* val) {
-    const long ld = ps.ld;
-    const int n = ps.n, c0 = 9 * cam, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid < kBlkPairs) {  // iZ holds G_0 here
-        int r = 0, s = tid;
-        while (s > r) s -= ++r;  // tid = r (r + 1) / 2 + s, s <= r
-        val[tid] = ps.iZ[(c0 + r) + (long)(c0 + s) * ld];
-    }
+// The camera's block of iZ = sum_i c_i X^(i+1) and the outputs that read it:
+// cam_unc = (iZ(j,k) + iZ(k,j) / 2) d_j d_k, d = 1 / s (compute.cpp:176), and
+// the unscaled covariance block sig (compute.cpp:435). One CTA per camera, a
+// thread per element of the lower triangle.
+__global__ void __launch_bounds__(64) k_power_output(PowerSet ps, const double* __restrict__ s_cam,
+                                                     double* __restrict__ cam_unc, double* __restrict__ sig) {
+    const int p = threadIdx.x;
+    if (p >= kBlkPairs) return;
+    const long cam = blockIdx.x, c0 = 9 * cam;
+    int r, s;
+    lower_pair(p, r, s);
+    const double* c = ps.te->c;
+    const long at = (c0 + r) + (c0 + s) * ps.ld;
+    double v = c[0] * ps.M[0][at];
+    v += c[1] * ps.M[1][at];
+    v += c[2] * ps.M[2][at];
+    v += c[3] * ps.M[3][at];
     for (int q = 1; q <= 4; ++q) {
-        if (ps.te->skip[q]) continue;  // the same word for every thread of the CTA
-        const double* cq = ps.te->c + 4 * q;
-        const double k0 = cq[0], k1 = cq[1], k2 = cq[2], k3 = cq[3];
-        const double* P = ps.M[q + 2];  // X^4, X^8, X^12, X^16
-        double acc[kBlkPairs];
-#pragma unroll
-        for (int p = 0; p < kBlkPairs; ++p) acc[p] = 0.0;
-        for (int k = tid; k < n; k += kBlkThreads) {
-            double g[9], x[9];
-#pragma unroll
-            for (int i = 0; i < 9; ++i) {
-                const long o = k + (long)(c0 + i) * ld;
-                double v = k0 * ps.M[0][o];
-                v += k1 * ps.M[1][o];
-                v += k2 * ps.M[2][o];
-                v += k3 * ps.M[3][o];
-                g[i] = v;
-                x[i] = P[o];
-            }
-#pragma unroll
-            for (int r = 0, p = 0; r < 9; ++r)
-#pragma unroll
-                for (int s = 0; s <= r; ++s, ++p) acc[p] = fma(g[r], x[s], acc[p]);
-        }
-#pragma unroll
-        for (int p = 0; p < kBlkPairs; ++p) {
-            double a = acc[p];
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) a += __shfl_xor_sync(0xffffffffu, a, d);
-            if (lane == 0) red[warp][p] = a;
-        }
-        __syncthreads();
-        if (tid < kBlkPairs) {
-            double t = red[0][tid];
-#pragma unroll
-            for (int w = 1; w < kBlkThreads / 32; ++w) t += red[w][tid];
-            val[tid] += t;
-        }
-        __syncthreads();  // red is reused by the next block
+        if (ps.te->skip[q]) continue;
+        const double* b = ps.blk + (cam * 16 + 4 * (q - 1)) * kBlkPairs + p;
+        double t = c[4 * q] * b[0];
+        t += c[4 * q + 1] * b[kBlkPairs];
+        t += c[4 * q + 2] * b[2 * kBlkPairs];
+        t += c[4 * q + 3] * b[3 * kBlkPairs];
+        v += t;
     }
-    if (tid < kBlkPairs) {
-        int r = 0, s = tid;
-        while (s > r) s -= ++r;
-        ps.iZ[(c0 + r) + (long)(c0 + s) * ld] = val[tid];
-        ps.iZ[(c0 + s) + (long)(c0 + r) * ld] = val[tid];
-    }
-}
-
-__global__ void __launch_bounds__(kBlkThreads) k_taylor_blocks(PowerSet ps) {
-    __shared__ double red[kBlkThreads / 32][kBlkPairs];
-    __shared__ double val[kBlkPairs];
-    taylor_camera_block(ps, blockIdx.x, red, val);
-}
-
-// The same over the cameras of many sets: blk holds the sets' column offsets
-// (multiples of 9), so set m owns the cameras [blk[m] / 9, blk[m + 1] / 9).
-__global__ void __launch_bounds__(kBlkThreads) k_taylor_blocks_grouped(const PowerSet* __restrict__ sets, int nsets,
-                                                                       const long* __restrict__ blk) {
-    const int m = set_of_block(blk, nsets, 9L * blockIdx.x);
-    __shared__ double red[kBlkThreads / 32][kBlkPairs];
-    __shared__ double val[kBlkPairs];
-    taylor_camera_block(sets[m], (int)(blockIdx.x - blk[m] / 9), red, val);
+    const double dr = 1.0 / s_cam[c0 + r], ds = 1.0 / s_cam[c0 + s];
+    sig[81 * cam + 9 * r + s] = v * dr * ds;
+    sig[81 * cam + 9 * s + r] = v * ds * dr;
+    cam_unc[45 * cam + s * 9 - (s * (s - 1)) / 2 + (r - s)] = (v + v / 2) * ds * dr;  // row s, column r
 }
 
 }  // namespace
 
-void launch_taylor_blocks(const PowerSet& ps, cudaStream_t st) {
-    k_taylor_blocks<<<ps.n / 9, kBlkThreads, 0, st>>>(ps);
+void launch_power_blocks(const PowerSet& ps, bool past_15, const int* skip, cudaStream_t st) {
+    if (past_15)
+        k_power_blocks<4, 1><<<ps.n / 9, kBlkThreads, 0, st>>>(ps, skip);
+    else
+        k_power_blocks<1, 3><<<ps.n / 9, kBlkThreads, 0, st>>>(ps, skip);
     count_launch();
 }
 
-void launch_taylor_blocks_grouped(const PowerSet* d_sets, int nsets, const long* d_blk_cols, long nblk_cols,
-                                  cudaStream_t st) {
+void launch_power_blocks_grouped(const PowerSet* d_sets, int nsets, const long* d_blk_cols, long nblk_cols, bool past_15,
+                                 cudaStream_t st) {
     if (nsets <= 0 || nblk_cols < 9) return;
-    k_taylor_blocks_grouped<<<(unsigned)(nblk_cols / 9), kBlkThreads, 0, st>>>(d_sets, nsets, d_blk_cols);
-    count_launch();
-}
-
-void launch_power_diag(const PowerSet& ps, int jlo, int jhi, const int* skip, cudaStream_t st) {
-    if (jlo == 2 && jhi == 16) {
-        k_power_diag<2, 16><<<ps.n, kDiagThreads, 0, st>>>(ps, skip);
-    } else {
-        k_power_diag<17, 20><<<ps.n, kDiagThreads, 0, st>>>(ps, skip);
-    }
+    const unsigned cams = (unsigned)(nblk_cols / 9);
+    if (past_15)
+        k_power_blocks_grouped<4, 1><<<cams, kBlkThreads, 0, st>>>(d_sets, nsets, d_blk_cols);
+    else
+        k_power_blocks_grouped<1, 3><<<cams, kBlkThreads, 0, st>>>(d_sets, nsets, d_blk_cols);
     count_launch();
 }
 
 void launch_power_decide(TeState* te, const unsigned long long* dmax, const TaylorCoefs& k, int ilo, int ihi,
                          cudaStream_t st) {
     k_power_decide<<<1, 32, 0, st>>>(te, dmax, k, ilo, ihi);
-    count_launch();
-}
-
-void launch_power_combine(const PowerSet& ps, int q, double* out, const int* skip, cudaStream_t st) {
-    const long total = (long)ps.n * ps.n;
-    k_power_combine<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(ps, q, out, skip);
-    count_launch();
-}
-
-void launch_power_diag_grouped(const PowerSet* d_sets, int nsets, const long* d_blk_cols, long nblk, int jlo,
-                               int jhi, bool skip_if_done_early, cudaStream_t st) {
-    if (nsets <= 0) return;
-    if (jlo == 2 && jhi == 16) {
-        k_power_diag_grouped<2, 16><<<(unsigned)nblk, kDiagThreads, 0, st>>>(d_sets, nsets, d_blk_cols,
-                                                                             skip_if_done_early ? 1 : 0);
-    } else {
-        k_power_diag_grouped<17, 20><<<(unsigned)nblk, kDiagThreads, 0, st>>>(d_sets, nsets, d_blk_cols,
-                                                                              skip_if_done_early ? 1 : 0);
-    }
     count_launch();
 }
 
@@ -314,10 +277,8 @@ void launch_power_decide_grouped(const PowerSet* d_sets, int nsets, const double
     count_launch();
 }
 
-void launch_power_combine_grouped(const PowerSet* d_sets, int nsets, const long* d_blk_elems, long nblk, int q,
-                                  cudaStream_t st) {
-    if (nsets <= 0) return;
-    k_power_combine_grouped<<<(unsigned)nblk, 256, 0, st>>>(d_sets, nsets, d_blk_elems, q);
+void launch_power_output(const PowerSet& ps, const double* s_cam, double* cam_unc, double* sig, cudaStream_t st) {
+    k_power_output<<<ps.n / 9, 64, 0, st>>>(ps, s_cam, cam_unc, sig);
     count_launch();
 }
 
