@@ -854,6 +854,7 @@ int unc_context_create(int device, unc_context** out) {
         c->task_ctas = c->sm_count;
         prepare_assembly_kernels();
         prepare_point_kernels();
+        prepare_power_kernels();
         prepare_dense_kernels();
         prepare_mixed_kernels();
         e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);

@@ -351,7 +351,7 @@ int launch_group(unc_batch* b, GroupRun& g) {
     launch_unequilibrate_grouped(g.dd.dense, n, g.dd.blk_elems, g.nblk_elems, sm);  // X in Z, iZ = X
     // the Taylor series from blocked powers (powers.cu), every step over all scenes
     auto slice = [&](int set) {
-        mixed_slice_grouped(g.dd.slice + (size_t)set * n, n, g.dd.row_start, g.total_rows, sm);
+        mixed_slice_grouped(g.slices, g.dd.slice + (size_t)set * n, n, g.dd.row_start, g.total_rows, sm);
     };
     auto gemm = [&](int set) {  // product `set` with its slices (power_product_slices)
         const int k = power_product_slices(set, g.slices);
@@ -481,7 +481,7 @@ int prepare_group(unc_batch* b, GroupRun& g, int nt) {
         };
         const SliceDef sd[kSliceSets] = {{s.b.Z, 0}, {s.b.add, 1}, {s.b.tmp, 1}, {s.b.p4, 2}, {s.b.p8, 3}};
         for (int q = 0; q < kSliceSets; ++q)
-            hdd.slice[(size_t)q * n + i] = MixedSliceJob{sd[q].src, ld, N, g.slices, s.buf[sd[q].buf], rows, kp,
+            hdd.slice[(size_t)q * n + i] = MixedSliceJob{sd[q].src, ld, N, s.buf[sd[q].buf], rows, kp,
                                                          s.ex[sd[q].buf], nullptr, nullptr, nullptr};
         // products: A map, B map, A / B exponent buffers, output, skip
         const CUtensorMap* dm = g.dd.maps + kMaps * i;
@@ -669,6 +669,7 @@ int unc_batch_create(int device, unc_batch** out) {
     if (e == cudaSuccess) {
         prepare_assembly_kernels();
         prepare_point_kernels();
+        prepare_power_kernels();
         prepare_dense_kernels();
         prepare_mixed_kernels();
         prepare_task_kernels();

@@ -308,6 +308,7 @@ struct TaylorCoefs {
 // The camera blocks and diagonal maxima from X .. X^12 (past_15: those with
 // X^16), unless *skip; grouped: over the cameras of every set (d_blk_cols: the
 // sets' column offsets).
+void prepare_power_kernels();  // kernel attributes (before any stream capture)
 void launch_power_blocks(const PowerSet& ps, bool past_15, const int* skip, cudaStream_t st);
 void launch_power_blocks_grouped(const PowerSet* d_sets, int nsets, const long* d_blk_cols, long nblk_cols, bool past_15,
                                  cudaStream_t st);
@@ -384,7 +385,7 @@ MixedOperand mixed_fewer_slices(const MixedOperand& op, int slices, bool as_b, b
 struct MixedSliceJob {  // k_slice_rows of one matrix
     const double* A;
     long lda;
-    int n, S;
+    int n;
     int8_t* out;
     int rows_pad, kp;
     int* exps;
@@ -405,7 +406,7 @@ struct MixedGemmJob {  // one lower-triangle symmetric product C = P X (mirrored
     const int* skip;
 };
 // block b of the launch slices row b - row_start[m] of job m (row_start: njobs + 1 ints)
-void mixed_slice_grouped(const MixedSliceJob* d_jobs, int njobs, const int* d_row_start, int total_rows,
+void mixed_slice_grouped(int slices, const MixedSliceJob* d_jobs, int njobs, const int* d_row_start, int total_rows,
                          cudaStream_t st);
 // the lower-triangle 128 x nt tiles of an n x n product, as (job, m0, n0, 0)
 void mixed_lower_tiles(int job, int n, int nt, std::vector<int4>& out);

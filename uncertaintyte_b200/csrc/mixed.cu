@@ -168,11 +168,14 @@ __device__ __forceinline__ double pow2(int e) {
 // 1.5 2^(52 - 7s) rounds the remainder to that unit (to nearest, ties to even)
 // and leaves the digit in the sum's low bits, so a digit is three additions and
 // no conversion; the row stays in registers between its maximum and its digits
-// up to kSliceKept elements. n = 1800, five slices: 19 -> 8 us.
+// up to kSliceKept elements. The slice count is a template parameter and the
+// digits' bytes are gathered by byte permutes: issue slots bound it. n = 1800, five
+// slices: 19 -> 13.5 us.
 // Y (optional): Y += te->coef * A on the way (the Taylor update iZ += k add of
 // the power being sliced, compute.cpp:64-71).
 constexpr int kSlicePasses = 4;  // 1024 elements each
-__device__ __forceinline__ void slice_row(int j, const double* __restrict__ A, long lda, int n, int S,
+template <int S>
+__device__ __forceinline__ void slice_row(int j, const double* __restrict__ A, long lda, int n,
                                           int8_t* __restrict__ out, int rows_pad, int kp, int* __restrict__ exps,
                                           double* Y, const TeState* te, bool lower, double* red) {
     const double* col = A + (long)j * lda;
@@ -227,17 +230,20 @@ __device__ __forceinline__ void slice_row(int j, const double* __restrict__ A, l
         if (k >= kp) return;
 #pragma unroll
         for (int u = 0; u < 4; ++u) v[u] *= sc;
-        double unit = 1.5 * 35184372088832.0;  // 1.5 2^45
-        for (int s = 0; s < S; ++s) {
-            unsigned word = 0;
+        int8_t* dst = row + k;
+#pragma unroll
+        for (int s = 0; s < S; ++s, dst += plane) {
+            const double unit = 1.5 * (double)(1LL << (45 - 7 * s));
+            unsigned d[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const double r = v[u] + unit;
                 v[u] -= r - unit;
-                word |= ((unsigned)__double2loint(r) & 0xffu) << (8 * u);
+                d[u] = (unsigned)__double2loint(r);
             }
-            *reinterpret_cast<unsigned*>(row + s * plane + k) = word;
-            unit *= 1.0 / 128.0;
+            // the four low bytes
+            *reinterpret_cast<unsigned*>(dst) =
+                __byte_perm(__byte_perm(d[0], d[1], 0x0040), __byte_perm(d[2], d[3], 0x0040), 0x5410);
         }
     };
 #pragma unroll
@@ -249,17 +255,19 @@ __device__ __forceinline__ void slice_row(int j, const double* __restrict__ A, l
     }
 }
 
-__global__ void __launch_bounds__(256) k_slice_rows(const double* __restrict__ A, long lda, int n, int S,
+template <int S>
+__global__ void __launch_bounds__(256) k_slice_rows(const double* __restrict__ A, long lda, int n,
                                                    int8_t* __restrict__ out, int rows_pad, int kp,
                                                    int* __restrict__ exps, const int* skip, double* Y,
                                                    const TeState* te, int lower) {
     if (skip && *skip) return;
     __shared__ double red[8];
-    slice_row(blockIdx.x, A, lda, n, S, out, rows_pad, kp, exps, Y, te, lower != 0, red);
+    slice_row<S>(blockIdx.x, A, lda, n, out, rows_pad, kp, exps, Y, te, lower != 0, red);
 }
 
 // The same over the rows of many matrices (a batch): block b slices row
 // b - row_start[m] of matrix m, row_start[m] <= b < row_start[m + 1].
+template <int S>
 __global__ void __launch_bounds__(256) k_slice_rows_grouped(const MixedSliceJob* __restrict__ jobs, int njobs,
                                                            const int* __restrict__ row_start) {
     int lo = 0, hi = njobs - 1;
@@ -271,7 +279,7 @@ __global__ void __launch_bounds__(256) k_slice_rows_grouped(const MixedSliceJob*
     const MixedSliceJob& jb = jobs[lo];
     if (jb.skip && *jb.skip) return;
     __shared__ double red[8];
-    slice_row(b - row_start[lo], jb.A, jb.lda, jb.n, jb.S, jb.out, jb.rows_pad, jb.kp, jb.exps, jb.Y, jb.te, false, red);
+    slice_row<S>(b - row_start[lo], jb.A, jb.lda, jb.n, jb.out, jb.rows_pad, jb.kp, jb.exps, jb.Y, jb.te, false, red);
 }
 
 // One 128 x NT output tile at (m0, n0): TMA producer, MMA issuer, epilogue.
@@ -654,10 +662,13 @@ MixedOperand mixed_fewer_slices(const MixedOperand& op, int slices, bool as_b, b
     return r;
 }
 
-void mixed_slice_grouped(const MixedSliceJob* d_jobs, int njobs, const int* d_row_start, int total_rows,
+void mixed_slice_grouped(int slices, const MixedSliceJob* d_jobs, int njobs, const int* d_row_start, int total_rows,
                          cudaStream_t st) {
     if (total_rows <= 0) return;
-    k_slice_rows_grouped<<<total_rows, 256, 0, st>>>(d_jobs, njobs, d_row_start);
+    const auto kern = slices == 5   ? k_slice_rows_grouped<5>
+                      : slices == 4 ? k_slice_rows_grouped<4>
+                                    : k_slice_rows_grouped<3>;
+    kern<<<total_rows, 256, 0, st>>>(d_jobs, njobs, d_row_start);
     count_launch();
 }
 
@@ -719,8 +730,11 @@ void mixed_gemm_grouped(int slices, int nt, const MixedGemmJob* d_jobs, const in
 
 void mixed_slice(const double* A, int lda, MixedOperand& op, cudaStream_t st, const int* skip, double* Y,
                  const TeState* te, bool lower) {
-    k_slice_rows<<<op.n, 256, 0, st>>>(A, lda, op.n, op.slices, op.buf, op.rows, op.kp, op.exps, skip, Y, te,
-                                       lower ? 1 : 0);
+    const auto kern = op.slices == 5   ? k_slice_rows<5>
+                      : op.slices == 4 ? k_slice_rows<4>
+                      : op.slices == 3 ? k_slice_rows<3>
+                                       : k_slice_rows<kGramSlices>;
+    kern<<<op.n, 256, 0, st>>>(A, lda, op.n, op.buf, op.rows, op.kp, op.exps, skip, Y, te, lower ? 1 : 0);
     count_launch();
 }
 

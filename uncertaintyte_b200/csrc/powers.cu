@@ -43,59 +43,84 @@ __device__ __forceinline__ void lower_pair(int p, int& r, int& s) {
 // The camera's blocks of X^(4q) X^(r+1) for q in [Q0, Q0 + NQ) and r = 0..3,
 // lower triangles, into ps.blk; their diagonals, and with Q0 = 1 those of X^2,
 // X^3, X^4, into the maxima ps.dmax (over the non-negative values; a non-finite
-// one becomes +inf). One CTA per camera, eight warps: warp (r, half) takes the
-// columns of X^(r+1) over half of the rows against those of the NQ powers: a DMMA
-// per power for the leading 8 x 8 part, ordinary multiply-adds for row 8. A
-// lane's 16-byte load holds the rows k = 8 j + 2 t and the next, which go to two
-// DMMA steps. Reading every power once bounds the kernel (the six or seven
-// matrices of the series; they were read three times when the diagonals, the
-// first four terms and the blocks were kernels of their own: 126 us at n = 1800).
+// one becomes +inf). One CTA per camera: the camera's nine columns of every
+// power are streamed through shared memory, kBlkK rows at a time in kBlkStages
+// asynchronous stages (reading each power once bounds the kernel; with loads
+// straight into registers its latency did: 110 us at n = 1800, 9.0 ms at 18000;
+// now 67 us and 4.0 ms, 59 % of the copy bandwidth). Eight warps:
+// warp (r, half) multiplies the columns of X^(r+1) with those of the NQ powers over
+// every other 8 rows: a DMMA per power for the leading 8 x 8 part, ordinary
+// multiply-adds for row 8. A lane's 16-byte read holds the rows k = 8 j + 2 t
+// and the next, which go to two DMMA steps.
+constexpr int kBlkK = 32, kBlkStages = 4, kBlkStride = kBlkK + 8;  // column stride: conflict-free 16-byte reads
+template <int NQ>
+constexpr int blk_slots() { return 4 + (NQ == 3 ? 2 : 1); }  // X .. X^4, then the powers that are not X^4
+template <int NQ>
+constexpr size_t blk_smem() { return sizeof(double) * kBlkStages * blk_slots<NQ>() * 9 * kBlkStride; }
+
 template <int Q0, int NQ>
-__device__ __forceinline__ void power_blocks(const PowerSet& ps, int cam, double (*red)[4][NQ][kBlkPairs],
+__device__ __forceinline__ void power_blocks(const PowerSet& ps, int cam, double* sm, double (*red)[4][NQ][kBlkPairs],
                                              double (*dia)[3][9], unsigned long long* top) {
+    static_assert((Q0 == 1 && NQ == 3) || (Q0 == 4 && NQ == 1), "X^4, X^8, X^12 or X^16");
+    constexpr int kSlots = blk_slots<NQ>(), kStage = kSlots * 9 * kBlkStride;
     const int n = ps.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int r = warp & 3, half = warp >> 2;
     const long ld = ps.ld, c0 = 9L * cam;
-    const int steps = (n + 7) / 8, s0 = half ? steps / 2 : 0, s1 = half ? steps : steps / 2;
-    const double* const A = ps.M[r] + c0 * ld;
+    const int stages = (n + kBlkK - 1) / kBlkK;
+    auto issue = [&](int s) {
+        if (s < stages) {
+            double* st = sm + (s % kBlkStages) * kStage;
+            for (int q = tid; q < kSlots * 9 * (kBlkK / 2); q += kBlkThreads) {
+                const int col = q / (kBlkK / 2), k2 = q % (kBlkK / 2) * 2, slot = col / 9;
+                const double* M = ps.M[slot < 4 ? slot : (Q0 == 1 ? slot : 6)];
+                const int left = n - (s * kBlkK + k2), bytes = left >= 2 ? 16 : (left == 1 ? 8 : 0);
+                const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(st + col * kBlkStride + k2));
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst),
+                             "l"(bytes ? M + (c0 + col - 9 * slot) * ld + s * kBlkK + k2 : M), "r"(bytes)
+                             : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
     double c[NQ][2], row[NQ], corner[NQ], d[2][2];  // d: diagonals of X X (X^2 X^2 in warp r = 1) and X X^2
 #pragma unroll
     for (int q = 0; q < NQ; ++q) c[q][0] = c[q][1] = row[q] = corner[q] = 0.0;
     d[0][0] = d[0][1] = d[1][0] = d[1][1] = 0.0;
-    auto load = [&](const double* M, int col, int k) {
-        double2 v = make_double2(0.0, 0.0);
-        if (k + 1 < n) v = *reinterpret_cast<const double2*>(M + col * ld + k);
-        else if (k < n) v.x = M[col * ld + k];
-        return v;
-    };
-    for (int s = s0; s < s1; ++s) {
-        const int k = 8 * s + 2 * t;
-        const double2 a = load(A, g, k), a8 = load(A, 8, k);
-        double2 b[NQ], b8[NQ];
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const double* B = ps.M[Q0 + q + 2] + c0 * ld;
-            b[q] = load(B, g, k);
-            b8[q] = load(B, 8, k);
-        }
+    for (int s = 0; s < kBlkStages - 1; ++s) issue(s);
+    for (int s = 0; s < stages; ++s) {
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kBlkStages - 2) : "memory");
+        __syncthreads();
+        issue(s + kBlkStages - 1);
+        const double* st = sm + (s % kBlkStages) * kStage;
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                         : "+d"(c[q][0]), "+d"(c[q][1])
-                         : "d"(a.x), "d"(b[q].x));
-            asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                         : "+d"(c[q][0]), "+d"(c[q][1])
-                         : "d"(a.y), "d"(b[q].y));
-            row[q] = fma(a8.y, b[q].y, fma(a8.x, b[q].x, row[q]));
-            corner[q] = fma(a8.y, b8[q].y, fma(a8.x, b8[q].x, corner[q]));
-        }
-        if (Q0 == 1 && r < 2) {
-            d[0][0] = fma(a.y, a.y, fma(a.x, a.x, d[0][0]));
-            d[0][1] = fma(a8.y, a8.y, fma(a8.x, a8.x, d[0][1]));
-            if (r == 0) {
-                const double2 x = load(ps.M[1] + c0 * ld, g, k), x8 = load(ps.M[1] + c0 * ld, 8, k);
-                d[1][0] = fma(a.y, x.y, fma(a.x, x.x, d[1][0]));
-                d[1][1] = fma(a8.y, x8.y, fma(a8.x, x8.x, d[1][1]));
+        for (int j = 0; j < kBlkK / 16; ++j) {
+            const double* at = st + 8 * (2 * j + half) + 2 * t;
+            auto read = [&](int slot, int col) {
+                return *reinterpret_cast<const double2*>(at + (9 * slot + col) * kBlkStride);
+            };
+            const double2 a = read(r, g), a8 = read(r, 8);
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                const int slot = Q0 == 1 ? 3 + q : 4;
+                const double2 b = read(slot, g), b8 = read(slot, 8);
+                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                             : "+d"(c[q][0]), "+d"(c[q][1])
+                             : "d"(a.x), "d"(b.x));
+                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                             : "+d"(c[q][0]), "+d"(c[q][1])
+                             : "d"(a.y), "d"(b.y));
+                row[q] = fma(a8.y, b.y, fma(a8.x, b.x, row[q]));
+                corner[q] = fma(a8.y, b8.y, fma(a8.x, b8.x, corner[q]));
+            }
+            if (Q0 == 1 && r < 2) {
+                d[0][0] = fma(a.y, a.y, fma(a.x, a.x, d[0][0]));
+                d[0][1] = fma(a8.y, a8.y, fma(a8.x, a8.x, d[0][1]));
+                if (r == 0) {
+                    const double2 x = read(1, g), x8 = read(1, 8);
+                    d[1][0] = fma(a.y, x.y, fma(a.x, x.x, d[1][0]));
+                    d[1][1] = fma(a8.y, x8.y, fma(a8.x, x8.x, d[1][1]));
+                }
             }
         }
     }
@@ -150,10 +175,11 @@ __device__ __forceinline__ void power_blocks(const PowerSet& ps, int cam, double
 
 template <int Q0, int NQ>
 __global__ void __launch_bounds__(kBlkThreads, 2) k_power_blocks(PowerSet ps, const int* skip) {
+    extern __shared__ __align__(16) double sm[];
     __shared__ double red[2][4][NQ][kBlkPairs], dia[2][3][9];
     __shared__ unsigned long long top[32];
     if (skip && *skip) return;
-    power_blocks<Q0, NQ>(ps, blockIdx.x, red, dia, top);
+    power_blocks<Q0, NQ>(ps, blockIdx.x, sm, red, dia, top);
 }
 
 __device__ __forceinline__ int set_of_block(const long* __restrict__ blk, int nsets, long b) {
@@ -170,12 +196,13 @@ __device__ __forceinline__ int set_of_block(const long* __restrict__ blk, int ns
 template <int Q0, int NQ>
 __global__ void __launch_bounds__(kBlkThreads, 2)
     k_power_blocks_grouped(const PowerSet* __restrict__ sets, int nsets, const long* __restrict__ cols) {
+    extern __shared__ __align__(16) double sm[];
     __shared__ double red[2][4][NQ][kBlkPairs], dia[2][3][9];
     __shared__ unsigned long long top[32];
     const int m = set_of_block(cols, nsets, 9L * blockIdx.x);
     const PowerSet ps = sets[m];
     if (Q0 > 1 && ps.te->skip[0]) return;
-    power_blocks<Q0, NQ>(ps, (int)(blockIdx.x - cols[m] / 9), red, dia, top);
+    power_blocks<Q0, NQ>(ps, (int)(blockIdx.x - cols[m] / 9), sm, red, dia, top);
 }
 
 // The reference's stop rule (compute.cpp:145-155) over iterations ilo..ihi.
@@ -245,11 +272,23 @@ __global__ void __launch_bounds__(64) k_power_output(PowerSet ps, const double* 
 
 }  // namespace
 
+void prepare_power_kernels() {
+    static std::atomic<unsigned long long> attr{0};
+    once_per_device(attr, [] {
+        auto set = [](const void* f, size_t bytes) {
+            return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+        };
+        return set((const void*)k_power_blocks<1, 3>, blk_smem<3>()) && set((const void*)k_power_blocks<4, 1>, blk_smem<1>()) &&
+               set((const void*)k_power_blocks_grouped<1, 3>, blk_smem<3>()) &&
+               set((const void*)k_power_blocks_grouped<4, 1>, blk_smem<1>());
+    });
+}
+
 void launch_power_blocks(const PowerSet& ps, bool past_15, const int* skip, cudaStream_t st) {
     if (past_15)
-        k_power_blocks<4, 1><<<ps.n / 9, kBlkThreads, 0, st>>>(ps, skip);
+        k_power_blocks<4, 1><<<ps.n / 9, kBlkThreads, blk_smem<1>(), st>>>(ps, skip);
     else
-        k_power_blocks<1, 3><<<ps.n / 9, kBlkThreads, 0, st>>>(ps, skip);
+        k_power_blocks<1, 3><<<ps.n / 9, kBlkThreads, blk_smem<3>(), st>>>(ps, skip);
     count_launch();
 }
 
@@ -258,9 +297,9 @@ void launch_power_blocks_grouped(const PowerSet* d_sets, int nsets, const long* 
     if (nsets <= 0 || nblk_cols < 9) return;
     const unsigned cams = (unsigned)(nblk_cols / 9);
     if (past_15)
-        k_power_blocks_grouped<4, 1><<<cams, kBlkThreads, 0, st>>>(d_sets, nsets, d_blk_cols);
+        k_power_blocks_grouped<4, 1><<<cams, kBlkThreads, blk_smem<1>(), st>>>(d_sets, nsets, d_blk_cols);
     else
-        k_power_blocks_grouped<1, 3><<<cams, kBlkThreads, 0, st>>>(d_sets, nsets, d_blk_cols);
+        k_power_blocks_grouped<1, 3><<<cams, kBlkThreads, blk_smem<3>(), st>>>(d_sets, nsets, d_blk_cols);
     count_launch();
 }
 
