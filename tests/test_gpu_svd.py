@@ -45,6 +45,18 @@ def test_pinv_known_spectrum(n, null):
     assert np.abs(got - ref).max() / np.abs(ref).max() < 1e-10
 
 
+@pytest.mark.parametrize("n,null", [(2, 1), (9, 3), (17, 8), (40, 22), (65, 24), (257, 16), (6600, 24)])
+def test_pinv_projector(n, null):
+    """P = I - V V^T is its own pseudo-inverse: subspace blocks of every width (2 to 32 columns) and
+    size, down to fewer rows than the cluster has CTAs and up to columns past its shared memory.
+    Every kept eigenvalue is 1, so the inverse adds a few n eps: 1e-11 covers n = 6600."""
+    rng = np.random.default_rng(n)
+    V, _ = np.linalg.qr(rng.standard_normal((n, null)))
+    P = np.eye(n) - V @ V.T
+    got = _pinv_gpu(0.5 * (P + P.T), null)
+    assert np.abs(got - P).max() < 1e-11
+
+
 def test_pinv_epsilon_rule():
     n = 200
     A, Q, lam = _psd(n, 0, seed=5)

@@ -13,28 +13,18 @@
 // signs are arbitrary (as with the reference's EigenSolver).
 #include "../../include/uncte.h"
 #include "internal.h"
+#include "rotation.cuh"
 
 namespace unc {
 namespace {
 
 constexpr int kMaxDim = 9;
 
-// The angle of the rotation that clears a_pq, from the tangent: entries so
-// large or small that their squares leave the FP64 range.
-__device__ __noinline__ void rotation_by_tangent(double d, double h, double& c, double& s, double& t) {
-    const double th = d / h;
-    t = fabs(th) > 1e100 ? 0.5 / th : (th >= 0.0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
-    c = 1.0 / sqrt(t * t + 1.0);
-    s = t * c;
-}
-
 // One D x D block on L lanes, everything in registers: every lane of a block
 // carries the whole upper triangle and applies every rotation to it, so the
 // rotations need no shared memory, shuffle or barrier; the rows of V are dealt
 // to the lanes (D / L each). The chain of dependent rotations bounds the
-// kernel, so a rotation takes two reciprocal square roots and no division:
-// with d = a_qq - a_pp, h = 2 a_pq and r = 1 / sqrt(d^2 + h^2),
-//   cos^2 = x = (1 + |d| r) / 2,  c = x / sqrt(x),  |s| = |h| r / (2 sqrt(x)).
+// kernel.
 template <int D, int L>
 __global__ void __launch_bounds__(128) k_block_eigen(const double* __restrict__ packed, int nblk, int src, int off,
                                                      double* vals, double* vecs) {
@@ -70,20 +60,8 @@ __global__ void __launch_bounds__(128) k_block_eigen(const double* __restrict__ 
 #pragma unroll
             for (int q = p + 1; q < D; ++q) {
                 const double apq = a[p][q], app = a[p][p], aqq = a[q][q];
-                const double pr = fabs(app * aqq);
-                const bool small = fabs(apq) > 1e-140 ? apq * apq <= 1e-34 * pr : fabs(apq) <= 1e-17 * sqrt(pr);
-                if (apq == 0.0 || small) continue;
-                const double d = aqq - app, h = 2.0 * apq, m = fma(d, d, h * h);
                 double c, s, t;
-                if (m > 1e-280 && m < 1e280) {
-                    const double r = rsqrt(m), x = fma(0.5 * fabs(d), r, 0.5), rs = rsqrt(x);
-                    c = x * rs;
-                    s = 0.5 * fabs(h) * r * rs;
-                    if (d != 0.0 && (d < 0.0) != (h < 0.0)) s = -s;
-                    t = s * rs;
-                } else {
-                    rotation_by_tangent(d, h, c, s, t);
-                }
+                if (!sym_rotation(app, aqq, apq, c, s, t)) continue;
                 a[p][p] = fma(-t, apq, app);
                 a[q][q] = fma(t, apq, aqq);
                 a[p][q] = 0.0;

@@ -436,7 +436,7 @@ void mixed_gemm(const MixedOperand& a, const MixedOperand& b, double* C, int ldc
 // Scratch of the PSD pseudo-inverse (n x ld matrices and p x n blocks).
 struct PinvBuffers {
     double *G, *T, *W, *Tt;        // shifted inverse, Cholesky-inverse scratch
-    double *X, *Y, *MX, *MX2;      // n x 32 subspace blocks
+    double *X, *Y, *MX;            // n x 32 subspace blocks
     double *H, *Wr, *S;            // 32 x 32
     double *theta, *res, *e;
     int* state;                    // counters of the tile tasks

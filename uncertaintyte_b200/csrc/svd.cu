@@ -15,7 +15,7 @@
 //   1. G = (M + s I)^{-1}, s = 1e-13 max_i M_ii, by the Cholesky inverse of
 //      dense.cu (equilibrated); the removed directions are G's dominant ones.
 //   2. Subspace iteration on G with p = removed + 8 vectors: Y = G X,
-//      Gram-Schmidt (twice), Rayleigh-Ritz with M (p x p cyclic Jacobi), until
+//      Gram-Schmidt (twice), Rayleigh-Ritz with M (p x p Jacobi rotations), until
 //      the Ritz residuals of the removed vectors stop shrinking.
 //   3. B = M + c V_R V_R^T with c the smallest kept Ritz value: SPD when every
 //      kept eigenvalue is positive, with the removed directions lifted.
@@ -26,17 +26,19 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <cooperative_groups.h>
 #include <cstring>
 #include <vector>
 
 #include "../../include/uncte.h"
 #include "internal.h"
+#include "rotation.cuh"
 
 namespace unc {
 
 namespace {
 
-constexpr int kMaxBlock = 32;  // largest subspace block (the p x p kernels run in one warp)
+constexpr int kMaxBlock = 32;  // largest subspace block (a row of the p x p matrices is a lane)
 
 #define SVD_CK(call)                                                                              \
     do {                                                                                          \
@@ -162,84 +164,139 @@ __global__ void __launch_bounds__(256) k_gram(const double* __restrict__ A, long
     if (threadIdx.x == 0) G[i + j * ldg] = s;
 }
 
-// Orthonormalise the p columns of Y in place: Gram-Schmidt run twice per
+// Orthonormalise the p <= 32 columns of Y in place: Gram-Schmidt run twice per
 // column (the second pass restores orthogonality lost to cancellation). A
 // column that vanishes (dependent on the earlier ones) restarts from a random
-// vector (status bit 1); if that fails three times status bit 2 is set. Each
-// thread owns a fixed set of rows, so threads only meet in the reductions.
-__global__ void __launch_bounds__(1024) k_orthonormalize(double* Y, int n, long ld, int p, unsigned long long seed,
-                                                         int* status) {
-    __shared__ double red[33];
-    const int t = threadIdx.x, nt = blockDim.x;
+// vector (status bit 1); if that fails three times status bit 2 is set.
+// The columns depend on one another, so 2 p steps follow each other: the products
+// of the column with all earlier ones (a warp per product), their sum over the rows,
+// the subtraction. Barriers and latency bound a step. A cluster of CTAs shares the rows, each with its rows of all
+// columns in shared memory (`shared`: they fit), and sends its partial products to
+// the others: one cluster barrier per step (two buffers take turns). 15 columns of
+// 1590 rows: 70 us; 133 us in one CTA (bounded by its shared-memory reads), 235 us
+// with a reduction for every earlier column and pass.
+// The squared norm after the second pass is |y|^2 - sum d^2 of that pass's own
+// products d: what it subtracts is rounding error of the first.
+constexpr int kOrthoCtas = 8, kOrthoThreads = 256;
+constexpr size_t kOrthoSharedMax = 200 * 1024;
+__global__ void __cluster_dims__(kOrthoCtas, 1, 1) __launch_bounds__(kOrthoThreads)
+    k_orthonormalize(double* Yg, int n, long ldg, int p, int shared, unsigned long long seed, int* status) {
+    extern __shared__ __align__(16) double ortho_sm[];
+    __shared__ double part[2][kOrthoCtas][32], dot[32], scale, norm0;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank();
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int row0 = (int)((long)rank * n / kOrthoCtas), m = (int)((long)(rank + 1) * n / kOrthoCtas) - row0;
+    Yg += row0;
+    double* const Y = shared ? ortho_sm : Yg;
+    const long ld = shared ? m : ldg;
+    if (shared)
+        for (int r = t; r < m; r += kOrthoThreads)
+#pragma unroll 8
+            for (int j = 0; j < p; ++j) Y[r + j * ld] = Yg[r + j * ldg];
+    cluster.sync();  // every CTA runs: its shared memory may be written
+    int step = 0;
     for (int j = 0; j < p; ++j) {
         double* y = Y + j * ld;
         bool done = false;
         for (int attempt = 0; attempt < 3 && !done; ++attempt) {
-            double s0 = 0.0;
-            for (int r = t; r < n; r += nt) s0 += y[r] * y[r];
-            const double n0 = sqrt(block_sum(s0, red));
-            for (int pass = 0; pass < 2; ++pass)
-                for (int i = 0; i < j; ++i) {
+            for (int pass = 0; pass < 2; ++pass, step ^= 1) {
+                for (int i = warp; i <= j; i += kOrthoThreads / 32) {  // j: the squared norm
                     const double* q = Y + i * ld;
-                    double d = 0.0;
-                    for (int r = t; r < n; r += nt) d += q[r] * y[r];
-                    d = block_sum(d, red);
-                    for (int r = t; r < n; r += nt) y[r] -= d * q[r];
+                    double d[4] = {0.0, 0.0, 0.0, 0.0};
+                    for (int r = lane; r < m; r += 128)
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+                            if (r + 32 * u < m) d[u] = fma(q[r + 32 * u], y[r + 32 * u], d[u]);
+                    double v = (d[0] + d[1]) + (d[2] + d[3]);
+#pragma unroll
+                    for (int k = 16; k > 0; k >>= 1) v += __shfl_xor_sync(0xffffffffu, v, k);
+                    if (lane < kOrthoCtas) *cluster.map_shared_rank(&part[step][rank][i], lane) = v;
                 }
-            double s1 = 0.0;
-            for (int r = t; r < n; r += nt) s1 += y[r] * y[r];
-            const double n1 = sqrt(block_sum(s1, red));
-            if (n1 > 0.0 && n1 > 1e-10 * n0) {
-                const double inv = 1.0 / n1;
-                for (int r = t; r < n; r += nt) y[r] *= inv;
-                done = true;
-            } else {
-                if (t == 0) atomicOr(status, 1);
-                for (int r = t; r < n; r += nt) y[r] = uniform_pm1(seed + 7919ULL * (attempt + 1), j, r);
+                cluster.sync();
+                if (warp == 0) {  // the same sums in every CTA
+                    double v = 0.0;
+                    if (lane <= j)
+#pragma unroll
+                        for (int k = 0; k < kOrthoCtas; ++k) v += part[step][k][lane];
+                    dot[lane] = lane < j ? v : 0.0;
+                    double sq = lane < j ? v * v : 0.0;
+#pragma unroll
+                    for (int k = 16; k > 0; k >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, k);
+                    if (lane == j) {
+                        if (pass == 0) {
+                            norm0 = sqrt(v);
+                        } else {
+                            const double n1 = sqrt(v - sq);
+                            scale = n1 > 0.0 && n1 > 1e-10 * norm0 ? 1.0 / n1 : 0.0;  // 0: restart
+                        }
+                    }
+                }
+                __syncthreads();
+                const double f = pass ? scale : 1.0;
+                done = pass && f != 0.0;
+                for (int r = t; r < m; r += kOrthoThreads) {
+                    double d[4] = {y[r], 0.0, 0.0, 0.0};
+                    for (int k = 0; k < j; k += 4)
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) d[u] = fma(-dot[k + u], Y[r + min(k + u, j - 1) * ld], d[u]);
+                    y[r] = f != 0.0 ? ((d[0] + d[1]) + (d[2] + d[3])) * f
+                                    : uniform_pm1(seed + 7919ULL * (attempt + 1), j, row0 + r);
+                }
+                if (f == 0.0 && rank == 0 && t == 0) atomicOr(status, 1);
+                __syncthreads();
             }
         }
-        if (!done && t == 0) atomicOr(status, 2);
+        if (!done && rank == 0 && t == 0) atomicOr(status, 2);
+        if (shared)
+            for (int r = t; r < m; r += kOrthoThreads) Yg[r + j * ldg] = y[r];
     }
 }
 
-// Eigen-decomposition of the symmetric p x p matrix H (p <= 32) by cyclic
-// Jacobi rotations in one warp (lane = row). Outputs ascending eigenvalues
-// theta and the matching orthonormal eigenvectors as the columns of Wr.
-// Rotation: t = sgn(th) / (|th| + sqrt(th^2 + 1)), th = (a_bb - a_aa) / (2 a_ab),
-// c = 1 / sqrt(t^2 + 1), s = t c (Golub & Van Loan, symmetric Schur 2 x 2);
-// off-diagonal entries below 1e-17 sqrt(|a_aa a_bb|) are left alone.
-__global__ void __launch_bounds__(32) k_small_jacobi(const double* __restrict__ H, int ldh, int p, double* theta,
+// Eigen-decomposition of the symmetric p x p matrix H (p <= 32) by Jacobi
+// rotations. Outputs ascending eigenvalues theta and the matching orthonormal
+// eigenvectors as the columns of Wr.
+// One warp per pair of a round-robin round (the pairs of a round are disjoint:
+// column m - 1 stays, the others move round a circle), lane = row, then column:
+// a sweep is a chain of m - 1 rotations, not of p (p - 1) / 2 (p = 15: 45 us; 240 us
+// for the cyclic order in one warp).
+__global__ void __launch_bounds__(512) k_small_jacobi(const double* __restrict__ H, int ldh, int p, double* theta,
                                                      double* Wr, int ldw) {
     __shared__ double A[kMaxBlock][kMaxBlock + 1], V[kMaxBlock][kMaxBlock + 1];
-    const int l = threadIdx.x;
-    for (int c = 0; c < p; ++c)
-        if (l < p) {
+    __shared__ int stop;
+    const int l = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5, m = 2 * nw;  // m: p rounded up to even
+    if (l < p)
+        for (int c = w; c < p; c += nw) {
             A[l][c] = 0.5 * (H[l + c * ldh] + H[c + l * ldh]);
             V[l][c] = (l == c) ? 1.0 : 0.0;
         }
-    __syncwarp();
+    __syncthreads();
     for (int sweep = 0; sweep < 60; ++sweep) {
-        double off = 0.0, dg = 0.0;
-        if (l < p) {
-            for (int c = 0; c < l; ++c) off += A[l][c] * A[l][c];
-            dg = A[l][l] * A[l][l];
-        }
+        if (w == 0) {
+            double off = 0.0, dg = 0.0;
+            if (l < p) {
+                for (int c = 0; c < l; ++c) off += A[l][c] * A[l][c];
+                dg = A[l][l] * A[l][l];
+            }
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            off += __shfl_xor_sync(0xffffffffu, off, d);
-            dg += __shfl_xor_sync(0xffffffffu, dg, d);
+            for (int d = 16; d > 0; d >>= 1) {
+                off += __shfl_xor_sync(0xffffffffu, off, d);
+                dg += __shfl_xor_sync(0xffffffffu, dg, d);
+            }
+            if (l == 0) stop = off <= 1e-30 * dg;
         }
-        if (off <= 1e-30 * dg) break;
-        for (int a = 0; a < p - 1; ++a)
-            for (int b = a + 1; b < p; ++b) {
-                const double apq = A[a][b], aa = A[a][a], bb = A[b][b];
-                if (apq == 0.0 || fabs(apq) <= 1e-17 * sqrt(fabs(aa * bb))) continue;
-                const double th = (bb - aa) / (2.0 * apq);
-                const double t = fabs(th) > 1e100 ? 0.5 / th
-                                                  : (th >= 0.0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
-                const double c = 1.0 / sqrt(t * t + 1.0), s = t * c;
+        __syncthreads();
+        if (stop) break;
+        for (int round = 0; round < m - 1; ++round) {
+            const int i = (round + w) % (m - 1), j = w == 0 ? m - 1 : (round - w + m - 1) % (m - 1);
+            const int a = min(i, j), b = max(i, j);
+            bool rotate = b < p;
+            double c = 1.0, s = 0.0, t = 0.0;
+            if (rotate) {
+                rotate = sym_rotation(A[a][a], A[b][b], A[a][b], c, s, t);
                 __syncwarp();
-                if (l < p) {
+                if (rotate && l < p) {  // columns a and b: no other warp's in this round
                     const double x = A[l][a], y = A[l][b];
                     A[l][a] = c * x - s * y;
                     A[l][b] = s * x + c * y;
@@ -247,39 +304,194 @@ __global__ void __launch_bounds__(32) k_small_jacobi(const double* __restrict__ 
                     V[l][a] = c * vx - s * vy;
                     V[l][b] = s * vx + c * vy;
                 }
-                __syncwarp();
-                if (l < p) {
-                    const double x = A[a][l], y = A[b][l];
-                    A[a][l] = c * x - s * y;
-                    A[b][l] = s * x + c * y;
-                }
-                __syncwarp();
             }
+            __syncthreads();
+            if (rotate && l < p) {  // rows a and b
+                const double x = A[a][l], y = A[b][l];
+                A[a][l] = c * x - s * y;
+                A[b][l] = s * x + c * y;
+            }
+            __syncthreads();
+        }
     }
-    if (l < p) {
-        const double w = A[l][l];
+    if (w == 0 && l < p) {
+        const double v = A[l][l];
         int rank = 0;
         for (int i = 0; i < p; ++i) {
             const double u = A[i][i];
-            rank += (u < w) || (u == w && i < l);
+            rank += (u < v) || (u == v && i < l);
         }
-        theta[rank] = w;
+        theta[rank] = v;
         for (int r = 0; r < p; ++r) Wr[r + rank * ldw] = V[r][l];
     }
 }
 
-// res_j = || MX(:, j) - theta_j X(:, j) ||
-__global__ void __launch_bounds__(256) k_resid(const double* __restrict__ MX, const double* __restrict__ X, long ld,
-                                               int n, const double* __restrict__ theta, double* res) {
-    __shared__ double red[33];
-    const int j = blockIdx.x;
+// C = A B, A n x n column-major (ld even, 16-byte aligned), B and C n x p,
+// p <= 8 NT <= 32: one CTA per 16 rows, its warps a share of k each, the
+// shares added in warp order. A lane's 16-byte load is rows 2g and 2g + 1 of one
+// column, the A operands of two 8 x 8 x 4 FP64 tensor-core tiles; B comes from
+// the cache, a batch of steps in flight. Load latency bounds it at the sizes of one
+// wave, reading A above (n = 1590, p = 15: 12 us; the tile kernel of the square
+// products has 25 tiles here, each a chain over all of k: 31 us).
+constexpr int kTallWarps = 16;
+template <int NT>
+__global__ void __launch_bounds__(32 * kTallWarps) k_tall_product(const double* __restrict__ A, long lda,
+                                                      const double* __restrict__ B, long ldb, int n, int p, double* C,
+                                                      long ldc) {
+    extern __shared__ double tall_red[];
+    double(*red)[NT][8][16 + 1] = reinterpret_cast<double(*)[NT][8][16 + 1]>(tall_red);
+    constexpr int kTallBatch = NT < 4 ? 7 : 6;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int r = 16 * blockIdx.x + 2 * g;
+    const int steps = (n + 3) / 4, s0 = (int)((long)warp * steps / kTallWarps), s1 = (int)((long)(warp + 1) * steps / kTallWarps);
+    double c[2][NT][2];
+#pragma unroll
+    for (int q = 0; q < NT; ++q) c[0][q][0] = c[0][q][1] = c[1][q][0] = c[1][q][1] = 0.0;
+    for (int s = s0; s < s1; s += kTallBatch) {  // a batch of loads in flight, then its products
+        double2 a[kTallBatch];
+        double v[kTallBatch][NT];
+#pragma unroll
+        for (int u = 0; u < kTallBatch; ++u) {
+            const int k = 4 * (s + u) + t;
+            const bool in = s + u < s1 && k < n;
+            const double* src = A + r + k * lda;
+            a[u] = make_double2(0.0, 0.0);
+            if (in && r + 1 < n) a[u] = __ldg(reinterpret_cast<const double2*>(src));
+            else if (in && r < n) a[u].x = __ldg(src);
+#pragma unroll
+            for (int q = 0; q < NT; ++q) v[u][q] = in && 8 * q + g < p ? __ldg(B + k + (8 * q + g) * ldb) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < kTallBatch; ++u)
+#pragma unroll
+            for (int q = 0; q < NT; ++q) {
+                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                             : "+d"(c[0][q][0]), "+d"(c[0][q][1])
+                             : "d"(a[u].x), "d"(v[u][q]));
+                asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                             : "+d"(c[1][q][0]), "+d"(c[1][q][1])
+                             : "d"(a[u].y), "d"(v[u][q]));
+            }
+    }
+#pragma unroll
+    for (int q = 0; q < NT; ++q)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) red[warp][q][2 * t + e][2 * g + h] = c[h][q][e];
+    __syncthreads();
+    for (int e = threadIdx.x; e < NT * 128; e += 32 * kTallWarps) {
+        const int row = e & 15, col = e >> 4;
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < kTallWarps; ++w) v += red[w][col >> 3][col & 7][row];
+        if (16 * blockIdx.x + row < n && col < p) C[16L * blockIdx.x + row + col * ldc] = v;
+    }
+}
+
+void tall_product(const double* A, long lda, const double* B, long ldb, int n, int p, double* C, long ldc,
+                  cudaStream_t sm) {
+    const unsigned grid = (unsigned)((n + 15) / 16);
+    auto launch = [&](auto kern, int nt) {
+        const size_t smem = sizeof(double) * kTallWarps * nt * 8 * 17;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        kern<<<grid, 32 * kTallWarps, smem, sm>>>(A, lda, B, ldb, n, p, C, ldc);
+    };
+    if (p <= 8) launch(k_tall_product<1>, 1);
+    else if (p <= 16) launch(k_tall_product<2>, 2);
+    else if (p <= 24) launch(k_tall_product<3>, 3);
+    else launch(k_tall_product<4>, 4);
+    count_launch();
+}
+
+// C += f A1 B1^T - A2 B2^T (A2 optional) with kk columns each, A1 replaced by
+// A1 - S when S is given: one pass over C (n x n), 64 x 64 tiles, 4 x 4 elements
+// per thread, the panels through shared memory eight columns at a time. Reading
+// and writing C bounds it (n = 1590, rank 7: 14 us; 29 us per update with the tile
+// kernel of the square products, and three updates where the last step has one).
+constexpr int kRankK = 8;
+__global__ void __launch_bounds__(256) k_rank_update(double* C, int n, long ld, int kk, double f,
+                                                     const double* __restrict__ A1, const double* __restrict__ S,
+                                                     const double* __restrict__ B1, const double* __restrict__ A2,
+                                                     const double* __restrict__ B2, long ldp) {
+    __shared__ double pa[2][kRankK][64], pb[2][kRankK][64];
+    const int i0 = 64 * blockIdx.x, j0 = 64 * blockIdx.y, t = threadIdx.x, ti = t & 15, tj = t >> 4;
+    double acc[4][4] = {};
+    for (int k0 = 0; k0 < kk; k0 += kRankK) {
+        for (int e = t; e < kRankK * 64; e += 256) {
+            const int k = k0 + e / 64, x = e % 64, i = i0 + x, j = j0 + x;
+            const bool ki = k < kk && i < n, kj = k < kk && j < n;
+            pa[0][e / 64][x] = ki ? f * (S ? A1[i + k * ldp] - S[i + k * ldp] : A1[i + k * ldp]) : 0.0;
+            pb[0][e / 64][x] = kj ? B1[j + k * ldp] : 0.0;
+            pa[1][e / 64][x] = ki && A2 ? -A2[i + k * ldp] : 0.0;
+            pb[1][e / 64][x] = kj && A2 ? B2[j + k * ldp] : 0.0;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (h && !A2) break;
+#pragma unroll
+            for (int k = 0; k < kRankK; ++k)
+#pragma unroll
+                for (int y = 0; y < 4; ++y) {
+                    const double b = pb[h][k][tj + 16 * y];
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) acc[x][y] = fma(pa[h][k][ti + 16 * x], b, acc[x][y]);
+                }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int y = 0; y < 4; ++y)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const int i = i0 + ti + 16 * x, j = j0 + tj + 16 * y;
+            if (i < n && j < n) C[i + j * ld] += acc[x][y];
+        }
+}
+
+void rank_update(double* C, int n, long ld, int kk, double f, const double* A1, const double* S, const double* B1,
+                 const double* A2, const double* B2, long ldp, cudaStream_t sm) {
+    const unsigned tiles = (unsigned)((n + 63) / 64);
+    k_rank_update<<<dim3(tiles, tiles), 256, 0, sm>>>(C, n, ld, kk, f, A1, S, B1, A2, B2, ldp);
+    count_launch();
+}
+
+// The Ritz vectors X = Q Wr and the squares of their residuals M X_j - theta_j X_j
+// from MQ = M Q, summed over rows [part n / kRitzParts, ..) into res[part][j]: a
+// CTA per column and part.
+constexpr int kRitzParts = 8;
+__global__ void __launch_bounds__(256) k_ritz(const double* __restrict__ Q, const double* __restrict__ MQ, long ld,
+                                              int n, int p, const double* __restrict__ Wr, int ldw,
+                                              const double* __restrict__ theta, double* X, double* res) {
+    __shared__ double red[33], w[kMaxBlock];
+    const int j = blockIdx.x, part = blockIdx.y;
+    if (threadIdx.x < kMaxBlock) w[threadIdx.x] = threadIdx.x < p ? Wr[threadIdx.x + j * ldw] : 0.0;
+    __syncthreads();
+    const double th = theta[j];
+    const int r1 = (int)((long)(part + 1) * n / kRitzParts);
     double s = 0.0;
-    for (int r = threadIdx.x; r < n; r += blockDim.x) {
-        const double d = MX[r + j * ld] - theta[j] * X[r + j * ld];
-        s += d * d;
+    for (int r = (int)((long)part * n / kRitzParts) + threadIdx.x; r < r1; r += blockDim.x) {
+        double x = 0.0, mx = 0.0;
+        for (int i = 0; i < p; i += 8) {
+            double q[8], m[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                q[u] = i + u < p ? Q[r + (i + u) * ld] : 0.0;
+                m[u] = i + u < p ? MQ[r + (i + u) * ld] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                x = fma(q[u], w[i + u], x);
+                mx = fma(m[u], w[i + u], mx);
+            }
+        }
+        X[r + j * ld] = x;
+        const double d = mx - th * x;
+        s = fma(d, d, s);
     }
     s = block_sum(s, red);
-    if (threadIdx.x == 0) res[j] = sqrt(s);
+    if (threadIdx.x == 0) res[part * kMaxBlock + j] = s;
 }
 
 // Upper triangle (00 01 02 11 12 22) of every 3 x 3 point block on the diagonal.
@@ -328,12 +540,11 @@ size_t pinv_carve(char* base, int n, int ld, PinvBuffers& b) {
     b.X = c.take<double>(blk);
     b.Y = c.take<double>(blk);
     b.MX = c.take<double>(blk);
-    b.MX2 = c.take<double>(blk);
     b.H = c.take<double>(kMaxBlock * kMaxBlock);
     b.Wr = c.take<double>(kMaxBlock * kMaxBlock);
     b.S = c.take<double>(kMaxBlock * kMaxBlock);
     b.theta = c.take<double>(kMaxBlock);
-    b.res = c.take<double>(kMaxBlock);
+    b.res = c.take<double>(kRitzParts * kMaxBlock);
     b.e = c.take<double>((size_t)n + 64);
     b.state = c.take<int>(spd_task_state_ints(n));
     b.err = c.take<int>(4);
@@ -357,7 +568,6 @@ int pinv_psd(double* M, int n, int ld, int remove_n, double eps, const PinvBuffe
     SVD_CK(cudaMemsetAsync(b.X, 0, sizeof(double) * blk, sm));
     SVD_CK(cudaMemsetAsync(b.Y, 0, sizeof(double) * blk, sm));
     SVD_CK(cudaMemsetAsync(b.MX, 0, sizeof(double) * blk, sm));
-    SVD_CK(cudaMemsetAsync(b.MX2, 0, sizeof(double) * blk, sm));
     SVD_CK(cudaMemsetAsync(b.H, 0, sizeof(double) * kMaxBlock * kMaxBlock, sm));
     SVD_CK(cudaMemsetAsync(b.Wr, 0, sizeof(double) * kMaxBlock * kMaxBlock, sm));
     SVD_CK(cudaMemsetAsync(b.S, 0, sizeof(double) * kMaxBlock * kMaxBlock, sm));
@@ -405,23 +615,24 @@ int pinv_psd(double* M, int n, int ld, int remove_n, double eps, const PinvBuffe
         k_fill_random<<<(unsigned)((tot + 255) / 256), 256, 0, sm>>>(b.X, n, ld, p, 0x5eedULL);
         count_launch();
     }
-    std::vector<double> th(p), rs(p);
+    std::vector<double> th(p), rs(kRitzParts * kMaxBlock);
     double best = DBL_MAX;
     int stall = 0, it = 0, kk = 0;
     SVD_CK(cudaMemsetAsync(b.err, 0, sizeof(int) * 2, sm));
+    const size_t cols_bytes = sizeof(double) * (size_t)((n + kOrthoCtas - 1) / kOrthoCtas) * p;
+    const size_t ortho_smem = cols_bytes <= kOrthoSharedMax ? cols_bytes : 0;
+    SVD_CK(cudaFuncSetAttribute(k_orthonormalize, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOrthoSharedMax));
     for (it = 0; it < 60; ++it) {
-        gemm_f64(n, p, n, 1.0, b.G, ld, b.X, ld, 0.0, b.Y, ld, nullptr, sm);  // Y = G X
-        k_orthonormalize<<<1, 1024, 0, sm>>>(b.Y, n, ld, p, 0x9e37ULL + (unsigned long long)it, b.err + 1);
-        count_launch();
-        gemm_f64(n, p, n, 1.0, M, ld, b.Y, ld, 0.0, b.MX, ld, nullptr, sm);  // M Q
+        tall_product(b.G, ld, b.X, ld, n, p, b.Y, ld, sm);  // Y = G X
+        k_orthonormalize<<<kOrthoCtas, kOrthoThreads, ortho_smem, sm>>>(b.Y, n, ld, p, ortho_smem > 0,
+                                                                        0x9e37ULL + (unsigned long long)it, b.err + 1);
+        tall_product(M, ld, b.Y, ld, n, p, b.MX, ld, sm);  // M Q
         k_gram<<<dim3(p, p), 256, 0, sm>>>(b.Y, ld, b.MX, ld, n, b.H, kMaxBlock);  // Q^T M Q
-        k_small_jacobi<<<1, 32, 0, sm>>>(b.H, kMaxBlock, p, b.theta, b.Wr, kMaxBlock);
-        gemm_f64(n, p, p, 1.0, b.Y, ld, b.Wr, kMaxBlock, 0.0, b.X, ld, nullptr, sm);     // Ritz vectors
-        gemm_f64(n, p, p, 1.0, b.MX, ld, b.Wr, kMaxBlock, 0.0, b.MX2, ld, nullptr, sm);  // M X
-        k_resid<<<p, 256, 0, sm>>>(b.MX2, b.X, ld, n, b.theta, b.res);
-        count_launch(3);
+        k_small_jacobi<<<1, 32 * ((p + 1) / 2), 0, sm>>>(b.H, kMaxBlock, p, b.theta, b.Wr, kMaxBlock);
+        k_ritz<<<dim3(p, kRitzParts), 256, 0, sm>>>(b.Y, b.MX, ld, n, p, b.Wr, kMaxBlock, b.theta, b.X, b.res);
+        count_launch(4);
         SVD_CK(cudaMemcpyAsync(th.data(), b.theta, sizeof(double) * p, cudaMemcpyDeviceToHost, sm));
-        SVD_CK(cudaMemcpyAsync(rs.data(), b.res, sizeof(double) * p, cudaMemcpyDeviceToHost, sm));
+        SVD_CK(cudaMemcpyAsync(rs.data(), b.res, sizeof(double) * rs.size(), cudaMemcpyDeviceToHost, sm));
         SVD_CK(cudaStreamSynchronize(sm));
         if (remove_n > 0) {
             kk = remove_n;
@@ -430,7 +641,12 @@ int pinv_psd(double* M, int n, int ld, int remove_n, double eps, const PinvBuffe
             for (int j = 0; j < p; ++j) kk += fabs(th[j]) <= eps;
         }
         double conv = 0.0;
-        for (int j = 0; j < std::max(kk, 1); ++j) conv = std::max(conv, rs[j]);
+        for (int j = 0; j < std::max(kk, 1); ++j) {
+            double sq = 0.0;
+            for (int q = 0; q < kRitzParts; ++q) sq += rs[q * kMaxBlock + j];
+            conv = sq <= DBL_MAX ? std::max(conv, std::sqrt(sq)) : HUGE_VAL;
+            if (conv > DBL_MAX) break;
+        }
         if (!(conv <= DBL_MAX)) return svd_fail(UNC_ERR_SINGULAR, "non-finite Ritz residual");
         inf.residual = conv;
         // stop once the residuals of the removed vectors no longer shrink
@@ -469,17 +685,15 @@ int pinv_psd(double* M, int n, int ld, int remove_n, double eps, const PinvBuffe
         return svd_fail(UNC_ERR_SINGULAR, "the matrix has more (near-)null directions than are removed");
 
     // 3. B = M + c V_R V_R^T, inverted in place
-    gemm_f64_mode(n, n, kk, c, b.X, ld, b.X, ld, 1.0, M, ld, nullptr, GEMM_TRANS_B, sm);
+    rank_update(M, n, ld, kk, c, b.X, nullptr, b.X, nullptr, nullptr, ld, sm);
     if (int rc = inverse_in_place(M, n, ld, b, sm)) return rc;
 
     // 4. P B^{-1} P = B^{-1} - Z V^T - V Z^T + V (V^T Z) V^T, Z = B^{-1} V
-    gemm_f64(n, kk, n, 1.0, M, ld, b.X, ld, 0.0, b.Y, ld, nullptr, sm);
+    tall_product(M, ld, b.X, ld, n, kk, b.Y, ld, sm);
     k_gram<<<dim3(kk, kk), 256, 0, sm>>>(b.X, ld, b.Y, ld, n, b.S, kMaxBlock);
     count_launch();
-    gemm_f64_mode(n, n, kk, -1.0, b.Y, ld, b.X, ld, 1.0, M, ld, nullptr, GEMM_TRANS_B, sm);
-    gemm_f64_mode(n, n, kk, -1.0, b.X, ld, b.Y, ld, 1.0, M, ld, nullptr, GEMM_TRANS_B, sm);
     gemm_f64(n, kk, kk, 1.0, b.X, ld, b.S, kMaxBlock, 0.0, b.MX, ld, nullptr, sm);
-    gemm_f64_mode(n, n, kk, 1.0, b.MX, ld, b.X, ld, 1.0, M, ld, nullptr, GEMM_TRANS_B, sm);
+    rank_update(M, n, ld, kk, 1.0, b.MX, b.Y, b.X, b.X, b.Y, ld, sm);
     SVD_CK(cudaGetLastError());
     return UNC_OK;
 }
