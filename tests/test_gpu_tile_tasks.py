@@ -39,6 +39,17 @@ def test_task_inverse_matches_numpy(n):
     assert np.max(np.abs(got - got.T)) / np.max(np.abs(ref)) < TOL  # both triangles written
 
 
+@pytest.mark.parametrize("n", [1920, 1921, 2368, 2369, 2624, 2625])
+def test_task_inverse_at_group_sizes(n):
+    """Either side of the tile counts at which tasks take one, two, three and four terms; the
+    condition number is about 5, so a few n eps bound the error."""
+    A = _spd(n, n)
+    got = _inverse(A)
+    ref = np.linalg.inv(A)
+    assert np.max(np.abs(got - ref)) / np.max(np.abs(ref)) < TOL
+    np.testing.assert_array_equal(got, _inverse(A))
+
+
 def test_task_inverse_bitwise_repeatable():
     A = _spd(700, 7)
     first = _inverse(A)

@@ -200,14 +200,15 @@ __device__ __forceinline__ void chol_leaf_load(const double* A, long lda, int k0
 // Factorisation of the block in S (after chol_leaf_load and a barrier), T_kk
 // in Ts (lower 16 x 16 blocks, the diagonal ones with zeros above the diagonal)
 // and written to T at (k0, k0). One CTA of LEAF_THREADS threads. Warp 4 calls
-// beside(q) during panel q: the caller's own work (no block barrier in it).
-template <class F>
+// beside(q) during panel q, all threads last() after the panels: the caller's own work
+// (no block barrier in it).
+template <class F, class G>
 __device__ __forceinline__ void chol_leaf_factor(int k0, int kb, double* T, long ldt, int* err, double* S, double* Ts,
-                                                 F&& beside) {
+                                                 F&& beside, G&& last) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
     // the warps beside (A): 1, 2, 3, 5, 6, 7 (warp 4 shares warp 0's scheduler and FP64 pipe)
     const int worker = warp < 4 ? warp - 1 : warp - 2;
-    constexpr int kWorkers = 6, kSideThreads = LEAF_THREADS - 32;
+    constexpr int kWorkers = 6;
     auto S_ = [S](int r, int c) { return leaf_block(S, r, c); };
     auto T_ = [Ts](int r, int c) { return leaf_block(Ts, r, c); };
 #pragma unroll 1
@@ -216,7 +217,6 @@ __device__ __forceinline__ void chol_leaf_factor(int k0, int kb, double* T, long
             leaf_panel(S_(q, q), T_(q, q), lane, err);
         } else if (warp == 4) {
             beside(q);
-            if (q > 0) named_barrier(1, kSideThreads);
         } else if (q > 0) {
             // beside panel q: the updates of panel p = q - 1 that panel q does not need
             const int p = q - 1;
@@ -238,7 +238,7 @@ __device__ __forceinline__ void chol_leaf_factor(int k0, int kb, double* T, long
                         if (item++ % kWorkers == worker)
                             leaf_gather(T_(i, p), S_(i, p), T_(p, p), true, f & 1, f >> 1, g, t);
             }
-            named_barrier(1, kSideThreads);
+            named_barrier(1, 32 * kWorkers);
             {
                 int item = 0;
                 for (int i = q; i < 4; ++i)
@@ -257,6 +257,7 @@ __device__ __forceinline__ void chol_leaf_factor(int k0, int kb, double* T, long
         if (warp < 3) leaf_update(S_(q + 1, q + 1), S_(q + 1, q), S_(q + 1, q), warp > 0, warp > 1, g, t);
         __syncthreads();
     }
+    last();
     for (int s = warp; s < 6; s += LEAF_THREADS / 32) leaf_finish(T_(3, s >> 1), T_(3, 3), s & 1, g, t);
     __syncthreads();
     const int i = tid & (NB - 1);
@@ -272,7 +273,7 @@ __device__ __forceinline__ void chol_leaf_tile(const double* A, long lda, int k0
                                                int* err, double* lsm) {
     chol_leaf_load(A, lda, k0, kb, lsm);
     __syncthreads();
-    chol_leaf_factor(k0, kb, T, ldt, err, lsm, lsm + LEAF_TILE, [](int) {});
+    chol_leaf_factor(k0, kb, T, ldt, err, lsm, lsm + LEAF_TILE, [](int) {}, [] {});
 }
 
 }  // namespace unc

@@ -64,7 +64,7 @@ constexpr int SLICE = 32, STREAM_STAGES = 3;      // k of a slice
 constexpr int SLD = SLICE + 4;                    // stride of a slice of rows (k contiguous)
 constexpr int SLOT = TB * SLD > SLICE * TLD ? TB * SLD : SLICE * TLD;  // doubles of one operand's slice
 constexpr size_t DAG_SMEM = sizeof(double) * (2 * STREAM_STAGES * SLOT > 3 * LEAF_TILE ? 2 * STREAM_STAGES * SLOT : 3 * LEAF_TILE);
-constexpr int GROUP = 4;                          // consecutive k of a group
+constexpr int MAX_GROUP = 4;                      // consecutive k of a group, at most
 constexpr long kDagSpin = 1L << 22;      // polls of one dependency before the kernel gives up
 constexpr int kMaxTilesN = 56;           // tasks are used up to n = 56 * 64
 
@@ -270,6 +270,14 @@ struct TaskMatrix {
     }
 };
 
+// The lower 8 x 8 blocks of a 64 x 64 tile dealt to eight warps, four or five each and
+// nine or ten to the two warps of a scheduler (its FP64 pipe takes one DMMA per 16
+// cycles; n = 1351: 364 -> 350 us): nibbles 0 and 1 the block rows of slots 0-2 and
+// 3-4, nibbles 2-6 the block columns of the slots, nibble 7 whether slot 4 is used.
+// Warp 6 repeats its slot 1 as slot 2. Two warps of a scheduler with 32 x 16 blocks took 16.
+__constant__ const unsigned kDiagBlocks[8] = {0x14321077u, 0x14321066u, 0x14321055u, 0x14321044u,
+                                              0x03321033u, 0x00021002u, 0x16511061u, 0x05576557u};
+
 // POTRF(k): A(k,k) -= L(k,k-1) L(k,k-1)^T, the leaf, T(k,k) published, then
 // L(k+1,k) = A(k+1,k) T(k,k)^T with T(k,k) still in shared memory (Bs), published.
 // A(k+1,k) is fetched beside the leaf once its updates are in. chained: called
@@ -278,7 +286,9 @@ struct TaskMatrix {
 // flag: three shared ints. False when a wait gave up.
 __device__ bool potrf(const TaskMatrix& m, int k, bool chained, bool& diag_in, double* sm, int* flag) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
-    const int wm = (warp & 1) * 32, wn = (warp >> 1) * 16;
+    // column blocks 0, 16, 48, 32: the product with a lower triangle takes warps w and
+    // w + 4, which share a scheduler, the same time in sum
+    const int wm = (warp & 1) * 32, wn = ((warp >> 1) ^ (warp >> 2)) * 16;
     double *As = sm, *Bs = sm + LEAF_TILE, *S = sm + 2 * LEAF_TILE;
     const bool below = k + 1 < m.tiles();
     if (chained && k > 0 && !diag_in) {
@@ -290,30 +300,51 @@ __device__ bool potrf(const TaskMatrix& m, int k, bool chained, bool& diag_in, d
     if (k > 0 && !chained) load_tile(As, m.tile(m.A, k, k - 1), m.ld, m.ext(k), m.ext(k - 1), tid);
     tile_wait();
     __syncthreads();
-    Acc acc = {};
     if (k > 0) {
-        if (wn < wm + 32) tile_mma(As, As, wm, wn, g, t4, 0, TB, acc);  // lower blocks only
-        tile_elements(TB, TB, wm, wn, g, t4, acc, [&](int r, int c, double& v) {
-            if (c <= r) S[c * TLD + r] -= v;
-        });
+        // S -= As As^T, lower 8 x 8 blocks only, four or five per warp (kDiagBlocks)
+        const unsigned tab = kDiagBlocks[warp];
+        const int rows[2] = {(int)(tab & 7u) * 8, (int)(tab >> 4 & 7u) * 8};
+        const bool five = (tab >> 28) != 0u;
+        int cols[5];
+        double c[5][2], d[5][2];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            cols[q] = (int)(tab >> (8 + 4 * q) & 7u) * 8;
+            c[q][0] = c[q][1] = 0.0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) d[q][h] = S[(cols[q] + 2 * t4 + h) * TLD + rows[q / 3] + g];
+        }
+#pragma unroll 4
+        for (int kk = 0; kk < TB; kk += 4) {
+            const double* at = As + (kk + t4) * TLD + g;
+            const double a[2] = {at[rows[0]], at[rows[1]]};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) dmma(c[q][0], c[q][1], a[q / 3], at[cols[q]]);
+            if (five) dmma(c[4][0], c[4][1], a[1], at[cols[4]]);
+        }
+#pragma unroll
+        for (int q = 0; q < 5; ++q)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int col = cols[q] + 2 * t4 + h, row = rows[q / 3] + g;
+                if (col <= row && (q < 4 || five) && !(q == 2 && cols[2] == cols[1]))
+                    S[col * TLD + row] = d[q][h] - c[q][h];
+            }
     }
     if (tid == 0) flag[0] = 0;
     __syncthreads();
-    // warp 4: A(k+1,k) into As in two halves of 32 columns, beside two panels (a
-    // whole tile takes this one warp longer than a panel)
-    int halves = 0;
-    chol_leaf_factor(TB * k, m.ext(k), m.T, m.ld, m.err, S, Bs, [&](int q) {
-        if (!below || halves == 2 || q == 0) return;
-        if (halves == 0) {
-            int ready = 0;
-            if (lane == 0) ready = ld_acquire(m.ver + tri(k + 1, k)) >= k;
-            if (!__shfl_sync(0xffffffffu, ready, 0)) return;
-            if (lane == 0) flag[0] = 1;
-        }
-        for (const int stop = q == 3 ? 2 : halves + 1; halves < stop; ++halves)
-            load_tile(As + halves * 32 * TLD, m.tile(m.A, k + 1, k) + halves * 32 * m.ld, m.ld, m.ext(k + 1),
-                      m.ext(k) - halves * 32, lane, 32, 32);
-    });
+    // A(k+1,k) into As before the leaf's last products when warp 4 has seen its updates
+    // (one warp's loads of a tile take longer than a panel: 1.8 us more per step)
+    chol_leaf_factor(
+        TB * k, m.ext(k), m.T, m.ld, m.err, S, Bs,
+        [&](int q) {
+            if (!below || q < 2) return;
+            for (int poll = q; poll < 5; poll += 2)  // the last panel: twice
+                if (lane == 0 && !flag[0] && ld_acquire(m.ver + tri(k + 1, k)) >= k) flag[0] = 1;
+        },
+        [&] {
+            if (flag[0]) load_tile(As, m.tile(m.A, k + 1, k), m.ld, m.ext(k + 1), m.ext(k), tid);
+        });
     tile_wait();
     __syncthreads();
     if (tid == 0) {
@@ -335,10 +366,7 @@ __device__ bool potrf(const TaskMatrix& m, int k, bool chained, bool& diag_in, d
     __syncthreads();
     diag_in = flag[2];
     if (diag_in) load_tile(S, m.tile(m.A, k + 1, k + 1), m.ld, TB, TB, tid);
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
+    Acc acc = {};
     tile_mma(As, Bs, wm, wn, g, t4, 0, wn + 16, acc);
     if (chained) {
         __syncthreads();  // As is read no more
@@ -347,7 +375,7 @@ __device__ bool potrf(const TaskMatrix& m, int k, bool chained, bool& diag_in, d
     double* L = m.tile(m.A, k + 1, k);
     tile_elements(m.ext(k + 1), m.ext(k), wm, wn, g, t4, acc, [&](int r, int c, double& v) { L[r + (long)c * m.ld] = v; });
     __syncthreads();
-    if (tid == 0) {
+    if (tid == 32 * 5) {  // warp 5: its share of the next update is short
         __threadfence();
         atomicExch(m.lrdy + tri(k + 1, k), 1);
     }
@@ -528,24 +556,37 @@ __global__ void __launch_bounds__(DAG_THREADS, DAG_CTAS)
     }
 }
 
+// Consecutive terms of one tile that a task takes, by the number of tiles: the
+// work of a step grows with nt^2, the chain's time for it does not. While the
+// CTAs keep up with single terms a group only delays its tile; beyond that the
+// longer groups save the CTAs a load and a store of the tile per term. Single,
+// pairs, threes and fours, with the product (us): n = 1800 505, 525, 539, 572;
+// 2300 816, 700, 725, 794; 2432 951, 808, 787, 845; 2752 1355, 1130, 1076, 1056.
+// Without the product a step has about two thirds of the work: n = 1984 497, 510,
+// 534, 550; 2400 714, 649, 667, 728; 2701 969, 841, 834, 863; 3584 1994, 1645,
+// 1566, 1538.
+int group_size(int nt, bool product) {
+    const int load = product ? nt : nt - 4;
+    return load <= 30 ? 1 : load <= 37 ? 2 : load <= 41 ? 3 : MAX_GROUP;
+}
+
 // The task list of nt x nt tiles in the order described above; without the
 // product, T = L^{-1} only (no PACC). At step s panel s, T's row s - 1 and the
-// product terms of T's row s become available. A tile that is not needed in the
-// next two steps takes its terms in groups of GROUP, whose ends fall on another
-// step for each of GROUP neighbouring tiles, so that every step has its share of
-// them and none floods the CTAs that the chain waits for; one that is needed in
-// the step after next takes the rest of its group, so that only a single term is
-// left when the next step waits for it. The last two product terms are single
-// ones (a short tail). Below kGroupTiles the CTAs keep up with single terms and a
-// group would only delay its tile (n = 600: 173 us single, 188 us in groups; equal at 1800;
-// n = 2752: 1606 and 1102 us).
-constexpr int kGroupTiles = 32;
+// product terms of T's row s - 1 become available (T's row s is final at the end
+// of step s: its product terms come a step later, where they do not wait for it;
+// n = 1800: 562 -> 504 us). A tile that is not needed in the next two steps takes
+// its terms in groups, whose ends fall on another step for each of the group's
+// size of neighbouring tiles, so that every step has its share of them and none
+// floods the CTAs that the chain waits for; one that is needed in the step after
+// next takes the rest of its group, so that only a single term is left when the
+// next step waits for it. The last two product terms are single ones (a short
+// tail).
 std::vector<int4> build_tasks(int nt, bool product = true) {
     std::vector<int4> v;
     auto add = [&v](int ty, int i, int j, int first, int last) {
         v.push_back(make_int4(ty, i, j, first | (last - first + 1) << 16));
     };
-    const int size = nt < kGroupTiles ? 1 : GROUP;
+    const int size = group_size(nt, product);
     // tile (i, j): terms first_of(i, j, s) .. s are one group at step s when ends(i, j, s)
     auto ends = [size](int i, int j, int s) { return (s + i + j) % size == size - 1; };
     auto first_of = [size](int i, int j, int s) { return std::max(0, s - (s + i + j) % size); };
@@ -573,12 +614,13 @@ std::vector<int4> build_tasks(int nt, bool product = true) {
                     if (r == s + 1 || ends(r, c, p)) add(K_TACC, r, c, std::max(c, first_of(r, c, p)), p);
         }
         for (int c = 0; c < s; ++c) add(K_TFIN, s, c, 0, 0);
-        for (int r = 0; product && r <= s; ++r)
-            for (int c = 0; c <= r; ++c) {
-                const bool last = s == nt - 1;
-                if (last || s == nt - 2 || ends(r, c, s))
-                    add(K_PACC, r, c, last ? s : std::max(r, first_of(r, c, s)), s);
-            }
+        for (int k = s - 1; product && k <= (s == nt - 1 ? s : s - 1); ++k)
+            for (int r = 0; r <= k; ++r)
+                for (int c = 0; c <= r; ++c) {
+                    const bool last = k == nt - 1;
+                    if (last || k == nt - 2 || ends(r, c, k))
+                        add(K_PACC, r, c, last ? k : std::max(r, first_of(r, c, k)), k);
+                }
     }
     return v;
 }
