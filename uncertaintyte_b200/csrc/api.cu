@@ -180,8 +180,8 @@ size_t carve(char* base, const Plan& pl, bool host_io, long long nnz, int nrows,
     s.is_cam = c.take<double>((size_t)pl.C * 9);
     s.Vraw = c.take<double>((size_t)pl.P * 6);
     s.Mp = c.take<double>((size_t)pl.P * 6);
-    s.Q = c.take<double>((size_t)pl.nobs * 27);
-    s.cam_part = c.take<double>(45 * camera_tile_slots(pl.C, pl.nobs));
+    s.Q = c.take<double>(((size_t)pl.nobs + 1) * 27);
+    s.cam_part = c.take<double>(90 * camera_tile_slots(pl.C, pl.nobs));
     s.Ucam = c.take<double>(81 * (size_t)pl.C);
     s.err = c.take<int>(4);
     b.amax = c.take<unsigned long long>(4);

@@ -434,16 +434,47 @@ __device__ __forceinline__ void ut9_inv(int el, int& j, int& k) {
 }
 
 // One pass over the tile's Jacobian records:
-//   * the partial sums of U = sum_o Jc_o^T Jc_o: the six upper 3 x 3 blocks by
-//     six lanes of a warp (18 multiply-adds per 12 shared reads), four
-//     observations per warp at a time, the partials added over lanes, then warps;
+//   * the partial sums of U = sum_o Jc_o^T Jc_o;
 //   * Q_o = W_o M_p, W_o = Jc_o^T Jp_o, M_p M_p^T = the inverse of the point's
 //     block (k_point_blocks): the record the Schur complement reads, not yet
 //     scaled by the camera's column norms. Written in position order, so the
-//     tile's records are one contiguous store of 27 doubles each.
-// The records (192 bytes in, 216 out per observation) bound the kernel.
+//     tile's records are one contiguous store of 27 doubles each;
+//   * the partial sums of Q_o Q_o^T, the self terms of the Schur complement's
+//     diagonal block (formed here, where the records are in shared memory, and
+//     not in the column kernel: 29 us of a column's first CTA at 200 cameras).
+// Shared-memory instructions and the latency of the scattered records bound the
+// kernel (192 bytes in and 216 out per observation are 22 us at 342,000), so both
+// sums are outer products on the FP64 tensor cores: a third of the reads (57 us at
+// that size; as much for U alone with ordinary multiply-adds).
 constexpr size_t kCamTileSmem = sizeof(double) * kObsTile * 27;
 static_assert(27 >= kRecStride, "the staged records fit the Q records' space");
+
+// sum_k x_k x_k^T over k in [k0, k1), a multiple of 4 apart, x_k in R^9, by one warp:
+// x(k, e) is element e of x_k. out: the 45 upper elements.
+template <class F>
+__device__ __forceinline__ void outer_sum(int k0, int k1, F&& x, double* out) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    double c[2] = {0.0, 0.0}, row = 0.0, corner = 0.0;
+#pragma unroll 4
+    for (int k = k0 + t; k < k1; k += 4) {
+        const double a = x(k, g), a8 = x(k, 8);
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                     : "+d"(c[0]), "+d"(c[1])
+                     : "d"(a), "d"(a));
+        row = fma(a8, a, row);
+        corner = fma(a8, a8, corner);
+    }
+#pragma unroll
+    for (int d = 1; d < 4; d <<= 1) {
+        row += __shfl_xor_sync(0xffffffffu, row, d);
+        corner += __shfl_xor_sync(0xffffffffu, corner, d);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        if (g >= 2 * t + h) out[ut9(2 * t + h, g)] = c[h];
+    if (t == 0) out[ut9(g, 8)] = row;
+    if (lane == 0) out[ut9(8, 8)] = corner;
+}
 
 __global__ void __launch_bounds__(kObsTile, 2)
     k_camera_tiles(int num_cams, const double* __restrict__ J, const int* __restrict__ cam_ptr,
@@ -451,10 +482,10 @@ __global__ void __launch_bounds__(kObsTile, 2)
                    double* __restrict__ part, double* __restrict__ Q) {
     extern __shared__ __align__(16) double sj[];
     __shared__ int ids[kObsTile];
-    __shared__ double red[kObsTile / 32][54];
+    __shared__ double red[kObsTile / 32][2][45];
     ObsTile tile;
     if (!find_tile(cam_ptr, num_cams, blockIdx.x, tile)) return;
-    const int n = tile.end - tile.begin, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int n = tile.end - tile.begin, t = threadIdx.x, warp = t >> 5;
     stage_records(sj, ids, J, cam_obs, tile);
     double m[6] = {0, 0, 0, 0, 0, 0};
     if (t < n) {
@@ -467,33 +498,12 @@ __global__ void __launch_bounds__(kObsTile, 2)
             m[2 * k + 1] = v.y;
         }
     }
-    double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    if (lane < 24) {
-        const int sub = lane % 6, grp = lane / 6;
-        const int bj = sub < 3 ? 0 : (sub < 5 ? 1 : 2), bk = sub < 3 ? sub : (sub < 5 ? sub - 2 : 2);
-        for (int i = 4 * warp + grp; i < n; i += kObsTile / 8) {
-            const double* r = sj + i * kRecStride;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                double x[3], y[3];
-#pragma unroll
-                for (int a = 0; a < 3; ++a) {
-                    x[a] = r[12 * h + 3 * bj + a];
-                    y[a] = r[12 * h + 3 * bk + a];
-                }
-#pragma unroll
-                for (int a = 0; a < 3; ++a)
-#pragma unroll
-                    for (int b = 0; b < 3; ++b) acc[3 * a + b] = fma(x[a], y[b], acc[3 * a + b]);
-            }
-        }
-    }
-#pragma unroll
-    for (int e = 0; e < 9; ++e) {  // over the four observations of the warp (lanes 6 apart; 24.. hold zeros)
-        acc[e] += __shfl_down_sync(0xffffffffu, acc[e], 12);
-        acc[e] += __shfl_down_sync(0xffffffffu, acc[e], 6);
-        if (lane < 6) red[warp][9 * lane + e] = acc[e];
-    }
+    // U: k = 2 observation + row
+    const int i0 = 32 * warp;
+    outer_sum(2 * i0, 2 * (i0 + 32), [&](int k, int e) {
+        const int i = k >> 1;
+        return i < n ? sj[i * kRecStride + 12 * (k & 1) + e] : 0.0;
+    }, red[warp][0]);
     double q[27];
     if (t < n) {
         const double* r = sj + t * kRecStride;
@@ -512,40 +522,46 @@ __global__ void __launch_bounds__(kObsTile, 2)
 #pragma unroll
         for (int e = 0; e < 27; ++e) sj[27 * t + e] = q[e];
     }
-    if (t < 45) {
-        int j, k;
-        ut9_inv(t, j, k);
-        const int bj = j / 3, bk = k / 3, sub = bj == 0 ? bk : (bj == 1 ? bk + 2 : 5);
-        const int e = 9 * sub + 3 * (j % 3) + k % 3;
-        double v = red[0][e];
-        for (int w = 1; w < kObsTile / 32; ++w) v += red[w][e];
-        part[45L * blockIdx.x + t] = v;
-    }
     __syncthreads();
     double* out = Q + 27L * tile.begin;
     for (int i = t; i < 27 * n; i += kObsTile) out[i] = sj[i];
+    // the self terms: k = 3 observation + component
+    outer_sum(3 * i0, 3 * (i0 + 32), [&](int k, int e) {
+        const int i = k / 3;
+        return i < n ? sj[24 * i + k + 3 * e] : 0.0;
+    }, red[warp][1]);
+    __syncthreads();
+    if (t < 90) {
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < kObsTile / 32; ++w) v += red[w][t / 45][t % 45];
+        part[90L * blockIdx.x + t] = v;
+    }
 }
 
 // One warp per camera: U = sum of the camera's tile partials, column norms
-// s = sqrt(diag U), scaled block U/(s s) written as a full 9 x 9 block
-// (column-major, 81 per camera). J <- J diag(1/s) skips s == 0
+// s = sqrt(diag U), scaled block U/(s s) less the scaled self terms, written as a
+// full 9 x 9 block (column-major, 81 per camera). J <- J diag(1/s) skips s == 0
 // (ScaledSparseMatrix.cpp:352-356).
 __global__ void __launch_bounds__(128) k_camera_gram_reduce(int num_cams, const int* __restrict__ cam_ptr,
                                                             const double* __restrict__ part, double* __restrict__ s_cam,
-                                                            double* __restrict__ is_cam, double* __restrict__ U) {
-    __shared__ double sh[4][45];
+                                                            double* __restrict__ is_cam, double* __restrict__ U,
+                                                            double* __restrict__ zero_record) {
+    __shared__ double sh[4][90];
+    if (blockIdx.x == 0 && threadIdx.x < 27) zero_record[threadIdx.x] = 0.0;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int cam = blockIdx.x * 4 + w;
     if (cam >= num_cams) return;
     const int k0 = tile_base(cam_ptr, cam), k1 = tile_base(cam_ptr, cam + 1);
-    double a0 = 0.0, a1 = 0.0;
-    for (int k = k0; k < k1; ++k) {
-        a0 += part[45L * k + lane];
-        if (lane < 13) a1 += part[45L * k + 32 + lane];
-    }
+    double a[3] = {0.0, 0.0, 0.0};
+    for (int k = k0; k < k1; ++k)
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+            if (32 * q + lane < 90) a[q] += part[90L * k + 32 * q + lane];
     double* u = sh[w];
-    u[lane] = a0;
-    if (lane < 13) u[32 + lane] = a1;
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+        if (32 * q + lane < 90) u[32 * q + lane] = a[q];
     __syncwarp();
     if (lane < 9) {
         const double v = sqrt(u[ut9(lane, lane)]);
@@ -556,9 +572,10 @@ __global__ void __launch_bounds__(128) k_camera_gram_reduce(int num_cams, const 
         int j, k;
         ut9_inv(el, j, k);
         const double sj = sqrt(u[ut9(j, j)]), sk = sqrt(u[ut9(k, k)]);
-        double v = u[el];
-        if (sj != 0) v *= 1.0 / sj;
-        if (sk != 0) v *= 1.0 / sk;
+        double v = u[el], self = u[45 + el];
+        if (sj != 0) v *= 1.0 / sj, self *= 1.0 / sj;
+        if (sk != 0) v *= 1.0 / sk, self *= 1.0 / sk;
+        v -= self;
         U[81L * cam + j + 9 * k] = v;
         U[81L * cam + k + 9 * j] = v;
     }
@@ -571,7 +588,7 @@ void launch_camera_blocks(const SceneDev& s, cudaStream_t st) {
     k_camera_tiles<<<slots, kObsTile, kCamTileSmem, st>>>(s.num_cams, s.J, s.cam_ptr, s.cam_obs, s.obs_pt, s.Mp, s.cam_part,
                                                           s.Q);
     k_camera_gram_reduce<<<(s.num_cams + 3) / 4, 128, 0, st>>>(s.num_cams, s.cam_ptr, s.cam_part, s.s_cam, s.is_cam,
-                                                                s.Ucam);
+                                                                s.Ucam, s.Q + 27L * s.num_obs);
     count_launch(2);
 }
 

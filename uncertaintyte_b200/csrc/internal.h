@@ -115,7 +115,7 @@ struct SceneDev {
     double* Mp;           // 6*num_points M_p, M_p M_p^T = V_p^{-1} (k_point_blocks), or nullptr
     double* Q;            // 27*num_obs by position: Q_o = W_o M_p, 9x3 row-major (W_o = J_c^T J_p); after the
                           // Schur stage 6 per position: the observation's share of its point's covariance
-    double* cam_part;     // 45 * camera_tile_slots(): per-tile partial sums of the camera blocks
+    double* cam_part;     // 90 * camera_tile_slots(): per-tile partial sums of the camera blocks and self terms
     double* Ucam;         // 81*num_cams scaled camera blocks U (9 x 9, column-major)
     int* err;             // device error bits
 };

@@ -20,9 +20,9 @@
 //     covers the rows of one or two records (216 bytes each), where a thread per
 //     row of a record made each touch thirty cache lines: the record loads bound
 //     the kernel. The block is stored (subtracted from U on the diagonal, read
-//     back and updated for the second and later chunks). The self terms
-//     Q_o' Q_o'^T of the diagonal block are summed by all warps over contiguous
-//     ranges and added in warp order.
+//     back and updated for the second and later chunks). U comes with the self
+//     terms Q_o' Q_o'^T of the diagonal block already subtracted
+//     (k_camera_tiles); only a camera that sees a point twice adds to it here.
 // Scenes with few cameras split every column over several CTAs (camera ca's
 // block to CTA (cb - ca) mod parts, in every chunk), so that the grid covers
 // the SMs.
@@ -40,12 +40,13 @@ constexpr int kSzWarps = kSzThreads / 32;
 constexpr int kSzChunk = 2048;        // owner observations per chunk, at most
 constexpr int kSzParts = 8192;        // partner entries per chunk, at most
 constexpr int kSzMaskWords = 6144;    // run-mask words (also the entries' owners and the camera scan)
-constexpr int kSzSegCap = 256;        // run entries staged per warp at a time
+constexpr int kSzPad = 16;            // terms past the end of a run that its steps read
+constexpr int kSzSegCap = 256 - kSzPad;  // run entries staged per warp at a time
 constexpr unsigned short kNoSlot = 0xFFFF;
 
 static_assert(kSzMaskWords >= kSchurMaxCams, "the camera scan reuses the mask words");
 static_assert(kSzMaskWords * 2 >= kSzParts, "the entries' owners (16-bit) reuse the mask words");
-static_assert(kSzWarps * kSzSegCap * 2 >= kSzChunk, "the point-list starts reuse the run buffers");
+static_assert(kSzWarps * (kSzSegCap + kSzPad) * 2 >= kSzChunk, "the point-list starts reuse the run buffers");
 static_assert(kSzParts <= 65536 && kSzChunk <= 65536, "owners are 16-bit");
 static_assert(kSchurMaxCams < kNoSlot, "slot ids are 16-bit");
 
@@ -57,15 +58,14 @@ struct SzShared {
     unsigned short* slot_of;      // [C] slot of a camera, kNoSlot when none
     unsigned short* cam_of_slot;  // [C]
     int* tmp;             // [kSzWarps + 4] scan scratch and broadcast words
-    double* self;         // [kSzWarps][45] the chunk's self terms: the warps' sums, then their sum in [0]
-    int2* runbuf;         // [kSzWarps][kSzSegCap] staged run entries (partner, owner), one buffer per warp
+    uint2* runbuf;        // [kSzWarps][kSzSegCap + kSzPad] staged terms (partner, owner), one buffer per warp
     int* sb;              // [kSzChunk] start of each observation's partners (aliases runbuf)
     unsigned short* seg;  // [kSzParts] observation of each entry (aliases mask)
 };
 
 // Shared-memory layout (byte offsets; every array starts 16-byte aligned).
 struct SzOffsets {
-    size_t mask, off, part_o, tmp, self, runbuf, part_c, slot_of, cam_of_slot, total;
+    size_t mask, off, part_o, tmp, runbuf, part_c, slot_of, cam_of_slot, total;
 };
 __host__ __device__ constexpr size_t sz_align(size_t x) { return (x + 15) & ~size_t(15); }
 __host__ __device__ inline SzOffsets sz_offsets(int C) {
@@ -74,9 +74,8 @@ __host__ __device__ inline SzOffsets sz_offsets(int C) {
     o.off = sz_align(o.mask + sizeof(unsigned) * kSzMaskWords);
     o.part_o = sz_align(o.off + sizeof(int) * (kSzChunk + 1));
     o.tmp = sz_align(o.part_o + sizeof(int) * kSzParts);
-    o.self = sz_align(o.tmp + sizeof(int) * (kSzWarps + 4));
-    o.runbuf = sz_align(o.self + sizeof(double) * 45 * kSzWarps);
-    o.part_c = sz_align(o.runbuf + sizeof(int2) * kSzWarps * kSzSegCap);
+    o.runbuf = sz_align(o.tmp + sizeof(int) * (kSzWarps + 4));
+    o.part_c = sz_align(o.runbuf + sizeof(uint2) * kSzWarps * (kSzSegCap + kSzPad));
     o.slot_of = sz_align(o.part_c + sizeof(unsigned short) * kSzParts);
     o.cam_of_slot = sz_align(o.slot_of + sizeof(unsigned short) * (size_t)C);
     o.total = sz_align(o.cam_of_slot + sizeof(unsigned short) * (size_t)C);
@@ -90,8 +89,7 @@ __device__ __forceinline__ SzShared sz_layout(char* base, int C) {
     s.off = reinterpret_cast<int*>(base + o.off);
     s.part_o = reinterpret_cast<int*>(base + o.part_o);
     s.tmp = reinterpret_cast<int*>(base + o.tmp);
-    s.self = reinterpret_cast<double*>(base + o.self);
-    s.runbuf = reinterpret_cast<int2*>(base + o.runbuf);
+    s.runbuf = reinterpret_cast<uint2*>(base + o.runbuf);
     s.part_c = reinterpret_cast<unsigned short*>(base + o.part_c);
     s.slot_of = reinterpret_cast<unsigned short*>(base + o.slot_of);
     s.cam_of_slot = reinterpret_cast<unsigned short*>(base + o.cam_of_slot);
@@ -133,34 +131,35 @@ __device__ int sz_scan(int* a, int n, int* tmp) {
 // The sum of Q_P Q_O^T over the terms of a run, by one warp: lane (g, t) holds
 // C(g, 2t), C(g, 2t + 1) in c, and its share (its k) of C(8, g), C(g, 8) and
 // C(8, 8) in row, col, corner. Four terms are k = 12: three DMMA steps, lane t's
-// k of step s being 4 s + t (component k % 3 of term k / 3).
+// k of step s being 4 s + t (component k % 3 of term k / 3). A term is the two
+// records' positions; terms past the end of a run name the zero record, so that a
+// load is one address and no test. The loads' latency bounds a run: two steps are
+// in flight while one is summed (200 cameras, 60 terms per block: the kernel
+// 230 -> 202 us with the tests gone, the second step ahead and the self terms summed
+// where the records are made).
 struct SzSum {
-    int g, t, q[3], at[3], at8[3];  // per step: term, offset of its element of row g and of row 8
+    int g, t, q[3];
+    const double *at[3], *at8[3];  // per step: the lane's element of row g and of row 8 of record 0
     double c[2] = {0.0, 0.0}, row = 0.0, col = 0.0, corner = 0.0;
 
-    __device__ explicit SzSum(int lane) : g(lane >> 2), t(lane & 3) {
+    __device__ SzSum(int lane, const double* Q) : g(lane >> 2), t(lane & 3) {
 #pragma unroll
         for (int s = 0; s < 3; ++s) {
             const int k = 4 * s + t;
             q[s] = k / 3;
-            at[s] = 3 * g + k % 3;
-            at8[s] = 24 + k % 3;
+            at[s] = Q + 3 * g + k % 3;
+            at8[s] = Q + 24 + k % 3;
         }
     }
-    // term(e): the records' element offsets (27 x position) of term e, x < 0 past the end
     template <class F>
-    __device__ void load(int e0, F&& term, const double* __restrict__ Q, double (&a)[3], double (&b)[3], double (&a8)[3],
-                         double (&b8)[3]) const {
+    __device__ void load(int e0, F&& term, double (&a)[3], double (&b)[3], double (&a8)[3], double (&b8)[3]) const {
 #pragma unroll
         for (int s = 0; s < 3; ++s) {
-            const int2 po = term(e0 + q[s]);
-            const bool ok = po.x >= 0;
-            const double* P = Q + 27L * po.x;
-            const double* O = Q + 27L * po.y;
-            a[s] = ok ? __ldg(P + at[s]) : 0.0;
-            b[s] = ok ? __ldg(O + at[s]) : 0.0;
-            a8[s] = ok ? __ldg(P + at8[s]) : 0.0;
-            b8[s] = ok ? __ldg(O + at8[s]) : 0.0;
+            const uint2 po = term(e0 + q[s]);
+            a[s] = __ldg(at[s] + 27L * po.x);
+            b[s] = __ldg(at[s] + 27L * po.y);
+            a8[s] = __ldg(at8[s] + 27L * po.x);
+            b8[s] = __ldg(at8[s] + 27L * po.y);
         }
     }
     __device__ void add(const double (&a)[3], const double (&b)[3], const double (&a8)[3], const double (&b8)[3]) {
@@ -174,17 +173,21 @@ struct SzSum {
             corner = fma(a8[s], b8[s], corner);
         }
     }
-    // terms 0 .. n - 1; the next step's records are in flight while a step is summed
+    // terms 0 .. n - 1 (term(e) answers up to e < n + kSzPad)
     template <class F>
-    __device__ void run(int n, F&& term, const double* __restrict__ Q) {
-        double a[2][3], b[2][3], a8[2][3], b8[2][3];
-        load(0, term, Q, a[0], b[0], a8[0], b8[0]);
-        for (int e = 0; e < n; e += 8) {
-            load(e + 4, term, Q, a[1], b[1], a8[1], b8[1]);
+    __device__ void run(int n, F&& term) {
+        double a[3][3], b[3][3], a8[3][3], b8[3][3];
+        load(0, term, a[0], b[0], a8[0], b8[0]);
+        load(4, term, a[1], b[1], a8[1], b8[1]);
+        for (int e = 0; e < n; e += 12) {
+            load(e + 8, term, a[2], b[2], a8[2], b8[2]);
             add(a[0], b[0], a8[0], b8[0]);
             if (e + 4 >= n) break;
-            load(e + 8, term, Q, a[0], b[0], a8[0], b8[0]);
+            load(e + 12, term, a[0], b[0], a8[0], b8[0]);
             add(a[1], b[1], a8[1], b8[1]);
+            if (e + 8 >= n) break;
+            load(e + 16, term, a[1], b[1], a8[1], b8[1]);
+            add(a[2], b[2], a8[2], b8[2]);
         }
     }
     // the shares of row 8 and column 8 added over the k lanes
@@ -209,15 +212,16 @@ struct SzSum {
 
 // One block: the terms of slot s (camera ca <= cb) over the chunk, pass u (the
 // (u+1)-th partner of camera ca of each marked observation), then the block
-// stored in both triangles (the diagonal: U minus the terms, both ways round,
-// and the self terms). The run is staged in the warp's buffer segment by
-// segment. first: the position of the chunk's observation 0. Warp-level.
-__device__ void sz_block(const SzShared& sh, int2* buf, int s, int ca, int cb, int first, int W, int u, bool store,
-                         const double* __restrict__ Q, const double* __restrict__ is_cam,
+// stored in both triangles (the diagonal: U minus the terms, both ways round). The run is staged in the warp's buffer segment by
+// segment. first: the position of the chunk's observation 0; zero: the zero
+// record's position. Warp-level.
+__device__ void sz_block(const SzShared& sh, uint2* buf, int s, int ca, int cb, int first, int zero, int W, int u,
+                         bool store, const double* __restrict__ Q, const double* __restrict__ is_cam,
                          const double* __restrict__ U, double* Z, long ldz) {
     const int lane = threadIdx.x & 31;
     const unsigned* mk = sh.mask + (size_t)s * W;
-    SzSum sum(lane);
+    SzSum sum(lane, Q);
+    const uint2 none = make_uint2((unsigned)zero, (unsigned)zero);
     for (int wi = 0; wi < W;) {
         // stage a segment of the run: the marked observations j in order (32
         // mask words per step, a prefix scan of their bit counts gives every
@@ -237,22 +241,23 @@ __device__ void sz_block(const SzShared& sh, int2* buf, int s, int ca, int cb, i
             const int take = __popc(__ballot_sync(0xffffffffu, lane < nw && nseg + incl <= kSzSegCap));
             if (lane < take) {
                 int pos = nseg + incl - c;
-                for (unsigned bb = word; bb; bb &= bb - 1u) buf[pos++].y = 32 * (wi + lane) + (__ffs(bb) - 1);
+                for (unsigned bb = word; bb; bb &= bb - 1u) buf[pos++].y = 32u * (wi + lane) + (__ffs(bb) - 1);
             }
             nseg += __shfl_sync(0xffffffffu, incl, take - 1);
             wi += take;
         }
         __syncwarp();
         for (int e = lane; e < nseg; e += 32) {
-            const int j = buf[e].y;
+            const int j = (int)buf[e].y;
             const int t1 = sh.off[j + 1];
             int t = sh.off[j], c = 0;
             for (; t < t1; ++t)
                 if (sh.part_c[t] == ca && c++ == u) break;
-            buf[e] = t < t1 ? make_int2(sh.part_o[t], first + j) : make_int2(-1, 0);
+            buf[e] = t < t1 ? make_uint2((unsigned)sh.part_o[t], (unsigned)(first + j)) : none;
         }
+        if (lane < kSzPad) buf[nseg + lane] = none;
         __syncwarp();
-        sum.run(nseg, [&](int e) { return e < nseg ? buf[e] : make_int2(-1, 0); }, Q);
+        sum.run(nseg, [&](int e) { return buf[e]; });
         __syncwarp();  // the buffer is refilled next
     }
     sum.finish();
@@ -277,7 +282,6 @@ __device__ void sz_block(const SzShared& sh, int2* buf, int s, int ca, int cb, i
         if (r > q) continue;
         const long row = 9L * cb + r, col = 9L * cb + q;
         double v = blk[9 * r + q] + blk[9 * q + r];
-        if (u == 0) v += sh.self[q * (q + 1) / 2 + r];
         v *= __ldg(is_cam + row) * __ldg(is_cam + col);
         double* up = Z + row + col * ldz;
         v = (store ? U[81L * cb + e] : *up) - v;
@@ -285,27 +289,6 @@ __device__ void sz_block(const SzShared& sh, int2* buf, int s, int ca, int cb, i
         Z[col + row * ldz] = v;
     }
     __syncwarp();
-}
-
-// The self terms sum Q_o Q_o^T over positions [first, first + len) into
-// sh.self[0 .. 45) (element r <= q at q (q + 1) / 2 + r): warp w sums a
-// contiguous share, the shares are added in warp order. Block-level.
-__device__ void sz_self(const SzShared& sh, int first, int len, const double* __restrict__ Q) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int j0 = (int)((long)warp * len / kSzWarps), j1 = (int)((long)(warp + 1) * len / kSzWarps);
-    SzSum sum(lane);
-    sum.run(j1 - j0, [&](int e) { const int p = j0 + e < j1 ? first + j0 + e : -1; return make_int2(p, p); }, Q);
-    sum.finish();
-    sum.elements([&](int r, int q, double v) {
-        if (r <= q) sh.self[45 * warp + q * (q + 1) / 2 + r] = v;
-    });
-    __syncthreads();
-    double v = 0.0;
-    if (threadIdx.x < 45)
-        for (int w = 0; w < kSzWarps; ++w) v += sh.self[45 * w + threadIdx.x];
-    __syncthreads();
-    if (threadIdx.x < 45) sh.self[threadIdx.x] = v;
-    __syncthreads();
 }
 
 // The terms of the partners of rank u (their camera's (u+1)-th observation of
@@ -337,7 +320,7 @@ __device__ bool sz_masks(const SzShared& sh, int len, int K, int W, int u) {
 __global__ void __launch_bounds__(kSzThreads, 2)
     k_schur_columns(int C, const int* __restrict__ cam_ptr, const int2* __restrict__ pt_list,
                     const int2* __restrict__ pos_list, const double* __restrict__ Q, const double* __restrict__ is_cam,
-                    const double* __restrict__ U, double* Z, long ldz, int parts) {
+                    const double* __restrict__ U, double* Z, long ldz, int parts, int zero) {
     extern __shared__ __align__(16) char sz_smem[];
     const SzShared sh = sz_layout(sz_smem, C);
     const int cb = C - 1 - (int)(blockIdx.x / parts);  // the most partners (cameras <= cb) first
@@ -404,7 +387,7 @@ __global__ void __launch_bounds__(kSzThreads, 2)
                 }
             }
         }
-        if (tid == 0) sh.slot_of[cb] = 0;  // the diagonal block always has a slot (its self terms)
+        if (tid == 0) sh.slot_of[cb] = 0;  // the diagonal block always has a slot (U)
         __syncthreads();
         int K = 0, W = 0;
         for (;;) {
@@ -432,9 +415,6 @@ __global__ void __launch_bounds__(kSzThreads, 2)
                 }
         }
         __syncthreads();
-        // the self terms of the chunk's observations, once each (part 0 has the diagonal block)
-        const int taken = skip > 0;  // j0's was in its first piece
-        if (part == 0) sz_self(sh, base + j0 + taken, len - taken, Q);
         for (int u = 0;; ++u) {
             const bool more = sz_masks(sh, len, K, W, u);
             if (tid == 0) sh.tmp[kSzWarps + 1] = 0;  // slot cursor: warps take slots as they finish
@@ -448,8 +428,8 @@ __global__ void __launch_bounds__(kSzThreads, 2)
                 if (s < 0) break;
                 const int ca = sh.cam_of_slot[s];
                 if ((cb - ca) % parts != part) continue;
-                sz_block(sh, sh.runbuf + warp * kSzSegCap, s, ca, cb, base + j0, W, u, first_chunk && u == 0, Q, is_cam, U,
-                         Z, ldz);
+                sz_block(sh, sh.runbuf + warp * (kSzSegCap + kSzPad), s, ca, cb, base + j0, zero, W, u, first_chunk && u == 0,
+                         Q, is_cam, U, Z, ldz);
             }
             __syncthreads();
             if (!more) break;
@@ -487,7 +467,7 @@ int launch_schur_columns(const SceneDev& s, double* Z, int ldz, cudaStream_t st)
     // few cameras: split every column so that the grid covers about two waves of CTAs
     const int parts = std::max(1, std::min(8, (4 * device_sms() + C - 1) / C));
     k_schur_columns<<<C * parts, kSzThreads, smem, st>>>(C, s.cam_ptr, s.pt_list, s.pos_list, s.Q, s.is_cam, s.Ucam, Z,
-                                                         ldz, parts);
+                                                         ldz, parts, s.num_obs);
     count_launch();
     return UNC_OK;
 }
