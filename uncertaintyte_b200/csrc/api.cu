@@ -553,6 +553,8 @@ int run_pipeline(unc_context* ctx, const unc_options* o, int num_rows, long long
         }
         if (err & ERRBIT_LAYOUT)
             return fail(UNC_ERR_LAYOUT, "Jacobian rows are not in the 2 x (9 camera + 3 point) observation layout");
+        if (err & ERRBIT_SCHUR_CAP)
+            return fail(UNC_ERR_TOO_LARGE, "an observation shares its point with more observations than the Schur stage holds");
         if (err & (ERRBIT_SINGULAR | ERRBIT_NONFINITE))
             return fail(UNC_ERR_SINGULAR, "singular point block or non-finite value");
         return UNC_OK;
@@ -789,6 +791,8 @@ int run_pipeline(unc_context* ctx, const unc_options* o, int num_rows, long long
     }
     if (err & ERRBIT_LAYOUT)
         return fail(UNC_ERR_LAYOUT, "Jacobian rows are not in the 2 x (9 camera + 3 point) observation layout");
+    if (err & ERRBIT_SCHUR_CAP)
+        return fail(UNC_ERR_TOO_LARGE, "an observation shares its point with more observations than the Schur stage holds");
     if (err & (ERRBIT_SINGULAR | ERRBIT_NONFINITE))
         return fail(UNC_ERR_SINGULAR, "non-positive pivot or non-finite value while inverting Z + lambda*I");
     if (err & ERRBIT_TIMEOUT)

@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kIndexThreads)
 
 // pt_ptr (and a copy of it, advanced by the placing) from the counts and the blocks' sums.
 __global__ void __launch_bounds__(kIndexThreads)
-    k_index_points(int num_points, const int* __restrict__ pt_sums, int* pt_cnt, int* __restrict__ pt_ptr) {
+    k_index_points(int num_points, const int* __restrict__ pt_sums, int* pt_cnt, int* __restrict__ pt_ptr, int* err) {
     __shared__ int buf[kScanItems], tmp[kIndexWarps];
     const int t = threadIdx.x, p0 = blockIdx.x * kScanItems;
     int before = 0;
@@ -271,7 +271,11 @@ __global__ void __launch_bounds__(kIndexThreads)
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) before += __shfl_xor_sync(0xffffffffu, before, d);
     if ((t & 31) == 0) tmp[t >> 5] = before;
-    for (int i = t; i < kScanItems; i += kIndexThreads) buf[i] = p0 + i < num_points ? pt_cnt[p0 + i] : 0;
+    for (int i = t; i < kScanItems; i += kIndexThreads) {
+        const int cnt = p0 + i < num_points ? pt_cnt[p0 + i] : 0;
+        buf[i] = cnt;
+        if (cnt > kSchurMaxList) atomicOr(err, ERRBIT_SCHUR_CAP);
+    }
     __syncthreads();
     before = 0;
     for (int q = 0; q < kIndexWarps; ++q) before += tmp[q];
@@ -372,7 +376,7 @@ void launch_build_index(SceneDev& s, cudaStream_t st) {
                                                                             hist, pt_cnt);
         k_index_scan<<<x.point_blocks + x.cam_blocks, kIndexThreads, sizeof(int) * std::max(range, kIndexThreads), st>>>(
             x.point_blocks, P, pt_cnt, pt_sums, x.chunks, c0, range, hist, totals, s.cam_ptr, ticket);
-        if (x.point_blocks) k_index_points<<<x.point_blocks, kIndexThreads, 0, st>>>(P, pt_sums, pt_cnt, s.pt_ptr);
+        if (x.point_blocks) k_index_points<<<x.point_blocks, kIndexThreads, 0, st>>>(P, pt_sums, pt_cnt, s.pt_ptr, s.err);
         k_index_place<<<x.chunks, kIndexThreads, sizeof(int) * kIndexWarps * range, st>>>(
             n, x.per_chunk, c0, range, s.obs_cam, s.obs_pt, hist, s.cam_ptr, pt_cnt, s.cam_obs, s.pt_tmp);
         count_launch(x.point_blocks ? 4 : 3);

@@ -627,6 +627,7 @@ int run_group(unc_batch* b, GroupRun& g, const int* const* rows, const int* cons
         const TeState& te = tes[i];
         int rc = UNC_OK;
         if (err & ERRBIT_LAYOUT) rc = UNC_ERR_LAYOUT;
+        else if (err & ERRBIT_SCHUR_CAP) rc = UNC_ERR_TOO_LARGE;
         else if (err & (ERRBIT_SINGULAR | ERRBIT_NONFINITE)) rc = UNC_ERR_SINGULAR;
         else if (err & ERRBIT_TIMEOUT) rc = UNC_ERR_CUDA;
         else if (te.bad) rc = UNC_ERR_SINGULAR;

@@ -18,6 +18,7 @@ enum : int {
     ERRBIT_LAYOUT = 1,      // observation rows not 12 entries / columns out of range
     ERRBIT_SINGULAR = 2,    // non-positive or non-finite pivot
     ERRBIT_NONFINITE = 4,   // NaN / Inf produced
+    ERRBIT_SCHUR_CAP = 32,  // a point has more observations than the Schur stage takes (kSchurMaxList)
     ERRBIT_TIMEOUT = 16,    // a bounded device wait ran out (tensor-core pipeline)
 };
 
@@ -132,7 +133,9 @@ void launch_point_blocks(const SceneDev& s, cudaStream_t st);
 void launch_camera_blocks(const SceneDev& s, cudaStream_t st);
 // The Schur complement Z = U - W V^-1 W^T (schur.cu) over a zeroed Z: the
 // diagonal blocks from s.Ucam, every co-visible camera-pair block written in
-// both triangles, bitwise symmetric. UNC_ERR_TOO_LARGE above kSchurMaxCams.
+// both triangles, bitwise symmetric. UNC_ERR_TOO_LARGE above kSchurMaxCams;
+// nothing is written when ERRBIT_SCHUR_CAP is set.
+constexpr int kSchurMaxList = 12288;  // observations of one point
 constexpr int kSchurMaxCams = 5120;  // above the dense path's limit (9 C <= 46000)
 int launch_schur_columns(const SceneDev& s, double* Z, int ldz, cudaStream_t st);
 size_t schur_columns_smem(int num_cams);

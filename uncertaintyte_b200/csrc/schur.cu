@@ -320,7 +320,9 @@ __device__ bool sz_masks(const SzShared& sh, int len, int K, int W, int u) {
 __global__ void __launch_bounds__(kSzThreads, 2)
     k_schur_columns(int C, const int* __restrict__ cam_ptr, const int2* __restrict__ pt_list,
                     const int2* __restrict__ pos_list, const double* __restrict__ Q, const double* __restrict__ is_cam,
-                    const double* __restrict__ U, double* Z, long ldz, int parts, int zero) {
+                    const double* __restrict__ U, double* Z, long ldz, int parts, int zero,
+                    const int* __restrict__ err) {
+    if (*err & ERRBIT_SCHUR_CAP) return;
     extern __shared__ __align__(16) char sz_smem[];
     const SzShared sh = sz_layout(sz_smem, C);
     const int cb = C - 1 - (int)(blockIdx.x / parts);  // the most partners (cameras <= cb) first
@@ -467,7 +469,7 @@ int launch_schur_columns(const SceneDev& s, double* Z, int ldz, cudaStream_t st)
     // few cameras: split every column so that the grid covers about two waves of CTAs
     const int parts = std::max(1, std::min(8, (4 * device_sms() + C - 1) / C));
     k_schur_columns<<<C * parts, kSzThreads, smem, st>>>(C, s.cam_ptr, s.pt_list, s.pos_list, s.Q, s.is_cam, s.Ucam, Z,
-                                                         ldz, parts, s.num_obs);
+                                                         ldz, parts, s.num_obs, s.err);
     count_launch();
     return UNC_OK;
 }
