@@ -230,22 +230,23 @@ def measured_peaks():
 def stage_rooflines(stats, num_cams: int, num_points: int, num_obs: int):
     """HBM rooflines of the assembly and Schur stages from their CUDA-event
     times and the algorithmic bytes per unit: assembly reads 296 B and writes
-    432 B per observation (J values, columns and row pointers in; W and Y out)
-    plus 72 B per point (V) and 648 B per camera (U); the Schur stage reads W
-    and Y (432 B per observation) and U (648 B per camera) and writes Z once
-    (8 N^2 B, N = 9 cameras)."""
+    216 B per observation (J values, columns and row pointers in; the record
+    Q = W M out, M M^T the inverse of the point's block) plus 96 B per point (V
+    and M) and 648 B per camera (U); the Schur stage reads Q (216 B per
+    observation) and U (648 B per camera) and writes Z once (8 N^2 B, N = 9
+    cameras)."""
     peak, src, _ = measured_peaks()
     N = 9 * num_cams
-    asm_b = 728.0 * num_obs + 72.0 * num_points + 648.0 * num_cams
+    asm_b = 512.0 * num_obs + 96.0 * num_points + 648.0 * num_cams
     asm_t = sum(stats[k] for k in ("time_create_j", "time_fix_j", "time_norm_j", "time_multiply_jj"))
-    sch_b = 432.0 * num_obs + 648.0 * num_cams + 8.0 * N * N
+    sch_b = 216.0 * num_obs + 648.0 * num_cams + 8.0 * N * N
     sch_t = stats["time_compose_z"]
     out = {}
     for name, b, t, what in (("roofline_assembly", asm_b, asm_t, "validation, index, J^T J blocks, column norms, "
-                              "point blocks and inverses, W and Y records, zeroing of the dense work buffers"),
-                             ("roofline_schur", sch_b, sch_t, "zeroing of Z, then one CTA per camera column: "
-                                                                "partner lists, run masks, block sums in registers, "
-                                                                "both triangles written")):
+                              "point blocks and their inverses' factors, Q records"),
+                             ("roofline_schur", sch_b, sch_t, "one CTA per camera column and share of its blocks: "
+                                                                "partner lists, run masks, block sums on the FP64 "
+                                                                "tensor cores, both triangles written")):
         ach = b / t / 1e9 if t > 0 else None
         out[name] = {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                      "frac": ach / peak if ach else None, "algorithmic_bytes": b, "seconds": t,
@@ -528,7 +529,7 @@ def run_ours(a):
             peak64 = _fp64_peak_tflops(torch, dev, n=nd, reps=3)
             ach = prod_flops / prod_s / 1e12
             fp64["product_kernel"] = {
-                "kernel": "k_gemm_f64 (DMMA m8n8k4, 128x128 lower tiles, symmetric product)",
+                "kernel": "k_gemm_f64 (DMMA m8n8k4, 64x64 lower tiles, symmetric product)",
                 "achieved_tflops": ach, "cublas_dgemm_tflops": peak64, "frac_of_cublas": ach / peak64,
                 "launches": n_prod, "flops_per_launch": prod_flops / n_prod,
                 "note": f"algorithmic N^2(N+1) flops of the lower-triangle product over its CUDA-event time; "

@@ -190,9 +190,8 @@ int unc_jacob_write_binary(const char* path, const unc_jacob_header* header, con
                            const double* values);
 
 /* Device bytes one unc_compute call needs for this Jacobian (host arrays):
- * the workspace with the input copies, the Schur pair list (counted from the
- * point columns of the rows) and the int8 slices of the mixed modes. -1 for
- * invalid options. No counterpart in the reference (admission control). */
+ * the workspace with the input copies, the records of the sparse stage and the
+ * int8 slices of the mixed modes. -1 for invalid options. No counterpart in the reference (admission control). */
 long long unc_request_bytes(const unc_options* opt, int num_rows, int num_cols, const int* rows,
                             const int* cols);
 
