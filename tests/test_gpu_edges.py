@@ -97,6 +97,27 @@ def test_mixed_product_of_any_leading_dimension(n, ld):
     assert torch.equal(out[0], out[1])
 
 
+@pytest.mark.parametrize("power", [-900, 0, 900])
+def test_mixed_product_of_scaled_and_zero_rows(power):
+    """A row's exponent is that of its largest entry: operands scaled by a power of two give the same
+    digits, so exactly the scaled result, and rows of zeros give zeros."""
+    import torch
+    n = 200
+    g = torch.Generator(device="cuda").manual_seed(7)
+    P = torch.randn(n, n, dtype=torch.float64, device="cuda", generator=g)
+    X = torch.randn(n, n, dtype=torch.float64, device="cuda", generator=g)
+    P, X = P + P.T, X + X.T
+    P[17], P[:, 17] = 0.0, 0.0
+    out = []
+    for scale in (1.0, 2.0 ** power):
+        p, c = P * scale, torch.full((n, n), 5.0, dtype=torch.float64, device="cuda")
+        native.gemm_mixed_device(n, p.data_ptr(), X.data_ptr(), n, c.data_ptr(), 5)
+        torch.cuda.synchronize()
+        out.append(c)
+    assert torch.equal(out[0] * 2.0 ** power, out[1])
+    assert (out[0][:, 17] == 0).all()
+
+
 @pytest.mark.parametrize("cams,points,obs", [(5200, 800, 12000), (2, 1, 3000), (40, 1025, 9000)])
 def test_index_of_unsorted_observations(cams, points, obs):
     """J^T J of observations in random order, some of them repeated: more cameras than one pass of
