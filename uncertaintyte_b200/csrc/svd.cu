@@ -259,7 +259,7 @@ __global__ void __cluster_dims__(kOrthoCtas, 1, 1) __launch_bounds__(kOrthoThrea
 // eigenvectors as the columns of Wr.
 // One warp per pair of a round-robin round (the pairs of a round are disjoint:
 // column m - 1 stays, the others move round a circle), lane = row, then column:
-// a sweep is a chain of m - 1 rotations, not of p (p - 1) / 2 (p = 15: 45 us; 240 us
+// a sweep is a chain of m - 1 rotations, not of p (p - 1) / 2 (p = 15: 40 us; 240 us
 // for the cyclic order in one warp).
 __global__ void __launch_bounds__(512) k_small_jacobi(const double* __restrict__ H, int ldh, int p, double* theta,
                                                      double* Wr, int ldw) {
@@ -288,8 +288,9 @@ __global__ void __launch_bounds__(512) k_small_jacobi(const double* __restrict__
         }
         __syncthreads();
         if (stop) break;
-        for (int round = 0; round < m - 1; ++round) {
-            const int i = (round + w) % (m - 1), j = w == 0 ? m - 1 : (round - w + m - 1) % (m - 1);
+        int i = w, j = m - 1 - w;  // both move round the circle of m - 1; column m - 1 stays with warp 0
+        for (int round = 0; round < m - 1; ++round, i = i + 1 < m - 1 ? i + 1 : 0,
+                 j = w == 0 ? j : (j + 1 < m - 1 ? j + 1 : 0)) {
             const int a = min(i, j), b = max(i, j);
             bool rotate = b < p;
             double c = 1.0, s = 0.0, t = 0.0;
