@@ -24,7 +24,9 @@ constexpr int kMaxDim = 9;
 // carries the whole upper triangle and applies every rotation to it, so the
 // rotations need no shared memory, shuffle or barrier; the rows of V are dealt
 // to the lanes (D / L each). The chain of dependent rotations bounds the
-// kernel.
+// kernel. The order is the cyclic one: the signs of the vectors follow from it (rounds
+// of disjoint pairs, their angles found side by side, took 65 us for 2000 9 x 9
+// blocks against 84, with other signs).
 template <int D, int L>
 __global__ void __launch_bounds__(128) k_block_eigen(const double* __restrict__ packed, int nblk, int src, int off,
                                                      double* vals, double* vecs) {
