@@ -20,9 +20,10 @@ constexpr int NB = 64;  // leaf size
 //  (A) warp 0 factors the 16 x 16 diagonal block in registers, two columns per
 //      step: with pivot d, e below it and f the next diagonal entry,
 //      1/L(p,p) = d^-1/2 and 1/L(p+1,p+1) = (d f - e^2)^-1/2 d^1/2, whose two
-//      reciprocal square roots run side by side, and the next step's d, e, f are
-//      formed by every lane from broadcast values (one shuffle latency per
-//      step). Lanes 0..15 hold the block's rows, lanes 16..31 the rows of the
+//      reciprocal square roots are one call, half of the warp's lanes taking the
+//      one and half the other (two calls follow one another: n = 1351 432 us
+//      instead of 421), and the next step's d, e, f are formed by every lane from
+//      broadcast values (one shuffle latency per step). Lanes 0..15 hold the block's rows, lanes 16..31 the rows of the
 //      identity, which the same instructions turn into D_q = L_qq^{-1}.
 //  (B) the rows below: X = A_iq D_q^T on the FP64 tensor cores (DMMA);
 //  (C) the next diagonal block takes its rank-16 update; the rest of the
@@ -116,16 +117,6 @@ __device__ __forceinline__ void leaf_finish(double* W, const double* D, int fj, 
     }
 }
 
-// 1 / sqrt(d) for a normal d > 0: the hardware's approximation (about 2^-22) and one
-// third-order Householder step, y (1 + e/2 + 3 e^2/8) with e = 1 - d y^2. No
-// branch, so that two of them overlap in the panel's dependent chain.
-__device__ __forceinline__ double rsqrt_step(double d) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(d));
-    const double e = fma(-(d * y), y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 // (A): one warp; the diagonal block Sb becomes L_qq, Db receives L_qq^{-1}.
 __device__ __forceinline__ void leaf_panel(double* Sb, double* Db, int lane, int* err) {
     constexpr unsigned kAll = 0xffffffffu;
@@ -146,7 +137,9 @@ __device__ __forceinline__ void leaf_panel(double* Sb, double* Db, int lane, int
             en = __shfl_sync(kAll, a[p + 2], p + 3);
             fn = __shfl_sync(kAll, a[p + 3], p + 3);
         }
-        const double r0 = rsqrt_step(d), det = fma(d, f, -(e * e)), rd = rsqrt_step(det);
+        const double det = fma(d, f, -(e * e)), r = rsqrt(lane < LEAF_PW ? d : det);
+        const double other = __shfl_xor_sync(kAll, r, LEAF_PW);
+        const double r0 = lane < LEAF_PW ? r : other, rd = lane < LEAF_PW ? other : r;
         bad |= !(d >= kTiny && det >= kTiny && d <= kHuge && det <= kHuge);
         const double r1 = rd * (d * r0);
         const double x0 = a[p] * r0;
