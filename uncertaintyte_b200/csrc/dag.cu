@@ -89,12 +89,16 @@ __device__ bool wait_ge(const int* flag, int v, const int* abort, long spin) {
     return false;
 }
 
-// One warp: the same for one flag per lane (nullptr: none), polled together.
+// One warp: the same for one flag per lane (nullptr: none), polled together. The
+// lanes leave together: one lane reads the abort flag and the warp votes on what it
+// read (with a read per lane, some could see the flag and leave while the others
+// wait for them at the next vote).
 __device__ bool wait_all(const int* flag, int v, const int* abort, long spin) {
+    const int lane = threadIdx.x & 31;
     for (long it = 0; it < spin; ++it) {
         const bool ok = !flag || ld_acquire(flag) >= v;
         if (__all_sync(0xffffffffu, ok)) return true;
-        if (ld_acquire(abort)) return false;
+        if (__any_sync(0xffffffffu, lane == 0 && ld_acquire(abort) != 0)) return false;
         __nanosleep(32);
     }
     return false;
