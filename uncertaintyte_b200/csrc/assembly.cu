@@ -602,11 +602,17 @@ void launch_camera_blocks(const SceneDev& s, cudaStream_t st) {
 // it), its Cholesky factor L, M_p = diag(1/s) L^{-T}. The reference inverts the
 // scaled block by its adjugate (ScaledSparseMatrix.cpp:219-228) and multiplies
 // W V^{-1} W^T; with the factor one record Q = W M per observation gives the
-// same product as Q Q^T. A block that is not positive definite leaves a
-// non-finite or huge M_p, which the inverse of Z reports.
+// same product as Q Q^T.
+// A singular block (a point seen once, or only along one ray) sets
+// ERRBIT_SINGULAR: the scaled block's last pivot, taken in the order that puts the
+// larger second pivot first, is at most (64 + n) eps for n observations. In that
+// order rounding leaves at most about 16 eps of a zero pivot (200,000 blocks of
+// rank two, rows up to 1e-6 from parallel), besides n eps of the block's sums; in
+// the fixed order it can leave any size, of either sign, when the first two
+// columns are close. 64 eps is where k_point_cov drops an eigenvalue.
 __global__ void k_point_blocks(int num_points, const double* __restrict__ J, const int* __restrict__ pt_ptr,
                                const int2* __restrict__ pt_list, const int* __restrict__ cam_obs,
-                               double* __restrict__ Vraw, double* __restrict__ Mp) {
+                               double* __restrict__ Vraw, double* __restrict__ Mp, int* err) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= num_points) return;
     double v00 = 0, v01 = 0, v02 = 0, v11 = 0, v12 = 0, v22 = 0;
@@ -647,6 +653,12 @@ __global__ void k_point_blocks(int num_points, const double* __restrict__ J, con
     const double a = v00 * i0 * i0, bb = v01 * i0 * i1, c = v02 * i0 * i2;
     const double e = v11 * i1 * i1, f = v12 * i1 * i2, k = v22 * i2 * i2;
     const double r0 = 1.0 / sqrt(a), l10 = bb * r0, l20 = c * r0;
+    {
+        const double p1 = e - l10 * l10, p2 = k - l20 * l20, g = f - l20 * l10;
+        const double top = fmax(p1, p2), least = (64.0 + n) * 2.220446049250313e-16;
+        // the last pivot min(p1, p2) - g^2 / top > least (false for a NaN)
+        if (!(top > least && fma(fmin(p1, p2), top, -(g * g)) > least * top)) atomicOr(err, ERRBIT_SINGULAR);
+    }
     const double r1 = 1.0 / sqrt(e - l10 * l10), l21 = (f - l20 * l10) * r1;
     const double r2 = 1.0 / sqrt(k - l20 * l20 - l21 * l21);
     o[0] = r0 * i0;
@@ -660,7 +672,7 @@ __global__ void k_point_blocks(int num_points, const double* __restrict__ J, con
 void launch_point_blocks(const SceneDev& s, cudaStream_t st) {
     if (s.num_points == 0) return;
     k_point_blocks<<<(s.num_points + 127) / 128, 128, 0, st>>>(s.num_points, s.J, s.pt_ptr, s.pt_list, s.cam_obs, s.Vraw,
-                                                               s.Mp);
+                                                               s.Mp, s.err);
     count_launch();
 }
 
