@@ -29,7 +29,9 @@
 // No floating-point atomics, no device-to-host round trip: the result is
 // bitwise repeatable and the stage can be captured in a graph. A camera that
 // observes a point more than once gives more than one term per (slot,
-// observation); those extra terms are added by further passes.
+// observation): a run of neighbouring entries, since the lists are ordered by
+// camera. A chunk that has such a run expands it where the terms are staged, so
+// the work is the number of terms whatever the multiplicities.
 #include "internal.h"
 
 namespace unc {
@@ -210,26 +212,52 @@ struct SzSum {
     }
 };
 
-// One block: the terms of slot s (camera ca <= cb) over the chunk, pass u (the
-// (u+1)-th partner of camera ca of each marked observation), then the block
-// stored in both triangles (the diagonal: U minus the terms, both ways round). The run is staged in the warp's buffer segment by
-// segment. first: the position of the chunk's observation 0; zero: the zero
-// record's position. Warp-level.
-__device__ void sz_block(const SzShared& sh, uint2* buf, int s, int ca, int cb, int first, int zero, int W, int u,
+// The first partner of camera c among observation j's (one exists; ordered by camera).
+__device__ __forceinline__ int sz_first(const SzShared& sh, int j, int c) {
+    int t = sh.off[j], end = sh.off[j + 1];
+    while (end - t > 16) {
+        const int m = (t + end) >> 1;
+        if (sh.part_c[m] < c) t = m + 1; else end = m + 1;
+    }
+    while (t < end && sh.part_c[t] != c) ++t;
+    return t;
+}
+
+// The end of the run of equal cameras that starts at entry t of observation j.
+__device__ __forceinline__ int sz_run_end(const SzShared& sh, int j, int t) {
+    int lo = t + 1, hi = sh.off[j + 1];
+    while (lo < hi) {
+        const int m = (lo + hi) >> 1;
+        if (sh.part_c[m] == sh.part_c[t]) lo = m + 1; else hi = m;
+    }
+    return lo;
+}
+
+// One block: the terms of slot s (camera ca <= cb) over the chunk, then the block
+// stored in both triangles (the diagonal: U minus the terms, both ways round). The
+// run is staged in the warp's buffer segment by segment. repeats: some observation
+// of the chunk has several partners in a camera; the segments are at most 32
+// observations then, one per lane, and a segment whose terms do not fit is staged
+// again for the next of them, so that only its start and `skip` stay in registers
+// over the sum (200 cameras: the kernel 208 us without repeats, 210 so, 218 with the
+// lanes' entries kept). first: the position of the chunk's observation 0; zero: the
+// zero record's position. Warp-level.
+__device__ void sz_block(const SzShared& sh, uint2* buf, int s, int ca, int cb, int first, int zero, int W, bool repeats,
                          bool store, const double* __restrict__ Q, const double* __restrict__ is_cam,
                          const double* __restrict__ U, double* Z, long ldz) {
     const int lane = threadIdx.x & 31;
     const unsigned* mk = sh.mask + (size_t)s * W;
     SzSum sum(lane, Q);
     const uint2 none = make_uint2((unsigned)zero, (unsigned)zero);
-    for (int wi = 0; wi < W;) {
+    for (int wi = 0, skip = 0; wi < W;) {
         // stage a segment of the run: the marked observations j in order (32
         // mask words per step, a prefix scan of their bit counts gives every
         // lane its place), then each entry's partner, one entry per lane
-        int nseg = 0;
-        while (wi < W && nseg <= kSzSegCap - 32) {
-            const int nw = min(32, W - wi);
-            const unsigned word = lane < nw ? mk[wi + lane] : 0u;
+        const int cap = repeats ? 32 : kSzSegCap;
+        int nseg = 0, next = wi;
+        while (next < W && nseg <= cap - 32) {
+            const int nw = min(32, W - next);
+            const unsigned word = lane < nw ? mk[next + lane] : 0u;
             const int c = __popc(word);
             int incl = c;
 #pragma unroll
@@ -238,23 +266,50 @@ __device__ void sz_block(const SzShared& sh, uint2* buf, int s, int ca, int cb, 
                 if (lane >= d) incl += y;
             }
             // whole words that fit (a prefix of the lanes: incl grows with the lane)
-            const int take = __popc(__ballot_sync(0xffffffffu, lane < nw && nseg + incl <= kSzSegCap));
+            const int take = __popc(__ballot_sync(0xffffffffu, lane < nw && nseg + incl <= cap));
             if (lane < take) {
                 int pos = nseg + incl - c;
-                for (unsigned bb = word; bb; bb &= bb - 1u) buf[pos++].y = 32u * (wi + lane) + (__ffs(bb) - 1);
+                for (unsigned bb = word; bb; bb &= bb - 1u) buf[pos++].y = 32u * (next + lane) + (__ffs(bb) - 1);
             }
             nseg += __shfl_sync(0xffffffffu, incl, take - 1);
-            wi += take;
+            next += take;
         }
         __syncwarp();
-        for (int e = lane; e < nseg; e += 32) {
-            const int j = (int)buf[e].y;
-            const int t1 = sh.off[j + 1];
-            int t = sh.off[j], c = 0;
-            for (; t < t1; ++t)
-                if (sh.part_c[t] == ca && c++ == u) break;
-            buf[e] = t < t1 ? make_uint2((unsigned)sh.part_o[t], (unsigned)(first + j)) : none;
+        if (!repeats) {
+            for (int e = lane; e < nseg; e += 32) {
+                const int j = (int)buf[e].y;
+                buf[e] = make_uint2((unsigned)sh.part_o[sz_first(sh, j, ca)], (unsigned)(first + j));
+            }
+        } else {
+            int j = 0, t = 0, n = 0;  // this lane's observation and its entries [t, t + n) of camera ca
+            if (lane < nseg) {
+                j = (int)buf[lane].y;
+                t = sz_first(sh, j, ca);
+                n = sz_run_end(sh, j, t) - t;
+            }
+            int incl = n;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += y;
+            }
+            const int total = __shfl_sync(0xffffffffu, incl, 31);
+            __syncwarp();
+            nseg = min(kSzSegCap, total - skip);  // the segment's terms [skip, skip + nseg)
+            for (int x = skip + lane; x - lane < skip + nseg; x += 32) {
+                int from = 0;  // the lane whose entries hold term x: as many lanes end at or before it
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1)
+                    if (__shfl_sync(0xffffffffu, incl, from + d - 1) <= x) from += d;
+                const int at = __shfl_sync(0xffffffffu, t + n - incl, from) + x;
+                const int owner = first + __shfl_sync(0xffffffffu, j, from);
+                if (x < skip + nseg) buf[x - skip] = make_uint2((unsigned)sh.part_o[at], (unsigned)owner);
+            }
+            skip += nseg;
+            if (skip < total) next = wi;
+            else skip = 0;
         }
+        wi = next;
         if (lane < kSzPad) buf[nseg + lane] = none;
         __syncwarp();
         sum.run(nseg, [&](int e) { return buf[e]; });
@@ -291,27 +346,20 @@ __device__ void sz_block(const SzShared& sh, uint2* buf, int s, int ca, int cb, 
     __syncwarp();
 }
 
-// The terms of the partners of rank u (their camera's (u+1)-th observation of
-// the point in the owner observation's list) into the run masks; true when
-// some partner has a higher rank (another pass is needed). Block-level.
-__device__ bool sz_masks(const SzShared& sh, int len, int K, int W, int u) {
+// The run masks of the chunk's entries; true when some camera has two entries at one
+// observation. Where the lists are long (one of more than 32 entries on average), the
+// block's threads share each of them. Block-level.
+__device__ bool sz_masks(const SzShared& sh, int len, int K, int W) {
     for (int k = threadIdx.x; k < K * W; k += kSzThreads) sh.mask[k] = 0u;
     __syncthreads();
+    const bool shared_list = sh.off[len] > 32 * len;
     int more = 0;
-    for (int j = threadIdx.x; j < len; j += kSzThreads) {
-        const int t0 = sh.off[j], t1 = sh.off[j + 1];
-        for (int t = t0; t < t1; ++t) {
+    for (int j = shared_list ? 0 : threadIdx.x; j < len; j += shared_list ? 1 : kSzThreads) {
+        const int t0 = sh.off[j], t1 = sh.off[j + 1], step = shared_list ? kSzThreads : 1;
+        for (int t = t0 + (shared_list ? threadIdx.x : 0); t < t1; t += step) {
             const unsigned short c = sh.part_c[t];
-            if (u == 0) {  // first occurrences: a second one finds its bit set
-                const unsigned bit = 1u << (j & 31);
-                const unsigned old = atomicOr(sh.mask + (size_t)sh.slot_of[c] * W + (j >> 5), bit);
-                more |= (old & bit) != 0u;
-            } else {
-                int r = 0;
-                for (int q = t0; q < t; ++q) r += sh.part_c[q] == c;
-                if (r == u) atomicOr(sh.mask + (size_t)sh.slot_of[c] * W + (j >> 5), 1u << (j & 31));
-                more |= r > u;
-            }
+            atomicOr(sh.mask + (size_t)sh.slot_of[c] * W + (j >> 5), 1u << (j & 31));
+            more |= t > t0 && sh.part_c[t - 1] == c;
         }
     }
     return __syncthreads_or(more) != 0;
@@ -366,10 +414,15 @@ __global__ void __launch_bounds__(kSzThreads, 2)
             __syncthreads();
         }
         // every entry: its observation (then its partner and camera, in parallel)
-        for (int j = tid; j < len; j += kSzThreads)
-            for (int i = sh.off[j]; i < sh.off[j + 1]; ++i) sh.seg[i] = (unsigned short)j;
-        __syncthreads();
         const int E = sh.off[len];
+        if (E > 32 * len) {  // long lists: the block's threads share each
+            for (int j = 0; j < len; ++j)
+                for (int i = sh.off[j] + tid; i < sh.off[j + 1]; i += kSzThreads) sh.seg[i] = (unsigned short)j;
+        } else {
+            for (int j = tid; j < len; j += kSzThreads)
+                for (int i = sh.off[j]; i < sh.off[j + 1]; ++i) sh.seg[i] = (unsigned short)j;
+        }
+        __syncthreads();
         for (int i = tid; i < E; i += 4 * kSzThreads) {  // four entries per thread in flight
             int2 l[4];
 #pragma unroll
@@ -417,25 +470,21 @@ __global__ void __launch_bounds__(kSzThreads, 2)
                 }
         }
         __syncthreads();
-        for (int u = 0;; ++u) {
-            const bool more = sz_masks(sh, len, K, W, u);
-            if (tid == 0) sh.tmp[kSzWarps + 1] = 0;  // slot cursor: warps take slots as they finish
-            __syncthreads();
-            for (;;) {  // this CTA's blocks: cameras ca with (cb - ca) mod parts == part, the same in
-                        // every chunk (slot numbers are not), so no block is updated by two CTAs
-                int q = 0;
-                if (lane == 0) q = atomicAdd(sh.tmp + kSzWarps + 1, 1);
-                q = __shfl_sync(0xffffffffu, q, 0);
-                const int s = K - 1 - q;
-                if (s < 0) break;
-                const int ca = sh.cam_of_slot[s];
-                if ((cb - ca) % parts != part) continue;
-                sz_block(sh, sh.runbuf + warp * (kSzSegCap + kSzPad), s, ca, cb, base + j0, zero, W, u, first_chunk && u == 0,
-                         Q, is_cam, U, Z, ldz);
-            }
-            __syncthreads();
-            if (!more) break;
+        if (tid == 0) sh.tmp[kSzWarps + 1] = 0;  // slot cursor: warps take slots as they finish
+        const bool repeats = sz_masks(sh, len, K, W);
+        for (;;) {  // this CTA's blocks: cameras ca with (cb - ca) mod parts == part, the same in
+                    // every chunk (slot numbers are not), so no block is updated by two CTAs
+            int q = 0;
+            if (lane == 0) q = atomicAdd(sh.tmp + kSzWarps + 1, 1);
+            q = __shfl_sync(0xffffffffu, q, 0);
+            const int s = K - 1 - q;
+            if (s < 0) break;
+            const int ca = sh.cam_of_slot[s];
+            if ((cb - ca) % parts != part) continue;
+            sz_block(sh, sh.runbuf + warp * (kSzSegCap + kSzPad), s, ca, cb, base + j0, zero, W, repeats, first_chunk, Q,
+                     is_cam, U, Z, ldz);
         }
+        __syncthreads();
         for (int s = tid; s < K; s += kSzThreads) sh.slot_of[sh.cam_of_slot[s]] = kNoSlot;
         __syncthreads();
         first_chunk = false;
