@@ -1235,6 +1235,7 @@ int unc_jtj_crs(int num_rows, int num_cols, const int* rows, const int* cols, co
     CK(cudaMemset(s.err, 0, 16));
     launch_repack_generic(nobs, cam_off, d_rows, d_cols, d_vals, d_J, s.obs_cam, s.obs_pt, s.err, sm);
     launch_build_index(s, sm);
+    launch_long_lists(s, sm);
     launch_point_blocks(s, sm);
     launch_unscaled_blocks(s, d_U, d_W, sm);
     CK(cudaDeviceSynchronize());

@@ -334,7 +334,9 @@ __global__ void __launch_bounds__(kIndexThreads)
 }
 
 // Every list entry to its rank in its point's list (ascending positions, so
-// ascending cameras); per position: its list's start and its rank in it.
+// ascending cameras); per position: its list's start and its rank in it. The count
+// is quadratic, so lists of more than kSchurMaxList entries are left alone: a solve
+// refuses them, J^T J and the SVD algorithms place them by k_index_long.
 __global__ void __launch_bounds__(kIndexThreads)
     k_index_rank(int num_cams, const int* __restrict__ cam_ptr, const int* __restrict__ cam_obs,
                  const int* __restrict__ obs_cam, const int* __restrict__ obs_pt, const int* __restrict__ pt_ptr,
@@ -347,10 +349,50 @@ __global__ void __launch_bounds__(kIndexThreads)
         return;
     }
     const int b = pt_ptr[p], e = pt_ptr[p + 1];
+    if (e - b > kSchurMaxList) {
+        pos_list[i] = make_int2(0, 0);
+        return;
+    }
     int rank = 0;
     for (int k = b; k < e; ++k) rank += pt_tmp[k].x < i;
     pt_list[b + rank] = make_int2(i, obs_cam[o]);
     pos_list[i] = make_int2(b, rank);
+}
+
+// The lists that k_index_rank leaves: one CTA walks the positions in order and keeps
+// those of the point. There are at most num_obs / kSchurMaxList such lists.
+__global__ void __launch_bounds__(kIndexThreads)
+    k_index_long(int num_cams, int num_points, const int* __restrict__ cam_ptr, const int* __restrict__ cam_obs,
+                 const int* __restrict__ obs_cam, const int* __restrict__ obs_pt, const int* __restrict__ pt_ptr,
+                 int2* __restrict__ pt_list) {
+    __shared__ int lists[kIndexThreads], count, found[kIndexWarps];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, n = cam_ptr[num_cams];
+    for (long p0 = (long)blockIdx.x * kIndexThreads; p0 < num_points; p0 += (long)gridDim.x * kIndexThreads) {
+        if (t == 0) count = 0;
+        __syncthreads();
+        if (p0 + t < num_points && pt_ptr[p0 + t + 1] - pt_ptr[p0 + t] > kSchurMaxList)
+            lists[atomicAdd(&count, 1)] = (int)p0 + t;
+        __syncthreads();
+        for (int q = 0; q < count; ++q) {
+            const int p = lists[q];
+            int at = pt_ptr[p];
+            for (int i0 = 0; i0 < n; i0 += kIndexThreads) {
+                const int i = i0 + t, o = i < n ? cam_obs[i] : -1;
+                const bool mine = o >= 0 && obs_pt[o] == p;
+                const unsigned votes = __ballot_sync(0xffffffffu, mine);
+                if (lane == 0) found[warp] = __popc(votes);
+                __syncthreads();
+                int before = at;
+                for (int w = 0; w < kIndexWarps; ++w) {
+                    before += w < warp ? found[w] : 0;
+                    at += found[w];
+                }
+                if (mine) pt_list[before + __popc(votes & ((1u << lane) - 1u))] = make_int2(i, obs_cam[o]);
+                __syncthreads();  // found is rewritten
+            }
+        }
+        __syncthreads();  // count is rewritten
+    }
 }
 
 size_t index_scratch_ints(int num_cams, int num_points) {
@@ -386,6 +428,14 @@ void launch_build_index(SceneDev& s, cudaStream_t st) {
             C, s.cam_ptr, s.cam_obs, s.obs_cam, s.obs_pt, s.pt_ptr, s.pt_tmp, s.pt_list, s.pos_list);
         count_launch();
     }
+}
+
+void launch_long_lists(const SceneDev& s, cudaStream_t st) {
+    if (s.num_obs <= kSchurMaxList || s.num_points == 0) return;
+    const int blocks = std::min((s.num_points + kIndexThreads - 1) / kIndexThreads, 4 * device_sms());
+    k_index_long<<<blocks, kIndexThreads, 0, st>>>(s.num_cams, s.num_points, s.cam_ptr, s.cam_obs, s.obs_cam, s.obs_pt,
+                                                   s.pt_ptr, s.pt_list);
+    count_launch();
 }
 
 // ------------------------------------------------------------------------
@@ -616,7 +666,9 @@ __global__ void k_point_blocks(int num_points, const double* __restrict__ J, con
     int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= num_points) return;
     double v00 = 0, v01 = 0, v02 = 0, v11 = 0, v12 = 0, v22 = 0;
-    const int b = pt_ptr[p], n = pt_ptr[p + 1] - b;
+    const int b = pt_ptr[p];
+    int n = pt_ptr[p + 1] - b;
+    if (Mp && n > kSchurMaxList) n = 0;  // refused (ERRBIT_SCHUR_CAP): its list was not placed
     for (int i0 = 0; i0 < n; i0 += 4) {  // four records in flight
         int o[4];
         double x[4][3], y[4][3];
@@ -643,7 +695,7 @@ __global__ void k_point_blocks(int num_points, const double* __restrict__ J, con
     V[0] = v00; V[1] = v01; V[2] = v02; V[3] = v11; V[4] = v12; V[5] = v22;
     if (!Mp) return;
     double* o = Mp + 6L * p;
-    if (n == 0) {  // unobserved or fixed point: unused
+    if (n == 0) {  // unobserved, fixed or refused point: unused
         o[0] = o[1] = o[2] = o[3] = o[4] = o[5] = 0.0;
         return;
     }

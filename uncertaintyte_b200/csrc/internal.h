@@ -125,6 +125,8 @@ void launch_validate_obs(const SceneDev& s, cudaStream_t st);
 // Camera observations are processed in tiles of 256; slots = C + num_obs/256 + 1.
 size_t camera_tile_slots(int num_cams, int num_obs);
 void launch_build_index(SceneDev& s, cudaStream_t st);
+// After it, where points of more than kSchurMaxList observations are taken (not in a solve): their lists.
+void launch_long_lists(const SceneDev& s, cudaStream_t st);
 size_t index_scratch_ints(int num_cams, int num_points);
 // Point blocks and, unless s.Mp is nullptr, their inverse factors.
 void launch_point_blocks(const SceneDev& s, cudaStream_t st);

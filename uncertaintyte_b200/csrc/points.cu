@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(128) k_point_cov(int num_points, int3 fix, int
     if (has_fix && (p == fix.x || p == fix.y || p == fix.z)) return;  // fixed points are skipped
     double* out = pt_unc + 6L * p;
     const int b = pt_ptr[p], e = pt_ptr[p + 1];
-    if (b == e) {  // pinv of an empty A: zero covariance
+    if (b == e || e - b > kSchurMaxList) {  // pinv of an empty A: zero covariance; a refused point's list is not there
         out[0] = out[1] = out[2] = out[3] = out[4] = out[5] = 0.0;
         return;
     }

@@ -791,6 +791,7 @@ int svd_pipeline(char* ws, const unc_options* o, int num_rows, long long nnz, co
     SVD_CK(cudaEventRecord(ev[1], sm));
     launch_validate_obs(s, sm);
     launch_build_index(s, sm);
+    launch_long_lists(s, sm);
     SVD_CK(cudaEventRecord(ev[2], sm));
     // dense J^T J, unscaled (compute.cpp:189-199)
     SVD_CK(cudaMemsetAsync(L.M, 0, sizeof(double) * (size_t)n * ld, sm));
