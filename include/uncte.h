@@ -317,6 +317,10 @@ int unc_dense_inverse_noalloc(double* d_A, int n, int lda, void* stream);
  * device stays usable. A schedule with a task left out cannot complete, which
  * is how a test makes a wait run out. No counterpart in the reference. */
 int unc_spd_inverse_tasks_bounded(double* d_A, int n, int lda, long long poll_limit, int skip_task, void* stream);
+/* The same with a launch of at most `ctas` thread blocks, as when no more of
+ * them find room on the device: the schedule completes with any number of them
+ * and gives the same bytes. */
+int unc_spd_inverse_tasks_resident(double* d_A, int n, int lda, int ctas, void* stream);
 
 /* The order in which the tile-task form of unc_dense_inverse_device (n <= 3584)
  * runs its 64 x 64 tile tasks; no counterpart in the reference (its inverse is

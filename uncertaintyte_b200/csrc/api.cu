@@ -802,8 +802,9 @@ int run_pipeline(unc_context* ctx, const unc_options* o, int num_rows, long long
 }
 
 // SDM::inv on the GPU (unc_dense_inverse_device). poll_limit / skip_task are
-// passed to the tile-task form (n <= 3584): 0 / -1 for the regular schedule.
-int dense_inverse(double* d_A, int n, int lda, void* stream, long long poll_limit, int skip_task) {
+// passed to the tile-task form (n <= 3584): 0 / -1 for the regular schedule;
+// max_grid: its CTAs at most (0: as many as are useful).
+int dense_inverse(double* d_A, int n, int lda, void* stream, long long poll_limit, int skip_task, int max_grid = 0) {
     g_last_error.clear();
     if (!d_A || n <= 0 || lda < n || (lda & 1)) return fail(UNC_ERR_INVALID_ARG, "bad matrix arguments");
     cudaStream_t sm = (cudaStream_t)stream;
@@ -814,7 +815,8 @@ int dense_inverse(double* d_A, int n, int lda, void* stream, long long poll_limi
     Scratch mem;
     CK(mem.alloc(wsd * sizeof(double) + 256, sm));
     double* ws = static_cast<double*>(mem.p);
-    SpdScratch scratch{ws, ws + mat, ws + 2 * mat, reinterpret_cast<int*>(ws + 3 * mat), device_sms(), poll_limit, skip_task};
+    SpdScratch scratch{ws, ws + mat, ws + 2 * mat, reinterpret_cast<int*>(ws + 3 * mat), device_sms(), poll_limit, skip_task,
+                       max_grid};
     double* e = ws + 3 * mat + state_d;
     int* err = reinterpret_cast<int*>(ws + wsd);
     int h_err = 0;
@@ -1174,6 +1176,13 @@ int unc_spd_inverse_tasks_bounded(double* d_A, int n, int lda, long long poll_li
     if (!spd_tasks_apply(n)) return fail(UNC_ERR_INVALID_ARG, "the tile-task inverse takes n in 1..3584");
     if (poll_limit < 1 || poll_limit > (1LL << 22)) return fail(UNC_ERR_INVALID_ARG, "poll_limit must be in 1..2^22");
     return dense_inverse(d_A, n, lda, stream, poll_limit, skip_task);
+}
+
+int unc_spd_inverse_tasks_resident(double* d_A, int n, int lda, int ctas, void* stream) {
+    g_last_error.clear();
+    if (!spd_tasks_apply(n)) return fail(UNC_ERR_INVALID_ARG, "the tile-task inverse takes n in 1..3584");
+    if (ctas < 1) return fail(UNC_ERR_INVALID_ARG, "ctas must be at least 1");
+    return dense_inverse(d_A, n, lda, stream, 0, -1, ctas);
 }
 
 int unc_jtj_crs(int num_rows, int num_cols, const int* rows, const int* cols, const double* values,

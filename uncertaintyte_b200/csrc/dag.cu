@@ -34,8 +34,9 @@
 // in shared memory when POTRF(k+1) needs it and the next tiles are fetched
 // beside the leaf, and the SM's second CTA leaves it the FP64 pipe (it retires
 // once a CTA elsewhere takes tasks). The other CTAs' tasks still depend only on
-// earlier entries and on the chain, so one resident CTA beside the chain's is
-// enough to complete.
+// earlier entries and on the chain. Where none of them is resident to take the
+// entries before POTRF(k), the chain's CTA takes those itself while it waits
+// (chain_wait), in list order, so that it completes alone as well.
 //
 // Counters (ints, zeroed before the launch): cursor, abort flag, 1 + the SM of the
 // chain, CTAs on other SMs, then per
@@ -282,85 +283,143 @@ struct TaskMatrix {
 __constant__ const unsigned kDiagBlocks[8] = {0x14321077u, 0x14321066u, 0x14321055u, 0x14321044u,
                                               0x03321033u, 0x00021002u, 0x16511061u, 0x05576557u};
 
+// The chain's place (shared): where it goes on after the entry `taken`, which its CTA
+// runs meanwhile.
+struct Chain {
+    int step;      // 2 k, or 2 k + 1 when POTRF(k) has its T(k,k) and waits for A(k+1,k); -1: not this CTA's
+    int taken;     // the entry to run
+    int patience;  // polls of a wait before the CTA takes entries itself
+};
+enum : int { CHAIN_GAVE_UP = 0, CHAIN_ON = 1, CHAIN_TAKEN = 2 };
+constexpr int kChainPatience = 512;
+
+// The chain's wait for *counter >= v before or in POTRF(k). Once `patience` polls have
+// passed without it and the entries before POTRF(k) are not all claimed, it claims
+// the next of them for its own CTA (CHAIN_TAKEN). Such an entry depends on entries
+// before itself only: claimed by CTAs that run, run here already, or diagonal tasks
+// that are done. Never at or past POTRF(k) (place, see append_places): those may wait
+// for it. The first time takes longer than any wait beside other CTAs; from then on
+// entries are taken without delay. flag: a shared int.
+__device__ int chain_wait(const TaskMatrix& m, Chain* chain, int* cursor, const int4* place, const int* counter, int v,
+                          int* flag) {
+    if (threadIdx.x == 0) {
+        int r = CHAIN_GAVE_UP;
+        for (long it = 0; it < m.spin && r == CHAIN_GAVE_UP; ++it) {
+            if (ld_acquire(counter) >= v) {
+                r = CHAIN_ON;
+            } else if (ld_acquire(m.abort)) {
+                break;
+            } else if (it >= chain->patience) {
+                const int next = ld_acquire(cursor);
+                if (next < place->x && atomicCAS(cursor, next, next + 1) == next) {
+                    chain->taken = next;
+                    chain->patience = 0;
+                    r = CHAIN_TAKEN;
+                }
+            }
+            if (r == CHAIN_GAVE_UP) __nanosleep(32);
+        }
+        if (r == CHAIN_GAVE_UP) m.give_up();
+        flag[0] = r;
+    }
+    __syncthreads();
+    return flag[0];
+}
+
 // POTRF(k): A(k,k) -= L(k,k-1) L(k,k-1)^T, the leaf, T(k,k) published, then
 // L(k+1,k) = A(k+1,k) T(k,k)^T with T(k,k) still in shared memory (Bs), published.
-// A(k+1,k) is fetched beside the leaf once its updates are in. chained: called
-// in order by one CTA: L(k,k-1) is left in As by the call before, which also
-// fetched A(k,k) into S when diag_in. Otherwise the caller has waited for both.
-// flag: three shared ints. False when a wait gave up.
-__device__ bool potrf(const TaskMatrix& m, int k, bool chained, bool& diag_in, double* sm, int* flag) {
+// A(k+1,k) is fetched beside the leaf once its updates are in. chained: called in
+// order by one CTA: L(k,k-1) is left in As by the call before (unless gone: other
+// tasks ran since), which also fetched A(k,k) into S when diag_in; at a wait the call
+// may return CHAIN_TAKEN, to be repeated with gone (and chain->step odd: from T(k,k)
+// on) after the entry taken. Otherwise the caller has waited for both. flag: three
+// shared ints.
+template <bool chained>
+__device__ __forceinline__ int potrf(const TaskMatrix& m, int k, Chain* chain, int* cursor, const int4* place, bool gone,
+                                     bool& diag_in, double* sm, int* flag) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     // column blocks 0, 16, 48, 32: the product with a lower triangle takes warps w and
     // w + 4, which share a scheduler, the same time in sum
     const int wm = (warp & 1) * 32, wn = ((warp >> 1) ^ (warp >> 2)) * 16;
     double *As = sm, *Bs = sm + LEAF_TILE, *S = sm + 2 * LEAF_TILE;
     const bool below = k + 1 < m.tiles();
-    if (chained && k > 0 && !diag_in) {
-        if (tid == 0) flag[0] = m.wait(m.ver + tri(k, k), k - 1) || m.give_up();
+    const bool from_panel = chained && (chain->step & 1);  // T(k,k) is there
+    if (!from_panel) {
+        if (chained && k > 0 && !diag_in) {
+            const int r = chain_wait(m, chain, cursor, place + k, m.ver + tri(k, k), k - 1, flag);
+            if (r != CHAIN_ON) return r;
+        }
+        if (!diag_in) chol_leaf_load(m.A, m.ld, TB * k, m.ext(k), S);
+        if (k > 0 && (!chained || gone)) load_tile(As, m.tile(m.A, k, k - 1), m.ld, m.ext(k), m.ext(k - 1), tid);
+        tile_wait();
         __syncthreads();
-        if (!flag[0]) return false;
-    }
-    if (!diag_in) chol_leaf_load(m.A, m.ld, TB * k, m.ext(k), S);
-    if (k > 0 && !chained) load_tile(As, m.tile(m.A, k, k - 1), m.ld, m.ext(k), m.ext(k - 1), tid);
-    tile_wait();
-    __syncthreads();
-    if (k > 0) {
-        // S -= As As^T, lower 8 x 8 blocks only, four or five per warp (kDiagBlocks)
-        const unsigned tab = kDiagBlocks[warp];
-        const int rows[2] = {(int)(tab & 7u) * 8, (int)(tab >> 4 & 7u) * 8};
-        const bool five = (tab >> 28) != 0u;
-        int cols[5];
-        double c[5][2], d[5][2];
+        if (k > 0) {
+            // S -= As As^T, lower 8 x 8 blocks only, four or five per warp (kDiagBlocks)
+            const unsigned tab = kDiagBlocks[warp];
+            const int rows[2] = {(int)(tab & 7u) * 8, (int)(tab >> 4 & 7u) * 8};
+            const bool five = (tab >> 28) != 0u;
+            int cols[5];
+            double c[5][2], d[5][2];
 #pragma unroll
-        for (int q = 0; q < 5; ++q) {
-            cols[q] = (int)(tab >> (8 + 4 * q) & 7u) * 8;
-            c[q][0] = c[q][1] = 0.0;
+            for (int q = 0; q < 5; ++q) {
+                cols[q] = (int)(tab >> (8 + 4 * q) & 7u) * 8;
+                c[q][0] = c[q][1] = 0.0;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) d[q][h] = S[(cols[q] + 2 * t4 + h) * TLD + rows[q / 3] + g];
-        }
-#pragma unroll 4
-        for (int kk = 0; kk < TB; kk += 4) {
-            const double* at = As + (kk + t4) * TLD + g;
-            const double a[2] = {at[rows[0]], at[rows[1]]};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) dmma(c[q][0], c[q][1], a[q / 3], at[cols[q]]);
-            if (five) dmma(c[4][0], c[4][1], a[1], at[cols[4]]);
-        }
-#pragma unroll
-        for (int q = 0; q < 5; ++q)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int col = cols[q] + 2 * t4 + h, row = rows[q / 3] + g;
-                if (col <= row && (q < 4 || five) && !(q == 2 && cols[2] == cols[1]))
-                    S[col * TLD + row] = d[q][h] - c[q][h];
+                for (int h = 0; h < 2; ++h) d[q][h] = S[(cols[q] + 2 * t4 + h) * TLD + rows[q / 3] + g];
             }
-    }
-    if (tid == 0) flag[0] = 0;
-    __syncthreads();
-    // A(k+1,k) into As before the leaf's last products when warp 4 has seen its updates
-    // (one warp's loads of a tile take longer than a panel: 1.8 us more per step)
-    chol_leaf_factor(
-        TB * k, m.ext(k), m.T, m.ld, m.err, S, Bs,
-        [&](int q) {
-            if (!below || q < 2) return;
-            for (int poll = q; poll < 5; poll += 2)  // the last panel: twice
-                if (lane == 0 && !flag[0] && ld_acquire(m.ver + tri(k + 1, k)) >= k) flag[0] = 1;
-        },
-        [&] {
-            if (flag[0]) load_tile(As, m.tile(m.A, k + 1, k), m.ld, m.ext(k + 1), m.ext(k), tid);
-        });
-    tile_wait();
-    __syncthreads();
-    if (tid == 0) {
-        __threadfence();
-        atomicExch(m.lrdy + tri(k, k), 1);
-        atomicExch(m.trdy + tri(k, k), 1);
-    }
-    if (!below) return true;
-    if (!flag[0]) {
-        if (tid == 0) flag[1] = m.wait(m.ver + tri(k + 1, k), k) || m.give_up();
+#pragma unroll 4
+            for (int kk = 0; kk < TB; kk += 4) {
+                const double* at = As + (kk + t4) * TLD + g;
+                const double a[2] = {at[rows[0]], at[rows[1]]};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) dmma(c[q][0], c[q][1], a[q / 3], at[cols[q]]);
+                if (five) dmma(c[4][0], c[4][1], a[1], at[cols[4]]);
+            }
+#pragma unroll
+            for (int q = 0; q < 5; ++q)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int col = cols[q] + 2 * t4 + h, row = rows[q / 3] + g;
+                    if (col <= row && (q < 4 || five) && !(q == 2 && cols[2] == cols[1]))
+                        S[col * TLD + row] = d[q][h] - c[q][h];
+                }
+        }
+        if (tid == 0) flag[0] = 0;
         __syncthreads();
-        if (!flag[1]) return false;
+        // A(k+1,k) into As before the leaf's last products when warp 4 has seen its updates
+        // (one warp's loads of a tile take longer than a panel: 1.8 us more per step)
+        chol_leaf_factor(
+            TB * k, m.ext(k), m.T, m.ld, m.err, S, Bs,
+            [&](int q) {
+                if (!below || q < 2) return;
+                for (int poll = q; poll < 5; poll += 2)  // the last panel: twice
+                    if (lane == 0 && !flag[0] && ld_acquire(m.ver + tri(k + 1, k)) >= k) flag[0] = 1;
+            },
+            [&] {
+                if (flag[0]) load_tile(As, m.tile(m.A, k + 1, k), m.ld, m.ext(k + 1), m.ext(k), tid);
+            });
+        tile_wait();
+        __syncthreads();
+        if (tid == 0) {
+            __threadfence();
+            atomicExch(m.lrdy + tri(k, k), 1);
+            atomicExch(m.trdy + tri(k, k), 1);
+        }
+    }
+    if (!below) return CHAIN_ON;
+    if (from_panel || !flag[0]) {
+        if (chained) {
+            const int r = chain_wait(m, chain, cursor, place + k, m.ver + tri(k + 1, k), k, flag + 1);
+            if (r != CHAIN_ON) {
+                if (tid == 0) chain->step = 2 * k + 1;
+                return r;
+            }
+            if (from_panel) load_tile(Bs, m.tile(m.T, k, k), m.ld, m.ext(k), m.ext(k), tid);
+        } else {
+            if (tid == 0) flag[1] = m.wait(m.ver + tri(k + 1, k), k) || m.give_up();
+            __syncthreads();
+            if (!flag[1]) return CHAIN_GAVE_UP;
+        }
         load_tile(As, m.tile(m.A, k + 1, k), m.ld, m.ext(k + 1), m.ext(k), tid);
         tile_wait();
     }
@@ -378,26 +437,32 @@ __device__ bool potrf(const TaskMatrix& m, int k, bool chained, bool& diag_in, d
     }
     double* L = m.tile(m.A, k + 1, k);
     tile_elements(m.ext(k + 1), m.ext(k), wm, wn, g, t4, acc, [&](int r, int c, double& v) { L[r + (long)c * m.ld] = v; });
+    if (chained && tid == 0) chain->step = 2 * k + 2;
     __syncthreads();
     if (tid == 32 * 5) {  // warp 5: its share of the next update is short
         __threadfence();
         atomicExch(m.lrdy + tri(k + 1, k), 1);
     }
-    return true;
+    return CHAIN_ON;
 }
 
-// Every POTRF(k) of one matrix, in order, by the calling CTA.
-__device__ bool run_chain(const TaskMatrix& m, double* sm, int* flag) {
-    bool diag_in = false;
-    for (int k = 0; k < m.tiles(); ++k)
-        if (!potrf(m, k, true, diag_in, sm, flag)) return false;
-    return true;
+// Every POTRF(k) of one matrix from chain->step on, in order, by the calling CTA;
+// place: of POTRF(0 ..) in the list.
+__device__ __forceinline__ int run_chain(const TaskMatrix& m, Chain* chain, int* cursor, const int4* place, double* sm,
+                                         int* flag) {
+    bool diag_in = false, gone = true;  // k = 0 needs no tile of before
+    for (int k = chain->step >> 1; k < m.tiles(); ++k, gone = false) {
+        const int r = potrf<true>(m, k, chain, cursor, place, gone, diag_in, sm, flag);
+        if (r != CHAIN_ON) return r;
+    }
+    return CHAIN_ON;
 }
 
 // One tile task (type, i, j, k with its count), run by all DAG_THREADS threads of
 // the block; warp 0 waits for its dependencies first. Returns false when a wait
 // gave up (ERRBIT_TIMEOUT and the abort flag are set): the caller stops taking
-// tasks.
+// tasks. kDiagonal: POTRF may be among them.
+template <bool kDiagonal>
 __device__ __forceinline__ bool run_task(const TaskMatrix& m, int type, int i, int j, int kc, double* sm, int* flag) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, t4 = lane & 3;
@@ -435,9 +500,9 @@ __device__ __forceinline__ bool run_task(const TaskMatrix& m, int type, int i, i
     }
     __syncthreads();
     if (!flag[0]) return false;
-    if (type == K_POTRF) {
+    if (kDiagonal && type == K_POTRF) {
         bool diag_in = false;
-        return potrf(m, k, false, diag_in, sm, flag);
+        return potrf<false>(m, k, nullptr, nullptr, nullptr, false, diag_in, sm, flag) != CHAIN_GAVE_UP;
     }
     auto ref = [&](double* M, int r, int c) { return TileRef{m.tile(M, r, c), m.ext(r), m.ext(c)}; };
     Acc acc = {}, prev = {};
@@ -501,36 +566,49 @@ __global__ void __launch_bounds__(DAG_THREADS, DAG_CTAS)
                         int* state, int ntri, int* err, long spin) {
     extern __shared__ __align__(16) double sm[];
     __shared__ int s_task, flag[3];
+    __shared__ Chain chain;
     int* const cursor = state;
     int* const chain_sm = state + 2;  // 1 + the SM that runs the chain
     int* const others = state + 3;    // CTAs that take tasks on other SMs until the list is done
     const TaskMatrix m(A, T, O, n, ld, state, ntri, err, state + 1, spin);
-    bool counted = false, chain = false;  // thread 0
+    bool counted = false, begin = false, ran_chain = false;  // thread 0
+    if (threadIdx.x == 0) chain = Chain{-1, 0, (int)min((long)kChainPatience, spin / 2)};
     while (true) {
         if (threadIdx.x == 0) {
-            const int at = ld_acquire(chain_sm), here = sm_id() + 1;
-            if (at != 0 && at != here && !counted) {
-                atomicAdd(others, 1);
-                counted = true;
+            if (begin) chain.step = 0;
+            begin = false;
+            if (chain.step < 0) {
+                const int at = ld_acquire(chain_sm), here = sm_id() + 1;
+                if (at != 0 && at != here && !counted) {
+                    atomicAdd(others, 1);
+                    counted = true;
+                }
+                // beside the chain, unless nobody else is there to do the tasks
+                const bool retire = at == here && !ran_chain && ld_acquire(others) > 0;
+                s_task = retire ? ntasks : atomicAdd(cursor, 1);
             }
-            // beside the chain, unless nobody else is there to do the tasks
-            const bool retire = at == here && !chain && ld_acquire(others) > 0;
-            s_task = retire ? ntasks : atomicAdd(cursor, 1);
         }
         __syncthreads();
-        const int task = s_task;
-        if (task >= ntasks) break;
-        const int4 tk = tasks[task];
-        if (tk.x != K_POTRF) {
-            if (!run_task(m, tk.x, tk.y, tk.z, tk.w, sm, flag)) break;
-        } else if (tk.y == 0) {
-            if (threadIdx.x == 0) {
-                chain = true;
+        int4 tk;
+        if (chain.step < 0) {
+            if (s_task >= ntasks) break;
+            tk = tasks[s_task];
+            if (threadIdx.x == 0 && tk.x == K_POTRF && tk.y == 0) {
+                begin = ran_chain = true;  // the chain, from the next round on
                 atomicExch(chain_sm, sm_id() + 1);
             }
-            if (!run_chain(m, sm, flag)) break;
+        } else {
+            const int r = run_chain(m, &chain, cursor, tasks + ntasks, sm, flag);
+            if (r == CHAIN_GAVE_UP) break;
+            __syncthreads();
+            tk = tasks[chain.taken];
+            if (r == CHAIN_ON) {  // all done: among the others from now on
+                tk.x = K_POTRF;
+                if (threadIdx.x == 0) chain.step = -1;
+            }
         }
-        __syncthreads();  // s_task and flag are rewritten
+        if (tk.x != K_POTRF && !run_task<false>(m, tk.x, tk.y, tk.z, tk.w, sm, flag)) break;
+        __syncthreads();  // s_task, flag and the chain's place are rewritten
     }
 }
 
@@ -555,7 +633,7 @@ __global__ void __launch_bounds__(DAG_THREADS, DAG_CTAS)
         const int4 tk = tasks[task];
         const SpdTaskMatrix& d = mats[tk.x >> 3];
         const TaskMatrix m(d.A, d.T, d.O, d.n, d.ld, d.state, d.ntri, d.err, ctl + 1, spin);
-        if (!run_task(m, tk.x & 7, tk.y, tk.z, tk.w, sm, flag)) break;
+        if (!run_task<true>(m, tk.x & 7, tk.y, tk.z, tk.w, sm, flag)) break;
         __syncthreads();
     }
 }
@@ -637,9 +715,17 @@ std::vector<int4> single_tasks(const std::vector<int4>& v) {
     return out;
 }
 
+// After the list the places of POTRF(0 .. nt - 1) in it, for the chain (0 where one is left out).
+void append_places(std::vector<int4>& v, int nt) {
+    std::vector<int> place(nt, 0);
+    for (size_t q = 0; q < v.size(); ++q)
+        if (v[q].x == K_POTRF) place[v[q].y] = (int)q;
+    for (int p : place) v.push_back(make_int4(p, 0, 0, 0));
+}
+
 struct TaskLists {
     std::mutex mu;
-    std::map<std::tuple<int, int, bool>, std::pair<int4*, int>> lists;  // (device, nt, product) -> device copy
+    std::map<std::tuple<int, int, bool>, std::pair<int4*, int>> lists;  // (device, nt, product) -> device copy, tasks
     std::map<int, cudaStream_t> upload;                          // device -> upload stream
 };
 TaskLists& task_lists() {
@@ -664,7 +750,9 @@ int spd_tasks_prepare(int n, bool product) {
     TaskLists& tl = task_lists();
     std::lock_guard<std::mutex> lock(tl.mu);
     if (tl.lists.count({dev, nt, product})) return UNC_OK;
-    const std::vector<int4> h = build_tasks(nt, product);
+    std::vector<int4> h = build_tasks(nt, product);
+    const int ntasks = (int)h.size();
+    append_places(h, nt);
     // upload on a private non-blocking stream: a copy on the legacy default
     // stream would wait for every other stream's work (a serving process runs
     // several requests at once)
@@ -688,12 +776,12 @@ int spd_tasks_prepare(int n, bool product) {
         return cudaFuncSetAttribute(k_spd_inverse_tasks, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)DAG_SMEM) == cudaSuccess;
     });
-    tl.lists[{dev, nt, product}] = {d, (int)h.size()};
+    tl.lists[{dev, nt, product}] = {d, ntasks};
     return UNC_OK;
 }
 
 int chol_inverse_tasks(double* A, int n, int lda, double* T, double* O, int* state, int* err, cudaStream_t st,
-                       int max_ctas, long long poll_limit, int skip_task) {
+                       int max_ctas, long long poll_limit, int skip_task, int max_grid) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return UNC_ERR_CUDA;
     const int nt = (n + TB - 1) / TB;
@@ -712,6 +800,8 @@ int chol_inverse_tasks(double* A, int n, int lda, double* T, double* O, int* sta
     if (skip_task >= 0 && skip_task < unc_spd_task_list(n, nullptr, 0)) {
         std::vector<int4> h = single_tasks(build_tasks(nt, O != nullptr));
         h.erase(h.begin() + skip_task);
+        const int left = (int)h.size();
+        append_places(h, nt);
         if (cudaMallocAsync(reinterpret_cast<void**>(&own), sizeof(int4) * h.size(), st) != cudaSuccess)
             return UNC_ERR_OUT_OF_MEMORY;
         if (cudaMemcpyAsync(own, h.data(), sizeof(int4) * h.size(), cudaMemcpyHostToDevice, st) != cudaSuccess ||
@@ -719,9 +809,10 @@ int chol_inverse_tasks(double* A, int n, int lda, double* T, double* O, int* sta
             cudaFreeAsync(own, st);
             return UNC_ERR_CUDA;
         }
-        list = {own, (int)h.size()};
+        list = {own, left};
     }
-    const int grid = std::max(1, std::min(DAG_CTAS * std::min(device_sms(), max_ctas), list.second));
+    int grid = std::max(1, std::min(DAG_CTAS * std::min(device_sms(), max_ctas), list.second));
+    if (max_grid > 0) grid = std::min(grid, max_grid);
     k_spd_inverse_tasks<<<grid, DAG_THREADS, DAG_SMEM, st>>>(A, T, O, n, lda, list.first, list.second, state, ntri,
                                                              err, spin);
     count_launch();

@@ -534,7 +534,8 @@ int spd_inverse(double* A, int n, int lda, double shift, double* e, const SpdScr
                 cudaStream_t st) {
     launch_shift_equilibrate(A, n, lda, shift, e, err, st);
     if (s.state && spd_tasks_apply(n)) {
-        if (int r = chol_inverse_tasks(A, n, lda, s.T, s.W, s.state, err, st, s.max_ctas, s.poll_limit, s.skip_task))
+        if (int r = chol_inverse_tasks(A, n, lda, s.T, s.W, s.state, err, st, s.max_ctas, s.poll_limit, s.skip_task,
+                                       s.max_grid))
             return r;
         launch_unequilibrate_from(s.W, A, n, lda, e, Y, st);
         return UNC_OK;

@@ -195,6 +195,7 @@ struct SpdScratch {
     int max_ctas = 148;        // SMs that the tile tasks may cover
     long long poll_limit = 0;  // as chol_inverse_tasks
     int skip_task = -1;
+    int max_grid = 0;
 };
 // Uploads the task lists that an inverse of order n uses (once per device and
 // size; outside any stream capture).
@@ -229,9 +230,10 @@ int spd_tasks_prepare(int n, bool product = true);
 // do the results.
 // poll_limit (> 0): polls of one dependency before a wait gives up (default
 // and maximum 2^22); skip_task >= 0 leaves that task out of the schedule, which
-// can then not complete: only for tests of the bounded waits.
+// can then not complete: only for tests of the bounded waits; max_grid > 0 bounds
+// the CTAs of the launch.
 int chol_inverse_tasks(double* A, int n, int lda, double* T, double* O, int* state, int* err, cudaStream_t st,
-                       int max_ctas = 148, long long poll_limit = 0, int skip_task = -1);
+                       int max_ctas = 148, long long poll_limit = 0, int skip_task = -1, int max_grid = 0);
 // One matrix of a grouped tile-task inverse: A (lower triangle) becomes L, T
 // receives L^{-1}, O = A^{-1}; state: spd_task_state_ints(n) zeroed ints; err:
 // the matrix's error word.
