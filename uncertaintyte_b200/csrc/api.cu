@@ -1242,7 +1242,7 @@ int unc_jtj_crs(int num_rows, int num_cols, const int* rows, const int* cols, co
     CK(cudaMemcpy(d_cols, cols, sizeof(int) * (size_t)nnz, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(d_vals, values, sizeof(double) * (size_t)nnz, cudaMemcpyHostToDevice));
     CK(cudaMemset(s.err, 0, 16));
-    launch_repack_generic(nobs, cam_off, d_rows, d_cols, d_vals, d_J, s.obs_cam, s.obs_pt, s.err, sm);
+    launch_repack_generic(nobs, C, P, d_rows, d_cols, d_vals, d_J, s.obs_cam, s.obs_pt, s.err, sm);
     launch_build_index(s, sm);
     launch_long_lists(s, sm);
     launch_point_blocks(s, sm);

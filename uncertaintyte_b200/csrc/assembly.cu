@@ -73,7 +73,7 @@ void launch_validate_obs(const SceneDev& s, cudaStream_t st) {
 
 // Generic repack for J^T J export: rows of 12 (camera + point) or 9 (camera
 // only) entries; writes the 24-value observation record with zero point part.
-__global__ void k_repack_generic(int num_obs, int cam_off, const int* __restrict__ rows,
+__global__ void k_repack_generic(int num_obs, int num_cams, int num_points, const int* __restrict__ rows,
                                  const int* __restrict__ cols, const double* __restrict__ vals,
                                  double* __restrict__ J, int* obs_cam, int* obs_pt, int* err) {
     int o = blockIdx.x * blockDim.x + threadIdx.x;
@@ -83,8 +83,10 @@ __global__ void k_repack_generic(int num_obs, int cam_off, const int* __restrict
     bool bad = n0 != n1 || (n0 != 12 && n0 != 9);
     int cam = -1, pt = -1;
     double* out = J + 24L * o;
+    const int cam_off = kCamParams * num_cams;
     if (!bad) {
         cam = cols[r0] / kCamParams;
+        bad = cols[r0] < 0 || cam >= num_cams;
         for (int j = 0; j < 9; ++j) {
             bad |= cols[r0 + j] != cam * 9 + j || cols[r1 + j] != cam * 9 + j;
             out[j] = vals[r0 + j];
@@ -92,6 +94,7 @@ __global__ void k_repack_generic(int num_obs, int cam_off, const int* __restrict
         }
         if (n0 == 12) {
             pt = (cols[r0 + 9] - cam_off) / 3;
+            bad |= cols[r0 + 9] < cam_off || pt >= num_points;
             for (int j = 0; j < 3; ++j) {
                 bad |= cols[r0 + 9 + j] != cam_off + 3 * pt + j || cols[r1 + 9 + j] != cam_off + 3 * pt + j;
                 out[9 + j] = vals[r0 + 9 + j];
@@ -109,11 +112,11 @@ __global__ void k_repack_generic(int num_obs, int cam_off, const int* __restrict
     obs_pt[o] = pt;
 }
 
-void launch_repack_generic(int num_obs, int cam_off, const int* rows, const int* cols,
+void launch_repack_generic(int num_obs, int num_cams, int num_points, const int* rows, const int* cols,
                            const double* vals, double* J, int* obs_cam, int* obs_pt, int* err,
                            cudaStream_t st) {
     if (num_obs == 0) return;
-    k_repack_generic<<<(num_obs + 255) / 256, 256, 0, st>>>(num_obs, cam_off, rows, cols, vals, J,
+    k_repack_generic<<<(num_obs + 255) / 256, 256, 0, st>>>(num_obs, num_cams, num_points, rows, cols, vals, J,
                                                             obs_cam, obs_pt, err);
     count_launch();
 }

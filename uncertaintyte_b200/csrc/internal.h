@@ -143,7 +143,7 @@ int launch_schur_columns(const SceneDev& s, double* Z, int ldz, cudaStream_t st)
 size_t schur_columns_smem(int num_cams);
 void prepare_schur_columns();  // kernel attributes (before any stream capture)
 // Generic 9/12-entry-row repack for the J^T J export (camera-only rows allowed).
-void launch_repack_generic(int num_obs, int cam_off, const int* rows, const int* cols,
+void launch_repack_generic(int num_obs, int num_cams, int num_points, const int* rows, const int* cols,
                            const double* vals, double* J, int* obs_cam, int* obs_pt, int* err,
                            cudaStream_t st);
 void launch_unscaled_blocks(const SceneDev& s, double* U, double* W, cudaStream_t st);
