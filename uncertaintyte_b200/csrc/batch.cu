@@ -82,9 +82,7 @@ struct Scene {
 struct Layout {
     size_t in_bytes = 0, out_bytes = 0, total = 0;
     // device regions (offsets)
-    size_t mixed_off = 0, mixed_bytes = 0;
     size_t zero_off = 0, zero_bytes = 0;  // dag states + control words
-    size_t amax_off = 0, amax_bytes = 0;
     size_t stat_off = 0, stat_bytes = 0;  // error words + Taylor states
     size_t desc_off = 0, desc_bytes = 0;  // descriptors uploaded from the host
 };
@@ -274,14 +272,12 @@ void lay_out(char* base, std::vector<Scene>& sc, int slices, int nt, Layout& L, 
         carve(base ? at : nullptr, s.pl, false, 0, s.pl.nobs * 2, s.b);
     }
     c.off = (c.off + 255) & ~size_t(255);
-    L.mixed_off = c.off;
     for (auto& s : sc) {
         const size_t sb = mixed_slice_bytes_nt(s.pl.N, slices, nt);
         for (int q = 0; q < 4; ++q) s.buf[q] = c.take<int8_t>(sb);
         for (int q = 0; q < 4; ++q) s.ex[q] = c.take<int>((size_t)s.pl.N + 64);
     }
     c.off = (c.off + 255) & ~size_t(255);
-    L.mixed_bytes = c.off - L.mixed_off;
     // zero at the start of the dense stage: tile-task counters of every scene,
     // the powers' diagonal maxima, control words (last)
     L.zero_off = c.off;
@@ -290,10 +286,6 @@ void lay_out(char* base, std::vector<Scene>& sc, int slices, int nt, Layout& L, 
     c.take<int>(4);
     c.off = (c.off + 255) & ~size_t(255);
     L.zero_bytes = c.off - L.zero_off;
-    L.amax_off = c.off;
-    for (auto& s : sc) s.b.amax = c.take<unsigned long long>(4);
-    c.off = (c.off + 255) & ~size_t(255);
-    L.amax_bytes = c.off - L.amax_off;
     // status words read back at the end: error words, then Taylor states
     L.stat_off = c.off;
     int* errs = c.take<int>(4 * sc.size());
@@ -348,7 +340,7 @@ int launch_group(unc_batch* b, GroupRun& g) {
     launch_shift_equilibrate_grouped(g.dd.dense, n, g.dd.blk_rows, g.nblk_rows, g.dd.blk_elems, g.nblk_elems, sm);
     int* ctl = reinterpret_cast<int*>(g.dbase + g.L.zero_off + g.L.zero_bytes - 256);
     if (int r = chol_inverse_tasks_grouped(g.dd.mats, g.dd.tasks, (int)g.ntasks, ctl, sm, device_sms())) return r;
-    launch_unequilibrate_grouped(g.dd.dense, n, g.dd.blk_elems, g.nblk_elems, sm);  // X in Z, iZ = X
+    launch_unequilibrate_grouped(g.dd.dense, n, g.dd.blk_elems, g.nblk_elems, sm);  // X in Z
     // the Taylor series from blocked powers (powers.cu), every step over all scenes
     auto slice = [&](int set) {
         mixed_slice_grouped(g.slices, g.dd.slice + (size_t)set * n, n, g.dd.row_start, g.total_rows, sm);
@@ -464,7 +456,7 @@ int prepare_group(unc_batch* b, GroupRun& g, int nt) {
             hdd.maps[kMaps * i + m] = op[m].map;
         }
         const int rows = op[0].rows, kp = op[0].kp;
-        hdd.dense[i] = DenseJob{s.b.Z, s.b.add, s.b.e, ld, N, s.lambda, s.b.s.err, s.b.te, s.b.amax};
+        hdd.dense[i] = DenseJob{s.b.Z, s.b.add, s.b.e, ld, N, s.lambda, s.b.s.err, s.b.te};
         hdd.blk_rows[i] = br;
         hdd.blk_elems[i] = be;
         hdd.blk_cols[i] = bc;
@@ -481,8 +473,7 @@ int prepare_group(unc_batch* b, GroupRun& g, int nt) {
         };
         const SliceDef sd[kSliceSets] = {{s.b.Z, 0}, {s.b.add, 1}, {s.b.tmp, 1}, {s.b.p4, 2}, {s.b.p8, 3}};
         for (int q = 0; q < kSliceSets; ++q)
-            hdd.slice[(size_t)q * n + i] = MixedSliceJob{sd[q].src, ld, N, s.buf[sd[q].buf], rows, kp,
-                                                         s.ex[sd[q].buf], nullptr, nullptr, nullptr};
+            hdd.slice[(size_t)q * n + i] = MixedSliceJob{sd[q].src, ld, N, s.buf[sd[q].buf], rows, kp, s.ex[sd[q].buf]};
         // products: A map, B map, A / B exponent buffers, output, skip
         const CUtensorMap* dm = g.dd.maps + kMaps * i;
         struct GemmDef {

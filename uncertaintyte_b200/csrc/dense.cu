@@ -430,21 +430,9 @@ void gemm_f64_mode(int M, int N, int K, double alpha, const double* A, int lda, 
         launch_gemm<32>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, amax, mode, st, ws, ws_doubles, skip);
 }
 
-void gemm_f64_ex(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
-                 double beta, double* C, int ldc, unsigned long long* amax, bool lower_only, cudaStream_t st,
-                 bool trans_b) {
-    gemm_f64_mode(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, amax,
-                  (lower_only ? GEMM_LOWER : 0) | (trans_b ? GEMM_TRANS_B : 0), st);
-}
-
 void gemm_f64(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
               double beta, double* C, int ldc, unsigned long long* amax, cudaStream_t st) {
-    gemm_f64_ex(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, amax, false, st, false);
-}
-
-void gemm_f64_tri(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
-                  double beta, double* C, int ldc, cudaStream_t st) {
-    gemm_f64_ex(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, nullptr, true, st, false);
+    gemm_f64_mode(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, amax, 0, st);
 }
 
 // ------------------------------------------------------------------------
@@ -617,22 +605,8 @@ void launch_unequilibrate(double* X, int n, int lda, const double* e, double* Y,
     launch_scale(X, X, n, lda, e, Y, false, st);
 }
 
-__global__ void k_axpy(double* Y, const double* __restrict__ X, double k, int n, long ld) {
-    long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    long total = (long)n * n;
-    if (idx >= total) return;
-    int c = (int)(idx / n), r = (int)(idx - (long)c * n);
-    long o = r + c * ld;
-    Y[o] = Y[o] + k * X[o];
-}
-
-void launch_axpy(double* Y, const double* X, double k, int n, int ld, cudaStream_t st) {
-    long total = (long)n * n;
-    k_axpy<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(Y, X, k, n, ld);
-    count_launch();
-}
-
-__device__ __forceinline__ void te_decide_one(TeState* s, const unsigned long long* amax_bits, double k) {
+__global__ void k_te_decide(TeState* s, const unsigned long long* amax_bits, double k) {
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
     if (s->done) return;
     double amax = __longlong_as_double((long long)*amax_bits);
     amax = fmax(amax, 2.2250738585072014e-308);  // absMax starts at DBL_MIN (ScaledDenseMatrix.cpp:208)
@@ -646,11 +620,6 @@ __device__ __forceinline__ void te_decide_one(TeState* s, const unsigned long lo
     if (s->iters < 20) s->change[s->iters] = change;
     s->iters += 1;
     s->coef = k;
-}
-
-__global__ void k_te_decide(TeState* s, const unsigned long long* amax_bits, double k) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    te_decide_one(s, amax_bits, k);
 }
 
 __device__ __forceinline__ void te_init_one(TeState* s) {
@@ -706,11 +675,6 @@ __global__ void k_te_init_grouped(const DenseJob* __restrict__ jobs, int njobs) 
     if (m < njobs) te_init_one(jobs[m].te);
 }
 
-__global__ void k_te_decide_grouped(const DenseJob* __restrict__ jobs, int njobs, const double* __restrict__ k) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m < njobs) te_decide_one(jobs[m].te, jobs[m].amax, k[m]);
-}
-
 void launch_shift_equilibrate_grouped(const DenseJob* d_jobs, int njobs, const long* d_blk_rows, long nblk_rows,
                                       const long* d_blk_elems, long nblk_elems, cudaStream_t st) {
     if (njobs <= 0) return;
@@ -731,12 +695,6 @@ long scale_blocks_grouped(int n) { return scale_blocks(n); }
 void launch_te_init_grouped(const DenseJob* d_jobs, int njobs, cudaStream_t st) {
     if (njobs <= 0) return;
     k_te_init_grouped<<<(njobs + 127) / 128, 128, 0, st>>>(d_jobs, njobs);
-    count_launch();
-}
-
-void launch_te_decide_grouped(const DenseJob* d_jobs, int njobs, const double* d_k, cudaStream_t st) {
-    if (njobs <= 0) return;
-    k_te_decide_grouped<<<(njobs + 127) / 128, 128, 0, st>>>(d_jobs, njobs, d_k);
     count_launch();
 }
 
@@ -766,8 +724,6 @@ void launch_axpy_te(double* Y, const double* X, const TeState* s, int n, int ld,
     k_axpy_te<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(Y, X, s, n, ld);
     count_launch();
 }
-
-void launch_zero(double* p, size_t n, cudaStream_t st) { cudaMemsetAsync(p, 0, n * sizeof(double), st); }
 
 // Camera output: for camera c and j <= k in its block,
 //   camUnc = (iZ(j,k) + iZ(k,j)/2) * d_j * d_k,  d = 1/s   (compute.cpp:176)

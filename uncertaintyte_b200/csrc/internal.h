@@ -153,19 +153,13 @@ void launch_unscaled_blocks(const SceneDev& s, double* U, double* W, cudaStream_
 // epilogue folds max|C| into *amax (bit pattern of a non-negative double).
 void gemm_f64(int M, int N, int K, double alpha, const double* A, int lda, const double* B,
               int ldb, double beta, double* C, int ldc, unsigned long long* amax, cudaStream_t st);
-// General form: lower_only skips output tiles strictly above the diagonal
-// (symmetric results; GEMM_MIRROR of gemm_f64_mode writes the other triangle too).
-// trans_b: B(k, n) is read from B[n + k * ldb] (the transpose of a column-major matrix).
-void gemm_f64_ex(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
-                 double beta, double* C, int ldc, unsigned long long* amax, bool lower_only, cudaStream_t st,
-                 bool trans_b = false);
-// Mode bits of gemm_f64_mode. The k-range bits restrict the k loop of the
-// output tile at (m0, n0) when an operand is triangular (terms outside the
-// range are zero): KLO_M k >= m0, KLO_N k >= n0, KHI_M k < m0 + 64,
-// KHI_N k < n0 + 64 (tile size 64 x 64).
+// Mode bits of gemm_f64_mode. The k-range bits restrict the k loop of the output
+// tile at (m0, n0) when an operand is triangular (terms outside the range are
+// zero): KLO_M k >= m0, KLO_N k >= n0, KHI_M k < m0 + B, KHI_N k < n0 + B, B the
+// side of the tile (64, or 32 where 64 x 64 tiles are fewer than the SMs).
 enum : int {
-    GEMM_LOWER = 1,
-    GEMM_TRANS_B = 2,
+    GEMM_LOWER = 1,    // tiles strictly above the diagonal are skipped
+    GEMM_TRANS_B = 2,  // B(k, n) is read from B[n + k * ldb]
     GEMM_KLO_M = 4,
     GEMM_KLO_N = 8,
     GEMM_KHI_M = 16,
@@ -182,9 +176,6 @@ enum : int {
 void gemm_f64_mode(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
                    double beta, double* C, int ldc, unsigned long long* amax, int mode, cudaStream_t st,
                    double* ws = nullptr, size_t ws_doubles = 0, const int* skip = nullptr);
-// Same, skipping output tiles strictly above the diagonal (symmetric updates).
-void gemm_f64_tri(int M, int N, int K, double alpha, const double* A, int lda, const double* B, int ldb,
-                  double beta, double* C, int ldc, cudaStream_t st);
 // Scratch of an SPD inverse of order n: T (receives L^{-1}; its tiles above the
 // diagonal are neither read nor written) and W, n x lda each; ws: n x lda doubles of split-K
 // partial sums, or unused by the tile tasks; state: spd_task_state_ints(n) ints
@@ -257,9 +248,6 @@ int chol_inverse_tasks_grouped(const SpdTaskMatrix* d_mats, const int4* d_tasks,
                                cudaStream_t st, int max_ctas, long long poll_limit = 0);
 // per context: the largest grid of the tile-task inverse (148 unless set)
 void context_set_task_ctas(unc_context* c, int max_ctas);
-// Y <- Y + k*X  (N x N, column-major)
-void launch_axpy(double* Y, const double* X, double k, int n, int ld, cudaStream_t st);
-
 // Device-side control of the Taylor loop (compute.cpp:141-160): the stop rule
 // runs on the device so that the host never waits inside the loop.
 struct TeState {
@@ -342,7 +330,6 @@ struct DenseJob {
     double lambda;
     int* err;
     TeState* te;
-    const unsigned long long* amax;
 };
 // Z += lambda I and the symmetric equilibration of every job (as launch_shift_equilibrate).
 void launch_shift_equilibrate_grouped(const DenseJob* d_jobs, int njobs, const long* d_blk_rows, long nblk_rows,
@@ -352,11 +339,7 @@ void launch_unequilibrate_grouped(const DenseJob* d_jobs, int njobs, const long*
                                   cudaStream_t st);
 long scale_blocks_grouped(int n);
 void launch_te_init_grouped(const DenseJob* d_jobs, int njobs, cudaStream_t st);
-// the stop rule of every job with its coefficient d_k[m]
-void launch_te_decide_grouped(const DenseJob* d_jobs, int njobs, const double* d_k, cudaStream_t st);
-// Y <- Y + s->coef * X unless s->done.
 void launch_axpy_te(double* Y, const double* X, const TeState* s, int n, int ld, cudaStream_t st);
-void launch_zero(double* p, size_t n, cudaStream_t st);
 // Camera output (a+b/2 quirk) and the unscaled 9x9 camera covariance blocks.
 void launch_camera_output(const double* iZ, int ldz, const double* s_cam, int num_cams,
                           double* cam_unc, double* sig, cudaStream_t st);
@@ -396,9 +379,6 @@ struct MixedSliceJob {  // k_slice_rows of one matrix
     int8_t* out;
     int rows_pad, kp;
     int* exps;
-    double* Y;            // optional Taylor update Y += te->coef * A
-    const TeState* te;
-    const int* skip;      // optional: return when *skip != 0
 };
 struct MixedGemmJob {  // one lower-triangle symmetric product C = P X (mirrored)
     const CUtensorMap* tA;  // 64-byte aligned maps in device memory

@@ -297,9 +297,8 @@ __global__ void __launch_bounds__(256) k_slice_rows_grouped(const MixedSliceJob*
         if (row_start[mid] <= b) lo = mid; else hi = mid - 1;
     }
     const MixedSliceJob& jb = jobs[lo];
-    if (jb.skip && *jb.skip) return;
     __shared__ uint2 red[8];
-    slice_row<S>(b - row_start[lo], jb.A, jb.lda, jb.n, jb.out, jb.rows_pad, jb.kp, jb.exps, jb.Y, jb.te, false, red);
+    slice_row<S>(b - row_start[lo], jb.A, jb.lda, jb.n, jb.out, jb.rows_pad, jb.kp, jb.exps, nullptr, nullptr, false, red);
 }
 
 // x exactly: 2^52 + 2^31 + x is the double with x + 2^31 in its low word.
