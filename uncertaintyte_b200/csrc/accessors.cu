@@ -24,9 +24,10 @@ constexpr int kMaxDim = 9;
 // carries the whole upper triangle and applies every rotation to it, so the
 // rotations need no shared memory, shuffle or barrier; the rows of V are dealt
 // to the lanes (D / L each). The chain of dependent rotations bounds the
-// kernel. The order is the cyclic one: the signs of the vectors follow from it (rounds
-// of disjoint pairs, their angles found side by side, took 65 us for 2000 9 x 9
-// blocks against 84, with other signs).
+// kernel. The order is the cyclic one by rows, from which the signs of the vectors
+// follow. Rounds of a round-robin tournament, their angles found side by side, took
+// 65 us for 200 9 x 9 blocks against 84, but gave other signs (pairs that share an
+// index change their order there; walking them by p + q would not change it).
 template <int D, int L>
 __global__ void __launch_bounds__(128) k_block_eigen(const double* __restrict__ packed, int nblk, int src, int off,
                                                      double* vals, double* vecs) {

@@ -392,7 +392,7 @@ __device__ __forceinline__ int potrf(const TaskMatrix& m, int k, Chain* chain, i
             TB * k, m.ext(k), m.T, m.ld, m.err, S, Bs,
             [&](int q) {
                 if (!below || q < 2) return;
-                for (int poll = q; poll < 5; poll += 2)  // the last panel: twice
+                for (int poll = q; poll < 5; poll += 2)  // the third panel: twice
                     if (lane == 0 && !flag[0] && ld_acquire(m.ver + tri(k + 1, k)) >= k) flag[0] = 1;
             },
             [&] {

@@ -19,11 +19,11 @@
 // symmetric, so their columns are their rows and the column-major FP64
 // matrices are read as K-major operands.
 //
-// Kernel layout: 128 threads. Warp 0 lane 0 issues the TMA loads of the S
+// Kernel layout: 256 threads. Warp 0 lane 0 issues the TMA loads of the S
 // slices of both operands per 64-byte K block (3-stage mbarrier pipeline);
 // warp 1 lane 0 issues the tcgen05.mma (M = 128, N = up to 256, K = 32 bytes:
 // one A slice against several adjacent B slices) and commits each stage back
-// to the producer; all four warps then read the
+// to the producer; all eight warps then read the
 // accumulators with tcgen05.ld and write FP64. Every mbarrier wait has an
 // iteration limit after which the kernel records ERRBIT_TIMEOUT and unwinds
 // (TMEM is always freed).
@@ -168,7 +168,7 @@ __device__ __forceinline__ double pow2(int e) {
 // 1.5 2^(52 - 7s) rounds the remainder to that unit (to nearest, ties to even)
 // and leaves the digit in the sum's low bits, so a digit is three additions and
 // no conversion; the row stays in registers between its maximum and its digits
-// up to kSliceKept elements. The slice count is a template parameter and the
+// up to 1024 kSlicePasses elements. The slice count is a template parameter and the
 // digits' bytes are gathered by byte permutes: issue slots bound it, so the maximum is
 // taken over the high words, as integers. n = 1800, five slices: 19 -> 13.5 us, and 4 us
 // less in a solve for the integer maximum (4.8 million warp instructions, 8.8 before).

@@ -124,8 +124,8 @@ extern "C" int unc_dense_inverse_noalloc(double* d_A, int n, int lda, void* stre
     double* Tt = ws + 2 * kMat;
     double* e = ws + 3 * kMat;
     int* err = reinterpret_cast<int*>(e + kEq);
-    // the previous call's contents stay in the array: clear what must start at
-    // zero (T above its diagonal blocks, the padding rows, the error word)
+    // the previous call's contents stay in the array: the error word must start at
+    // zero (the matrices need not: nothing of them is read before it is written)
     cudaError_t ce = cudaMemsetAsync(T, 0, sizeof(double) * mat, sm);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(W, 0, sizeof(double) * mat, sm);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(Tt, 0, sizeof(double) * mat, sm);

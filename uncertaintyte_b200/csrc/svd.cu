@@ -563,7 +563,7 @@ int pinv_psd(double* M, int n, int ld, int remove_n, double eps, const PinvBuffe
         return svd_fail(UNC_ERR_UNSUPPORTED, "at most 31 singular values can be removed");
     if (int rc = spd_prepare(n)) return svd_fail(rc, "tile-task inverse: cannot upload the task list");
     const size_t mat = (size_t)n * ld, blk = (size_t)ld * kMaxBlock;
-    // every scratch matrix starts finite (the GEMM reads padding rows in pairs)
+    // nothing below reads what it has not written: cleared so that the scratch holds nothing of earlier calls
     SVD_CK(cudaMemsetAsync(b.W, 0, sizeof(double) * mat, sm));
     SVD_CK(cudaMemsetAsync(b.Tt, 0, sizeof(double) * mat, sm));
     SVD_CK(cudaMemsetAsync(b.X, 0, sizeof(double) * blk, sm));
