@@ -87,13 +87,15 @@ __global__ void __launch_bounds__(128) k_block_eigen(const double* __restrict__ 
     }
     double* const w = vals + blk * D;
     double* const e = vecs ? vecs + blk * (D * D) : nullptr;
+    double key[D];  // a NaN counts as infinity, so that the ranks are a permutation and every place is written
+#pragma unroll
+    for (int j = 0; j < D; ++j) key[j] = a[j][j] == a[j][j] ? a[j][j] : __longlong_as_double(0x7ff0000000000000LL);
 #pragma unroll
     for (int j = 0; j < D; ++j) {  // descending order, ties by index
-        const double ev = a[j][j];
         int rank = 0;
 #pragma unroll
-        for (int i = 0; i < D; ++i) rank += (a[i][i] > ev) || (a[i][i] == ev && i < j);
-        if (part == j / R) w[rank] = ev;
+        for (int i = 0; i < D; ++i) rank += (key[i] > key[j]) || (key[i] == key[j] && i < j);
+        if (part == j / R) w[rank] = a[j][j];
         if (e) {
 #pragma unroll
             for (int r = 0; r < R; ++r) e[rank * D + part * R + r] = v[r][j];
